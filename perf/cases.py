@@ -167,34 +167,55 @@ def _gguf(rows, cols, gtype, gen):
     return out.view(-1)
 
 
-def prepare(case, seed):
-    E, k, d, mid, T = case["experts"], case["topk"], case["d"], case["mid"], case["tokens"]
+def _draw_inputs(case, seed):
+    """The raw weights and inputs of a case, on the GPU, from the seed alone."""
+    E, d, mid, T = case["experts"], case["d"], case["mid"], case["tokens"]
     gen = torch.Generator(device="cuda")
     gen.manual_seed(seed)
-    op = pkg.MoeOperator(E, k, d, mid, max(T, 16), has_shared=case["shared"])
+    raw = {}
     if case["fmt"] == "q4cp":
-        op.load_q4cp(0, _q4cp(E * 2 * mid, d, gen), _q4cp(E * d, mid, gen))
+        raw["gate_up"], raw["down"] = _q4cp(E * 2 * mid, d, gen), _q4cp(E * d, mid, gen)
     elif case["fmt"] == "i4r":
-        op.load_i4r(0, _i4r(E * 2 * mid, d, gen), _i4r(E * d, mid, gen), _planes(d, gen), _planes(2 * mid, gen),
-                    _planes(mid, gen), _planes(d, gen))
+        raw["gate_up"], raw["down"] = _i4r(E * 2 * mid, d, gen), _i4r(E * d, mid, gen)
+        raw["planes"] = _planes(d, gen), _planes(2 * mid, gen), _planes(mid, gen), _planes(d, gen)
     else:
         gu, dn = GGUF_TYPES[case["fmt"]]
-        op.load_gguf(0, _gguf(E * mid, d, gu, gen), _gguf(E * mid, d, gu, gen), _gguf(E * d, mid, dn, gen),
-                     type_gu=gu, type_dn=dn)
+        raw["gate"], raw["up"], raw["down"] = _gguf(E * mid, d, gu, gen), _gguf(E * mid, d, gu, gen), _gguf(E * d, mid, dn, gen)
     if case["shared"]:
-        gate_w = torch.empty(d, device="cuda").normal_(0.0, 0.02, generator=gen).bfloat16()
-        op.load_shared_q4cp(0, _q4cp(mid, d, gen), _q4cp(mid, d, gen), _q4cp(d, mid, gen), gate_w)
-    x = torch.empty(T, d, device="cuda").normal_(0.0, 1.0, generator=gen).bfloat16()
-    logits = torch.empty(T, E, device="cuda").normal_(0.0, 1.0, generator=gen)
+        raw["sh_gate_w"] = torch.empty(d, device="cuda").normal_(0.0, 0.02, generator=gen).bfloat16()
+        raw["shared"] = _q4cp(mid, d, gen), _q4cp(mid, d, gen), _q4cp(d, mid, gen)
+    raw["x"] = torch.empty(T, d, device="cuda").normal_(0.0, 1.0, generator=gen).bfloat16()
+    raw["logits"] = torch.empty(T, E, device="cuda").normal_(0.0, 1.0, generator=gen)
     if case["skew"]:
-        logits += torch.from_numpy(synth.zipf_bias(synth.rng_for(seed, 77), E, strength=case["skew"])).cuda()
+        raw["logits"] += torch.from_numpy(synth.zipf_bias(synth.rng_for(seed, 77), E, strength=case["skew"])).cuda()
+    if case["entry"] == "moe_hidden":
+        raw["router"] = torch.empty(E, d, device="cuda").normal_(0.0, 0.02, generator=gen).bfloat16()
+    elif case["entry"] == "moe_b_hc":
+        raw["w4"] = torch.empty(T, 4, device="cuda").normal_(0.0, 2.0, generator=gen)
+        raw["residual"] = torch.empty(T, 4, d, device="cuda").normal_(0.0, 1.0, generator=gen).bfloat16()
+    return raw
+
+
+def prepare(case, seed):
+    E, k, d, mid, T = case["experts"], case["topk"], case["d"], case["mid"], case["tokens"]
+    raw = _draw_inputs(case, seed)
+    op = pkg.MoeOperator(E, k, d, mid, max(T, 16), has_shared=case["shared"])
+    if case["fmt"] == "q4cp":
+        op.load_q4cp(0, raw["gate_up"], raw["down"])
+    elif case["fmt"] == "i4r":
+        op.load_i4r(0, raw["gate_up"], raw["down"], *raw["planes"])
+    else:
+        gu, dn = GGUF_TYPES[case["fmt"]]
+        op.load_gguf(0, raw["gate"], raw["up"], raw["down"], type_gu=gu, type_dn=dn)
+    if case["shared"]:
+        op.load_shared_q4cp(0, *raw["shared"], raw["sh_gate_w"])
+    x, logits = raw["x"], raw["logits"]
     state = {"case": case, "op": op, "x": x, "logits": logits, "out": torch.empty(T, d, dtype=torch.bfloat16, device="cuda")}
     entry = case["entry"]
     if entry == "moe_hidden":
-        op.load_router(0, torch.empty(E, d, device="cuda").normal_(0.0, 0.02, generator=gen).bfloat16())
+        op.load_router(0, raw["router"])
     elif entry == "moe_b_hc":
-        state["w4"] = torch.empty(T, 4, device="cuda").normal_(0.0, 2.0, generator=gen)
-        state["residual"] = torch.empty(T, 4, d, device="cuda").normal_(0.0, 1.0, generator=gen).bfloat16()
+        state["w4"], state["residual"] = raw["w4"], raw["residual"]
     elif entry == "moe_q4w_run":
         state["ids"] = torch.zeros(T, 16, dtype=torch.int32, device="cuda")
         state["w"] = torch.zeros(T, 16, device="cuda")
@@ -203,6 +224,7 @@ def prepare(case, seed):
         for n in ("x", "logits", "out"):
             state[n] = state[n].cpu().pin_memory()
     torch.cuda.synchronize()
+    del raw
     torch.cuda.empty_cache()  # the source tensors may be freed once they are loaded
     return state
 
@@ -260,3 +282,112 @@ def tolerance(case):
     1.5e-3 in the 2-norm and by one bf16 step (7.8e-3) at most; the residual write-back, which adds the result to a
     state of norm 1 before it rounds, by 2.4e-4. Four times that is stated."""
     return {"rel": 1e-3 if case["entry"] == "moe_b_hc" else 6e-3, "max": 0.032}
+
+
+# ------------------------------------------------------------------ the same in 64 bits
+def _f16_at(blocks, byte):
+    return blocks[:, byte:byte + 2].contiguous().view(torch.float16).double()
+
+
+def _nibbles(codes):
+    """Low nibbles, then high nibbles: [n][bytes] -> [n][2][bytes]."""
+    return torch.stack([codes & 15, codes >> 4], 1)
+
+
+def _q4cp_rows(blob, rows, cols, r0, n):
+    """Rows r0 .. r0+n-1; byte i of a row holds columns 2i and 2i+1."""
+    stride = ((cols // 32 * 2) + 15) & ~15
+    codes = blob[64 + r0 * cols // 2:64 + (r0 + n) * cols // 2].view(n, -1)
+    book = blob[:64].view(torch.float32).double()
+    off = 64 + rows * cols // 2
+    sc = blob[off + r0 * stride:off + (r0 + n) * stride].view(n, stride)[:, :cols // 32 * 2].contiguous().view(torch.float16).double()
+    return book[_nibbles(codes).transpose(1, 2).reshape(n, cols).long()] * sc.repeat_interleave(32, 1)
+
+
+def _i4r_rows(blob, rows, cols, r0, n):
+    codes = blob[r0 * cols // 2:(r0 + n) * cols // 2].view(n, -1)
+    off, per = rows * cols // 2, cols // 128
+    sc = blob[off + r0 * per * 2:off + (r0 + n) * per * 2].view(torch.float16).view(n, per).double()
+    return (_nibbles(codes).transpose(1, 2).reshape(n, cols).double() - 8.0) * sc.repeat_interleave(128, 1)
+
+
+_GRID = (-127, -104, -83, -65, -49, -35, -22, -10, 1, 13, 25, 38, 53, 69, 89, 113)
+
+
+def _gguf_rows(blob, cols, gtype, r0, n):
+    per, size = {pkg.GGML_Q4_K: (256, 144), pkg.GGML_Q5_K: (256, 176), pkg.GGML_Q5_1: (32, 24),
+                 pkg.GGML_IQ4_XS: (256, 136), pkg.GGML_Q8_0: (32, 34)}[gtype]
+    b = blob.view(-1, size)[r0 * (cols // per):(r0 + n) * (cols // per)]
+    nb = b.shape[0]
+    if gtype == pkg.GGML_Q8_0:
+        w = _f16_at(b, 0) * b[:, 2:].contiguous().view(torch.int8).double()
+    elif gtype == pkg.GGML_Q5_1:
+        bits = torch.stack([b[:, 4 + j // 8] >> (j % 8) & 1 for j in range(32)], 1)
+        w = _f16_at(b, 0) * (_nibbles(b[:, 8:]).reshape(nb, 32) + 16 * bits).double() + _f16_at(b, 2)
+    elif gtype == pkg.GGML_IQ4_XS:
+        low = torch.stack([b[:, 4 + i // 2] >> (4 * (i % 2)) & 15 for i in range(8)], 1)
+        high = torch.stack([b[:, 2 + i // 4] >> (2 * (i % 4)) & 3 for i in range(8)], 1)
+        sc = _f16_at(b, 0) * ((low | high << 4).double() - 32.0)
+        grid = torch.tensor(_GRID, dtype=torch.float64, device=b.device)
+        w = sc[:, :, None] * grid[_nibbles(b[:, 8:].reshape(nb * 8, 16)).reshape(nb, 8, 32).long()]
+    else:
+        p = b[:, 4:16].int()
+        sc = torch.cat([p[:, 0:4] & 63, (p[:, 8:12] & 15) | (p[:, 0:4] >> 6 << 4)], 1).double() * _f16_at(b, 0)
+        mn = torch.cat([p[:, 4:8] & 63, (p[:, 8:12] >> 4) | (p[:, 4:8] >> 6 << 4)], 1).double() * _f16_at(b, 2)
+        q = _nibbles(b[:, -128:].reshape(nb * 4, 32)).reshape(nb, 8, 32).int()
+        if gtype == pkg.GGML_Q5_K:
+            q = q + 16 * torch.stack([b[:, 16:48] >> i & 1 for i in range(8)], 1)
+        w = sc[:, :, None] * q.double() - mn[:, :, None]
+    return w.reshape(n, cols)
+
+
+def _hadamard(v):
+    """128-point orthonormal Hadamard transform of every block of the last axis."""
+    h = torch.ones(1, 1, dtype=torch.float64, device=v.device)
+    for _ in range(7):
+        h = torch.cat([torch.cat([h, h], 1), torch.cat([h, -h], 1)], 0)
+    return (v.reshape(-1, 128) @ h).reshape(v.shape) / math.sqrt(128.0)
+
+
+def exact(case, seed):
+    """The layer in 64 bits: softmax, top-k, renormalised weights, SwiGLU experts, shared expert behind its sigmoid gate."""
+    E, k, d, mid, fmt = case["experts"], case["topk"], case["d"], case["mid"], case["fmt"]
+    raw = _draw_inputs(case, seed)
+    x = raw["x"].double()
+    logits = x @ raw["router"].double().T if case["entry"] == "moe_hidden" else raw["logits"].double()
+    w, ids = torch.topk(torch.softmax(logits, 1), k, dim=1)
+    w = w / w.sum(1, keepdim=True)
+    xin = x
+    if fmt == "i4r":
+        pre_gu, post_gu, pre_dn, post_dn = [p.double() for p in raw["planes"]]
+        xin = _hadamard(x * pre_gu)
+    y = torch.zeros_like(x)
+    silu = torch.nn.functional.silu
+    for e in range(E):
+        tok, slot = torch.nonzero(ids == e, as_tuple=True)
+        if not len(tok):
+            continue
+        if fmt in ("q4cp", "i4r"):
+            rows = _q4cp_rows if fmt == "q4cp" else _i4r_rows
+            gu = rows(raw["gate_up"], E * 2 * mid, d, e * 2 * mid, 2 * mid)
+            dn = rows(raw["down"], E * d, mid, e * d, d)
+        else:
+            tg, td = GGUF_TYPES[fmt]
+            gu = torch.cat([_gguf_rows(raw[n], d, tg, e * mid, mid) for n in ("gate", "up")])
+            dn = _gguf_rows(raw["down"], mid, td, e * d, d)
+        z = xin[tok] @ gu.T
+        if fmt == "i4r":
+            z = _hadamard(z) * post_gu
+        h = silu(z[:, :mid]) * z[:, mid:]
+        if fmt == "i4r":
+            h = _hadamard(h * pre_dn)
+        y.index_add_(0, tok, (h @ dn.T) * w[tok, slot, None])
+    if fmt == "i4r":
+        y = _hadamard(y) * post_dn
+    if case["shared"]:
+        g, u, dn = raw["shared"]
+        h = silu(x @ _q4cp_rows(g, mid, d, 0, mid).T) * (x @ _q4cp_rows(u, mid, d, 0, mid).T)
+        y += torch.sigmoid(x @ raw["sh_gate_w"].double())[:, None] * (h @ _q4cp_rows(dn, d, mid, 0, d).T)
+    if case["entry"] == "moe_b_hc":
+        return raw["residual"].double() + 2.0 * torch.sigmoid(raw["w4"].double() / 4.0)[:, :, None] * y[:, None, :]
+    return y
