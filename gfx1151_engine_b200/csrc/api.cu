@@ -43,7 +43,6 @@ struct b200moe_ctx {
   void* hid = nullptr;      // [rows][mid] fp32 (GEMV path) or fp16 (tensor-core path)
   void* pairs = nullptr;    // [rows][d]   fp32 or fp16
   __half* x_sorted = nullptr;
-  __half* x_rot = nullptr;  // [max_tokens][d] fp16: rotated activations of hgn v2 i4r layers (allocated by the first such load)
   int dec_rows = 0;
   RouterPlan* rplan = nullptr;     // router logits from hidden states
   const float* hc_w4 = nullptr;    // set for the duration of b200moe_forward_hc: the combine
@@ -445,7 +444,6 @@ int b200moe_load_i4r(b200moe_handle h, int layer, const void* gate_up_src, size_
   L.i4r = false;
   std::vector<void*> tmp;
   cudaError_t e = cudaSuccess;
-  if (!h->x_rot) e = dev_alloc(h, &h->x_rot, (size_t)c.max_tokens * d);
   static const float kBook[32] = {-8, -7, -6, -5, -4, -3, -2, -1, 0, 1, 2, 3, 4, 5, 6, 7,
                                   -8, -7, -6, -5, -4, -3, -2, -1, 0, 1, 2, 3, 4, 5, 6, 7};
   const uint8_t* src = nullptr;
@@ -693,7 +691,7 @@ static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const
   // stay the default.
   static const bool fused_env = getenv("B200MOE_FUSED_DECODE") != nullptr && atoi(getenv("B200MOE_FUSED_DECODE")) != 0;
   const bool fused = fused_env || c.decode_impl == B200MOE_DECODE_FUSED;
-  if (L.i4r && (c.gemm_impl == B200MOE_GEMM_SIMT || !h->tc || !h->x_rot))
+  if (L.i4r && (c.gemm_impl == B200MOE_GEMM_SIMT || !h->tc))
     return fail(h, B200MOE_ERR_UNSUPPORTED, "forward: hgn v2 i4r layers run on the tensor-core path only");
   if (fused && !L.i4r && c.gemm_impl == B200MOE_GEMM_AUTO && T <= h->decode_max && T <= decode_max_tokens() &&
       ((uintptr_t)x & 15) == 0 && (size_t)T * (k + (shared ? 1 : 0)) <= (size_t)h->dec_rows &&
@@ -709,6 +707,9 @@ static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const
     h->launches += 1;
     return B200MOE_OK;
   }
+  const bool simt = !L.i4r && (c.gemm_impl == B200MOE_GEMM_SIMT ||
+                                (c.gemm_impl == B200MOE_GEMM_AUTO && T <= h->decode_max));
+  const uint16_t* gate_w = nullptr;  // set: the shared expert's gate is still to be computed
   static const bool slow_router = getenv("B200MOE_EXACT_ROUTER") != nullptr;  // A/B: the general routing body for every call
   if (logits && !slow_router && T <= decode_max_tokens() && T * k <= 128 && d % 8 == 0 && (!shared || ((uintptr_t)x & 15) == 0)) {
     // decode / verify: the compact router (ids from the logits' order, general body only on a near-tie)
@@ -727,15 +728,15 @@ static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const
       stride = kIdStride;
     }
     CU_TRY(h, launch_route(h->rb, ids, w, stride, T, k, E, h->tile_cap, st, &n));
-    if (shared) {
+    if (shared && simt) {
       CU_TRY(h, launch_shared_gate(x, L.sh_gate_w, T, d, k, h->rb, st));
       n++;
+    } else if (shared) {
+      gate_w = L.sh_gate_w;  // tensor-core path: computed with the activations' rows, launch_scatter_f16
     }
   }
   if (ev) CU_TRY(h, cudaEventRecord(ev[1], st));
   const int pairs = T * k;
-  const bool simt = !L.i4r && (c.gemm_impl == B200MOE_GEMM_SIMT ||
-                                (c.gemm_impl == B200MOE_GEMM_AUTO && T <= h->decode_max));
   if (simt && c.gemm_impl != B200MOE_GEMM_SIMT && T > h->decode_max)
     return fail(h, B200MOE_ERR_BAD_ARG, "forward: T exceeds the GEMV path's workspace");
   // (the shared expert's images are q4cp: it can ride along only with q4cp routed experts)
@@ -784,11 +785,10 @@ static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const
     if (!h->tc) return fail(h, B200MOE_ERR_UNSUPPORTED, "tensor-core path not available on this handle");
     const int rows = pairs + (shared ? T : 0);
     if (L.i4r) {
-      // hgn v2 i4r (rotate.cu): rotate the tokens once, gather the rotated rows, plain GEMM into
+      // hgn v2 i4r (rotate.cu): rotate the tokens once into their rows, plain GEMM into
       // the pair buffer (2*mid <= d columns of it), then the Hadamard / SwiGLU / Hadamard step
-      CU_TRY(h, launch_rot_in(x, L.rot, T, d, h->x_rot, st));
-      CU_TRY(h, launch_gather_f16(h->x_rot, h->rb.tokidx, rows, d, h->x_sorted, st, true));
-      n += 2;
+      CU_TRY(h, launch_rot_in(x, L.rot, h->rb.pairids, T, k, d, h->x_sorted, st));
+      n++;
       if (ev) CU_TRY(h, cudaEventRecord(ev[2], st));
       CU_TRY(h, launch_raw_tc(h->tc, L.gu, h->rb.tiles, h->rb.n_tiles, h->max_tiles, (__half*)h->pairs, h->status_dev, st));
       CU_TRY(h, launch_i4r_mid((const __half*)h->pairs, L.rot + d, L.rot + d + 2 * mid, rows, mid, (__half*)h->hid, st));
@@ -807,7 +807,7 @@ static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const
       h->launches += n;
       return B200MOE_OK;
     }
-    CU_TRY(h, launch_gather_f16(x, h->rb.tokidx, rows, d, h->x_sorted, st));
+    CU_TRY(h, launch_scatter_f16(x, T, k, d, shared ? pairs : -1, h->x_sorted, gate_w, h->rb, st));
     n++;
     if (ev) CU_TRY(h, cudaEventRecord(ev[2], st));
     CU_TRY(h, launch_up_tc(h->tc, L.gu, h->rb.tiles, h->rb.n_tiles, h->max_tiles, (__half*)h->hid,
@@ -1117,8 +1117,6 @@ int b200moe_share_weights(b200moe_handle h, b200moe_handle owner) {
     }
     L = owner->layers[i];
     L.borrowed = true;
-    if (L.i4r && !h->x_rot)
-      CU_TRY(h, dev_alloc(h, &h->x_rot, (size_t)h->cfg.max_tokens * h->cfg.d_model));
   }
   if (h->place_dev && !h->place_borrowed) cudaFree(h->place_dev);
   if (h->source_of_placed_dev && !h->place_borrowed) cudaFree(h->source_of_placed_dev);
@@ -1184,12 +1182,9 @@ int b200moe_ep_route(b200moe_handle h, int layer, const void* x, int T, const fl
     n++;
   }
   CU_TRY(h, launch_route(h->rb, h->rb.topids, h->rb.topw, kIdStride, T, c.topk, c.experts, h->tile_cap, st, &n));
-  if (shared) {
-    // the shared expert stays on the token's own rank: its rows (token order) follow the routed ones
-    CU_TRY(h, launch_shared_gate(x, L.sh_gate_w, T, c.d_model, c.topk, h->rb, st));
-    n++;
-  }
-  CU_TRY(h, launch_gather_f16(x, h->rb.tokidx, T * c.topk + (shared ? T : 0), c.d_model, h->ep_x_send, st));
+  // the shared expert stays on the token's own rank: its rows (token order) follow the routed ones
+  CU_TRY(h, launch_scatter_f16(x, T, c.topk, c.d_model, shared ? T * c.topk : -1, h->ep_x_send,
+                               shared ? L.sh_gate_w : nullptr, h->rb, st));
   if (eoff_out)
     CU_TRY(h, cudaMemcpyAsync(eoff_out, h->rb.eoff, ((size_t)c.experts + 1) * 4, cudaMemcpyDeviceToDevice, st));
   h->launches += n + 2;

@@ -1,4 +1,4 @@
-// combine.cu -- the memory-bound ends of the path: the expert-sorted activation gather
+// combine.cu -- the memory-bound ends of the path: the activations in expert order
 // in front of the grouped GEMM and the weighted top-k combine behind it.
 //
 // Combine replaces k_moe_reduce_pw / k_moe_reduce_pw_sg
@@ -192,50 +192,53 @@ __device__ __forceinline__ float clamp_f16_range(float v) {
   return v != v ? v : fminf(fmaxf(v, -65504.f), 65504.f);
 }
 
-// plain row gather of fp16 rows (the source is already fp16: rotated activations of hgn v2 i4r layers)
-__global__ void __launch_bounds__(256)
-k_gather_rows16(const uint4* __restrict__ x, const int32_t* __restrict__ tokidx, int rows, int per_row,
-                uint4* __restrict__ xs) {
-  const int lane = threadIdx.x & 31;
-  const int n_warps = gridDim.x * (blockDim.x >> 5);
-  for (int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); row < rows; row += n_warps) {
-    const uint4* src = x + (size_t)tokidx[row] * per_row;
-    uint4* dst = xs + (size_t)row * per_row;
-    for (int v = lane; v < per_row; v += 32) dst[v] = src[v];
-  }
-}
-
-// x_sorted[row][:] = fp16(x[tokidx[row]][:]); bf16 -> fp16 is exact for 2^-14 <= |v| < 65520,
+// The activations of the grouped GEMM: x_sorted[row] = fp16(x[t]) for the k rows of token t (pairids)
+// and, with a shared expert, for row shared_row0 + t. bf16 -> fp16 is exact for 2^-14 <= |v| < 65520,
 // larger magnitudes (infinities included) saturate to the largest finite half, NaN stays NaN.
-// One warp per row: the token index is read once, a lane keeps four 16-byte loads in flight.
+// One block per token: a row is read and converted once and written k times. HBM bound (k*T*d*2
+// bytes written): gathering row by row in expert order re-read x k times, from HBM wherever x
+// does not fit L2 (16384 tokens x 4096: 392 us under the profiler's cold clocks).
+// With gw the block also computes the token's scalar sigmoid gate of the shared expert
+// (src/ref.cpp:623-626, 635; double sums) and appends the shared expert's row to the routing lists.
 __global__ void __launch_bounds__(256)
-k_gather_f16(const uint16_t* __restrict__ x, const int32_t* __restrict__ tokidx, int rows, int d,
-             __half* __restrict__ xs) {
-  const int lane = threadIdx.x & 31;
-  const int n_warps = gridDim.x * (blockDim.x >> 5);
-  const int per_row = d / 8;  // 16-byte pieces
-  for (int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); row < rows; row += n_warps) {
-    const uint4* src = (const uint4*)(x + (size_t)tokidx[row] * d);
-    uint4* dst = (uint4*)(xs + (size_t)row * d);
-    for (int v0 = lane; v0 < per_row; v0 += 128) {
-      uint4 u[4];
+k_scatter_f16(const uint16_t* __restrict__ x, const int32_t* __restrict__ pairids, int k, int d, int shared_row0,
+              __half* __restrict__ xs, const uint16_t* __restrict__ gw, int32_t* __restrict__ tokidx,
+              float* __restrict__ pw, float* __restrict__ sgate) {
+  __shared__ int s_row[kMaxTopK + 1];
+  __shared__ double s_gate[8];
+  const int t = blockIdx.x;
+  if (threadIdx.x < k) s_row[threadIdx.x] = pairids[(size_t)t * k + threadIdx.x];  // negative: dropped by the bucketing
+  if (threadIdx.x == k) s_row[k] = shared_row0 >= 0 ? shared_row0 + t : -1;
+  __syncthreads();
+  double g = 0;
+  for (int c = threadIdx.x; c < d / 8; c += 256) {
+    const uint4 u = ((const uint4*)(x + (size_t)t * d))[c];
+    const uint16_t* b = (const uint16_t*)&u;
+    uint4 o;
+    __half2* oh = (__half2*)&o;
 #pragma unroll
-      for (int i = 0; i < 4; i++)
-        if (v0 + 32 * i < per_row) u[i] = src[v0 + 32 * i];
+    for (int j = 0; j < 4; j++)
+      oh[j] = __floats2half2_rn(clamp_f16_range(bf16_bits_to_f32(b[2 * j])), clamp_f16_range(bf16_bits_to_f32(b[2 * j + 1])));
+    for (int s = 0; s <= k; s++)
+      if (s_row[s] >= 0) ((uint4*)(xs + (size_t)s_row[s] * d))[c] = o;
+    if (gw) {
+      const uint4 v = ((const uint4*)gw)[c];
+      const uint16_t* w = (const uint16_t*)&v;
 #pragma unroll
-      for (int i = 0; i < 4; i++) {
-        if (v0 + 32 * i < per_row) {
-          const uint16_t* b = (const uint16_t*)&u[i];
-          uint4 o;
-          __half2* oh = (__half2*)&o;
-#pragma unroll
-          for (int j = 0; j < 4; j++) {
-            oh[j] = __floats2half2_rn(clamp_f16_range(bf16_bits_to_f32(b[2 * j])), clamp_f16_range(bf16_bits_to_f32(b[2 * j + 1])));
-          }
-          dst[v0 + 32 * i] = o;
-        }
-      }
+      for (int j = 0; j < 8; j++) g += (double)bf16_bits_to_f32(w[j]) * (double)bf16_bits_to_f32(b[j]);
     }
+  }
+  if (!gw) return;
+#pragma unroll
+  for (int o = 16; o; o >>= 1) g += __shfl_xor_sync(0xffffffffu, g, o);
+  if ((threadIdx.x & 31) == 0) s_gate[threadIdx.x >> 5] = g;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; w++) g += s_gate[w];
+    const float v = sigmoid_f32((float)g);
+    sgate[t] = v;
+    tokidx[shared_row0 + t] = t;
+    pw[shared_row0 + t] = v;
   }
 }
 
@@ -270,19 +273,10 @@ cudaError_t launch_combine_f16_rot(const __half* pairs, const float* pw, const i
   return cudaGetLastError();
 }
 
-cudaError_t launch_gather_f16(const void* x_bf16, const int32_t* tokidx, int rows, int d,
-                              __half* x_sorted, cudaStream_t st, bool src_f16) {
-  static int sms = 0;
-  if (!sms) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) sms = 148;
-  }
-  int blocks = (rows + 7) / 8;
-  if (blocks > sms * 8) blocks = sms * 8;
-  if (blocks < 1) blocks = 1;
-  if (src_f16) k_gather_rows16<<<blocks, 256, 0, st>>>((const uint4*)x_bf16, tokidx, rows, d / 8, (uint4*)x_sorted);
-  else k_gather_f16<<<blocks, 256, 0, st>>>((const uint16_t*)x_bf16, tokidx, rows, d, x_sorted);
+cudaError_t launch_scatter_f16(const void* x_bf16, int T, int k, int d, int shared_row0, __half* x_sorted,
+                               const uint16_t* gate_w_bf16, const RouteBuffers& rb, cudaStream_t st) {
+  k_scatter_f16<<<T, 256, 0, st>>>((const uint16_t*)x_bf16, rb.pairids, k, d, shared_row0, x_sorted, gate_w_bf16, rb.tokidx,
+                                   rb.pw, rb.sgate);
   return cudaGetLastError();
 }
 

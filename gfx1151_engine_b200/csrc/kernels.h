@@ -88,7 +88,6 @@ cudaError_t launch_route_small(const RouteBuffers& rb, const float* logits, cons
                                const uint16_t* gate_w_bf16, int d, cudaStream_t st);
 cudaError_t launch_shared_gate(const void* x_bf16, const uint16_t* gate_w_bf16, int T, int d,
                                int k, const RouteBuffers& rb, cudaStream_t st);
-
 cudaError_t launch_apply_placement(int32_t* ids, int stride, int T, int k, int E, const int32_t* place,
                                    cudaStream_t st);
 cudaError_t launch_ep_merge_tails(__half* x_recv, const int32_t* segs, int n_seg, const int32_t* counts, int d,
@@ -177,12 +176,14 @@ cudaError_t launch_combine_f16(const __half* pairs, const float* pw, const int32
 cudaError_t launch_combine_f16_rot(const __half* pairs, const float* pw, const int32_t* pairids, int T,
                                    int k, int d, const float* rot_post, void* out_bf16, cudaStream_t st,
                                    const float* hc_w4 = nullptr, void* hc_state = nullptr);
-// src_f16: the source rows are fp16 already (rotated activations) instead of bf16
-cudaError_t launch_gather_f16(const void* x_bf16, const int32_t* tokidx, int rows, int d,
-                              __half* x_sorted, cudaStream_t st, bool src_f16 = false);
+// x_sorted rows of every token (pairids of rb) and, with shared_row0 >= 0, of the shared expert's row
+// block; gate_w_bf16 non-null: also the shared expert's gate and its rows of tokidx / pw.
+cudaError_t launch_scatter_f16(const void* x_bf16, int T, int k, int d, int shared_row0, __half* x_sorted,
+                               const uint16_t* gate_w_bf16, const RouteBuffers& rb, cudaStream_t st);
 
 // ---- rotate.cu (hgn v2 i4r: Hadamard steps around the two GEMMs) ----
-cudaError_t launch_rot_in(const void* x_bf16, const float* pre, int T, int d, __half* xr, cudaStream_t st);
+cudaError_t launch_rot_in(const void* x_bf16, const float* pre, const int32_t* pairids, int T, int k, int d,
+                          __half* x_sorted, cudaStream_t st);
 cudaError_t launch_i4r_mid(const __half* z, const float* svh_gu, const float* suh_dn, int rows, int mid, __half* hr,
                            cudaStream_t st);
 cudaError_t launch_f16_to_f32(const void* src_f16_dev, float* dst, int n, cudaStream_t st);

@@ -45,9 +45,12 @@ __device__ __forceinline__ uint32_t pack_f16x2_sat(float lo, float hi) {
   return r;
 }
 
-// xr[t][b*128 ..] = fp16( Hn(pre * x[t][b*128 ..]) ), one warp per (token, block)
+// x_sorted[row][b*128 ..] = fp16( Hn(pre * x[t][b*128 ..]) ) for the k rows of token t (pairids; negative:
+// dropped by the bucketing), one warp per (token, block): rotated once, written k times, no rotated
+// copy in token order in between
 __global__ void __launch_bounds__(256)
-k_rot_in(const uint16_t* __restrict__ x, const float* __restrict__ pre, int T, int d, __half* __restrict__ xr) {
+k_rot_in(const uint16_t* __restrict__ x, const float* __restrict__ pre, const int32_t* __restrict__ pairids, int T, int k,
+         int d, __half* __restrict__ x_sorted) {
   const int lane = threadIdx.x & 31;
   const int nb = d >> 7;
   const long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -62,7 +65,10 @@ k_rot_in(const uint16_t* __restrict__ x, const float* __restrict__ pre, int T, i
   uint2 o;
   o.x = pack_f16x2_sat(v[0] * kRs128, v[1] * kRs128);
   o.y = pack_f16x2_sat(v[2] * kRs128, v[3] * kRs128);
-  *(uint2*)(xr + off) = o;
+  for (int s = 0; s < k; s++) {
+    const int row = pairids[(size_t)t * k + s];
+    if (row >= 0) *(uint2*)(x_sorted + (size_t)row * d + b * 128 + lane * 4) = o;
+  }
 }
 
 __device__ __forceinline__ void load4(const __half* p, float (&v)[4]) {
@@ -112,10 +118,11 @@ __global__ void k_f16_to_f32(const uint16_t* __restrict__ src, float* __restrict
 
 }  // namespace
 
-cudaError_t launch_rot_in(const void* x_bf16, const float* pre, int T, int d, __half* xr, cudaStream_t st) {
+cudaError_t launch_rot_in(const void* x_bf16, const float* pre, const int32_t* pairids, int T, int k, int d,
+                          __half* x_sorted, cudaStream_t st) {
   const long long warps = (long long)T * (d >> 7);
   if (warps == 0) return cudaSuccess;
-  k_rot_in<<<(unsigned)((warps + 7) / 8), 256, 0, st>>>((const uint16_t*)x_bf16, pre, T, d, xr);
+  k_rot_in<<<(unsigned)((warps + 7) / 8), 256, 0, st>>>((const uint16_t*)x_bf16, pre, pairids, T, k, d, x_sorted);
   return cudaGetLastError();
 }
 
