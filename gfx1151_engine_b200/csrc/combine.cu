@@ -207,6 +207,8 @@ k_scatter_f16(const uint16_t* __restrict__ x, const int32_t* __restrict__ pairid
   __shared__ int s_row[kMaxTopK + 1];
   __shared__ double s_gate[8];
   const int t = blockIdx.x;
+  pdl_trigger();
+  pdl_wait();
   if (threadIdx.x < k) s_row[threadIdx.x] = pairids[(size_t)t * k + threadIdx.x];  // negative: dropped by the bucketing
   if (threadIdx.x == k) s_row[k] = shared_row0 >= 0 ? shared_row0 + t : -1;
   __syncthreads();
@@ -275,9 +277,8 @@ cudaError_t launch_combine_f16_rot(const __half* pairs, const float* pw, const i
 
 cudaError_t launch_scatter_f16(const void* x_bf16, int T, int k, int d, int shared_row0, __half* x_sorted,
                                const uint16_t* gate_w_bf16, const RouteBuffers& rb, cudaStream_t st) {
-  k_scatter_f16<<<T, 256, 0, st>>>((const uint16_t*)x_bf16, rb.pairids, k, d, shared_row0, x_sorted, gate_w_bf16, rb.tokidx,
-                                   rb.pw, rb.sgate);
-  return cudaGetLastError();
+  return launch_pdl(k_scatter_f16, dim3(T), dim3(256), 0, st, (const uint16_t*)x_bf16, rb.pairids, k, d, shared_row0, x_sorted,
+                    gate_w_bf16, rb.tokidx, rb.pw, rb.sgate);
 }
 
 }  // namespace b200moe

@@ -21,7 +21,7 @@ namespace {
 
 constexpr int kRouterWarps = 8;
 
-constexpr int kChunk = 512;  // pairs handled by one single-warp block of the bucketing kernels
+constexpr int kChunk = 512;  // pairs handled by one block (a thread per pair) of the bucketing kernels
 
 __device__ __forceinline__ double shfl_double(double v, int src) {
   int lo = __double2loint(v), hi = __double2hiint(v);
@@ -140,6 +140,8 @@ k_router_topk(const float* __restrict__ logits, int T, int E, int k, int32_t* __
   __shared__ float s_p[kRouterWarps][kMaxExperts];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t = blockIdx.x * kRouterWarps + warp;
+  pdl_trigger();
+  pdl_wait();
   if (t >= T) return;
   router_one_token(logits + (size_t)t * E, E, k, lane, s_p[warp], ids + (size_t)t * stride,
                    w + (size_t)t * stride, stride);
@@ -160,24 +162,22 @@ k_route_small(const float* __restrict__ logits, const int32_t* __restrict__ ids_
   route_small_body<16>(logits, ids_in, w_in, stride_in, T, E, k, x, gw, d, sc, o, RouteSmallOut{}, rb.status);
 }
 
-__global__ void __launch_bounds__(32)
+__global__ void __launch_bounds__(kChunk)
 k_route_count(const int32_t* __restrict__ ids, int stride, int pairs, int k, int E,
               int32_t* __restrict__ blockcnt, int32_t* __restrict__ status) {
   __shared__ int hist[kMaxExperts];
-  const int lane = threadIdx.x;
-  for (int e = lane; e < E; e += 32) hist[e] = 0;
-  __syncwarp();
-  const int base = blockIdx.x * kChunk;
-  for (int it = 0; it < kChunk / 32; it++) {
-    int p = base + it * 32 + lane;
-    if (p < pairs) {
-      const int e = ids[(size_t)(p / k) * stride + p % k];
-      if ((unsigned)e < (unsigned)E) atomicAdd(&hist[e], 1);  // ids outside [0, E) are dropped, never used as an index
-      else if (status && atomicCAS(status, 0, kStatusBadId) == 0) status[1] = e;
-    }
+  pdl_trigger();
+  for (int e = threadIdx.x; e < E; e += kChunk) hist[e] = 0;
+  pdl_wait();
+  __syncthreads();
+  const int p = blockIdx.x * kChunk + threadIdx.x;
+  if (p < pairs) {
+    const int e = ids[(size_t)(p / k) * stride + p % k];
+    if ((unsigned)e < (unsigned)E) atomicAdd(&hist[e], 1);  // ids outside [0, E) are dropped, never used as an index
+    else if (status && atomicCAS(status, 0, kStatusBadId) == 0) status[1] = e;
   }
-  __syncwarp();
-  for (int e = lane; e < E; e += 32) blockcnt[(size_t)blockIdx.x * E + e] = hist[e];
+  __syncthreads();
+  for (int e = threadIdx.x; e < E; e += kChunk) blockcnt[(size_t)blockIdx.x * E + e] = hist[e];
 }
 
 // One block of 512 threads: per-expert exclusive prefix over the chunk counts, expert
@@ -187,19 +187,23 @@ __global__ void __launch_bounds__(kMaxExperts)
 k_route_scan(int32_t* __restrict__ blockcnt, int nblk, int E, int pairs, int T, int tile_cap,
              int32_t* __restrict__ eoff, Run* __restrict__ runs, int32_t* __restrict__ n_runs,
              Tile* __restrict__ tiles, Tile* __restrict__ tiles_sh, int32_t* __restrict__ n_tiles) {
-  __shared__ int s_a[kMaxExperts], s_b[kMaxExperts], s_c[kMaxExperts];
-  const int e = threadIdx.x;
+  __shared__ __align__(16) int s_a[kMaxExperts];
+  __shared__ unsigned long long s_w[kMaxExperts / 32];
+  __shared__ int s_wc[kMaxExperts / 32];
+  const int e = threadIdx.x, lane = e & 31, warp = e >> 5;
+  pdl_trigger();
+  pdl_wait();
   int cnt = 0;
   if (e < E) {
-    // exclusive prefix down this expert's column of the chunk counts; the loads of eight
+    // exclusive prefix down this expert's column of the chunk counts; the loads of sixteen
     // rows are issued together so that the walk does not pay one memory latency per chunk
     int b = 0;
-    for (; b + 8 <= nblk; b += 8) {
-      int c[8];
+    for (; b + 16 <= nblk; b += 16) {
+      int c[16];
 #pragma unroll
-      for (int i = 0; i < 8; i++) c[i] = blockcnt[(size_t)(b + i) * E + e];
+      for (int i = 0; i < 16; i++) c[i] = blockcnt[(size_t)(b + i) * E + e];
 #pragma unroll
-      for (int i = 0; i < 8; i++) {
+      for (int i = 0; i < 16; i++) {
         blockcnt[(size_t)(b + i) * E + e] = cnt;
         cnt += c[i];
       }
@@ -210,41 +214,57 @@ k_route_scan(int32_t* __restrict__ blockcnt, int nblk, int E, int pairs, int T, 
       cnt += c;
     }
   }
-  // three inclusive scans side by side: counts, non-empty flags, full tiles
+  // three inclusive scans side by side: counts (low 32 bits) and non-empty flags, full tiles
   const int nfull = cnt / tile_cap, part = cnt % tile_cap;
-  s_a[e] = cnt;
-  s_b[e] = cnt > 0;
-  s_c[e] = nfull;
-  __syncthreads();
-  for (int o = 1; o < kMaxExperts; o <<= 1) {
-    int a = e >= o ? s_a[e - o] : 0, b = e >= o ? s_b[e - o] : 0, c = e >= o ? s_c[e - o] : 0;
-    __syncthreads();
-    s_a[e] += a;
-    s_b[e] += b;
-    s_c[e] += c;
-    __syncthreads();
+  unsigned long long ab = (unsigned long long)(uint32_t)cnt | (unsigned long long)(cnt > 0) << 32;
+  int c = nfull;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned long long u = __shfl_up_sync(0xffffffffu, ab, o);
+    const int v = __shfl_up_sync(0xffffffffu, c, o);
+    if (lane >= o) {
+      ab += u;
+      c += v;
+    }
   }
-  const int first = s_a[e] - cnt;
-  const int total_full = s_c[kMaxExperts - 1];
+  if (lane == 31) {
+    s_w[warp] = ab;
+    s_wc[warp] = c;
+  }
+  s_a[e] = part;
+  __syncthreads();
+  unsigned long long ab_all = 0;
+  int c_all = 0;
+#pragma unroll
+  for (int w = 0; w < kMaxExperts / 32; w++) {
+    const unsigned long long u = s_w[w];
+    const int v = s_wc[w];
+    if (w < warp) {
+      ab += u;
+      c += v;
+    }
+    ab_all += u;
+    c_all += v;
+  }
+  const int first = (int)(uint32_t)ab - cnt, total_full = c_all;
   if (e < E) eoff[e] = first;
   if (e == 0) {
-    eoff[E] = s_a[kMaxExperts - 1];  // pairs placed (= T*k unless ids outside [0, E) were dropped)
-    n_runs[0] = s_b[kMaxExperts - 1];
+    eoff[E] = (int)(uint32_t)ab_all;  // pairs placed (= T*k unless ids outside [0, E) were dropped)
+    n_runs[0] = (int)(ab_all >> 32);
     n_runs[1] = 1;  // the shared expert's run, kept at runs[kMaxExperts]
     runs[kMaxExperts] = Run{0, pairs, T};
   }
-  if (cnt > 0) runs[s_b[e] - 1] = Run{e, first, cnt};
-  const int full0 = s_c[e] - nfull;
+  if (cnt > 0) runs[(int)(ab >> 32) - 1] = Run{e, first, cnt};
+  const int full0 = c - nfull;
   for (int j = 0; j < nfull; j++) tiles[full0 + j] = Tile{e, first + j * tile_cap, tile_cap};
-  __syncthreads();
   // rank of the ragged tile among all ragged tiles: larger first, ties to the lower id
-  s_a[e] = part;
-  __syncthreads();
   int rank = 0, nparts = 0;
-  for (int o = 0; o < kMaxExperts; o++) {
-    int p = s_a[o];
-    nparts += p > 0;
-    rank += (p > part) || (p == part && o < e);
+#pragma unroll 4
+  for (int o = 0; o < kMaxExperts; o += 4) {
+    const int4 q = *(const int4*)(s_a + o);
+    nparts += (q.x > 0) + (q.y > 0) + (q.z > 0) + (q.w > 0);
+    rank += (q.x > part || (q.x == part && o < e)) + (q.y > part || (q.y == part && o + 1 < e)) +
+            (q.z > part || (q.z == part && o + 2 < e)) + (q.w > part || (q.w == part && o + 3 < e));
   }
   if (part > 0) tiles[total_full + rank] = Tile{e, first + nfull * tile_cap, part};
   // tiles of the shared expert: all T tokens in token order, rows behind the routed ones
@@ -257,49 +277,56 @@ k_route_scan(int32_t* __restrict__ blockcnt, int nblk, int E, int pairs, int T, 
   }
 }
 
-__global__ void __launch_bounds__(32)
+// Places in expert order, stable in the pair index. A thread per pair: pairs of one warp with the same
+// expert are told apart by their lanes, the warps' counts by a prefix over the block's 16 warps, so
+// that nothing is serial but that prefix (one warp walking the 512 pairs took 24 us at any T).
+__global__ void __launch_bounds__(kChunk)
 k_route_place(const int32_t* __restrict__ ids, const float* __restrict__ w, int stride, int pairs,
               int k, int E, const int32_t* __restrict__ blockcnt, const int32_t* __restrict__ eoff,
               int32_t* __restrict__ tokidx, float* __restrict__ pw, int32_t* __restrict__ pairids) {
-  __shared__ int cursor[kMaxExperts];
-  const int lane = threadIdx.x;
-  for (int e = lane; e < E; e += 32) cursor[e] = eoff[e] + blockcnt[(size_t)blockIdx.x * E + e];
-  __syncwarp();
-  const int base = blockIdx.x * kChunk;
-  for (int it = 0; it < kChunk / 32; it++) {
-    const int p = base + it * 32 + lane;
-    const bool live = p < pairs;
-    const unsigned act = __ballot_sync(0xffffffffu, live);
-    if (live) {
-      const int t = p / k, s = p % k;
-      const int e = ids[(size_t)t * stride + s];
-      const bool good = (unsigned)e < (unsigned)E;
-      const unsigned same = __match_any_sync(act, good ? e : -1);
-      const int leader = __ffs(same) - 1;
-      int start = 0;
-      if (good && lane == leader) {
-        start = cursor[e];
-        cursor[e] = start + __popc(same);
-      }
-      start = __shfl_sync(same, start, leader);
-      const int row = start + __popc(same & ((1u << lane) - 1u));
-      if (good) {
-        tokidx[row] = t;
-        pw[row] = w[(size_t)t * stride + s];
-      }
-      // slot in the token's reduce order: ascending expert id; equal ids keep their slot order,
-      // so every slot is written; a dropped pair's slot holds -1 (the combine skips it)
-      int rank = 0;
-      const int key = good ? e : kBadKey;
-      for (int q = 0; q < k; q++) {
-        const int eq = ids[(size_t)t * stride + q];
-        const int kq = (unsigned)eq < (unsigned)E ? eq : kBadKey;  // dropped pairs sort behind every expert
-        rank += (kq < key) || (kq == key && q < s);
-      }
-      pairids[(size_t)t * k + rank] = good ? row : -1;
+  __shared__ __align__(4) uint16_t before[kChunk / 32][kMaxExperts];  // pairs of an expert: per warp, then in the warps before
+  __shared__ int start[kMaxExperts];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  pdl_trigger();
+  for (int i = threadIdx.x; i < (int)sizeof(before) / 4; i += kChunk) ((uint32_t*)before)[i] = 0;
+  pdl_wait();
+  const int p = blockIdx.x * kChunk + threadIdx.x;
+  const bool live = p < pairs;
+  const int t = live ? p / k : 0, s = live ? p % k : 0;
+  const int e = live ? ids[(size_t)t * stride + s] : -1;
+  const bool good = (unsigned)e < (unsigned)E;
+  const float wt = live ? w[(size_t)t * stride + s] : 0.f;
+  for (int i = threadIdx.x; i < E; i += kChunk) start[i] = eoff[i] + blockcnt[(size_t)blockIdx.x * E + i];
+  __syncthreads();
+  const unsigned same = __match_any_sync(0xffffffffu, good ? e : -1);
+  if (good && lane == __ffs(same) - 1) before[warp][e] = (uint16_t)__popc(same);
+  __syncthreads();
+  for (int i = threadIdx.x; i < E; i += kChunk) {
+    int run = 0;
+#pragma unroll
+    for (int v = 0; v < kChunk / 32; v++) {
+      const int n = before[v][i];
+      before[v][i] = (uint16_t)run;
+      run += n;
     }
-    __syncwarp();
   }
+  __syncthreads();
+  if (!live) return;
+  const int row = good ? start[e] + before[warp][e] + __popc(same & ((1u << lane) - 1u)) : -1;
+  if (good) {
+    tokidx[row] = t;
+    pw[row] = wt;
+  }
+  // slot in the token's reduce order: ascending expert id; equal ids keep their slot order,
+  // so every slot is written; a dropped pair's slot holds -1 (the combine skips it)
+  int rank = 0;
+  const int key = good ? e : kBadKey;
+  for (int q = 0; q < k; q++) {
+    const int eq = ids[(size_t)t * stride + q];
+    const int kq = (unsigned)eq < (unsigned)E ? eq : kBadKey;  // dropped pairs sort behind every expert
+    rank += (kq < key) || (kq == key && q < s);
+  }
+  pairids[(size_t)t * k + rank] = row;
 }
 
 // Scalar sigmoid gate of the shared expert (src/ref.cpp:623-626, 635): one warp per token.
@@ -331,22 +358,24 @@ k_shared_gate(const uint16_t* __restrict__ x, const uint16_t* __restrict__ gw, i
 
 cudaError_t launch_router_topk(const float* logits, int T, int E, int k, int32_t* ids, float* w,
                                int stride, cudaStream_t st) {
-  k_router_topk<<<(T + kRouterWarps - 1) / kRouterWarps, kRouterWarps * 32, 0, st>>>(
-      logits, T, E, k, ids, w, stride);
-  return cudaGetLastError();
+  return launch_pdl(k_router_topk, dim3((T + kRouterWarps - 1) / kRouterWarps), dim3(kRouterWarps * 32), 0, st, logits, T, E,
+                    k, ids, w, stride);
 }
 
 cudaError_t launch_route(const RouteBuffers& rb, const int32_t* ids, const float* w, int stride,
                          int T, int k, int E, int tile_cap, cudaStream_t st, int* launches) {
   const int pairs = T * k;
   const int nblk = (pairs + kChunk - 1) / kChunk;
-  k_route_count<<<nblk, 32, 0, st>>>(ids, stride, pairs, k, E, rb.blockcnt, rb.status);
-  k_route_scan<<<1, kMaxExperts, 0, st>>>(rb.blockcnt, nblk, E, pairs, T, tile_cap, rb.eoff, rb.runs,
-                                           rb.n_runs, rb.tiles, rb.tiles_sh, rb.n_tiles);
-  k_route_place<<<nblk, 32, 0, st>>>(ids, w, stride, pairs, k, E, rb.blockcnt, rb.eoff, rb.tokidx,
-                                     rb.pw, rb.pairids);
+  // every kernel of the chain waits for the one before it: the launches overlap its tail
+  cudaError_t e = launch_pdl(k_route_count, dim3(nblk), dim3(kChunk), 0, st, ids, stride, pairs, k, E, rb.blockcnt, rb.status);
+  if (e == cudaSuccess)
+    e = launch_pdl(k_route_scan, dim3(1), dim3(kMaxExperts), 0, st, rb.blockcnt, nblk, E, pairs, T, tile_cap, rb.eoff, rb.runs,
+                   rb.n_runs, rb.tiles, rb.tiles_sh, rb.n_tiles);
+  if (e == cudaSuccess)
+    e = launch_pdl(k_route_place, dim3(nblk), dim3(kChunk), 0, st, ids, w, stride, pairs, k, E, rb.blockcnt, rb.eoff, rb.tokidx,
+                   rb.pw, rb.pairids);
   if (launches) *launches += 3;
-  return cudaGetLastError();
+  return e;
 }
 
 cudaError_t launch_shared_gate(const void* x_bf16, const uint16_t* gate_w_bf16, int T, int d, int k,
