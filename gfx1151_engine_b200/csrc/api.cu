@@ -815,7 +815,7 @@ static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const
     n++;
     if (shared) {
       CU_TRY(h, launch_up_tc(h->tc, L.sh_gu, h->rb.tiles_sh, h->rb.n_tiles + 1, h->max_tiles_sh,
-                             (__half*)h->hid, h->status_dev, st));
+                             (__half*)h->hid, h->status_dev, st, true));
       n++;
     }
     if (ev) CU_TRY(h, cudaEventRecord(ev[3], st));
@@ -824,7 +824,7 @@ static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const
     n++;
     if (shared) {
       CU_TRY(h, launch_down_tc(h->tc, L.sh_dn, h->rb.tiles_sh, h->rb.n_tiles + 1, h->max_tiles_sh,
-                               (__half*)h->pairs, h->status_dev, st));
+                               (__half*)h->pairs, h->status_dev, st, nullptr, nullptr, true));
       n++;
     }
     if (ev) CU_TRY(h, cudaEventRecord(ev[4], st));

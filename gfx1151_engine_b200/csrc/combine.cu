@@ -61,6 +61,8 @@ k_combine(const TP* __restrict__ pairs, const float* __restrict__ pw,
   const int t = blockIdx.x;
   __shared__ int s_row[kMaxTopK + 1];
   __shared__ float s_w[kMaxTopK + 1];
+  pdl_trigger();
+  pdl_wait();
   int n = k;
   if (threadIdx.x < k) {
     // a negative row marks a pair the bucketing dropped (expert id outside [0, E)): it adds nothing
@@ -254,25 +256,23 @@ cudaError_t launch_combine_f32(const float* pairs, const float* pw, const int32_
     return launch_pdl(k_combine_small, dim3(T, (d / 4 + 127) / 128), dim3(128), 0, st, pairs, pw, pairids, k, d, shared_row0,
                       (__nv_bfloat16*)out_bf16, hc);
   else
-    k_combine<float><<<dim3(T, (d + 2047) / 2048), 256, 0, st>>>(pairs, pw, pairids, k, d, shared_row0, (__nv_bfloat16*)out_bf16, hc);
-  return cudaGetLastError();
+    return launch_pdl(k_combine<float>, dim3(T, (d + 2047) / 2048), dim3(256), 0, st, pairs, pw, pairids, k, d, shared_row0,
+                      (__nv_bfloat16*)out_bf16, hc, nullptr);
 }
 
 cudaError_t launch_combine_f16(const __half* pairs, const float* pw, const int32_t* pairids, int T,
                                int k, int d, int shared_row0, void* out_bf16, cudaStream_t st,
                                const float* hc_w4, void* hc_state) {
-  k_combine<__half><<<dim3(T, (d + 2047) / 2048), 256, 0, st>>>(pairs, pw, pairids, k, d, shared_row0,
-                                       (__nv_bfloat16*)out_bf16, HcWriteBack{hc_w4, (uint16_t*)hc_state});
-  return cudaGetLastError();
+  return launch_pdl(k_combine<__half>, dim3(T, (d + 2047) / 2048), dim3(256), 0, st, pairs, pw, pairids, k, d, shared_row0,
+                    (__nv_bfloat16*)out_bf16, HcWriteBack{hc_w4, (uint16_t*)hc_state}, nullptr);
 }
 
 cudaError_t launch_combine_f16_rot(const __half* pairs, const float* pw, const int32_t* pairids, int T,
                                    int k, int d, const float* rot_post, void* out_bf16, cudaStream_t st,
                                    const float* hc_w4, void* hc_state) {
   if (d % 128 != 0 || !rot_post) return cudaErrorInvalidValue;
-  k_combine<__half, true><<<dim3(T, (d + 2047) / 2048), 256, 0, st>>>(pairs, pw, pairids, k, d, -1, (__nv_bfloat16*)out_bf16,
-                                                                      HcWriteBack{hc_w4, (uint16_t*)hc_state}, rot_post);
-  return cudaGetLastError();
+  return launch_pdl(k_combine<__half, true>, dim3(T, (d + 2047) / 2048), dim3(256), 0, st, pairs, pw, pairids, k, d, -1,
+                    (__nv_bfloat16*)out_bf16, HcWriteBack{hc_w4, (uint16_t*)hc_state}, rot_post);
 }
 
 cudaError_t launch_scatter_f16(const void* x_bf16, int T, int k, int d, int shared_row0, __half* x_sorted,

@@ -41,6 +41,8 @@
 // word, stops issuing work, and leaves after releasing its tensor memory.
 #include "tc.h"
 
+#include "kernels.h"
+
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
@@ -263,6 +265,7 @@ struct KParams {
   int l2_ahead;      // weight tiles are asked into L2 this many own pairs ahead of their register fetch (0: off)
   const int32_t* rowmap;    // down kernel, may be null: tile-list row r >= map_base[0] is written to output row
   const int32_t* map_base;  // rowmap[r - map_base[0]] (rows below map_base[0], and all rows without a map: to row r)
+  int beside;        // 1: runs beside the launch in front of it (see the wait in the set-up)
 };
 constexpr int kTraceSlots = 512;
 // Timeline stamps of CTA 0 (a debugging aid: build with -DB200MOE_TRACE and set
@@ -355,9 +358,8 @@ k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ C
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const Image img = p.img;
   const int KB = img.n_kblocks;
-  const int n_items = p.n_tiles[0] * img.n_mtiles;
 
-  // ---- set-up ----
+  // ---- set-up (weights and the CTA's own state only: it overlaps the tail of the kernel before) ----
   if (threadIdx.x == 0) {
     for (int i = 0; i < kNS; i++) mbar_init(bars + 8 * (kBarAFull + i), 9);  // 8 dequantising warps + relay
     for (int i = 0; i < kNBS; i++) {
@@ -386,6 +388,13 @@ k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ C
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
+  // The kernel before in the stream is complete behind this wait. The shared expert's launch (p.beside)
+  // has nothing to wait for but what the routed launch in front of it has waited for before it let this
+  // one start: its few CTAs fill SMs as the routed ones leave them, and it waits at its end instead, so
+  // that its completion still stands for both.
+  if (!p.beside) pdl_wait();
+  pdl_trigger();
+  const int n_items = p.n_tiles[0] * img.n_mtiles;
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -762,6 +771,7 @@ k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ C
   }
 
   // ---- teardown ----
+  if (p.beside) pdl_wait();
   __syncthreads();
   if (*abort_flag) {
     // give copies still in flight time to land before the CTA's shared memory goes away
@@ -791,7 +801,7 @@ cudaError_t encode_2d(PFN_cuTensorMapEncodeTiled_v12000 enc, CUtensorMap* map, c
 template <bool UP, bool DUAL, int FMT>
 cudaError_t launch(TcPlan* plan, const CUtensorMap* m, const Image& img,
                    const Tile* tiles, const int32_t* n_tiles, int max_tiles, __half* out, int out_ld,
-                   int32_t* status, cudaStream_t st, const int32_t* rowmap = nullptr, const int32_t* map_base = nullptr) {
+                   int32_t* status, cudaStream_t st, const int32_t* rowmap = nullptr, const int32_t* map_base = nullptr, bool beside = false) {
   constexpr int kSmemBytes = Map::kSmemBytes;
   static bool attr_set = false;  // one flag per template instance
   if (!attr_set) {
@@ -802,13 +812,12 @@ cudaError_t launch(TcPlan* plan, const CUtensorMap* m, const Image& img,
   }
   static const int l2_ahead = getenv("B200MOE_TC_L2_AHEAD") ? atoi(getenv("B200MOE_TC_L2_AHEAD")) : 3;
   KParams p{img, tiles, n_tiles, out, out_ld, status, (UP != (getenv("B200MOE_TC_TRACE_DOWN") != nullptr)) ? plan->trace : nullptr,
-            l2_ahead, rowmap, map_base};
+            l2_ahead, rowmap, map_base, beside ? 1 : 0};
   long long max_items = (long long)max_tiles * img.n_mtiles;
   const int usable = plan->sms - plan->margin > 1 ? plan->sms - plan->margin : 1;
   int grid = (int)(max_items < usable ? max_items : usable);
   if (grid < 1) grid = 1;
-  k_expert_tc<UP, DUAL, FMT><<<grid, kThreads, kSmemBytes, st>>>(m[0], m[1], m[2], m[3], p);
-  return cudaGetLastError();
+  return launch_pdl(k_expert_tc<UP, DUAL, FMT>, dim3(grid), dim3(kThreads), (size_t)kSmemBytes, st, m[0], m[1], m[2], m[3], p);
 }
 
 }  // namespace
@@ -865,28 +874,29 @@ void tc_destroy(TcPlan* plan) {
 }
 
 cudaError_t launch_up_tc(TcPlan* plan, const Image& img, const Tile* tiles, const int32_t* n_tiles,
-                         int max_tiles, __half* hid16, int32_t* status, cudaStream_t st) {
+                         int max_tiles, __half* hid16, int32_t* status, cudaStream_t st, bool beside) {
   if (img.fmt == kQ4K)
     return launch<true, false, kQ4K>(plan, plan->x, img, tiles, n_tiles, max_tiles, hid16, img.n_mtiles * 64, status, st);
   if (img.fmt == kQ51)  // Q5_K gate/up in the Q5_1 image form
     return launch<true, false, kQ51>(plan, plan->x, img, tiles, n_tiles, max_tiles, hid16, img.n_mtiles * 64, status, st);
   if (img.fmt != kQ4CP) return cudaErrorNotSupported;
   if (img.dual_book)
-    return launch<true, true, kQ4CP>(plan, plan->x, img, tiles, n_tiles, max_tiles, hid16, img.n_mtiles * 64, status, st);
+    return launch<true, true, kQ4CP>(plan, plan->x, img, tiles, n_tiles, max_tiles, hid16, img.n_mtiles * 64, status, st, nullptr,
+                                     nullptr, beside);
   return launch<true, false, kQ4CP>(plan, plan->x, img, tiles, n_tiles, max_tiles, hid16,
-                      img.n_mtiles * 64, status, st);
+                      img.n_mtiles * 64, status, st, nullptr, nullptr, beside);
 }
 
 cudaError_t launch_down_tc(TcPlan* plan, const Image& img, const Tile* tiles, const int32_t* n_tiles,
                            int max_tiles, __half* pairs16, int32_t* status, cudaStream_t st, const int32_t* rowmap,
-                           const int32_t* map_base) {
+                           const int32_t* map_base, bool beside) {
   if ((rowmap == nullptr) != (map_base == nullptr)) return cudaErrorInvalidValue;
   if (img.fmt == kQ51)
     return launch<false, false, kQ51>(plan, plan->h, img, tiles, n_tiles, max_tiles, pairs16, img.n_mtiles * 128, status, st,
                                       rowmap, map_base);
   if (img.fmt != kQ4CP) return cudaErrorNotSupported;
   return launch<false, false, kQ4CP>(plan, plan->h, img, tiles, n_tiles, max_tiles, pairs16,
-                       img.n_mtiles * 128, status, st, rowmap, map_base);
+                       img.n_mtiles * 128, status, st, rowmap, map_base, beside);
 }
 
 cudaError_t launch_raw_tc(TcPlan* plan, const Image& img, const Tile* tiles, const int32_t* n_tiles,

@@ -53,6 +53,8 @@ k_rot_in(const uint16_t* __restrict__ x, const float* __restrict__ pre, const in
          int d, __half* __restrict__ x_sorted) {
   const int lane = threadIdx.x & 31;
   const int nb = d >> 7;
+  pdl_trigger();
+  pdl_wait();
   const long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (w >= (long long)T * nb) return;
   const int t = (int)(w / nb), b = (int)(w % nb);
@@ -85,6 +87,8 @@ k_i4r_mid(const __half* __restrict__ z, const float* __restrict__ svh_gu, const 
           long long rows, int mid, __half* __restrict__ hr) {
   const int lane = threadIdx.x & 31;
   const int nb = mid >> 7;
+  pdl_trigger();
+  pdl_wait();
   const long long total = rows * nb;
   for (long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < total;
        w += (long long)gridDim.x * (blockDim.x >> 5)) {
@@ -122,8 +126,8 @@ cudaError_t launch_rot_in(const void* x_bf16, const float* pre, const int32_t* p
                           __half* x_sorted, cudaStream_t st) {
   const long long warps = (long long)T * (d >> 7);
   if (warps == 0) return cudaSuccess;
-  k_rot_in<<<(unsigned)((warps + 7) / 8), 256, 0, st>>>((const uint16_t*)x_bf16, pre, pairids, T, k, d, x_sorted);
-  return cudaGetLastError();
+  return launch_pdl(k_rot_in, dim3((unsigned)((warps + 7) / 8)), dim3(256), 0, st, (const uint16_t*)x_bf16, pre, pairids, T, k, d,
+                    x_sorted);
 }
 
 cudaError_t launch_i4r_mid(const __half* z, const float* svh_gu, const float* suh_dn, int rows, int mid, __half* hr,
@@ -132,8 +136,7 @@ cudaError_t launch_i4r_mid(const __half* z, const float* svh_gu, const float* su
   long long blocks = (warps + 7) / 8;
   if (blocks > 148 * 16) blocks = 148 * 16;
   if (blocks < 1) blocks = 1;
-  k_i4r_mid<<<(unsigned)blocks, 256, 0, st>>>(z, svh_gu, suh_dn, (long long)rows, mid, hr);
-  return cudaGetLastError();
+  return launch_pdl(k_i4r_mid, dim3((unsigned)blocks), dim3(256), 0, st, z, svh_gu, suh_dn, (long long)rows, mid, hr);
 }
 
 cudaError_t launch_f16_to_f32(const void* src_f16_dev, float* dst, int n, cudaStream_t st) {
