@@ -33,6 +33,13 @@ struct LayerWeights {
 
 }  // namespace
 
+// At most this many rows per expert on average: tiles of 64 rows and the GEMM kernels' narrow form, which
+// hides the latency of the weights. Beyond it the popular experts of a skewed routing have hundreds of
+// rows, and decoding their weights once per 64 rows costs more than that. Measured wide / narrow:
+// 1.5 rows on average (77 tokens, 512 experts of 4096 x 1024) 526 / 477 us, 10 rows (500 tokens, 2560 x 640)
+// 474 / 454, 40 rows (2048 tokens) 748 / 802; chunks of 1024 tokens (20 rows) lose 20 %.
+constexpr int kNarrowRows = 12;
+
 struct b200moe_ctx {
   b200moe_config cfg{};
   int decode_max = 16;
@@ -258,8 +265,10 @@ int b200moe_create(const b200moe_config* cfg, b200moe_handle* out) {
   const size_t pairs = (size_t)Tm * k;
   const size_t rows = pairs + (c.has_shared ? Tm : 0);
   h->max_rows = (int)rows;
-  h->max_tiles = (int)(pairs / h->tile_cap) + E + 1;
-  h->max_tiles_sh = Tm / h->tile_cap + 1;
+  // (calls with few rows per expert cut them into narrow tiles)
+  const size_t narrow_pairs = std::min(pairs, (size_t)kNarrowRows * E), narrow_tokens = std::min((size_t)Tm, narrow_pairs / k);
+  h->max_tiles = (int)std::max(pairs / h->tile_cap, narrow_pairs / kTcNarrowN) + E + 1;
+  h->max_tiles_sh = (int)std::max((size_t)(Tm / h->tile_cap), narrow_tokens / kTcNarrowN) + 1;
   const size_t dec_rows = (size_t)std::min(Tm, h->decode_max) * (k + (c.has_shared ? 1 : 0));
   const bool simt_all = c.gemm_impl == B200MOE_GEMM_SIMT;
   const size_t hid_bytes = std::max(rows * mid * (simt_all ? 4 : 2), dec_rows * mid * 4);
@@ -709,6 +718,8 @@ static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const
   }
   const bool simt = !L.i4r && (c.gemm_impl == B200MOE_GEMM_SIMT ||
                                 (c.gemm_impl == B200MOE_GEMM_AUTO && T <= h->decode_max));
+  const bool narrow = T * k <= kNarrowRows * E;
+  const TcLaunch routed{narrow, false}, beside{narrow, true};
   const uint16_t* gate_w = nullptr;  // set: the shared expert's gate is still to be computed
   static const bool slow_router = getenv("B200MOE_EXACT_ROUTER") != nullptr;  // A/B: the general routing body for every call
   if (logits && !slow_router && T <= decode_max_tokens() && T * k <= 128 && d % 8 == 0 && (!shared || ((uintptr_t)x & 15) == 0)) {
@@ -727,7 +738,7 @@ static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const
       w = h->rb.topw;
       stride = kIdStride;
     }
-    CU_TRY(h, launch_route(h->rb, ids, w, stride, T, k, E, h->tile_cap, st, &n));
+    CU_TRY(h, launch_route(h->rb, ids, w, stride, T, k, E, narrow ? kTcNarrowN : h->tile_cap, st, &n));
     if (shared && simt) {
       CU_TRY(h, launch_shared_gate(x, L.sh_gate_w, T, d, k, h->rb, st));
       n++;
@@ -790,11 +801,11 @@ static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const
       CU_TRY(h, launch_rot_in(x, L.rot, h->rb.pairids, T, k, d, h->x_sorted, st));
       n++;
       if (ev) CU_TRY(h, cudaEventRecord(ev[2], st));
-      CU_TRY(h, launch_raw_tc(h->tc, L.gu, h->rb.tiles, h->rb.n_tiles, h->max_tiles, (__half*)h->pairs, h->status_dev, st));
+      CU_TRY(h, launch_raw_tc(h->tc, L.gu, h->rb.tiles, h->rb.n_tiles, h->max_tiles, (__half*)h->pairs, h->status_dev, st, routed));
       CU_TRY(h, launch_i4r_mid((const __half*)h->pairs, L.rot + d, L.rot + d + 2 * mid, rows, mid, (__half*)h->hid, st));
       n += 2;
       if (ev) CU_TRY(h, cudaEventRecord(ev[3], st));
-      CU_TRY(h, launch_down_tc(h->tc, L.dn, h->rb.tiles, h->rb.n_tiles, h->max_tiles, (__half*)h->pairs, h->status_dev, st));
+      CU_TRY(h, launch_down_tc(h->tc, L.dn, h->rb.tiles, h->rb.n_tiles, h->max_tiles, (__half*)h->pairs, h->status_dev, st, routed));
       if (ev) CU_TRY(h, cudaEventRecord(ev[4], st));
       CU_TRY(h, launch_combine_f16_rot((const __half*)h->pairs, h->rb.pw, h->rb.pairids, T, k, d, L.rot + d + 3 * mid, out, st,
                                        h->hc_w4, h->hc_state));
@@ -811,20 +822,20 @@ static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const
     n++;
     if (ev) CU_TRY(h, cudaEventRecord(ev[2], st));
     CU_TRY(h, launch_up_tc(h->tc, L.gu, h->rb.tiles, h->rb.n_tiles, h->max_tiles, (__half*)h->hid,
-                           h->status_dev, st));
+                           h->status_dev, st, routed));
     n++;
     if (shared) {
       CU_TRY(h, launch_up_tc(h->tc, L.sh_gu, h->rb.tiles_sh, h->rb.n_tiles + 1, h->max_tiles_sh,
-                             (__half*)h->hid, h->status_dev, st, true));
+                             (__half*)h->hid, h->status_dev, st, beside));
       n++;
     }
     if (ev) CU_TRY(h, cudaEventRecord(ev[3], st));
     CU_TRY(h, launch_down_tc(h->tc, L.dn, h->rb.tiles, h->rb.n_tiles, h->max_tiles,
-                             (__half*)h->pairs, h->status_dev, st));
+                             (__half*)h->pairs, h->status_dev, st, routed));
     n++;
     if (shared) {
       CU_TRY(h, launch_down_tc(h->tc, L.sh_dn, h->rb.tiles_sh, h->rb.n_tiles + 1, h->max_tiles_sh,
-                               (__half*)h->pairs, h->status_dev, st, nullptr, nullptr, true));
+                               (__half*)h->pairs, h->status_dev, st, beside));
       n++;
     }
     if (ev) CU_TRY(h, cudaEventRecord(ev[4], st));
@@ -1224,7 +1235,7 @@ int b200moe_ep_experts_part(b200moe_handle h, int layer, const int32_t* eoff_all
                                     h->sms, st));
     CU_TRY(h, launch_up_tc(h->tc_ep, L.gu, h->ep_tiles, h->ep_counts, h->ep_max_tiles, h->ep_hid, h->status_dev, st));
     CU_TRY(h, launch_down_tc(h->tc_ep, L.dn, h->ep_tiles, h->ep_counts, h->ep_max_tiles, h->ep_pairs_recv, h->status_dev, st,
-                             h->ep_rowmap, h->ep_counts + 1));
+                             TcLaunch{false, false, h->ep_rowmap, h->ep_counts + 1}));
     h->launches += 4;
     return B200MOE_OK;
   }

@@ -62,7 +62,7 @@ namespace {
 
 constexpr int kNS = 2;    // tensor-memory A slots; a slot holds a pair of K blocks (64 columns)
 constexpr int kNBSMax = 3;
-constexpr int kBStage = kTcTileN * 128;  // bytes of one K block of activations: rows x 64 halfs
+constexpr int kNST = 8;                  // narrow tiles: stages of packed weights, a pair of K blocks each
 constexpr int kThreads = 768;           // 24 warps: 4 service, 16 dequantising, 4 epilogue
 constexpr int kAccCols = kTcTileN;       // columns per accumulator
 constexpr int kTmemA = 2 * kAccCols;     // first column of the A slots
@@ -76,19 +76,29 @@ static_assert(kTmemA + kNS * 64 <= 512, "tensor memory: two accumulators and the
 // boundary, so that a lookup address is ONE byte permute:
 //   bytes { lane*4 (+128), code byte, table >> 16, 0 }.
 // The first activation slot fits below the table, the other two above it.
+//
+// TN is the most rows a tile of the launch has. 192 (prefill chunks): the activation slots take all
+// there is. 64 (launches whose experts have few rows, where the MMAs are short and the packed weights
+// decide): all three slots lie below the table and the space above it is a ring of kNST pairs of
+// weight tiles (74 to 98 KB in flight per SM), which warp 2 fills with bulk copies. The dequantising
+// warps' register fetch of the wide form reaches one pair ahead, which is less than a load from L2
+// takes: on a 77-token prompt (1 to 3 rows per expert) 40 % of their time went into that wait.
+template <int TN>
 struct Map {
+  static constexpr int kBStage = TN * 128;             // bytes of one K block of activations: rows x 64 halfs
   static constexpr int kNBS = 3;                       // activation ring depth, in pairs of K blocks
   static constexpr int kOffLow = 2048;                 // the dynamic allocation must start at or below this
   static constexpr int kOffBar = 2048;                 // barriers and flags (1 KB)
   static constexpr int kOffU = 3072;                   // epilogue exchange + output tile (12 KB)
   static constexpr int kOffB0 = 15360;                 // activation slot 0 (1 KB aligned)
   static constexpr int kOffLut = 65536;                // 256 lines of 256 B
-  static constexpr int kOffB1 = 131072;                // activation slots 1, 2
-  static constexpr int kSmemEnd = kOffB1 + 2 * 2 * kBStage;
+  static constexpr int kOffB1 = 131072;                // wide: activation slots 1, 2; narrow: weight stages
+  static constexpr int kSmemEnd = TN == kTcTileN ? kOffB1 + 2 * 2 * kBStage : kOffB1 + kNST * 2 * tile_bytes(kQ51);
   static constexpr int kSmemBytes = kSmemEnd - 1024;   // dynamic bytes requested
-  static_assert(kOffB0 + 2 * kBStage <= kOffLut, "slot 0 overlaps the table");
+  static_assert(kOffB0 + (TN == kTcTileN ? 1 : kNBS) * 2 * kBStage <= kOffLut, "activation slots overlap the table");
   static_assert(kSmemEnd <= 233472, "shared memory map exceeds the SM");
   __host__ __device__ static constexpr uint32_t slot(uint32_t s) {
+    if (TN != kTcTileN) return (uint32_t)(kOffB0 + s * 2 * kBStage);
     return s == 0 ? (uint32_t)kOffB0 : (uint32_t)(kOffB1 + (s - 1) * 2 * kBStage);
   }
 };
@@ -98,7 +108,10 @@ constexpr int kBarAFull = 0,                   // [tensor-memory slot]: A of a p
               kBarBFull = kBarAFull + kNS,     // [activation slot]
               kBarDone = kBarBFull + kNBSMax,  // [activation slot]: all MMAs of a pair have completed
               kBarAccFull = kBarDone + kNBSMax,
-              kBarAccEmpty = kBarAccFull + 2, kNumBars = kBarAccEmpty + 2;
+              kBarAccEmpty = kBarAccFull + 2,
+              kBarCFull = kBarAccEmpty + 2,    // [weight stage] (narrow): a pair's packed tiles have landed
+              kBarCEmpty = kBarCFull + kNST,   // [weight stage]: the set's eight warps hold them in registers
+              kNumBars = kBarCEmpty + kNST;
 static_assert(kNumBars * 8 + 16 + 32 <= 1024, "barrier block too small");
 
 constexpr long long kWaitLimitNs = 2000000000ll;  // 2 s: far beyond any legitimate wait
@@ -330,7 +343,7 @@ struct GroupDecode<kQ51> {  // w = d*(q + 16*fifth bit) + m, src/gguf.h:360-374
   }
 };
 
-template <bool UP, bool DUAL, int FMT>
+template <bool UP, bool DUAL, int FMT, int TN>
 __global__ void __launch_bounds__(kThreads, 1)
 k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ CUtensorMap map64,
             const __grid_constant__ CUtensorMap map128, const __grid_constant__ CUtensorMap map192,
@@ -340,8 +353,9 @@ k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ C
   const uint32_t dyn0 = smem_u32(smem_raw);
   uint8_t* const smem = smem_raw - dyn0;
   constexpr uint32_t sbase = 0;
-  using M = Map;
-  constexpr int kNBS = M::kNBS, kOffLow = M::kOffLow, kOffU = M::kOffU, kOffBar = M::kOffBar,
+  using M = Map<TN>;
+  constexpr bool kNarrow = TN != kTcTileN;
+  constexpr int kBStage = M::kBStage, kNBS = M::kNBS, kOffLow = M::kOffLow, kOffU = M::kOffU, kOffBar = M::kOffBar,
                 kSmemEnd = M::kSmemEnd;
   {
     uint32_t dyn_size;
@@ -365,6 +379,10 @@ k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ C
     for (int i = 0; i < kNBS; i++) {
       mbar_init(bars + 8 * (kBarBFull + i), 1);    // activation producer (with byte count)
       mbar_init(bars + 8 * (kBarDone + i), 1);     // one tcgen05.commit per pair
+    }
+    for (int i = 0; i < kNST; i++) {
+      mbar_init(bars + 8 * (kBarCFull + i), 1);
+      mbar_init(bars + 8 * (kBarCEmpty + i), 8);
     }
     for (int i = 0; i < 2; i++) {
       mbar_init(bars + 8 * (kBarAccFull + i), 1);
@@ -431,7 +449,7 @@ k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ C
         const uint8_t* w_next =
             it + (int)gridDim.x < n_items ? img.tile(t_ahead.expert, (it + (int)gridDim.x) % img.n_mtiles, 0) : nullptr;
         for (int pp = 0; pp < NP && ok; pp++, pi++) {
-          if (p.l2_ahead > 0) {
+          if (!kNarrow && p.l2_ahead > 0) {
             int q = pp + 2 * p.l2_ahead;
             const uint8_t* b2 = w_this;
             if (q >= NP) {
@@ -543,8 +561,8 @@ k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ C
     };
     const int io_step = NP == 1 ? 2 : 1;  // a set visits every item, or every other one when an item is one pair
     int f_io = set / NP, f_pp = set % NP;
-    const uint8_t* f_base = item_base(f_io);
-    const uint8_t* f_next = item_base(f_io + io_step);
+    const uint8_t* f_base = kNarrow ? nullptr : item_base(f_io);
+    const uint8_t* f_next = kNarrow ? nullptr : item_base(f_io + io_step);
     // f_tile walks with the stream: the tile of K block 2 * f_pp + kblk of the current item
     const uint8_t* f_tile = f_base ? f_base + (size_t)(2 * f_pp + kblk) * tile_b : nullptr;
     const size_t step_b = 4 * tile_b;  // the set's next pair is two pairs = four K blocks further
@@ -577,15 +595,49 @@ k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ C
         f_tile = f_base ? f_base + (size_t)(2 * f_pp + kblk) * tile_b : nullptr;
       }
     };
-    fetch(ca, cb, sc);
+    if (!kNarrow) fetch(ca, cb, sc);
     bool mine = f_valid;  // the codes in (ca, cb, sc) are a K block of this thread's
     bool ok = true;
+    // narrow: the pair's tiles come from the ring of weight stages
+    uint32_t c_stage = (uint32_t)set, c_ph = 0;
+    int c_pp = set % NP;
+    auto from_ring = [&]() -> bool {
+      if (!__all_sync(0xffffffffu, mbar_wait(bars + 8 * (kBarCFull + c_stage), c_ph, abort_flag, p.status, 11))) return false;
+      mine = 2 * c_pp + kblk < KB;
+      if (mine) {
+        const uint8_t* pc = smem + M::kOffB1 + c_stage * (2 * (uint32_t)tile_b) + kblk * (uint32_t)tile_b + off_c;
+        ca = *(const uint4*)pc;
+        cb = *(const uint4*)(pc + 2048);
+        const uint8_t* pm = pc + (off_m - off_c);
+        if (FMT == kQ4CP) {
+          sc.a = *(const uint32_t*)pm;
+        } else if (FMT == kQ4K) {
+          const uint2 u = *(const uint2*)pm;
+          sc.a = u.x;
+          sc.b = u.y;
+        } else {
+          const uint4 u = *(const uint4*)pm;
+          sc = RowMetaTc{u.x, u.y, u.z, u.w};
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bars + 8 * (kBarCEmpty + c_stage));
+      c_stage += 2;
+      if (c_stage >= (uint32_t)kNST) {
+        c_stage -= kNST;
+        c_ph ^= 1;
+      }
+      for (c_pp += 2; c_pp >= NP;) c_pp -= NP;
+      return true;
+    };
+    static_assert(kNST % 2 == 0, "a set visits every other stage");
     static_assert(kNS == 2, "a set always fills the tensor-memory slot of its own index");
     const uint32_t aslot = (uint32_t)set;
     uint32_t qslot = (uint32_t)set % kNBS, qph = 0;  // (pi - kNS) % kNBS and ((pi - kNS) / kNBS) & 1, from pi == set + kNS on
     for (uint32_t pi = set; pi < total && ok; pi += 2) {
       if (lane == 0 && quarter == 0) TR(2 + kblk, pi, 0);
       uint32_t v[32];
+      if (kNarrow && !from_ring()) break;
       const bool mine_now = mine;
       if (mine_now) {
 #pragma unroll
@@ -610,8 +662,10 @@ k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ C
       // The codes are used up: the next own pair's go into the same registers (no second set, no
       // copies). They have the rest of this iteration and the wait of the next one to arrive, and
       // the producer thread's L2 prefetch has put them close.
-      fetch(ca, cb, sc);
-      mine = f_valid;
+      if (!kNarrow) {
+        fetch(ca, cb, sc);
+        mine = f_valid;
+      }
       if (lane == 0 && quarter == 0) TR(2 + kblk, pi, 1);
       if (pi >= (uint32_t)kNS) {
         // the slot is free once the MMAs of the pair that used it before (pi - kNS) have completed
@@ -634,6 +688,31 @@ k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ C
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(bars + 8 * (kBarAFull + aslot));
+    }
+  } else if (kNarrow && warp == 2) {
+    // ================= producer of packed weights (one bulk copy per pair of K blocks) ==========
+    if (lane == 0) {
+      constexpr uint32_t w_tile_b = tile_bytes(FMT);
+      uint32_t stage = 0, ph = 0;
+      bool ok = true;
+      Tile t_ahead = (int)blockIdx.x < n_items ? p.tiles[blockIdx.x / img.n_mtiles] : Tile{0, 0, 0};
+      for (int it = blockIdx.x; it < n_items && ok; it += gridDim.x) {
+        const uint8_t* src = img.tile(t_ahead.expert, it % img.n_mtiles, 0);
+        if (it + (int)gridDim.x < n_items) t_ahead = p.tiles[(it + gridDim.x) / img.n_mtiles];
+        for (int pp = 0; pp < NP; pp++, src += 2 * w_tile_b) {
+          ok = mbar_wait(bars + 8 * (kBarCEmpty + stage), ph ^ 1, abort_flag, p.status, 12, 64);
+          if (!ok) break;
+          const uint32_t bytes = (uint32_t)min(2, KB - 2 * pp) * w_tile_b, bar = bars + 8 * (kBarCFull + stage);
+          mbar_expect_tx(bar, bytes);
+          asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                           (uint32_t)M::kOffB1 + stage * (2 * w_tile_b)), "l"(src), "r"(bytes), "r"(bar)
+                       : "memory");
+          if (++stage == (uint32_t)kNST) {
+            stage = 0;
+            ph ^= 1;
+          }
+        }
+      }
     }
   } else if (warp == 3) {
     // ================= relay: "activations landed" folded into the A-slot barrier ==========
@@ -798,14 +877,14 @@ cudaError_t encode_2d(PFN_cuTensorMapEncodeTiled_v12000 enc, CUtensorMap* map, c
   return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
-template <bool UP, bool DUAL, int FMT>
-cudaError_t launch(TcPlan* plan, const CUtensorMap* m, const Image& img,
+template <bool UP, bool DUAL, int FMT, int TN>
+cudaError_t launch_n(TcPlan* plan, const CUtensorMap* m, const Image& img,
                    const Tile* tiles, const int32_t* n_tiles, int max_tiles, __half* out, int out_ld,
-                   int32_t* status, cudaStream_t st, const int32_t* rowmap = nullptr, const int32_t* map_base = nullptr, bool beside = false) {
-  constexpr int kSmemBytes = Map::kSmemBytes;
+                   int32_t* status, cudaStream_t st, const int32_t* rowmap, const int32_t* map_base, bool beside) {
+  constexpr int kSmemBytes = Map<TN>::kSmemBytes;
   static bool attr_set = false;  // one flag per template instance
   if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(k_expert_tc<UP, DUAL, FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(k_expert_tc<UP, DUAL, FMT, TN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          kSmemBytes);
     if (e != cudaSuccess) return e;
     attr_set = true;
@@ -817,7 +896,18 @@ cudaError_t launch(TcPlan* plan, const CUtensorMap* m, const Image& img,
   const int usable = plan->sms - plan->margin > 1 ? plan->sms - plan->margin : 1;
   int grid = (int)(max_items < usable ? max_items : usable);
   if (grid < 1) grid = 1;
-  return launch_pdl(k_expert_tc<UP, DUAL, FMT>, dim3(grid), dim3(kThreads), (size_t)kSmemBytes, st, m[0], m[1], m[2], m[3], p);
+  return launch_pdl(k_expert_tc<UP, DUAL, FMT, TN>, dim3(grid), dim3(kThreads), (size_t)kSmemBytes, st, m[0], m[1], m[2], m[3], p);
+}
+
+template <bool UP, bool DUAL, int FMT>
+cudaError_t launch(TcPlan* plan, const CUtensorMap* m, const Image& img,
+                   const Tile* tiles, const int32_t* n_tiles, int max_tiles, __half* out, int out_ld,
+                   int32_t* status, cudaStream_t st, const TcLaunch& o) {
+  if (o.narrow)
+    return launch_n<UP, DUAL, FMT, kTcNarrowN>(plan, m, img, tiles, n_tiles, max_tiles, out, out_ld, status, st, o.rowmap,
+                                               o.map_base, o.beside);
+  return launch_n<UP, DUAL, FMT, kTcTileN>(plan, m, img, tiles, n_tiles, max_tiles, out, out_ld, status, st, o.rowmap,
+                                           o.map_base, o.beside);
 }
 
 }  // namespace
@@ -874,35 +964,29 @@ void tc_destroy(TcPlan* plan) {
 }
 
 cudaError_t launch_up_tc(TcPlan* plan, const Image& img, const Tile* tiles, const int32_t* n_tiles,
-                         int max_tiles, __half* hid16, int32_t* status, cudaStream_t st, bool beside) {
-  if (img.fmt == kQ4K)
-    return launch<true, false, kQ4K>(plan, plan->x, img, tiles, n_tiles, max_tiles, hid16, img.n_mtiles * 64, status, st);
+                         int max_tiles, __half* hid16, int32_t* status, cudaStream_t st, const TcLaunch& o) {
+  const int ld = img.n_mtiles * 64;
+  if (img.fmt == kQ4K) return launch<true, false, kQ4K>(plan, plan->x, img, tiles, n_tiles, max_tiles, hid16, ld, status, st, o);
   if (img.fmt == kQ51)  // Q5_K gate/up in the Q5_1 image form
-    return launch<true, false, kQ51>(plan, plan->x, img, tiles, n_tiles, max_tiles, hid16, img.n_mtiles * 64, status, st);
+    return launch<true, false, kQ51>(plan, plan->x, img, tiles, n_tiles, max_tiles, hid16, ld, status, st, o);
   if (img.fmt != kQ4CP) return cudaErrorNotSupported;
-  if (img.dual_book)
-    return launch<true, true, kQ4CP>(plan, plan->x, img, tiles, n_tiles, max_tiles, hid16, img.n_mtiles * 64, status, st, nullptr,
-                                     nullptr, beside);
-  return launch<true, false, kQ4CP>(plan, plan->x, img, tiles, n_tiles, max_tiles, hid16,
-                      img.n_mtiles * 64, status, st, nullptr, nullptr, beside);
+  if (img.dual_book) return launch<true, true, kQ4CP>(plan, plan->x, img, tiles, n_tiles, max_tiles, hid16, ld, status, st, o);
+  return launch<true, false, kQ4CP>(plan, plan->x, img, tiles, n_tiles, max_tiles, hid16, ld, status, st, o);
 }
 
 cudaError_t launch_down_tc(TcPlan* plan, const Image& img, const Tile* tiles, const int32_t* n_tiles,
-                           int max_tiles, __half* pairs16, int32_t* status, cudaStream_t st, const int32_t* rowmap,
-                           const int32_t* map_base, bool beside) {
-  if ((rowmap == nullptr) != (map_base == nullptr)) return cudaErrorInvalidValue;
-  if (img.fmt == kQ51)
-    return launch<false, false, kQ51>(plan, plan->h, img, tiles, n_tiles, max_tiles, pairs16, img.n_mtiles * 128, status, st,
-                                      rowmap, map_base);
+                           int max_tiles, __half* pairs16, int32_t* status, cudaStream_t st, const TcLaunch& o) {
+  if ((o.rowmap == nullptr) != (o.map_base == nullptr)) return cudaErrorInvalidValue;
+  const int ld = img.n_mtiles * 128;
+  if (img.fmt == kQ51) return launch<false, false, kQ51>(plan, plan->h, img, tiles, n_tiles, max_tiles, pairs16, ld, status, st, o);
   if (img.fmt != kQ4CP) return cudaErrorNotSupported;
-  return launch<false, false, kQ4CP>(plan, plan->h, img, tiles, n_tiles, max_tiles, pairs16,
-                       img.n_mtiles * 128, status, st, rowmap, map_base, beside);
+  return launch<false, false, kQ4CP>(plan, plan->h, img, tiles, n_tiles, max_tiles, pairs16, ld, status, st, o);
 }
 
 cudaError_t launch_raw_tc(TcPlan* plan, const Image& img, const Tile* tiles, const int32_t* n_tiles,
-                          int max_tiles, __half* z16, int32_t* status, cudaStream_t st) {
+                          int max_tiles, __half* z16, int32_t* status, cudaStream_t st, const TcLaunch& o) {
   if (img.fmt != kQ4CP || img.paired) return cudaErrorNotSupported;
-  return launch<false, false, kQ4CP>(plan, plan->x, img, tiles, n_tiles, max_tiles, z16, img.n_mtiles * 128, status, st);
+  return launch<false, false, kQ4CP>(plan, plan->x, img, tiles, n_tiles, max_tiles, z16, img.n_mtiles * 128, status, st, o);
 }
 
 }  // namespace b200moe

@@ -366,7 +366,8 @@ cudaError_t launch_route(const RouteBuffers& rb, const int32_t* ids, const float
                          int T, int k, int E, int tile_cap, cudaStream_t st, int* launches) {
   const int pairs = T * k;
   const int nblk = (pairs + kChunk - 1) / kChunk;
-  // every kernel of the chain waits for the one before it: the launches overlap its tail
+  // Every kernel of the chain waits for the one before it: its launch and set-up overlap that one's tail.
+  // (These kernels with a thread per pair: 592 -> 559 us on a 77-token call, 531 -> 500 on 500 tokens.)
   cudaError_t e = launch_pdl(k_route_count, dim3(nblk), dim3(kChunk), 0, st, ids, stride, pairs, k, E, rb.blockcnt, rb.status);
   if (e == cudaSuccess)
     e = launch_pdl(k_route_scan, dim3(1), dim3(kMaxExperts), 0, st, rb.blockcnt, nblk, E, pairs, T, tile_cap, rb.eoff, rb.runs,

@@ -14,24 +14,31 @@ void tc_destroy(TcPlan* plan);
 // at the same time).
 void tc_set_sm_margin(TcPlan* plan, int sms);
 
-// Largest number of rows in one grouped-GEMM tile (the MMA N extent).
+// Largest number of rows in one grouped-GEMM tile (the MMA N extent), and in one of a narrow launch.
 constexpr int kTcTileN = 192;
+constexpr int kTcNarrowN = 64;
 
-// beside: the launch (of q4cp images) may run at the same time as the one in front of it in the stream, which must be
-// another of these launches on other rows; it is complete only when that one is.
+struct TcLaunch {
+  bool narrow = false;  // every tile of the list has at most kTcNarrowN rows
+  // The launch may run at the same time as the one in front of it in the stream, which must be another
+  // of these launches on other rows; it is complete only when that one is.
+  bool beside = false;
+  // down GEMM; rowmap + map_base (device, both or neither): result row r >= map_base[0] of the tile list goes
+  // to pairs16[rowmap[r - map_base[0]]] instead of pairs16[r].
+  const int32_t* rowmap = nullptr;
+  const int32_t* map_base = nullptr;
+};
+
 // gate/up GEMM + SwiGLU: hid16[row][mid] = silu(W_gate x) * (W_up x) for every row of every tile.
 cudaError_t launch_up_tc(TcPlan* plan, const Image& img, const Tile* tiles, const int32_t* n_tiles,
-                         int max_tiles, __half* hid16, int32_t* status, cudaStream_t st, bool beside = false);
+                         int max_tiles, __half* hid16, int32_t* status, cudaStream_t st, const TcLaunch& o = {});
 // down GEMM: pairs16[row][d] = W_down hid16[row].
-// rowmap + map_base (device, both or neither): result row r >= map_base[0] of the tile list goes to
-// pairs16[rowmap[r - map_base[0]]] instead of pairs16[r].
 cudaError_t launch_down_tc(TcPlan* plan, const Image& img, const Tile* tiles, const int32_t* n_tiles,
-                           int max_tiles, __half* pairs16, int32_t* status, cudaStream_t st,
-                           const int32_t* rowmap = nullptr, const int32_t* map_base = nullptr, bool beside = false);
+                           int max_tiles, __half* pairs16, int32_t* status, cudaStream_t st, const TcLaunch& o = {});
 
 // plain GEMM over the expert-sorted activations (no activation function): z16[row][n_mtiles*128] =
 // W x_sorted[row], for images whose rows are not gate/up pairs (hgn v2 i4r gate_up).
 cudaError_t launch_raw_tc(TcPlan* plan, const Image& img, const Tile* tiles, const int32_t* n_tiles,
-                          int max_tiles, __half* z16, int32_t* status, cudaStream_t st);
+                          int max_tiles, __half* z16, int32_t* status, cudaStream_t st, const TcLaunch& o = {});
 
 }  // namespace b200moe

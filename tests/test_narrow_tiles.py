@@ -1,0 +1,85 @@
+"""Calls with few rows per expert run the grouped GEMMs in their narrow form (tiles of at most 64 rows,
+weights through a ring of bulk copies; at most 12 rows per expert on average), longer ones in the wide
+form. Against the oracle where that form can go wrong -- K block counts that are odd, one, or fewer than
+the ring's stages, experts whose rows end just behind a tile, every weight format -- and bit for bit
+against the wide form on both sides of the rule: a row's sums do not depend on the tile it is in."""
+import numpy as np
+import pytest
+
+import gfx1151_engine_b200 as pkg
+import oracle
+from gfx1151_engine_b200 import synth
+from helpers import assert_output_close
+from test_gpu_parity import bits, make_op, run_layer
+
+pytestmark = pytest.mark.gpu
+
+
+def popular(logits, experts):
+    """All tokens take these experts (in addition to others): as many rows as the call has tokens."""
+    logits[:, list(experts)] += 20.0
+    return logits
+
+
+@pytest.mark.parametrize("T", [17, 64, 65, 129])
+@pytest.mark.parametrize("shape", [dict(experts=64, topk=2, d=128, mid=64, shared=True, book="random"),
+                                   dict(experts=64, topk=4, d=384, mid=192, shared=True),
+                                   dict(experts=48, topk=4, d=2560, mid=640, shared=False, book="random")])
+def test_narrow_tiles_against_oracle(cuda, shape, T):
+    spec = synth.LayerSpec(**shape)
+    if T * spec.topk > 12 * spec.experts:
+        pytest.skip("a wide call")
+    layer = synth.make_layer(spec, seed=81)
+    logits = popular(synth.make_logits(synth.rng_for(81, T), T, spec.experts), [3])
+    xb = synth.make_x(synth.rng_for(81, 9), T, spec.d)
+    op = make_op(cuda, spec, T, layer=layer)
+    y = run_layer(cuda, op, spec, xb, logits)
+    y_o, ids_o, _ = oracle.moe_forward(spec, layer, synth.bf16_bits_to_f32(xb), logits=logits)
+    assert np.array_equal(op.get_routing(T)[0][:, :spec.topk], ids_o[:, :spec.topk])
+    assert_output_close(y, y_o, "narrow %r T=%d" % (shape, T))
+    op.close()
+
+
+def test_both_sides_of_the_rule_agree(cuda):
+    """T*k = 12*E is the last narrow call; one token more runs wide."""
+    spec = synth.LayerSpec(experts=32, topk=4, d=512, mid=256, shared=True)
+    layer = synth.make_layer(spec, seed=82)
+    T = 12 * spec.experts // spec.topk
+    logits = popular(synth.make_logits(synth.rng_for(82, 1), T + 1, spec.experts, zipf=True), [5, 17])
+    xb = synth.make_x(synth.rng_for(82, 9), T + 1, spec.d)
+    op = make_op(cuda, spec, T + 1, layer=layer)
+    wide = run_layer(cuda, op, spec, xb, logits)
+    narrow = run_layer(cuda, op, spec, xb[:T], logits[:T])
+    assert np.array_equal(bits(narrow), bits(wide[:T]))
+    op.close()
+
+
+@pytest.mark.parametrize("types", [(pkg.GGML_Q4_K, pkg.GGML_Q5_1), (pkg.GGML_Q5_K, pkg.GGML_Q5_1), (pkg.GGML_Q8_0, pkg.GGML_Q8_0)])
+def test_narrow_gguf_equals_wide(cuda, types):
+    """The GGUF images (more metadata per tile, two planes for Q8_0): the same rows in a narrow and in a wide call."""
+    torch = cuda
+    E, k, d, mid = 16, 2, 512, 256
+    gen = np.random.default_rng(83)
+    size = {pkg.GGML_Q4_K: (256, 144), pkg.GGML_Q5_K: (256, 176), pkg.GGML_Q5_1: (32, 24), pkg.GGML_Q8_0: (32, 34)}
+
+    def blocks(rows, cols, t):
+        per, n = size[t]
+        b = gen.integers(0, 256, size=(rows * cols // per, n), dtype=np.uint8)
+        b[:, 0:2] = np.full(len(b), 1e-3 if per == 256 else 1e-2, "<f2").view(np.uint8).reshape(-1, 2)
+        if t != pkg.GGML_Q8_0:
+            b[:, 2:4] = np.full(len(b), 5e-4 if per == 256 else -1e-1, "<f2").view(np.uint8).reshape(-1, 2)
+        return torch.from_numpy(b.reshape(-1)).cuda()
+
+    T = 200
+    op = pkg.MoeOperator(E, k, d, mid, T)
+    op.load_gguf(0, blocks(E * mid, d, types[0]), blocks(E * mid, d, types[0]), blocks(E * d, mid, types[1]),
+                 type_gu=types[0], type_dn=types[1])
+    x = torch.randn(T, d, device="cuda").bfloat16()
+    logits = torch.randn(T, E, device="cuda")
+    out = torch.full((T, d), float("nan"), dtype=torch.bfloat16, device="cuda")
+    op.moe_b(0, x, logits, out)
+    few = torch.full((90, d), float("nan"), dtype=torch.bfloat16, device="cuda")
+    op.moe_b(0, x[:90].contiguous(), logits[:90].contiguous(), few)
+    op.synchronize()
+    assert torch.isfinite(out.float()).all() and torch.equal(few, out[:90])
+    op.close()
