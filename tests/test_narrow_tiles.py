@@ -83,3 +83,32 @@ def test_narrow_gguf_equals_wide(cuda, types):
     op.synchronize()
     assert torch.isfinite(out.float()).all() and torch.equal(few, out[:90])
     op.close()
+
+
+@pytest.mark.parametrize("T", [40, 200])
+def test_captured_call_replays(cuda, T):
+    """The chain's overlapping launches (and the shared expert's launch beside the routed one) in a CUDA
+    graph: replays with new inputs in the same buffers give what plain calls give."""
+    torch = cuda
+    spec = synth.LayerSpec(experts=16, topk=4, d=512, mid=256, shared=True)
+    layer = synth.make_layer(spec, seed=84)
+    op = make_op(torch, spec, T, layer=layer)
+    x = torch.randn(T, spec.d, device="cuda").bfloat16()
+    logits = torch.randn(T, spec.experts, device="cuda")
+    out = torch.empty(T, spec.d, dtype=torch.bfloat16, device="cuda")
+    op.moe_b(0, x, logits, out)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        op.moe_b(0, x, logits, out, stream=torch.cuda.current_stream().cuda_stream)
+    for _ in range(3):
+        x.copy_(torch.randn(T, spec.d, device="cuda"))
+        logits.copy_(torch.randn(T, spec.experts, device="cuda"))
+        out.fill_(float("nan"))
+        graph.replay()
+        replayed = out.clone()
+        op.moe_b(0, x, logits, out)
+        op.synchronize()
+        assert torch.equal(replayed, out)
+    del graph
+    op.close()
