@@ -720,15 +720,16 @@ static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const
                                 (c.gemm_impl == B200MOE_GEMM_AUTO && T <= h->decode_max));
   const bool narrow = T * k <= kNarrowRows * E;
   const TcLaunch routed{narrow, false}, beside{narrow, true};
+  const int tile_cap = narrow ? kTcNarrowN : h->tile_cap;
   const uint16_t* gate_w = nullptr;  // set: the shared expert's gate is still to be computed
   static const bool slow_router = getenv("B200MOE_EXACT_ROUTER") != nullptr;  // A/B: the general routing body for every call
   if (logits && !slow_router && T <= decode_max_tokens() && T * k <= 128 && d % 8 == 0 && (!shared || ((uintptr_t)x & 15) == 0)) {
     // decode / verify: the compact router (ids from the logits' order, general body only on a near-tie)
-    CU_TRY(h, launch_route_fast(h->rb, logits, T, k, E, x, shared ? L.sh_gate_w : nullptr, d, st));
+    CU_TRY(h, launch_route_fast(h->rb, logits, T, k, E, x, shared ? L.sh_gate_w : nullptr, d, tile_cap, st));
     n++;
   } else if (T * k <= route_small_max_pairs() && T <= 16) {
     CU_TRY(h, launch_route_small(h->rb, logits, ids, w, stride, T, k, E, x, shared ? L.sh_gate_w : nullptr,
-                                 d, st));
+                                 d, tile_cap, st));
     n++;
   } else {
     if (logits) {
@@ -738,7 +739,7 @@ static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const
       w = h->rb.topw;
       stride = kIdStride;
     }
-    CU_TRY(h, launch_route(h->rb, ids, w, stride, T, k, E, narrow ? kTcNarrowN : h->tile_cap, st, &n));
+    CU_TRY(h, launch_route(h->rb, ids, w, stride, T, k, E, tile_cap, st, &n));
     if (shared && simt) {
       CU_TRY(h, launch_shared_gate(x, L.sh_gate_w, T, d, k, h->rb, st));
       n++;

@@ -82,7 +82,8 @@ struct Run {
   int count;
 };
 
-// Work item of the grouped GEMM: at most 256 rows of one expert.
+// Work item of the grouped GEMM: rows of one expert, at most as many as the launch that reads the list takes
+// (kTcTileN, narrow launches kTcNarrowN: whoever writes a list cuts it to that).
 struct Tile {
   int expert;
   int first;

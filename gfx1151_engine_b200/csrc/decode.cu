@@ -98,6 +98,7 @@ struct DecParams {
   const uint16_t* x;            // bf16 [T][d]
   const uint16_t* gate_w;       // bf16 [d] (shared expert's gate) or null
   int T, E, k, d, mid;
+  int tile_cap;                 // most rows of a tile of the routed work list
   __half* hid;                  // workspace fp16 [T*k + T][mid]
   uint16_t* out;                // bf16 [T][d], or null with hc_state
   const float* hc_w4;
@@ -245,7 +246,7 @@ struct RouteOuts {
 
 // The general body, kept out of line: the fast path's instruction footprint stays small.
 __device__ __noinline__ void route_exact(const DecParams& p, RouteSmallScratch<kDecMaxT>* sc, const RouteOuts* o, int32_t* status) {
-  route_small_body<kDecMaxT, 2>(p.logits, p.ids, p.w, p.stride, p.T, p.E, p.k, p.x, nullptr, p.d, *sc, o->loc, o->glob, status);
+  route_small_body<kDecMaxT, 2>(p.logits, p.ids, p.w, p.stride, p.T, p.E, p.k, p.tile_cap, p.x, nullptr, p.d, *sc, o->loc, o->glob, status);
 }
 
 // Threads 0..511. Fills fs.key / fs.w (pair order) from the logits; returns false when the
@@ -353,7 +354,8 @@ __device__ __forceinline__ bool route_fast_select(const DecParams& p, FastScratc
 }
 
 // Threads 0..511: stable bucketing of the P = T*k pairs in fs.key / fs.w by expert (rank counting),
-// expert offsets, runs. Same definitions as the general body's.
+// expert offsets, runs. Same definitions as the general body's; its tiles are not cut: the experts that
+// route_fast_select gives a token are distinct, so none has more than T rows.
 __device__ __forceinline__ void route_fast_place(const DecParams& p, FastScratch& fs, const RouteSmallOut& loc,
                                                  const RouteSmallOut& glob) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -1038,7 +1040,7 @@ struct RouteFastParams {
   const float* logits;
   const uint16_t* x;
   const uint16_t* gate_w;  // null: no shared expert
-  int T, E, k, d;
+  int T, E, k, d, tile_cap;
   RouteBuffers rb;
 };
 
@@ -1049,7 +1051,7 @@ k_route_fast(const RouteFastParams q) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int T = q.T, P = q.T * q.k, d = q.d;
   DecParams p{};  // the fields the routing pieces read
-  p.logits = q.logits; p.x = q.x; p.gate_w = q.gate_w; p.T = q.T; p.E = q.E; p.k = q.k; p.d = q.d;
+  p.logits = q.logits; p.x = q.x; p.gate_w = q.gate_w; p.T = q.T; p.E = q.E; p.k = q.k; p.d = q.d; p.tile_cap = q.tile_cap;
   p.status = q.rb.status;
   pdl_trigger();
   pdl_wait();  // inputs may come from the previous kernel; the buffers written here may still be read by it
@@ -1141,6 +1143,7 @@ cudaError_t launch_decode(const Image& gu, const Image& dn, const Image* sh_gu, 
   p.logits = logits; p.ids = ids; p.w = w; p.stride = stride;
   p.x = (const uint16_t*)x_bf16; p.gate_w = gate_w;
   p.T = T; p.E = E; p.k = k; p.d = d; p.mid = mid;
+  p.tile_cap = route_small_max_pairs();  // (nothing reads this kernel's work list)
   p.hid = hid16; p.out = (uint16_t*)out_bf16; p.hc_w4 = hc_w4; p.hc_state = (uint16_t*)hc_state;
   p.rb = rb; p.bar = bar; p.status = status; p.trace = trace;
   return launch_pdl(k_decode, dim3(sms), dim3(kDecThreads), (size_t)smem, st, p);
@@ -1150,7 +1153,7 @@ cudaError_t launch_decode(const Image& gu, const Image& dn, const Image* sh_gu, 
 // Routing stage of a decode call (logits given, T <= decode_max_tokens(), T*k <= 128) in one launch;
 // same outputs as launch_route_small.
 cudaError_t launch_route_fast(const RouteBuffers& rb, const float* logits, int T, int k, int E, const void* x_bf16,
-                              const uint16_t* gate_w_bf16, int d, cudaStream_t st) {
+                              const uint16_t* gate_w_bf16, int d, int tile_cap, cudaStream_t st) {
   static bool attr_done = false;
   const int smem = (int)(sizeof(FastScratch) + sizeof(RouteSmallScratch<kDecMaxT>));
   if (!attr_done) {
@@ -1159,7 +1162,7 @@ cudaError_t launch_route_fast(const RouteBuffers& rb, const float* logits, int T
     attr_done = true;
   }
   RouteFastParams q{};
-  q.logits = logits; q.x = (const uint16_t*)x_bf16; q.gate_w = gate_w_bf16; q.T = T; q.E = E; q.k = k; q.d = d; q.rb = rb;
+  q.logits = logits; q.x = (const uint16_t*)x_bf16; q.gate_w = gate_w_bf16; q.T = T; q.E = E; q.k = k; q.d = d; q.tile_cap = tile_cap; q.rb = rb;
   return launch_pdl(k_route_fast, dim3(1), dim3(kDecThreads), (size_t)smem, st, q);
 }
 

@@ -81,11 +81,12 @@ cudaError_t launch_router_topk(const float* logits, int T, int E, int k, int32_t
 cudaError_t launch_route(const RouteBuffers& rb, const int32_t* ids, const float* w, int stride,
                          int T, int k, int E, int tile_cap, cudaStream_t st, int* launches);
 // Whole routing stage in one launch for T*k <= route_small_max_pairs(): logits != nullptr runs
-// the router too (ids/w ignored), gate_w_bf16 != nullptr adds the shared expert's gate.
+// the router too (ids/w ignored), gate_w_bf16 != nullptr adds the shared expert's gate. tile_cap: most rows
+// of one tile, as for launch_route.
 int route_small_max_pairs();
 cudaError_t launch_route_small(const RouteBuffers& rb, const float* logits, const int32_t* ids,
                                const float* w, int stride, int T, int k, int E, const void* x_bf16,
-                               const uint16_t* gate_w_bf16, int d, cudaStream_t st);
+                               const uint16_t* gate_w_bf16, int d, int tile_cap, cudaStream_t st);
 cudaError_t launch_shared_gate(const void* x_bf16, const uint16_t* gate_w_bf16, int T, int d,
                                int k, const RouteBuffers& rb, cudaStream_t st);
 cudaError_t launch_apply_placement(int32_t* ids, int stride, int T, int k, int E, const int32_t* place,
@@ -138,7 +139,7 @@ cudaError_t launch_decode(const Image& gu, const Image& dn, const Image* sh_gu, 
 // The routing stage alone with the decode kernel's compact router (logits given, T <= decode_max_tokens(),
 // T*k <= 128, x 16-byte aligned when gate_w_bf16 is given); same outputs as launch_route_small.
 cudaError_t launch_route_fast(const RouteBuffers& rb, const float* logits, int T, int k, int E, const void* x_bf16,
-                              const uint16_t* gate_w_bf16, int d, cudaStream_t st);
+                              const uint16_t* gate_w_bf16, int d, int tile_cap, cudaStream_t st);
 
 // Bounded wait (2 s) until n <= 32 flags written by other GPUs have reached `expected`; a
 // timeout sets status {3, flag index}.

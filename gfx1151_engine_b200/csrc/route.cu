@@ -150,7 +150,7 @@ k_router_topk(const float* __restrict__ logits, int T, int E, int k, int32_t* __
 // Decode / verify (T*k <= 256): the whole routing stage in ONE block (route_small.cuh).
 __global__ void __launch_bounds__(kMaxExperts, 1)
 k_route_small(const float* __restrict__ logits, const int32_t* __restrict__ ids_in,
-              const float* __restrict__ w_in, int stride_in, int T, int E, int k, RouteBuffers rb,
+              const float* __restrict__ w_in, int stride_in, int T, int E, int k, int tile_cap, RouteBuffers rb,
               const uint16_t* __restrict__ x, const uint16_t* __restrict__ gw, int d) {
   __shared__ RouteSmallScratch<16> sc;
   pdl_trigger();
@@ -159,7 +159,7 @@ k_route_small(const float* __restrict__ logits, const int32_t* __restrict__ ids_
   o.topids = rb.topids; o.topw = rb.topw; o.tokidx = rb.tokidx; o.pw = rb.pw; o.pairids = rb.pairids;
   o.eoff = rb.eoff; o.runs = rb.runs; o.shared_slot = kMaxExperts; o.n_runs = rb.n_runs; o.tiles = rb.tiles;
   o.tiles_sh = rb.tiles_sh; o.n_tiles = rb.n_tiles; o.sgate = rb.sgate;
-  route_small_body<16>(logits, ids_in, w_in, stride_in, T, E, k, x, gw, d, sc, o, RouteSmallOut{}, rb.status);
+  route_small_body<16>(logits, ids_in, w_in, stride_in, T, E, k, tile_cap, x, gw, d, sc, o, RouteSmallOut{}, rb.status);
 }
 
 __global__ void __launch_bounds__(kChunk)
@@ -561,9 +561,9 @@ cudaError_t launch_ep_merge_tails(__half* x_recv, const int32_t* segs, int n_seg
 
 cudaError_t launch_route_small(const RouteBuffers& rb, const float* logits, const int32_t* ids,
                                const float* w, int stride, int T, int k, int E, const void* x_bf16,
-                               const uint16_t* gate_w_bf16, int d, cudaStream_t st) {
-  return launch_pdl(k_route_small, dim3(1), dim3(kMaxExperts), 0, st, logits, ids, w, stride, T, E, k, rb, (const uint16_t*)x_bf16,
-                                           gate_w_bf16, d);
+                               const uint16_t* gate_w_bf16, int d, int tile_cap, cudaStream_t st) {
+  return launch_pdl(k_route_small, dim3(1), dim3(kMaxExperts), 0, st, logits, ids, w, stride, T, E, k, tile_cap, rb,
+                    (const uint16_t*)x_bf16, gate_w_bf16, d);
 }
 
 // Waits until every one of n flags (written by peer GPUs' copy engines behind their data)

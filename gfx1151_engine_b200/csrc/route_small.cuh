@@ -57,13 +57,14 @@ struct RouteSmallOut {
 // more warps, which do not take part)
 __device__ __forceinline__ void rs_sync() { asm volatile("bar.sync 1, 512;" ::: "memory"); }
 
-// Run by threads 0..511 of a block (tid = threadIdx.x < 512). Inputs as k_route_small's.
+// Run by threads 0..511 of a block (tid = threadIdx.x < 512). Inputs as k_route_small's; tile_cap: most rows
+// of one tile (T, at most 16, is below it).
 // GU: 16-byte pieces of the shared expert's gate product a lane loads before it uses any (a
 // register-hungry prefetch: 8 where the body has the whole SM's registers, 2 inside a larger kernel).
 template <int NROW, int GU = 8>
 __device__ __forceinline__ void route_small_body(
     const float* __restrict__ logits, const int32_t* __restrict__ ids_in, const float* __restrict__ w_in,
-    int stride_in, int T, int E, int k, const uint16_t* __restrict__ x, const uint16_t* __restrict__ gw, int d,
+    int stride_in, int T, int E, int k, int tile_cap, const uint16_t* __restrict__ x, const uint16_t* __restrict__ gw, int d,
     RouteSmallScratch<NROW>& sc, const RouteSmallOut& o1, const RouteSmallOut& o2, int32_t* status,
     unsigned long long* dbg = nullptr) {
 #define RS_STAMP(i)                                                     \
@@ -388,18 +389,34 @@ __device__ __forceinline__ void route_small_body(
       lt += kq < tid;
     }
   const unsigned active = __ballot_sync(0xffffffffu, cnt > 0);
-  if (lane == 0) s_wcnt[warp] = __popc(active);
+  // Ids may repeat within a token (a caller's, or the selection's on non-finite logits), so an expert can have
+  // up to T*k rows: the first tile_cap of them stand at the expert's place among the non-empty ones, the tiles
+  // cut from the rest behind all of those. Low half of the counts: non-empty experts, high half: such tiles.
+  int more = cnt > tile_cap ? (cnt - 1) / tile_cap : 0, more_upto = 0, more_warp = 0;
+  if (__any_sync(0xffffffffu, more > 0)) {
+    more_upto = more;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, more_upto, o);
+      if (lane >= o) more_upto += v;
+    }
+    more_warp = __shfl_sync(0xffffffffu, more_upto, 31);
+  }
+  if (lane == 0) s_wcnt[warp] = __popc(active) | more_warp << 16;
   rs_sync();
   RS_STAMP(6);
-  int before = __popc(active & ((1u << lane) - 1u)), n_active = 0;
+  int at = __popc(active & ((1u << lane) - 1u)) | (more_upto - more) << 16, all = 0;
   for (int w2 = 0; w2 < 16; w2++) {
-    if (w2 < warp) before += s_wcnt[w2];
-    n_active += s_wcnt[w2];
+    if (w2 < warp) at += s_wcnt[w2];
+    all += s_wcnt[w2];
   }
+  const int before = at & 0xffff, n_active = all & 0xffff;
   if (tid < E) RS_PUT(eoff, tid, lt);
   if (cnt > 0) {
     RS_PUT(runs, before, (Run{tid, lt, cnt}));
-    RS_PUT(tiles, before, (Tile{tid, lt, cnt}));
+    RS_PUT(tiles, before, (Tile{tid, lt, min(cnt, tile_cap)}));
+    for (int j = 1; j <= more; j++)
+      RS_PUT(tiles, n_active + (at >> 16) + j - 1, (Tile{tid, lt + j * tile_cap, min(cnt - j * tile_cap, tile_cap)}));
   }
   if (tid == 0) {
     RS_PUT(eoff, E, P - n_bad);  // pairs actually placed (thread 0 counted the dropped ones above)
@@ -407,7 +424,7 @@ __device__ __forceinline__ void route_small_body(
     RS_PUT(n_runs, 1, 1);
     if (o1.runs) o1.runs[o1.shared_slot] = Run{0, P, T};
     if (o2.runs) o2.runs[o2.shared_slot] = Run{0, P, T};
-    RS_PUT(n_tiles, 0, n_active);
+    RS_PUT(n_tiles, 0, n_active + (all >> 16));
     RS_PUT(n_tiles, 1, 1);
     RS_PUT(tiles_sh, 0, (Tile{0, P, T}));
   }

@@ -9,8 +9,10 @@ import pytest
 import gfx1151_engine_b200 as pkg
 import oracle
 from gfx1151_engine_b200 import synth
-from helpers import assert_output_close
+from helpers import assert_output_close, bf16_out_to_f32, bf16_tensor
+from oracle import i4r
 from test_gpu_parity import bits, make_op, run_layer
+from test_i4r_gpu import make_i4r_op, run as run_i4r
 
 pytestmark = pytest.mark.gpu
 
@@ -111,4 +113,62 @@ def test_captured_call_replays(cuda, T):
         op.synchronize()
         assert torch.equal(replayed, out)
     del graph
+    op.close()
+
+
+def tc_op(torch, E, k, d, mid, max_tokens, i4r_layer):
+    """A layer whose calls of every length run on the tensor cores: rotated experts, or q4cp with GEMM_TC."""
+    if i4r_layer is not None:
+        return make_i4r_op(torch, E, k, d, mid, max_tokens, i4r_layer)
+    spec = synth.LayerSpec(experts=E, topk=k, d=d, mid=mid)
+    return make_op(torch, spec, max_tokens, impl=pkg.GEMM_TC, layer=synth.make_layer(spec, seed=85))
+
+
+# experts with 72, 112 and 256 rows in narrow calls, 256 in a wide one (16 * 16 > 12 * 16)
+@pytest.mark.parametrize("rotated", [True, False])
+@pytest.mark.parametrize("E,k,T,idle", [(64, 8, 16, 9), (64, 16, 8, 7), (64, 16, 16, 16), (16, 16, 16, 16)])
+def test_repeated_ids_in_a_short_call(cuda, E, k, T, idle, rotated):
+    """A padded batch of at most 16 tokens whose idle rows carry one id in every slot: that expert has more
+    rows than a tile. Against the oracle (rotated layers), and bit for bit against the same tokens in a longer
+    call, whose routing is another kernel's."""
+    torch = cuda
+    d, mid, L = 512, 256, synth.make_i4r_layer(E, 512, 256, seed=85) if rotated else None
+    gen = synth.rng_for(85, T)
+    ids = np.zeros((40, 16), np.int32)
+    for t in range(40):
+        ids[t, :k] = gen.permutation(E)[:k]
+    ids[T - idle:T, :k] = 3
+    w = gen.uniform(0.2, 1.0, size=(40, 16)).astype(np.float32) / k
+    xb = synth.make_x(synth.rng_for(85, 9), 40, d)
+    op = tc_op(torch, E, k, d, mid, 40, L)
+
+    def run_ids(n):
+        out = torch.full((n, d), float("nan"), dtype=torch.bfloat16, device="cuda")
+        op.moe_q4w_run(0, bf16_tensor(torch, xb[:n], (n, d)), torch.from_numpy(ids[:n]).cuda(), torch.from_numpy(w[:n]).cuda(), out)
+        op.synchronize()
+        return bf16_out_to_f32(torch, out)
+
+    y = run_ids(T)
+    assert np.array_equal(bits(y), bits(run_ids(40)[:T]))
+    if rotated:
+        assert_output_close(y, i4r.moe_forward(E, d, mid, L, synth.bf16_bits_to_f32(xb[:T]), ids, w, k), "repeated ids T=%d" % T)
+    op.close()
+
+
+@pytest.mark.parametrize("rotated", [True, False])
+@pytest.mark.parametrize("E,k,T,bad", [(64, 8, 16, 11), (64, 16, 16, 11), (64, 16, 8, 7), (16, 16, 16, 15)])
+def test_many_non_finite_rows_in_a_short_call(cuda, E, k, T, bad, rotated):
+    """A token with NaN logits takes one id k times: with many of them that expert has more rows than a tile.
+    They are NaN, and the other tokens' bytes are what they are without them."""
+    torch = cuda
+    d, mid = 512, 256
+    op = tc_op(torch, E, k, d, mid, T, synth.make_i4r_layer(E, d, mid, seed=86) if rotated else None)
+    logits = synth.make_logits(synth.rng_for(86, T), T, E)
+    xb = synth.make_x(synth.rng_for(86, 9), T, d)
+    clean = run_i4r(torch, op, d, xb, logits)
+    logits[:bad - 1] = np.nan
+    logits[bad - 1] = -np.inf
+    y = run_i4r(torch, op, d, xb, logits)
+    assert np.isnan(y[:bad]).all() and np.isfinite(y[bad:]).all()
+    assert np.array_equal(bits(y[bad:]), bits(clean[bad:]))
     op.close()
