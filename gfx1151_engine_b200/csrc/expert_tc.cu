@@ -279,6 +279,7 @@ struct KParams {
   const int32_t* rowmap;    // down kernel, may be null: tile-list row r >= map_base[0] is written to output row
   const int32_t* map_base;  // rowmap[r - map_base[0]] (rows below map_base[0], and all rows without a map: to row r)
   int beside;        // 1: runs beside the launch in front of it (see the wait in the set-up)
+  int early_next;    // 1: the next launch of the stream may start its set-up while this one runs
 };
 constexpr int kTraceSlots = 512;
 // Timeline stamps of CTA 0 (a debugging aid: build with -DB200MOE_TRACE and set
@@ -411,7 +412,7 @@ k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ C
   // one start: its few CTAs fill SMs as the routed ones leave them, and it waits at its end instead, so
   // that its completion still stands for both.
   if (!p.beside) pdl_wait();
-  pdl_trigger();
+  if (p.early_next) pdl_trigger();
   const int n_items = p.n_tiles[0] * img.n_mtiles;
   tc_fence_before();
   __syncthreads();
@@ -891,12 +892,16 @@ cudaError_t launch_n(TcPlan* plan, const CUtensorMap* m, const Image& img,
   }
   static const int l2_ahead = getenv("B200MOE_TC_L2_AHEAD") ? atoi(getenv("B200MOE_TC_L2_AHEAD")) : 3;
   KParams p{img, tiles, n_tiles, out, out_ld, status, (UP != (getenv("B200MOE_TC_TRACE_DOWN") != nullptr)) ? plan->trace : nullptr,
-            l2_ahead, rowmap, map_base, beside ? 1 : 0};
+            l2_ahead, rowmap, map_base, beside ? 1 : 0, plan->margin == 0};
   long long max_items = (long long)max_tiles * img.n_mtiles;
   const int usable = plan->sms - plan->margin > 1 ? plan->sms - plan->margin : 1;
   int grid = (int)(max_items < usable ? max_items : usable);
   if (grid < 1) grid = 1;
-  return launch_pdl(k_expert_tc<UP, DUAL, FMT, TN>, dim3(grid), dim3(kThreads), (size_t)kSmemBytes, st, m[0], m[1], m[2], m[3], p);
+  // With a margin the free SMs belong to another stream's exchange kernels. The CTAs of a dependent launch
+  // would take them, shared memory and registers of a whole SM each, and only wait there: no early start
+  // then, neither of this launch nor (early_next) of the one behind it.
+  return launch_opt(plan->margin == 0, k_expert_tc<UP, DUAL, FMT, TN>, dim3(grid), dim3(kThreads), (size_t)kSmemBytes, st, m[0],
+                    m[1], m[2], m[3], p);
 }
 
 template <bool UP, bool DUAL, int FMT>

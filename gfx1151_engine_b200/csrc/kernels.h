@@ -14,12 +14,13 @@ namespace b200moe {
 // this one drains. A kernel launched this way must call pdl_wait() before it touches anything
 // an earlier kernel of the stream wrote (or still reads); pdl_trigger() lets its own successor
 // start early. B200MOE_NO_PDL=1 in the environment turns the attribute off (plain launches).
+// launch_opt(false, ...) is a plain launch of the same kernel.
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+inline cudaError_t launch_opt(bool dependent, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                               Args&&... args) {
   static const bool off = std::getenv("B200MOE_NO_PDL") != nullptr;
   cudaLaunchConfig_t cfg{};
@@ -31,8 +32,13 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = off ? 0 : 1;
+  cfg.numAttrs = off || !dependent ? 0 : 1;
   return cudaLaunchKernelEx(&cfg, kernel, KArgs(std::forward<Args>(args))...);
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                              Args&&... args) {
+  return launch_opt(true, kernel, grid, block, smem, st, std::forward<Args>(args)...);
 }
 #endif
 

@@ -5,6 +5,8 @@ another rank, so no kernel depends on a concurrent one. The result must equal th
 the same tokens up to the order of the combine's additions, and the split into an in-place own-rows
 pass (no copy of the rows that stay on a rank; the shared expert rides along) plus an other-rows pass
 must give the bytes of the single pass."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -149,3 +151,55 @@ def test_ep_with_shared_expert(cuda, world):
         op.ep_experts(0, eoff_all, part=0)
     assert e.value.status == 2
     op.close()
+
+
+def programmatic_edges(torch, enqueue):
+    """Edges of the captured launches along which a kernel may start before the one in front of it has ended."""
+    class EdgeData(ctypes.Structure):
+        _fields_ = [("from_port", ctypes.c_uint8), ("to_port", ctypes.c_uint8), ("type", ctypes.c_uint8),
+                    ("reserved", ctypes.c_uint8 * 5)]
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        enqueue(torch.cuda.current_stream())
+    get = ctypes.CDLL("libcuda.so.1").cuGraphGetEdges_v2
+    h, n = ctypes.c_void_p(graph.raw_cuda_graph()), ctypes.c_size_t(64)
+    src, dst, data = (ctypes.c_void_p * 64)(), (ctypes.c_void_p * 64)(), (EdgeData * 64)()
+    assert get(h, src, dst, data, ctypes.byref(n)) == 0 and n.value > 0
+    kinds = [data[i].type for i in range(n.value)]
+    graph.reset()
+    return sum(t == 1 for t in kinds), len(kinds)
+
+
+@pytest.mark.parametrize("shared", [False, True])
+def test_sm_margin_keeps_the_free_sms_free(cuda, shared):
+    """With ep_sm_margin the grouped GEMMs leave SMs to the exchange kernels of another stream: no GEMM launch
+    may start, and hold such an SM, while the one in front of it still runs. Without it they do start early."""
+    torch = cuda
+    spec = synth.LayerSpec(experts=16, topk=4, d=256, mid=128, shared=shared)
+    layer = synth.make_layer(spec, seed=96)
+    T = 64
+    pairs = T * spec.topk
+    rows = pairs + (T if shared else 0)
+    x = bf16_tensor(torch, synth.make_x(synth.rng_for(96, 9), T, spec.d), (T, spec.d))
+    logits = torch.from_numpy(synth.make_logits(synth.rng_for(96, 1), T, spec.experts)).cuda()
+    early, outs = {}, {}
+    for margin in (0, 16):
+        op = pkg.MoeOperator(spec.experts, spec.topk, spec.d, spec.mid, T, has_shared=shared, ep_sm_margin=margin)
+        op.load_q4cp(0, dev_bytes(torch, layer["gate_up"]), dev_bytes(torch, layer["down"]))
+        if shared:
+            op.load_shared_q4cp(0, dev_bytes(torch, layer["sh_gate"]), dev_bytes(torch, layer["sh_up"]),
+                                dev_bytes(torch, layer["sh_down"]), dev_bytes(torch, layer["sh_gate_w"]))
+        buf = {n: torch.zeros(rows, spec.d, dtype=torch.float16, device="cuda") for n in ("send", "recv", "pairs", "back")}
+        eoff = torch.zeros(spec.experts + 1, dtype=torch.int32, device="cuda")
+        op.ep_attach(buf["send"], buf["recv"], buf["pairs"], buf["back"], rows)
+        op.ep_route(0, x, logits, eoff_out=eoff)
+        part = 3 if shared else 0
+        buf["recv"][:pairs].copy_(buf["send"][:pairs])
+        op.ep_experts(0, eoff, part=part)
+        op.synchronize()
+        outs[margin] = buf["back" if shared else "pairs"].clone()
+        early[margin], total = programmatic_edges(torch, lambda st: op.ep_experts(0, eoff, stream=st, part=part))
+        assert total == (4 if shared else 2)
+        op.close()
+    assert early[0] >= 1 and early[16] == 0
+    assert torch.equal(outs[0], outs[16])
