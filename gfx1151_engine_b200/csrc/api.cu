@@ -33,12 +33,25 @@ struct LayerWeights {
 
 }  // namespace
 
-// At most this many rows per expert on average: tiles of 64 rows and the GEMM kernels' narrow form, which
-// hides the latency of the weights. Beyond it the popular experts of a skewed routing have hundreds of
-// rows, and decoding their weights once per 64 rows costs more than that. Measured wide / narrow:
-// 1.5 rows on average (77 tokens, 512 experts of 4096 x 1024) 526 / 477 us, 10 rows (500 tokens, 2560 x 640)
-// 474 / 454, 40 rows (2048 tokens) 748 / 802; chunks of 1024 tokens (20 rows) lose 20 %.
-constexpr int kNarrowRows = 12;
+// Calls with few rows per expert, at most this many on average: what decides there is the decoding of the
+// weights, once per tile, and the GEMM kernels' narrow form (tiles of 64 rows) hides the latency of the
+// weights. Measured wide / narrow, even routing: 77 tokens on 512 experts of 4096 x 1024 (1.5 rows) 903 / 798 us,
+// 614 tokens (12 rows) 1183 / 1061, 500 tokens on 512 of 2560 x 640 550 / 494. Longer calls run the wide form alone
+// (2048 tokens of 2560 x 640, 40 rows: 748 / 802).
+constexpr int kFewRows = 12;
+// In such a call the popular experts of a skewed routing have hundreds of rows all the same, and decoding their
+// weights once per 64 of them costs more than the narrow form gives (614 tokens, the benchmark's skew, 4096 x
+// 1024: wide 419, narrow 476). So tiles of more than 64 rows go on a list of their own, which the wide form runs
+// beside the narrow one: 407. Which experts those are only the device knows; the host bounds what they can
+// save, and k_route_scan counts it. The second launch costs its set-up and its last items, which nothing
+// fills: measured by the tiles saved x K per SM, in tiles of 4096 columns: 0.4 lose 5 %, 1.0 1 to 6 %, 1.5 +1 to -5 %, 2.0 even,
+// 2.7 gain 3 %, 3.9 7 %, 9 15 %. The line lies at 2 of them on each of 148 SMs: saved * (mid / 64 * d + d / 128 * mid) =
+// 2 * 148 * 4096, as saved * d * mid. (An empty second list costs 0 to 3 us of the call.)
+constexpr long long kMinSavedWork = 2ll * 148 * 4096 * 128 / 3;
+// The shared expert's rows stay in narrow tiles while its gate/up GEMM has at most this many of them times row
+// blocks: they fill SMs beside the routed ones, so that more and shorter items end earlier. Wide / narrow: 144
+// items (768 tokens, mid 768) 288 / 282 us, 384 (1536, mid 1024) 871 / 868, 576 (2304, mid 1024) 906 / 937.
+constexpr int kSharedNarrowItems = 384;
 
 struct b200moe_ctx {
   b200moe_config cfg{};
@@ -88,7 +101,7 @@ struct b200moe_ctx {
   bool prof = false;
   std::vector<cudaEvent_t> prof_ev;
   int prof_head = 0, prof_pending = 0;
-  int max_rows = 0, max_tiles = 0, max_tiles_sh = 0;
+  int max_rows = 0, max_tiles = 0, max_tiles_narrow = 0, max_tiles_sh = 0;
   std::string err;
 };
 
@@ -265,10 +278,10 @@ int b200moe_create(const b200moe_config* cfg, b200moe_handle* out) {
   const size_t pairs = (size_t)Tm * k;
   const size_t rows = pairs + (c.has_shared ? Tm : 0);
   h->max_rows = (int)rows;
-  // (calls with few rows per expert cut them into narrow tiles)
-  const size_t narrow_pairs = std::min(pairs, (size_t)kNarrowRows * E), narrow_tokens = std::min((size_t)Tm, narrow_pairs / k);
-  h->max_tiles = (int)std::max(pairs / h->tile_cap, narrow_pairs / kTcNarrowN) + E + 1;
-  h->max_tiles_sh = (int)std::max((size_t)(Tm / h->tile_cap), narrow_tokens / kTcNarrowN) + 1;
+  // (calls with few rows per expert cut them into narrow tiles, most calls the shared expert's)
+  h->max_tiles_narrow = (int)(std::min(pairs, (size_t)kFewRows * E) / kTcNarrowN) + E + 1;
+  h->max_tiles = std::max((int)(pairs / h->tile_cap) + E + 1, h->max_tiles_narrow);
+  h->max_tiles_sh = Tm / kTcNarrowN + 1;
   const size_t dec_rows = (size_t)std::min(Tm, h->decode_max) * (k + (c.has_shared ? 1 : 0));
   const bool simt_all = c.gemm_impl == B200MOE_GEMM_SIMT;
   const size_t hid_bytes = std::max(rows * mid * (simt_all ? 4 : 2), dec_rows * mid * 4);
@@ -287,8 +300,9 @@ int b200moe_create(const b200moe_config* cfg, b200moe_handle* out) {
   A(&h->rb.runs, (size_t)kMaxExperts + 1);
   A(&h->rb.n_runs, 2);
   A(&h->rb.tiles, (size_t)h->max_tiles);
+  A(&h->rb.tiles_narrow, (size_t)h->max_tiles_narrow);
   A(&h->rb.tiles_sh, (size_t)h->max_tiles_sh);
-  A(&h->rb.n_tiles, 2);
+  A(&h->rb.n_tiles, 3);
   A(&h->rb.sgate, (size_t)Tm);
   A((uint8_t**)&h->hid, hid_bytes);
   A((uint8_t**)&h->pairs, pair_bytes);
@@ -672,7 +686,7 @@ int b200moe_route(b200moe_handle h, const int32_t* topids_dev, const float* topw
   if (T == 0) return B200MOE_OK;
   int n = 0;
   CU_TRY(h, launch_route(h->rb, topids_dev, topw_dev, stride, T, h->cfg.topk, h->cfg.experts,
-                         h->tile_cap, (cudaStream_t)stream, &n));
+                         TileCut{h->tile_cap, h->tile_cap}, (cudaStream_t)stream, &n));
   h->launches += n;
   return B200MOE_OK;
 }
@@ -718,18 +732,21 @@ static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const
   }
   const bool simt = !L.i4r && (c.gemm_impl == B200MOE_GEMM_SIMT ||
                                 (c.gemm_impl == B200MOE_GEMM_AUTO && T <= h->decode_max));
-  const bool narrow = T * k <= kNarrowRows * E;
-  const TcLaunch routed{narrow, false}, beside{narrow, true};
-  const int tile_cap = narrow ? kTcNarrowN : h->tile_cap;
+  const bool few = T * k <= kFewRows * E;
+  const int min_saved = (int)(kMinSavedWork / ((long long)d * mid));
+  // (no expert saves more than two tiles in 2 * 64 + 1 rows; the small routing writes one list)
+  const bool split = few && T > 16 && T * k * 2 >= min_saved * (2 * kTcNarrowN + 1), narrow = few && !split;
+  const bool sh_narrow = few && (long long)(T / kTcNarrowN) * (mid / 64) <= kSharedNarrowItems;
+  const TileCut cut{narrow ? kTcNarrowN : h->tile_cap, sh_narrow ? kTcNarrowN : h->tile_cap, split ? kTcNarrowN : 0, min_saved};
   const uint16_t* gate_w = nullptr;  // set: the shared expert's gate is still to be computed
   static const bool slow_router = getenv("B200MOE_EXACT_ROUTER") != nullptr;  // A/B: the general routing body for every call
   if (logits && !slow_router && T <= decode_max_tokens() && T * k <= 128 && d % 8 == 0 && (!shared || ((uintptr_t)x & 15) == 0)) {
     // decode / verify: the compact router (ids from the logits' order, general body only on a near-tie)
-    CU_TRY(h, launch_route_fast(h->rb, logits, T, k, E, x, shared ? L.sh_gate_w : nullptr, d, tile_cap, st));
+    CU_TRY(h, launch_route_fast(h->rb, logits, T, k, E, x, shared ? L.sh_gate_w : nullptr, d, cut.routed, st));
     n++;
   } else if (T * k <= route_small_max_pairs() && T <= 16) {
     CU_TRY(h, launch_route_small(h->rb, logits, ids, w, stride, T, k, E, x, shared ? L.sh_gate_w : nullptr,
-                                 d, tile_cap, st));
+                                 d, cut.routed, st));
     n++;
   } else {
     if (logits) {
@@ -739,7 +756,7 @@ static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const
       w = h->rb.topw;
       stride = kIdStride;
     }
-    CU_TRY(h, launch_route(h->rb, ids, w, stride, T, k, E, tile_cap, st, &n));
+    CU_TRY(h, launch_route(h->rb, ids, w, stride, T, k, E, cut, st, &n));
     if (shared && simt) {
       CU_TRY(h, launch_shared_gate(x, L.sh_gate_w, T, d, k, h->rb, st));
       n++;
@@ -796,21 +813,34 @@ static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const
   } else {
     if (!h->tc) return fail(h, B200MOE_ERR_UNSUPPORTED, "tensor-core path not available on this handle");
     const int rows = pairs + (shared ? T : 0);
+    // One GEMM stage: its launches in one place, since those beside the first rely on being right behind it.
+    auto stage_tc = [&](auto launch, const Image& img, const Image* sh, __half* out16) -> cudaError_t {
+      const Tile* first = split ? h->rb.tiles_narrow : h->rb.tiles;
+      cudaError_t e = launch(h->tc, img, first, h->rb.n_tiles + (split ? 2 : 0), split ? h->max_tiles_narrow : h->max_tiles,
+                             out16, h->status_dev, st, TcLaunch{few, false});
+      if (e == cudaSuccess && sh)
+        e = launch(h->tc, *sh, h->rb.tiles_sh, h->rb.n_tiles + 1, h->max_tiles_sh, out16, h->status_dev, st,
+                   TcLaunch{sh_narrow, true});
+      if (e == cudaSuccess && split)
+        e = launch(h->tc, img, h->rb.tiles, h->rb.n_tiles, h->max_tiles, out16, h->status_dev, st, TcLaunch{false, true});
+      n += 1 + (sh ? 1 : 0) + (split ? 1 : 0);
+      return e;
+    };
     if (L.i4r) {
       // hgn v2 i4r (rotate.cu): rotate the tokens once into their rows, plain GEMM into
       // the pair buffer (2*mid <= d columns of it), then the Hadamard / SwiGLU / Hadamard step
       CU_TRY(h, launch_rot_in(x, L.rot, h->rb.pairids, T, k, d, h->x_sorted, st));
       n++;
       if (ev) CU_TRY(h, cudaEventRecord(ev[2], st));
-      CU_TRY(h, launch_raw_tc(h->tc, L.gu, h->rb.tiles, h->rb.n_tiles, h->max_tiles, (__half*)h->pairs, h->status_dev, st, routed));
+      CU_TRY(h, stage_tc(launch_raw_tc, L.gu, nullptr, (__half*)h->pairs));
       CU_TRY(h, launch_i4r_mid((const __half*)h->pairs, L.rot + d, L.rot + d + 2 * mid, rows, mid, (__half*)h->hid, st));
-      n += 2;
+      n++;
       if (ev) CU_TRY(h, cudaEventRecord(ev[3], st));
-      CU_TRY(h, launch_down_tc(h->tc, L.dn, h->rb.tiles, h->rb.n_tiles, h->max_tiles, (__half*)h->pairs, h->status_dev, st, routed));
+      CU_TRY(h, stage_tc(launch_down_tc, L.dn, nullptr, (__half*)h->pairs));
       if (ev) CU_TRY(h, cudaEventRecord(ev[4], st));
       CU_TRY(h, launch_combine_f16_rot((const __half*)h->pairs, h->rb.pw, h->rb.pairids, T, k, d, L.rot + d + 3 * mid, out, st,
                                        h->hc_w4, h->hc_state));
-      n += 2;
+      n++;
       if (ev) {
         CU_TRY(h, cudaEventRecord(ev[5], st));
         h->prof_head = (h->prof_head + 1) % kProfRing;
@@ -822,23 +852,9 @@ static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const
     CU_TRY(h, launch_scatter_f16(x, T, k, d, shared ? pairs : -1, h->x_sorted, gate_w, h->rb, st));
     n++;
     if (ev) CU_TRY(h, cudaEventRecord(ev[2], st));
-    CU_TRY(h, launch_up_tc(h->tc, L.gu, h->rb.tiles, h->rb.n_tiles, h->max_tiles, (__half*)h->hid,
-                           h->status_dev, st, routed));
-    n++;
-    if (shared) {
-      CU_TRY(h, launch_up_tc(h->tc, L.sh_gu, h->rb.tiles_sh, h->rb.n_tiles + 1, h->max_tiles_sh,
-                             (__half*)h->hid, h->status_dev, st, beside));
-      n++;
-    }
+    CU_TRY(h, stage_tc(launch_up_tc, L.gu, shared ? &L.sh_gu : nullptr, (__half*)h->hid));
     if (ev) CU_TRY(h, cudaEventRecord(ev[3], st));
-    CU_TRY(h, launch_down_tc(h->tc, L.dn, h->rb.tiles, h->rb.n_tiles, h->max_tiles,
-                             (__half*)h->pairs, h->status_dev, st, routed));
-    n++;
-    if (shared) {
-      CU_TRY(h, launch_down_tc(h->tc, L.sh_dn, h->rb.tiles_sh, h->rb.n_tiles + 1, h->max_tiles_sh,
-                               (__half*)h->pairs, h->status_dev, st, beside));
-      n++;
-    }
+    CU_TRY(h, stage_tc(launch_down_tc, L.dn, shared ? &L.sh_dn : nullptr, (__half*)h->pairs));
     if (ev) CU_TRY(h, cudaEventRecord(ev[4], st));
     CU_TRY(h, launch_combine_f16((const __half*)h->pairs, h->rb.pw, h->rb.pairids, T, k, d,
                                  shared ? pairs : -1, out, st, h->hc_w4, h->hc_state));
@@ -1193,7 +1209,7 @@ int b200moe_ep_route(b200moe_handle h, int layer, const void* x, int T, const fl
     CU_TRY(h, launch_apply_placement(h->rb.topids, kIdStride, T, c.topk, c.experts, h->place_dev, st));
     n++;
   }
-  CU_TRY(h, launch_route(h->rb, h->rb.topids, h->rb.topw, kIdStride, T, c.topk, c.experts, h->tile_cap, st, &n));
+  CU_TRY(h, launch_route(h->rb, h->rb.topids, h->rb.topw, kIdStride, T, c.topk, c.experts, TileCut{h->tile_cap, h->tile_cap}, st, &n));
   // the shared expert stays on the token's own rank: its rows (token order) follow the routed ones
   CU_TRY(h, launch_scatter_f16(x, T, c.topk, c.d_model, shared ? T * c.topk : -1, h->ep_x_send,
                                shared ? L.sh_gate_w : nullptr, h->rb, st));

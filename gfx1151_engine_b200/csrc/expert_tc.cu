@@ -77,8 +77,8 @@ static_assert(kTmemA + kNS * 64 <= 512, "tensor memory: two accumulators and the
 //   bytes { lane*4 (+128), code byte, table >> 16, 0 }.
 // The first activation slot fits below the table, the other two above it.
 //
-// TN is the most rows a tile of the launch has. 192 (prefill chunks): the activation slots take all
-// there is. 64 (launches whose experts have few rows, where the MMAs are short and the packed weights
+// TN is the most rows a tile of the launch has. 192 (wide form): the activation slots take all
+// there is. 64 (narrow form: tiles with few rows, whose MMAs are short, so that the packed weights
 // decide): all three slots lie below the table and the space above it is a ring of kNST pairs of
 // weight tiles (74 to 98 KB in flight per SM), which warp 2 fills with bulk copies. The dequantising
 // warps' register fetch of the wide form reaches one pair ahead, which is less than a load from L2
@@ -371,6 +371,12 @@ k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ C
   volatile int* abort_flag = (volatile int*)(smem + kOffBar + kNumBars * 8);
   uint32_t* tmem_slot = (uint32_t*)(smem + kOffBar + kNumBars * 8 + 8);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // (a launch beside another one starts only when its list is there, see below: with none, it just keeps the order)
+  if (p.beside && p.n_tiles[0] == 0) {
+    pdl_trigger();
+    if (blockIdx.x == 0) pdl_wait();
+    return;
+  }
   const Image img = p.img;
   const int KB = img.n_kblocks;
 
@@ -407,10 +413,11 @@ k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ C
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  // The kernel before in the stream is complete behind this wait. The shared expert's launch (p.beside)
-  // has nothing to wait for but what the routed launch in front of it has waited for before it let this
-  // one start: its few CTAs fill SMs as the routed ones leave them, and it waits at its end instead, so
-  // that its completion still stands for both.
+  // The kernel before in the stream is complete behind this wait. The shared expert's launch and the second
+  // list's (p.beside) have nothing to wait for but what the launch in front of the first of them has waited
+  // for before it let the next one start: their CTAs fill SMs as the others leave them, and the first CTA
+  // waits at the end instead, so that the completion of the last launch still stands for all. That needs
+  // the wait to stay in front of the trigger, and nothing else between these launches.
   if (!p.beside) pdl_wait();
   if (p.early_next) pdl_trigger();
   const int n_items = p.n_tiles[0] * img.n_mtiles;
@@ -851,7 +858,7 @@ k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ C
   }
 
   // ---- teardown ----
-  if (p.beside) pdl_wait();
+  if (p.beside && blockIdx.x == 0) pdl_wait();
   __syncthreads();
   if (*abort_flag) {
     // give copies still in flight time to land before the CTA's shared memory goes away

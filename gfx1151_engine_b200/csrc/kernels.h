@@ -13,7 +13,8 @@ namespace b200moe {
 // the next kernel of the stream may start its prologue (code-book tables, index setup) while
 // this one drains. A kernel launched this way must call pdl_wait() before it touches anything
 // an earlier kernel of the stream wrote (or still reads); pdl_trigger() lets its own successor
-// start early. B200MOE_NO_PDL=1 in the environment turns the attribute off (plain launches).
+// start early. (One exception: k_expert_tc launches with TcLaunch::beside rely on the wait of the
+// k_expert_tc launch in front of them, which triggers behind it.) B200MOE_NO_PDL=1 in the environment turns the attribute off (plain launches).
 // launch_opt(false, ...) is a plain launch of the same kernel.
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
@@ -77,18 +78,25 @@ struct RouteBuffers {
   Run* runs;         // [E+1] active experts in ascending id (+ the shared expert last)
   int32_t* n_runs;   // [2]: routed runs, 1 (the shared run sits at runs[kMaxExperts])
   Tile* tiles;       // grouped GEMM work list, large tiles first
+  Tile* tiles_narrow;  // a second one, of the tiles with few rows (see TileCut)
   Tile* tiles_sh;    // work list of the shared expert (all T tokens)
-  int32_t* n_tiles;  // [2]: routed, shared
+  int32_t* n_tiles;  // [3]: tiles, tiles_sh, tiles_narrow
   float* sgate;      // [T] sigmoid gate of the shared expert
   int32_t* status;   // the handle's status word (may be null): {4, id} when an expert id outside [0, E) was dropped
 };
 cudaError_t launch_router_topk(const float* logits, int T, int E, int k, int32_t* ids, float* w,
                                int stride, cudaStream_t st);
+// How the work lists are cut: at most `routed` rows in a tile of a routed expert, `shared` in one of the shared
+// expert. Routed tiles of at most `narrow` rows go on tiles_narrow instead of tiles (0: all on tiles) if tiles of
+// `routed` rows make at least min_saved fewer of them than tiles of `narrow` rows; else all rows are cut to that.
+struct TileCut {
+  int routed, shared, narrow = 0, min_saved = 0;
+};
 cudaError_t launch_route(const RouteBuffers& rb, const int32_t* ids, const float* w, int stride,
-                         int T, int k, int E, int tile_cap, cudaStream_t st, int* launches);
+                         int T, int k, int E, const TileCut& cut, cudaStream_t st, int* launches);
 // Whole routing stage in one launch for T*k <= route_small_max_pairs(): logits != nullptr runs
 // the router too (ids/w ignored), gate_w_bf16 != nullptr adds the shared expert's gate. tile_cap: most rows
-// of one tile, as for launch_route.
+// of one tile; all go on tiles.
 int route_small_max_pairs();
 cudaError_t launch_route_small(const RouteBuffers& rb, const float* logits, const int32_t* ids,
                                const float* w, int stride, int T, int k, int E, const void* x_bf16,

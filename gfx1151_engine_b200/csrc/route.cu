@@ -184,12 +184,12 @@ k_route_count(const int32_t* __restrict__ ids, int stride, int pairs, int k, int
 // offsets, the list of non-empty experts and the grouped-GEMM tile list (full tiles first,
 // then the ragged ones in descending size so that a static round-robin stays balanced).
 __global__ void __launch_bounds__(kMaxExperts)
-k_route_scan(int32_t* __restrict__ blockcnt, int nblk, int E, int pairs, int T, int tile_cap,
+k_route_scan(int32_t* __restrict__ blockcnt, int nblk, int E, int pairs, int T, TileCut cut,
              int32_t* __restrict__ eoff, Run* __restrict__ runs, int32_t* __restrict__ n_runs,
-             Tile* __restrict__ tiles, Tile* __restrict__ tiles_sh, int32_t* __restrict__ n_tiles) {
+             Tile* __restrict__ tiles, Tile* __restrict__ tiles_narrow, Tile* __restrict__ tiles_sh, int32_t* __restrict__ n_tiles) {
   __shared__ __align__(16) int s_a[kMaxExperts];
   __shared__ unsigned long long s_w[kMaxExperts / 32];
-  __shared__ int s_wc[kMaxExperts / 32];
+  __shared__ int s_wc[kMaxExperts / 32], s_saved[kMaxExperts / 32];
   const int e = threadIdx.x, lane = e & 31, warp = e >> 5;
   pdl_trigger();
   pdl_wait();
@@ -215,6 +215,17 @@ k_route_scan(int32_t* __restrict__ blockcnt, int nblk, int E, int pairs, int T, 
     }
   }
   // three inclusive scans side by side: counts (low 32 bits) and non-empty flags, full tiles
+  int tile_cap = cut.routed;
+  if (cut.narrow > 0) {
+    // two lists only where the wide tiles save enough of the narrow ones
+    const int saved = __reduce_add_sync(0xffffffffu, (cnt + cut.narrow - 1) / cut.narrow - (cnt + tile_cap - 1) / tile_cap);
+    if (lane == 0) s_saved[warp] = saved;
+    __syncthreads();
+    int all = 0;
+#pragma unroll
+    for (int w = 0; w < kMaxExperts / 32; w++) all += s_saved[w];
+    if (all < cut.min_saved) tile_cap = cut.narrow;
+  }
   const int nfull = cnt / tile_cap, part = cnt % tile_cap;
   unsigned long long ab = (unsigned long long)(uint32_t)cnt | (unsigned long long)(cnt > 0) << 32;
   int c = nfull;
@@ -232,7 +243,7 @@ k_route_scan(int32_t* __restrict__ blockcnt, int nblk, int E, int pairs, int T, 
     s_wc[warp] = c;
   }
   s_a[e] = part;
-  __syncthreads();
+  const int wide_parts = __syncthreads_count(part > cut.narrow);
   unsigned long long ab_all = 0;
   int c_all = 0;
 #pragma unroll
@@ -255,8 +266,14 @@ k_route_scan(int32_t* __restrict__ blockcnt, int nblk, int E, int pairs, int T, 
     runs[kMaxExperts] = Run{0, pairs, T};
   }
   if (cnt > 0) runs[(int)(ab >> 32) - 1] = Run{e, first, cnt};
+  // full tiles first, then the ragged ones from large to small: those with more than cut.narrow rows on tiles
+  const int n_wide = tile_cap > cut.narrow ? total_full + wide_parts : 0;
+  auto put = [&](int i, const Tile& t) {
+    if (i < n_wide) tiles[i] = t;
+    else tiles_narrow[i - n_wide] = t;
+  };
   const int full0 = c - nfull;
-  for (int j = 0; j < nfull; j++) tiles[full0 + j] = Tile{e, first + j * tile_cap, tile_cap};
+  for (int j = 0; j < nfull; j++) put(full0 + j, Tile{e, first + j * tile_cap, tile_cap});
   // rank of the ragged tile among all ragged tiles: larger first, ties to the lower id
   int rank = 0, nparts = 0;
 #pragma unroll 4
@@ -266,14 +283,15 @@ k_route_scan(int32_t* __restrict__ blockcnt, int nblk, int E, int pairs, int T, 
     rank += (q.x > part || (q.x == part && o < e)) + (q.y > part || (q.y == part && o + 1 < e)) +
             (q.z > part || (q.z == part && o + 2 < e)) + (q.w > part || (q.w == part && o + 3 < e));
   }
-  if (part > 0) tiles[total_full + rank] = Tile{e, first + nfull * tile_cap, part};
+  if (part > 0) put(total_full + rank, Tile{e, first + nfull * tile_cap, part});
   // tiles of the shared expert: all T tokens in token order, rows behind the routed ones
-  const int nsh = (T + tile_cap - 1) / tile_cap;
+  const int nsh = (T + cut.shared - 1) / cut.shared;
   for (int j = e; j < nsh; j += kMaxExperts)
-    tiles_sh[j] = Tile{0, pairs + j * tile_cap, min(tile_cap, T - j * tile_cap)};
+    tiles_sh[j] = Tile{0, pairs + j * cut.shared, min(cut.shared, T - j * cut.shared)};
   if (e == 0) {
-    n_tiles[0] = total_full + nparts;
+    n_tiles[0] = n_wide;
     n_tiles[1] = nsh;
+    n_tiles[2] = total_full + nparts - n_wide;
   }
 }
 
@@ -363,15 +381,15 @@ cudaError_t launch_router_topk(const float* logits, int T, int E, int k, int32_t
 }
 
 cudaError_t launch_route(const RouteBuffers& rb, const int32_t* ids, const float* w, int stride,
-                         int T, int k, int E, int tile_cap, cudaStream_t st, int* launches) {
+                         int T, int k, int E, const TileCut& cut, cudaStream_t st, int* launches) {
   const int pairs = T * k;
   const int nblk = (pairs + kChunk - 1) / kChunk;
   // Every kernel of the chain waits for the one before it: its launch and set-up overlap that one's tail.
   // (These kernels with a thread per pair: 592 -> 559 us on a 77-token call, 531 -> 500 on 500 tokens.)
   cudaError_t e = launch_pdl(k_route_count, dim3(nblk), dim3(kChunk), 0, st, ids, stride, pairs, k, E, rb.blockcnt, rb.status);
   if (e == cudaSuccess)
-    e = launch_pdl(k_route_scan, dim3(1), dim3(kMaxExperts), 0, st, rb.blockcnt, nblk, E, pairs, T, tile_cap, rb.eoff, rb.runs,
-                   rb.n_runs, rb.tiles, rb.tiles_sh, rb.n_tiles);
+    e = launch_pdl(k_route_scan, dim3(1), dim3(kMaxExperts), 0, st, rb.blockcnt, nblk, E, pairs, T, cut, rb.eoff, rb.runs,
+                   rb.n_runs, rb.tiles, rb.tiles_narrow, rb.tiles_sh, rb.n_tiles);
   if (e == cudaSuccess)
     e = launch_pdl(k_route_place, dim3(nblk), dim3(kChunk), 0, st, ids, w, stride, pairs, k, E, rb.blockcnt, rb.eoff, rb.tokidx,
                    rb.pw, rb.pairids);

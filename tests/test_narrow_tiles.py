@@ -116,6 +116,58 @@ def test_captured_call_replays(cuda, T):
     op.close()
 
 
+def ids_of_counts(E, k, T, counts):
+    """[T][16] distinct ids: expert e < len(counts) gets counts[e] tokens, the others share what is left."""
+    left, ids, rest = list(counts), np.zeros((T, 16), np.int32), len(counts)
+    for t in range(T):
+        # experts that need every token still to come first, then the fullest
+        pick = sorted((e for e in range(len(left)) if left[e] > 0), key=lambda e: -left[e])[:k]
+        for e in pick:
+            left[e] -= 1
+        while len(pick) < k:
+            pick.append(rest)
+            rest = len(counts) + (rest + 1 - len(counts)) % (E - len(counts))
+        ids[t, :k] = pick
+    assert not any(left)
+    return ids
+
+
+# Calls of T = 12*E/k tokens on a layer of 4096 x 1024, whose line for the second list lies at 12 tiles saved: rows
+# on both sides of a narrow tile (64) and of a full one (192), 13 saved; 16 experts just over a narrow tile, so
+# that every block has work in both forms; one tile short of the line; no expert over a narrow tile
+@pytest.mark.parametrize("fmt", ["q4cp", "i4r"])
+def test_both_forms_in_one_call(cuda, fmt):
+    """Tiles of more than 64 rows run in the wide form, the others of the same call in the narrow one: bit for
+    bit the rows of a call of one token more, which runs the wide form alone."""
+    torch = cuda
+    E, k, d, mid = 96, 4, 4096, 1024
+    T = 12 * E // k
+    if fmt == "i4r":
+        L = synth.make_i4r_layer(E, d, mid, seed=87)
+        op = make_i4r_op(torch, E, k, d, mid, T + 1, L)
+    else:
+        spec = synth.LayerSpec(experts=E, topk=k, d=d, mid=mid, shared=True)
+        op = make_op(torch, spec, T + 1, layer=synth.make_layer(spec, seed=87))
+    w = synth.rng_for(87, 1).uniform(0.2, 1.0, size=(T + 1, 16)).astype(np.float32) / k
+    xb = synth.make_x(synth.rng_for(87, 9), T + 1, d)
+    for counts in ([288, 257, 193, 130, 129, 65, 64], [65] * 16, [288, 257, 193, 130, 129, 64, 64], [64, 64]):
+        ids = ids_of_counts(E, k, T, counts)
+        ids = np.concatenate([ids, ids[-1:]])
+        outs = []
+        for n in (T, T + 1):
+            before = op.launches
+            out = torch.full((n, d), float("nan"), dtype=torch.bfloat16, device="cuda")
+            op.moe_q4w_run(0, bf16_tensor(torch, xb[:n], (n, d)), torch.from_numpy(ids[:n]).cuda(), torch.from_numpy(w[:n]).cuda(), out)
+            op.synchronize()
+            outs.append((bf16_out_to_f32(torch, out), op.launches - before))
+        assert np.isfinite(outs[0][0]).all() and np.array_equal(bits(outs[0][0]), bits(outs[1][0][:T])), counts
+        assert outs[0][1] == outs[1][1] + 2    # the second list's launch in both GEMM stages
+    if fmt == "i4r":
+        sel = np.arange(0, T, 97)
+        assert_output_close(outs[0][0][sel], i4r.moe_forward(E, d, mid, L, synth.bf16_bits_to_f32(xb[sel]), ids[sel], w[sel], k), fmt)
+    op.close()
+
+
 def tc_op(torch, E, k, d, mid, max_tokens, i4r_layer):
     """A layer whose calls of every length run on the tensor cores: rotated experts, or q4cp with GEMM_TC."""
     if i4r_layer is not None:
