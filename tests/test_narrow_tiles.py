@@ -1,6 +1,7 @@
 """Calls with few rows per expert run the grouped GEMMs in their narrow form (tiles of at most 64 rows,
 weights through a ring of bulk copies; at most 12 rows per expert on average), longer ones in the wide
-form. Against the oracle where that form can go wrong -- K block counts that are odd, one, or fewer than
+form; tiles of more than 64 rows in a call of the first kind are cut to 64 or run in the wide form beside the
+others. Against the oracle where that form can go wrong -- K block counts that are odd, one, or fewer than
 the ring's stages, experts whose rows end just behind a tile, every weight format -- and bit for bit
 against the wide form on both sides of the rule: a row's sums do not depend on the tile it is in."""
 import numpy as np
@@ -29,8 +30,7 @@ def popular(logits, experts):
                                    dict(experts=48, topk=4, d=2560, mid=640, shared=False, book="random")])
 def test_narrow_tiles_against_oracle(cuda, shape, T):
     spec = synth.LayerSpec(**shape)
-    if T * spec.topk > 12 * spec.experts:
-        pytest.skip("a wide call")
+    assert T * spec.topk <= 12 * spec.experts
     layer = synth.make_layer(spec, seed=81)
     logits = popular(synth.make_logits(synth.rng_for(81, T), T, spec.experts), [3])
     xb = synth.make_x(synth.rng_for(81, 9), T, spec.d)
@@ -56,19 +56,21 @@ def test_both_sides_of_the_rule_agree(cuda):
     op.close()
 
 
-@pytest.mark.parametrize("types", [(pkg.GGML_Q4_K, pkg.GGML_Q5_1), (pkg.GGML_Q5_K, pkg.GGML_Q5_1), (pkg.GGML_Q8_0, pkg.GGML_Q8_0)])
+@pytest.mark.parametrize("types", [(pkg.GGML_Q4_K, pkg.GGML_Q5_1), (pkg.GGML_Q5_K, pkg.GGML_Q5_1), (pkg.GGML_Q8_0, pkg.GGML_Q8_0),
+                                   (pkg.GGML_IQ4_XS, pkg.GGML_IQ4_XS)])
 def test_narrow_gguf_equals_wide(cuda, types):
     """The GGUF images (more metadata per tile, two planes for Q8_0): the same rows in a narrow and in a wide call."""
     torch = cuda
     E, k, d, mid = 16, 2, 512, 256
     gen = np.random.default_rng(83)
-    size = {pkg.GGML_Q4_K: (256, 144), pkg.GGML_Q5_K: (256, 176), pkg.GGML_Q5_1: (32, 24), pkg.GGML_Q8_0: (32, 34)}
+    size = {pkg.GGML_Q4_K: (256, 144), pkg.GGML_Q5_K: (256, 176), pkg.GGML_Q5_1: (32, 24), pkg.GGML_Q8_0: (32, 34), pkg.GGML_IQ4_XS: (256, 136)}
 
     def blocks(rows, cols, t):
         per, n = size[t]
         b = gen.integers(0, 256, size=(rows * cols // per, n), dtype=np.uint8)
-        b[:, 0:2] = np.full(len(b), 1e-3 if per == 256 else 1e-2, "<f2").view(np.uint8).reshape(-1, 2)
-        if t != pkg.GGML_Q8_0:
+        scale = 2e-5 if t == pkg.GGML_IQ4_XS else 1e-3 if per == 256 else 1e-2
+        b[:, 0:2] = np.full(len(b), scale, "<f2").view(np.uint8).reshape(-1, 2)
+        if t not in (pkg.GGML_Q8_0, pkg.GGML_IQ4_XS):
             b[:, 2:4] = np.full(len(b), 5e-4 if per == 256 else -1e-1, "<f2").view(np.uint8).reshape(-1, 2)
         return torch.from_numpy(b.reshape(-1)).cuda()
 
@@ -132,9 +134,9 @@ def ids_of_counts(E, k, T, counts):
     return ids
 
 
-# Calls of T = 12*E/k tokens on a layer of 4096 x 1024, whose line for the second list lies at 12 tiles saved: rows
-# on both sides of a narrow tile (64) and of a full one (192), 13 saved; 16 experts just over a narrow tile, so
-# that every block has work in both forms; one tile short of the line; no expert over a narrow tile
+# Calls of T = 12*E/k tokens on a layer of 4096 x 1024, whose line for the second list lies at 12 tiles saved: no
+# expert over a narrow tile (64 rows); 16 experts just over one, so that every block has work in both forms; rows on
+# both sides of a narrow tile and of a full one (192), 12 and 13 saved
 @pytest.mark.parametrize("fmt", ["q4cp", "i4r"])
 def test_both_forms_in_one_call(cuda, fmt):
     """Tiles of more than 64 rows run in the wide form, the others of the same call in the narrow one: bit for
@@ -150,7 +152,7 @@ def test_both_forms_in_one_call(cuda, fmt):
         op = make_op(torch, spec, T + 1, layer=synth.make_layer(spec, seed=87))
     w = synth.rng_for(87, 1).uniform(0.2, 1.0, size=(T + 1, 16)).astype(np.float32) / k
     xb = synth.make_x(synth.rng_for(87, 9), T + 1, d)
-    for counts in ([288, 257, 193, 130, 129, 65, 64], [65] * 16, [288, 257, 193, 130, 129, 64, 64], [64, 64]):
+    for counts in ([64, 64], [65] * 16, [288, 257, 193, 130, 129, 64, 64], [288, 257, 193, 130, 129, 65, 64]):
         ids = ids_of_counts(E, k, T, counts)
         ids = np.concatenate([ids, ids[-1:]])
         outs = []
@@ -162,6 +164,17 @@ def test_both_forms_in_one_call(cuda, fmt):
             outs.append((bf16_out_to_f32(torch, out), op.launches - before))
         assert np.isfinite(outs[0][0]).all() and np.array_equal(bits(outs[0][0]), bits(outs[1][0][:T])), counts
         assert outs[0][1] == outs[1][1] + 2    # the second list's launch in both GEMM stages
+    # captured: the launches beside each other, replayed with the last ids
+    x, i_dev, w_dev = bf16_tensor(torch, xb[:T], (T, d)), torch.zeros(T, 16, dtype=torch.int32, device="cuda"), torch.from_numpy(w[:T]).cuda()
+    out = torch.full((T, d), float("nan"), dtype=torch.bfloat16, device="cuda")
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        op.moe_q4w_run(0, x, i_dev, w_dev, out, stream=torch.cuda.current_stream().cuda_stream)
+    i_dev.copy_(torch.from_numpy(ids[:T]))
+    graph.replay()
+    torch.cuda.synchronize()
+    assert np.array_equal(bits(bf16_out_to_f32(torch, out)), bits(outs[0][0]))
+    del graph
     if fmt == "i4r":
         sel = np.arange(0, T, 97)
         assert_output_close(outs[0][0][sel], i4r.moe_forward(E, d, mid, L, synth.bf16_bits_to_f32(xb[sel]), ids[sel], w[sel], k), fmt)
