@@ -6,7 +6,7 @@ Workload ("config 3"): one 512-expert top-10 q4cp MoE 
 (d_model 4096, expert intermediate 1024, group 32, fp16 scales), a 16384-token prefill
 chunk per step and per GPU, bf16 activations ~ N(0,1), router logits ~ N(0,1) plus a
 per-expert Zipf(1.1) bias. Weights and inputs are synthetic (seeded); a step is one
-b200moe_forward call: router top-k, bucketing, activation gather, tcgen05 gate/up GEMM
+b200moe_forward call: router top-k, bucketing, activation rows in expert order, tcgen05 gate/up GEMM
 + SwiGLU, down GEMM, weighted combine.
 
 Prints ONE JSON line: value = tokens/s with inputs resident in HBM (CUDA events on the

@@ -12,17 +12,20 @@
 //   warp 0      producer of activation tiles: TMA tensor copies (128-byte swizzle, box of
 //               16/64/128/192 rows), one per K block, into a ring of 3 pair-slots in shared
 //               memory; the same thread asks for the packed weight tiles of a later pair to be
-//               brought into L2 (one bulk prefetch per pair)
+//               brought into L2 (one bulk prefetch per pair; wide form)
 //   warp 1      issues tcgen05.mma (A from tensor memory, B from shared memory): eight per
 //               pair behind ONE barrier wait and ONE commit; owns the tensor-memory allocation
+//   warp 2      narrow form (tiles of at most 64 rows, see Map): producer of packed weights, one
+//               bulk copy per pair into a ring of 8 stages in shared memory
 //   warp 3      relay: folds "activations of the pair have landed" into the barrier the MMA
 //               warp waits on, so that warp polls a single barrier
 //   warps 4-19  dequantise: two sets of eight warps alternate pairs (set s owns tensor-memory
-//               slot s); thread = one weight row of one K block. Packed codes come straight
-//               from global memory (a warp's 32 rows are 512 contiguous bytes) into ONE set of
-//               registers, refilled for the next own pair as soon as the decode has used them
-//               up, through a pointer that walks with the stream (the tile list is read one item
-//               ahead, never on the critical path); each code byte indexes a 256-entry half2
+//               slot s); thread = one weight row of one K block. Packed codes come, in the wide
+//               form, straight from global memory (a warp's 32 rows are 512 contiguous bytes) into
+//               ONE set of registers, refilled for the next own pair as soon as the decode has used
+//               them up, through a pointer that walks with the stream (the tile list is read one
+//               item ahead, never on the critical path), in the narrow form from warp 2's ring;
+//               each code byte indexes a 256-entry half2
 //               pair table replicated per lane in shared memory (bank-conflict free, the
 //               address is one byte permute); one half2 multiply by the group scale; the
 //               result goes straight into tensor memory (tcgen05.st) as the MMA's A operand
