@@ -193,7 +193,7 @@ SrcTensor q4cp_src(const uint8_t* blob, long long rows_total, long long cols,
 }
 
 // Turns the device status word (copied to status_host) into a return code and clears it on the
-// device. {1|2|3|5|6, site}: a bounded device-side wait gave up; {4, id}: a caller-supplied expert
+// device. {1|2|3|5|6|8, site}: a bounded device-side wait gave up; {4, id}: a caller-supplied expert
 // id outside [0, experts) was dropped by the bucketing; {7, token}: the router's near-tie list overflowed.
 int report_status(b200moe_handle h, cudaStream_t st) {
   const int code = h->status_host[0], detail = h->status_host[1];
@@ -777,11 +777,11 @@ static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const
   if (gemv) {
     // decode / verify: persistent dequant GEMV, routed and shared expert in one launch each
     if (ev) CU_TRY(h, cudaEventRecord(ev[2], st));
-    CU_TRY(h, launch_up_gemv(L.gu, shared ? &L.sh_gu : nullptr, x, d, mid, h->rb.tokidx, h->rb.runs,
-                             h->rb.n_runs, (__half*)h->hid, st));
+    CU_TRY(h, launch_up_gemv(L.gu, shared ? &L.sh_gu : nullptr, x, T, k, E, d, mid, h->rb.tokidx, h->rb.runs,
+                             h->rb.n_runs, (__half*)h->hid, h->status_dev, st));
     if (ev) CU_TRY(h, cudaEventRecord(ev[3], st));
-    CU_TRY(h, launch_down_gemv(L.dn, shared ? &L.sh_dn : nullptr, (const __half*)h->hid, d, mid,
-                               h->rb.runs, h->rb.n_runs, (float*)h->pairs, st));
+    CU_TRY(h, launch_down_gemv(L.dn, shared ? &L.sh_dn : nullptr, (const __half*)h->hid, T, k, E, d, mid,
+                               h->rb.runs, h->rb.n_runs, (float*)h->pairs, h->status_dev, st));
     if (ev) CU_TRY(h, cudaEventRecord(ev[4], st));
     CU_TRY(h, launch_combine_f32((const float*)h->pairs, h->rb.pw, h->rb.pairids, T, k, d,
                                  shared ? pairs : -1, out, st, h->hc_w4, h->hc_state));

@@ -8,24 +8,26 @@
 
 namespace b200moe {
 
-// ---- repacked weight tiles --------------------------------------------------------
-// Every quantised expert tensor is stored as tiles of 128 output rows x 64 K-elements:
-//   [expert][m_tile][k_block][tile bytes]
-// A tile starts with 4096 code bytes laid out [half h=0..1][row r=0..127][16 B]: the 16
-// bytes hold the 32 four-bit codes of row r for K = 64*kb + 32*h .. +31, low nibble =
-// even K (the nibble order of hgn q4cp, src/hgn.h:5-9 of the reference). The codes are
-// followed by per-(row, 32-group) metadata whose size depends on the source format.
-// A whole tile is one contiguous, 16-byte aligned object so that a single bulk async
-// copy brings it into shared memory, and a warp reading "its" rows touches 512
-// contiguous bytes.
+// ---- repacked weights ---------------------------------------------------------------
+// A quantised expert tensor is a grid of tiles of 128 output rows x 64 K elements, a tile four sub-blocks
+// of 32 rows. A sub-block is one contiguous object of whole 128-byte lines, {codes of half 0, codes of half 1,
+// metadata}: 512 code bytes per half h, 16 per row with the 32 four-bit codes of the row for
+// K = 64*kb + 32*h .. +31, low nibble = even K (the nibble order of hgn q4cp, src/hgn.h:5-9 of the reference), then
+// the rows' metadata, whose size depends on the source format. A plain image holds rows 32s .. 32s+31 of the
+// tile in sub-block s; a paired (gate/up) one gate rows 16s .. 16s+15 and the matching up rows 64+16s .. 64+16s+15.
+//   [expert][m_tile][sub-block 0..3][k_block][sub-block bytes]
+// The decode GEMV walks 16 hidden outputs (or 32 output rows) along K: one stream, a warp's K blocks one
+// bulk copy. A warp of the tensor-core kernel owns the 32 rows of a sub-block (or 16 rows of two): a
+// read of its rows of a half touches four whole lines.
 constexpr int kTileM = 128;
 constexpr int kTileK = 64;
-constexpr int kCodeBytes = kTileM * kTileK / 2;  // 4096
+constexpr int kSubRows = 32;
+constexpr int kSubCodes = kSubRows * kTileK / 2;  // 1024
 
 enum Format : int {
-  kQ4CP = 0,  // meta: [r]{fp16 scale of half 0, of half 1}                          -> 512 B
-  kQ4K = 1,   // meta: [r]{fp16 d, fp16 dmin, u8 sc0, u8 m0, u8 sc1, u8 m1}           -> 1024 B
-  kQ51 = 2    // meta: [r]{fp16 d0, fp16 m0, u32 fifth bits 0, fp16 d1, fp16 m1, u32 fifth bits 1} -> 2048 B
+  kQ4CP = 0,  // metadata of a row: {fp16 scale of half 0, of half 1}
+  kQ4K = 1,   // {fp16 d, fp16 dmin, u8 sc0, u8 m0, u8 sc1, u8 m1}
+  kQ51 = 2    // {fp16 d0, fp16 m0, u32 fifth bits 0, fp16 d1, fp16 m1, u32 fifth bits 1}
 };
 // kQ51, the fifth-bit word of a 32-group: bit i (i < 16) belongs to the LOW-nibble code of code
 // byte i (element 2i of the group), bit 16 + i to its high-nibble code (element 2i + 1). With the
@@ -48,10 +50,17 @@ __host__ __device__ inline uint32_t fifth_bit_of(uint32_t split, int j) {  // fi
 // followed by a block of the low nibbles (d' = d, m' = 0) -- and act_shift = 1. 16 d and 128 d are
 // exact in fp16, so every kernel reproduces d * q up to its usual single rounding.
 
-__host__ __device__ constexpr int meta_bytes(int fmt) {
-  return fmt == kQ4CP ? 512 : fmt == kQ4K ? 1024 : 2048;
+__host__ __device__ constexpr int meta_row_bytes(int fmt) { return fmt == kQ4CP ? 4 : fmt == kQ4K ? 8 : 16; }
+__host__ __device__ constexpr int sub_bytes(int fmt) { return kSubCodes + kSubRows * meta_row_bytes(fmt); }  // 1152, 1280, 1536
+__host__ __device__ constexpr int tile_bytes(int fmt) { return kTileM / kSubRows * sub_bytes(fmt); }
+// Where tile row r sits: its sub-block (bits 5 and up) and its place there.
+__host__ __device__ constexpr int tile_pos(int r, int paired) {
+  return paired ? ((r & 63) >> 4) * kSubRows + (r >> 6) * 16 + (r & 15) : r;
 }
-__host__ __device__ constexpr int tile_bytes(int fmt) { return kCodeBytes + meta_bytes(fmt); }
+// Inside a sub-block: the 16 code bytes of half 0 of the row at place `pos` (half 1 lies kHalfBytes further), its metadata.
+constexpr int kHalfBytes = kSubRows * 16;
+__host__ __device__ constexpr int code_offset(int pos) { return (pos & 31) * 16; }
+__host__ __device__ constexpr int meta_offset(int fmt, int pos) { return kSubCodes + (pos & 31) * meta_row_bytes(fmt); }
 
 // One repacked tensor set: n_experts x n_mtiles x n_kblocks tiles.
 struct Image {
@@ -65,13 +74,17 @@ struct Image {
   int act_shift = 0;  // 1: two-plane image of 8-bit codes (GGUF Q8_0): K block kb of the image multiplies the
                       //    activations of K block kb >> 1 -- the high and the low nibble plane of the same 64 columns
   float* book = nullptr;  // device [32]: code book of tile rows 0..63, then of rows 64..127
-  __host__ __device__ size_t tile_stride() const { return (size_t)tile_bytes(fmt); }
-  __host__ __device__ size_t expert_stride() const {
-    return (size_t)n_mtiles * n_kblocks * tile_bytes(fmt);
+  __host__ __device__ size_t mtile_stride() const { return (size_t)n_kblocks * tile_bytes(fmt); }
+  __host__ __device__ size_t expert_stride() const { return n_mtiles * mtile_stride(); }
+  __host__ __device__ uint8_t* mtile(int e, int mt) const { return data + ((size_t)e * n_mtiles + mt) * mtile_stride(); }
+  // from mtile(): the sub-block of tile row r in K block 0; the next K block lies sub_bytes(fmt) further
+  __host__ __device__ size_t row_sub(int r) const { return (size_t)(tile_pos(r, paired) >> 5) * n_kblocks * sub_bytes(fmt); }
+  // codes (half 0) and metadata of a tile row in K block kb
+  __host__ __device__ uint8_t* codes(int e, int mt, int kb, int r) const {
+    return mtile(e, mt) + row_sub(r) + (size_t)kb * sub_bytes(fmt) + code_offset(tile_pos(r, paired));
   }
-  __host__ __device__ const uint8_t* tile(int e, int mt, int kb) const {
-    return data + ((size_t)e * n_mtiles + mt) * n_kblocks * tile_bytes(fmt) +
-           (size_t)kb * tile_bytes(fmt);
+  __host__ __device__ uint8_t* meta(int e, int mt, int kb, int r) const {
+    return mtile(e, mt) + row_sub(r) + (size_t)kb * sub_bytes(fmt) + meta_offset(fmt, tile_pos(r, paired));
   }
 };
 

@@ -654,7 +654,7 @@ k_decode(const DecParams p) {
     }
   };
   auto finish_rec = [&](Rec& r, const Image& img, int expert, int mtile) {
-    r.base = img.data + ((size_t)expert * img.n_mtiles + mtile) * img.n_kblocks * tile_bytes(kQ4CP);
+    r.base = img.mtile(expert, mtile);
     const int cnt = r.info & 255;
     r.tok0 = res->tokidx[r.first];
     r.pw0 = res->pw[r.first];
@@ -668,7 +668,7 @@ k_decode(const DecParams p) {
   auto slot_base = [&](int s) -> uint32_t { return s == 0 ? slot_lo : slot_hi + (uint32_t)(s - 1) * kSlotBytes; };
   const uint32_t lut = 0x00010000u | (uint32_t)(lane * 4);  // address bytes {lane*4, code byte, 1, 0}: the table sits at 64 KB
   const uint32_t work = kOffTab + 128 + (uint32_t)lane * 4;  // work row R of this lane: work + R * 256
-  constexpr int tile_b = tile_bytes(kQ4CP);
+  constexpr int sub_b = sub_bytes(kQ4CP);
 
   // =========================== gate/up + SwiGLU ===========================
   // Units: the shared expert's sub-units first, then the routed ones. A task = 16 hidden outputs
@@ -747,8 +747,8 @@ k_decode(const DecParams p) {
         const uint8_t* base = (const uint8_t*)(((unsigned long long)a.y << 32) | a.x);
         const int info = (int)a.w, j = info >> 16, cnt = info & 255;
         const int row = (lane < 16 ? 0 : 48) + (j & 3) * 16 + lane;  // gate rows 0..63, up rows 64..127 of the tile
-        q_ptr = base + (size_t)kb0 * tile_b + row * 16;
-        q_mptr = base + (size_t)kb0 * tile_b + kCodeBytes + row * 4;
+        q_ptr = base + p.gu.row_sub(row) + (size_t)kb0 * sub_b + code_offset(tile_pos(row, 1));
+        q_mptr = base + p.gu.row_sub(row) + (size_t)kb0 * sub_b + meta_offset(kQ4CP, tile_pos(row, 1));
         const int tok = lane < 8 ? (int)b.x : (int)b.y;
         q_xp = lane < cnt * 8 ? p.x + (size_t)tok * d + kb0 * kTileK + (lane & 7) * 8 : nullptr;
       };
@@ -756,11 +756,11 @@ k_decode(const DecParams p) {
         if (q_task < nb && my_k > 0) {
           const uint32_t sb = slot_base(q_s);
           cp16(sb + lane * 16, q_ptr);
-          cp16(sb + 512 + lane * 16, q_ptr + 2048);
+          cp16(sb + 512 + lane * 16, q_ptr + kHalfBytes);
           cp4(sb + 1024 + lane * 4, q_mptr);
           if (q_xp) cp16(sb + 1280 + lane * 16, q_xp);
-          q_ptr += tile_b;
-          q_mptr += tile_b;
+          q_ptr += sub_b;
+          q_mptr += sub_b;
           if (q_xp) q_xp += kTileK;
           if (++q_ik == my_k) {
             q_ik = 0;
@@ -890,8 +890,8 @@ k_decode(const DecParams p) {
       item_units(q_it, ua, ub);
       const uint32_t sb = slot_base(q_s);
       const int row = (q_rb & 3) * 32 + lane;
-      const size_t koff = (size_t)(hb >> 1) * tile_b + (hb & 1) * 2048 + row * 16;
-      const size_t moff = (size_t)(hb >> 1) * tile_b + kCodeBytes + row * 4;
+      const size_t koff = p.dn.row_sub(row) + (size_t)(hb >> 1) * sub_b + (hb & 1) * kHalfBytes + code_offset(row);
+      const size_t moff = p.dn.row_sub(row) + (size_t)(hb >> 1) * sub_b + meta_offset(kQ4CP, row);
       const uint4 a0 = lds128(kOffRec + ua * 32);
       const uint8_t* base_a = (const uint8_t*)(((unsigned long long)a0.y << 32) | a0.x);
       if (with_w) {

@@ -1,415 +1,568 @@
-// expert_gemv.cu -- decode / speculative-verify path (T <= 16) for q4cp experts: a
-// bandwidth-oriented dequant GEMV. It takes the place of k_q4cp_gemv_gg, k_silu_mul_g and
-// k_q4cp_gemv_gd (src/gpu/parts/20_kernels_gemv.inc:1607-1764 of the reference): per
-// (token, expert) the 2*mid gate/up dot products, SwiGLU, then the d down dot products.
+// expert_gemv.cu -- decode / speculative-verify path (T <= 16): a bandwidth-oriented dequant GEMV. It
+// takes the place of k_q4cp_gemv_gg, k_silu_mul_g and k_q4cp_gemv_gd
+// (src/gpu/parts/20_kernels_gemv.inc:1607-1764 of the reference): per (token, expert) the 2*mid
+// gate/up dot products, SwiGLU, then the d down dot products.
 //
-// At one token the whole layer is ~78 MB of 4-bit weights and 138 M multiply-adds; what
-// decides the speed is (1) that DRAM sees long contiguous reads, (2) how many bytes each SM
-// keeps in flight, (3) how few instructions and shared-memory wavefronts turn a code into a
-// multiply-add.
-//   * A lane owns a weight ROW: in the tiled image the 32 rows of a warp are 512 contiguous
-//     bytes per half K block, so every load instruction of a warp is one long burst. (Lanes
-//     that split K instead -- the reference's mapping -- read 16-byte pieces 2 KB apart from
-//     this layout and reached 1 TB/s.) A lane's dot product needs no cross-lane reduction.
-//   * The 16 warps of a CTA split K of the same rows; their partial sums meet in shared
-//     memory and are added in a fixed order. The activations of the current token are staged
-//     in shared memory as fp16 and read by broadcast (one 16-byte load per 4 code bytes).
-//   * A code BYTE (two codes) is decoded by one lookup in a 256-entry half2 table that is
-//     replicated per lane in shared memory (no bank conflicts); a table line is 256 bytes, on
-//     a 64 KB boundary, so the lookup address is a single byte permute. The two products go
-//     into an fp32 accumulator with the mixed-precision multiply-add (f32 += f16 * f16):
-//     exact products, fp32 sums. The fp16 group scale multiplies the fp32 sum of a group once.
-//   * A warp's share of a task is at most four K blocks = eight 16-byte loads per lane; as
-//     soon as one K block has been consumed, the same registers receive the matching block
-//     of the CTA's NEXT task, so every SM keeps ~64 KB in flight while it computes.
-//   * Gate row r and up row r sit in lanes l and l+16 of the same warp: SwiGLU is a shuffle.
-//   * The kernels are persistent: (row of the permuted activations, row block) tasks are cut
-//     into one contiguous range per CTA; the tables are built once per CTA.
-// (mma.m16n8k16 retires every 2 cycles per SM and serves two tokens without giving up fp32 scales, but its
-// zero-padded activation operand costs load-pipe wavefronts, of which the lookups already take most:
-// 50 / 128 / 277 us against this form's 45 / 132 / 300 at T = 1 / 5 / 13 of the 4096 x 1024 layer.)
+// At one token the layer is ~78 MB of 4-bit weights and 138 M multiply-adds. What decides the speed is how many
+// shared-memory wavefronts and instructions turn a code into a multiply-add: a multiply-add GEMV on the same
+// image (a lane per row, two products per code byte, the activations read by broadcast) spent 37 wavefronts
+// on 512 code bytes, of which 16 were table lookups and 16 the activations, and stood at 2.7 TB/s. Here:
+//   * mma.m16n8k16 forms the products (exact) and sums (fp32). Its A operand is 16 weight rows: ldmatrix deals the
+//     packed codes of a row out to the four lanes of a quad, 8 codes each, a code BYTE becomes an fp16 pair. Scales
+//     stay in fp32: the K slots of the two 32-groups of a K block meet their activations in DIFFERENT columns of B
+//     (a column = a row of activations x a half), zeros elsewhere, so that a column is one group's unscaled sum.
+//     Eight columns = up to four rows of an expert in one pass over its weights.
+//   * B never moves: a warp owns at most four K blocks (its slice) of all the rows its team works on, and the
+//     activations of a slice are 4 registers per K block and lane (8 with the zeros).
+//   * q4cp: a code byte is decoded by one lookup in a 256-entry half2 table replicated per lane in shared memory
+//     (no bank conflicts; a line is 256 bytes, so the address is one byte permute): 32 of the 48 wavefronts per
+//     32 x 64 block, the load pipe is 76 % busy with them. GGUF: the codes are masked into fp16 bit patterns,
+//     code * 2^-24 (denormal, exact), no lookup; 2^24 goes into the fp32 constants.
+//   * Weights come by bulk copies into a ring of three slots of two K blocks per warp (110 KB in flight per SM), one
+//     copy and one wait per slot; the image keeps a slice's K blocks together (common.cuh).
+//   * A unit of work = 32 rows (16 hidden outputs: gate and up rows meet in one warp) over the whole K. The slices
+//     leave their sums in shared memory and go on; they take turns at adding up the unit BEFORE, in slice order, so
+//     that nobody waits at a barrier. A row's sums depend on nothing but its slice cut, a function of the shape.
+//   * Persistent; units are cut into equal contiguous shares per team. The shared expert has CTAs of its own, so
+//     that a CTA needs one image's tables.
+// us of the two kernels, the multiply-add form / this one, 4096 x 1024 with shared expert: T = 1 35 / 26, T = 5
+// 120 / 80, T = 13 288 / 177 (gate/up 4.85 TB/s); Q4_K / Q5_1 T = 5 128 / 88 (gate/up 5.0 TB/s, down 4.0: the
+// fifth bits); 64 experts of 2048 x 512, 16 tokens (2.2 rows an expert) 90 / 33.
 #include "kernels.h"
 
 namespace b200moe {
 
 namespace {
 
-constexpr int kGemvThreads = 512;     // 16 warps
-constexpr int kGemvWarps = kGemvThreads / 32;
-constexpr int kKpw = 4;               // K blocks per warp and task, at most
-constexpr int kGemvMaxRuns = 192;
-constexpr int kGemvMaxK = 4096;       // staged activations: 8 KB of fp16
-constexpr uint32_t kTab0 = 65536;     // absolute shared addresses of the two table blocks
-constexpr uint32_t kTab1 = 131072;
+constexpr int kWarps = 16;            // compute warps of a CTA
+constexpr int kThreads = kWarps * 32;
+constexpr int kRows = 4;              // rows of an expert that one pass over its weights serves
+constexpr int kRed = 4;               // partial-sum buffers of a team
+constexpr int kMaxSubs = 448;         // passes: every expert's rows in fours
+constexpr uint32_t kOffLow = 2048;    // the dynamic allocation must start at or below this (its absolute shared address)
+
+// Shared memory map, absolute shared addresses.
+// KPW: K blocks of a slice, at most.
+template <int FMT, int KPW>
+struct Map {
+  static constexpr int kGroup = KPW == 4 ? 2 : KPW;   // K blocks per ring slot
+  static constexpr int kGroups = KPW / kGroup;        // slots per unit
+  static constexpr uint32_t kLut = kOffLow;  // kQ4CP: 256 lines of {32 lanes x 4 B, first book}{32 x 4 B, second book}
+  static constexpr uint32_t kRing = kLut + (FMT == kQ4CP ? 65536u : 0u);
+  static constexpr uint32_t kSub = (uint32_t)sub_bytes(FMT), kSlot = kGroup * kSub;
+  static constexpr uint32_t kSlots = KPW == 3 ? 2 : 3;  // per warp
+  static constexpr uint32_t kScr = FMT == kQ4K ? 512 : 0;  // per warp: the rows' constants as floats
+  static constexpr uint32_t kPart = kRing + kWarps * kSlots * kSlot;          // partial sums [kRed][warp][32 rows][4]
+  static constexpr uint32_t kBar = kPart + kRed * kWarps * kSubRows * kRows * 4;
+  static constexpr uint32_t kBarFull = kBar;                                  // [warp][slot]
+  static constexpr uint32_t kBarSum = kBarFull + kWarps * kSlots * 8;         // [team][kRed]: the slices' sums are there
+  static constexpr uint32_t kBarFree = kBarSum + kWarps * kRed * 8;           // [team][kRed]: they have been taken
+  static constexpr uint32_t kSubs = kBarFree + kWarps * kRed * 8;             // int2 [kMaxSubs]
+  static constexpr uint32_t kScratch = kSubs + kMaxSubs * 8;
+  static constexpr uint32_t kEnd = kScratch + kWarps * kScr;
+  static constexpr int kBytes = (int)(kEnd - 1024);
+};
 
 struct GemvParams {
   Image img;             // routed experts
-  Image img_sh;          // shared expert (data == nullptr: none)
+  Image img_sh;          // shared expert
   const Run* runs;       // routed runs [n_runs[0]]; the shared run sits at runs[kMaxExperts]
   const int32_t* n_runs;
+  int n_sh;              // CTAs 0 .. n_sh-1 work on the shared expert, the others on the routed ones
   int K;                 // d (gate/up) or mid (down)
   int mid;
+  int slices, teams;     // warps that share a unit's K blocks; units in work at a time
   const uint16_t* x;     // gate/up: bf16 [T][d]
   const int32_t* tokidx;
   __half* hid;           // gate/up writes, down reads: fp16 [rows][mid] = silu(gate) * up
   float* out;            // down: pairs fp32 [rows][d]
+  int32_t* status;
 };
 
-__device__ __forceinline__ uint32_t lds_b32(uint32_t addr) {
+__device__ __forceinline__ uint32_t lds32(uint32_t a) {
   uint32_t v;
-  asm("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(addr));
+  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
   return v;
 }
-
-// acc += w.lo * x.lo + w.hi * x.hi with exact products and fp32 sums
-__device__ __forceinline__ void fma_pair(float& acc, uint32_t w, uint32_t x) {
-  asm("{\n\t.reg .b16 wl, wh, xl, xh;\n\t"
-      "mov.b32 {wl, wh}, %1;\n\t"
-      "mov.b32 {xl, xh}, %2;\n\t"
-      "fma.rn.f32.f16 %0, wl, xl, %0;\n\t"
-      "fma.rn.f32.f16 %0, wh, xh, %0;\n\t}"
-      : "+f"(acc)
-      : "r"(w), "r"(x));
+__device__ __forceinline__ uint2 lds64(uint32_t a) {
+  uint2 v;
+  asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a) : "memory");
+  return v;
 }
-
-// sum over one 16-byte chunk (32 codes of one group) of w[k] * x[k], as float.
-// lut: constant half of the lookup address { lane*4 (+128), -, table >> 16, 0 };
-// xs: shared address of the 32 fp16 activations of the group (same for all lanes: broadcast).
-__device__ __forceinline__ float chunk_dot(const uint4 c, uint32_t lut, uint32_t xs) {
-  const uint32_t w4[4] = {c.x, c.y, c.z, c.w};
-  float s0 = 0.f, s1 = 0.f;
-#pragma unroll
-  for (int q = 0; q < 4; q++) {
-    uint32_t x0, x1, x2, x3;
-    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(x0), "=r"(x1), "=r"(x2), "=r"(x3) : "r"(xs + q * 16));
-    fma_pair(s0, lds_b32(__byte_perm(w4[q], lut, 0x7604)), x0);
-    fma_pair(s1, lds_b32(__byte_perm(w4[q], lut, 0x7614)), x1);
-    fma_pair(s0, lds_b32(__byte_perm(w4[q], lut, 0x7624)), x2);
-    fma_pair(s1, lds_b32(__byte_perm(w4[q], lut, 0x7634)), x3);
-  }
-  return s0 + s1;
+__device__ __forceinline__ uint4 lds128(uint32_t a) {
+  uint4 v;
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
+  return v;
 }
-
-// Q5_1: the same with the fifth bits (bits i, 16 + i of qh belong to code byte i; shifted to bits
-// 14 and 30 they are the fp16 pair 2.0 / 0) added to the looked-up pair as 8 * 2.0 by one half2
-// multiply-add before the products: q + 16*bit <= 31 is exact in fp16.
-__device__ __forceinline__ float chunk_dot5(const uint4 c, uint32_t qh, uint32_t lut, uint32_t xs) {
-  const uint32_t w4[4] = {c.x, c.y, c.z, c.w};
-  float s0 = 0.f, s1 = 0.f;
-#pragma unroll
-  for (int q = 0; q < 4; q++) {
-    uint32_t x[4];
-    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]) : "r"(xs + q * 16));
-#pragma unroll
-    for (int b = 0; b < 4; b++) {
-      const int i = q * 4 + b;
-      const uint32_t u = (i <= 14 ? (qh << (14 - i)) : (qh >> 1)) & 0x40004000u;
-      const uint32_t pair = lds_b32(__byte_perm(w4[q], lut, 0x7604 | (b << 4)));
-      const __half2 w2 = __hfma2(*(const __half2*)&u, __float2half2_rn(8.f), *(const __half2*)&pair);
-      fma_pair((b & 1) ? s1 : s0, *(const uint32_t*)&w2, x[b]);
+__device__ __forceinline__ void sts32(uint32_t a, uint32_t v) { asm volatile("st.shared.b32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
+// the pair table does not change once it is built: these loads may be moved freely
+template <uint32_t BASE>
+__device__ __forceinline__ uint32_t lut32(uint32_t a) {
+  uint32_t v;
+  asm("ld.shared.b32 %0, [%1+%2];" : "=r"(v) : "r"(a), "n"(BASE));
+  return v;
+}
+__device__ __forceinline__ void ldsm4(uint32_t a, uint32_t* m) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(m[0]), "=r"(m[1]), "=r"(m[2]), "=r"(m[3]) : "r"(a) : "memory");
+}
+// c += a (16 rows x 16) * b (16 x 8), fp16 operands, fp32 sums
+__device__ __forceinline__ void mma16816(float* c, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void mma16816_first(float* c, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+      : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
+__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok) : "r"(bar), "r"(parity), "r"(20000u) : "memory");
+  return ok != 0;
+}
+// Bounded wait (2 s), all lanes of a warp. After one that gave up the warp waits no more: what it computes is
+// void, the status word tells.
+__device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, int32_t* status, int where) {
+  unsigned long long t0, t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
+  for (;;) {
+    if (mbar_try(bar, parity)) return false;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    if (t - t0 > 2000000000ull) {
+      if (status && atomicCAS(status, 0, 8) == 0) status[1] = where;
+      return true;
     }
   }
-  return s0 + s1;
+}
+__device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, bool& dead, int32_t* status, int where) {
+  if (!mbar_try(bar, parity) && !dead) dead = mbar_wait_slow(bar, parity, status, where);
 }
 
 // finite values saturate to the fp16 range, NaN stays NaN
 __device__ __forceinline__ float sat_f16(float v) { return v != v ? v : fminf(fmaxf(v, -65504.f), 65504.f); }
-__device__ __forceinline__ uint32_t pack_half2_sat(float a, float b) {
-  __half2 h = __floats2half2_rn(sat_f16(a), sat_f16(b));
-  return *(uint32_t*)&h;
+__device__ __forceinline__ uint32_t bf16x2_to_f16x2(uint32_t w) {
+  const __half2 h = __floats2half2_rn(sat_f16(__uint_as_float(w << 16)), sat_f16(__uint_as_float(w & 0xFFFF0000u)));
+  return *(const uint32_t*)&h;
 }
 
-
-
-struct GemvShared {
-  int first[kGemvMaxRuns + 2];  // unit prefix: rows before run i ("unit" = one row of the permuted activations)
-  float book[3][16];
-};
-
-// FMT: format of the image this kernel reads (gate/up: q4cp or Q4_K; down: q4cp or Q5_1). The
-// GGUF formats use the identity code book (table entry = the two code values) and fold their
-// affine constants into the group sums: Q4_K  sum w x = (d*sc) * sum q x - (dmin*m) * sum x,
-// Q5_1  sum w x = d * sum (q + 16 bit) x + m * sum x, with sum x per 32-group staged next to
-// the activations.
-template <bool UP, int FMT>
-__global__ void __launch_bounds__(kGemvThreads, 1)
+template <bool UP, int FMT, int KPW>
+__global__ void __launch_bounds__(kThreads, 1)
 k_gemv(const GemvParams p) {
+  using M = Map<FMT, KPW>;
   extern __shared__ __align__(16) uint8_t gsm[];
-  __shared__ GemvShared sh;
-  __shared__ __align__(16) __half xs[kGemvMaxK];   // activations of the current unit
-  __shared__ float xsum[kGemvMaxK / 32];            // their sums per 32-group (GGUF formats)
-  __shared__ float red[2][kGemvWarps][32];          // partial sums of the K slices, double-buffered by task
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t dyn0 = (uint32_t)__cvta_generic_to_shared(gsm);
-  uint8_t* const smem = gsm - dyn0;  // smem + A is the generic pointer of absolute shared address A
-  const bool has_sh = p.img_sh.data != nullptr;
-  const bool two = UP && has_sh && p.img_sh.dual_book;
-  pdl_trigger();
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   {
-    // The table blocks live at fixed absolute shared addresses: a launch whose dynamic
-    // allocation does not cover them is refused (uniform for the grid; the host sizes it).
+    // the map stands at fixed absolute shared addresses: a launch whose dynamic allocation does not
+    // cover it is refused (uniform for the grid; the host sizes it)
+    const uint32_t dyn0 = (uint32_t)__cvta_generic_to_shared(gsm);
     uint32_t dyn_size;
     asm volatile("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn_size));
-    if (dyn0 > kTab0 || dyn0 + dyn_size < (two ? kTab1 + 65536 : kTab0 + 65536)) return;
+    if (dyn0 > kOffLow || dyn0 + dyn_size < M::kEnd) return;
   }
-  // ---- code books and pair tables: weights only, nothing an earlier kernel of the stream
-  // writes, so this part may overlap that kernel's tail ----
-  if (threadIdx.x < 48) {
-    const int b = threadIdx.x >> 4, e = threadIdx.x & 15;
-    if (b == 0) sh.book[0][e] = p.img.book[e];
-    else if (has_sh && (b == 1 || two)) sh.book[b][e] = p.img_sh.book[(b - 1) * 16 + e];
+  const bool sh = (int)blockIdx.x < p.n_sh;
+  const Image& im = sh ? p.img_sh : p.img;
+  // ---- set-up that needs weights only, nothing an earlier kernel of the stream writes ----
+  if (tid < kWarps * (int)M::kSlots) mbar_init(M::kBarFull + tid * 8, 1);
+  if (tid < kWarps * kRed) {
+    mbar_init(M::kBarSum + tid * 8, p.slices);
+    mbar_init(M::kBarFree + tid * 8, 1);
   }
-  __syncthreads();
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  if (FMT == kQ4CP) {
+    // entry e = (f16(book[e & 15]), f16(book[e >> 4])); warp w writes the 16 lines whose high code is w
+    for (int b = 0; b < (UP && im.dual_book ? 2 : 1); b++) {
+      const uint32_t hi16 = (uint32_t)__half_as_ushort(__float2half_rn(__ldg(im.book + b * 16 + warp))) << 16;
+      const uint32_t mine = (uint32_t)__half_as_ushort(__float2half_rn(__ldg(im.book + b * 16 + (lane & 15))));
+      const uint32_t dst = M::kLut + (uint32_t)(warp * 16 * 256 + b * 128 + lane * 4);
+#pragma unroll
+      for (int c = 0; c < 16; c++) sts32(dst + c * 256, hi16 | __shfl_sync(0xffffffffu, mine, c));
+    }
+  }
+  if (UP) pdl_wait();
+  pdl_trigger();
+  // ---- passes: every expert's rows in fours ----
+  // (the down kernel reads the run list before its wait: the routing kernel was complete before any CTA of the
+  // gate/up kernel triggered)
+  __shared__ int s_cnt[kWarps];
+  int n_subs;
   {
-    // entry e = (f16(book[e & 15]), f16(book[e >> 4])), one 256-byte line per code byte:
-    // [32 lanes x 4 B of book A][32 lanes x 4 B of book B]. Block 0 holds the routed book (A)
-    // and the shared expert's first book (B); block 1 the shared expert's second book (rows
-    // 64..127 of its gate/up tiles, when that image has two books).
-    // Warp w writes the 16 lines whose high code is w; lane l writes copy l of each line.
-    const int nb = has_sh ? (two ? 3 : 2) : 1;
-    for (int b = 0; b < nb; b++) {
-      const uint32_t hi16 = (uint32_t)__half_as_ushort(__float2half_rn(sh.book[b][warp])) << 16;
-      uint8_t* dst = smem + (b == 2 ? kTab1 : kTab0) + (b == 1 ? 128 : 0) + (warp * 16) * 256 + lane * 4;
+    const int n_runs = sh ? 1 : min(p.n_runs[0], kThreads);
+    Run run{0, 0, 0};
+    if (tid < n_runs) run = sh ? p.runs[kMaxExperts] : p.runs[tid];
+    const int c = (run.count + kRows - 1) / kRows;
+    int incl = c;
 #pragma unroll
-      for (int c = 0; c < 16; c++)
-        *(uint32_t*)(dst + c * 256) = hi16 | (uint32_t)__half_as_ushort(__float2half_rn(sh.book[b][c]));
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
     }
+    if (lane == 31) s_cnt[warp] = incl;
+    __syncthreads();
+    int before = incl - c;
+    n_subs = 0;
+    for (int w = 0; w < kWarps; w++) {
+      const int v = s_cnt[w];
+      if (w < warp) before += v;
+      n_subs += v;
+    }
+    n_subs = min(n_subs, kMaxSubs);
+    for (int i = 0; i < c; i++)
+      if (before + i < kMaxSubs) {
+        sts32(M::kSubs + (before + i) * 8, (uint32_t)run.expert | (uint32_t)min(kRows, run.count - i * kRows) << 16);
+        sts32(M::kSubs + (before + i) * 8 + 4, (uint32_t)(run.first + i * kRows));
+      }
+    __syncthreads();
   }
-  pdl_wait();
-  // ---- unit prefix ----
-  const int n_routed = p.n_runs[0];
-  const int n_runs_all = min(n_routed + (has_sh ? 1 : 0), kGemvMaxRuns);
-  for (int i = threadIdx.x; i < n_runs_all; i += kGemvThreads)
-    sh.first[i] = (i < n_routed ? p.runs[i] : p.runs[kMaxExperts]).count;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int acc = 0;
-    for (int i = 0; i < n_runs_all; i++) {
-      const int c = sh.first[i];
-      sh.first[i] = acc;
-      acc += c;
-    }
-    sh.first[n_runs_all] = acc;
+  // ---- this team's share: units c0 .. c1-1 of all passes. A unit = one sub-block column, 32 tile rows over the whole K ----
+  const int KB = im.n_kblocks, ash = im.act_shift;
+  const int slice = warp % p.slices, team = warp / p.slices;
+  if (team >= p.teams) return;
+  const int kb0 = slice * KPW, nk = min(KPW, KB - kb0);
+  const int upr = im.n_mtiles * 4;  // units of a pass
+  int c0, n_units;
+  {
+    const int total = n_subs * upr;
+    const int n_ct = sh ? p.n_sh : (int)gridDim.x - p.n_sh, ci = sh ? (int)blockIdx.x : (int)blockIdx.x - p.n_sh;
+    const int nt = n_ct * p.teams, ti = ci * p.teams + team;
+    const int base = total / nt, rem = total % nt;
+    c0 = ti * base + min(ti, rem);
+    n_units = base + (ti < rem ? 1 : 0);
   }
-  __syncthreads();
-
-  // ---- geometry. gate/up: a task = 16 hidden outputs (lanes 0..15 the gate rows, lanes 16..31
-  // the matching up rows), every warp a K slice. down: a task = 64 output rows, warps = 2 row
-  // groups x 8 K slices. A warp's share of a task is kpw <= 4 K blocks ("items"). ----
-  const int KB = p.img.n_kblocks;        // image K blocks (twice p.K / 64 for a two-plane image of 8-bit codes)
-  const int ash = p.img.act_shift;       // an image K block multiplies the activations of K block (index >> ash)
-  constexpr int kSlices = UP ? kGemvWarps : kGemvWarps / 2;
-  const int slice = UP ? warp : warp >> 1;
-  const int kpw = (KB + kSlices - 1) / kSlices;  // <= kKpw (the host checks K)
-  const int kb0 = slice * kpw;
-  const int out_rows = UP ? p.mid : p.img.n_mtiles * kTileM;
-  const int tpu = UP ? out_rows / 16 : out_rows / 64;  // tasks per unit
-  const long long total = (long long)sh.first[n_runs_all] * tpu;
-  const long long base = total / gridDim.x, rem = total % gridDim.x;
-  const long long c0 = blockIdx.x * base + min((long long)blockIdx.x, rem), c1 = c0 + base + ((long long)blockIdx.x < rem ? 1 : 0);
-  constexpr size_t tile_b = tile_bytes(FMT);     // the routed and the shared image have the same format
-  constexpr int kMetaRow = FMT == kQ4CP ? 4 : FMT == kQ4K ? 8 : 16;  // bytes of metadata per tile row
-  const uint32_t xs_addr = (uint32_t)__cvta_generic_to_shared(xs);
-
-  uint4 cw[2 * kKpw];  // four item slots: codes of both halves of a K block ...
-  uint4 sw[kKpw];      // ... and the row's metadata of the K block (q4cp: .x = two fp16 scales)
-  int cur_tok = -1, buf = 0;
-  for (long long seg = c0; seg < c1;) {
-    // ---- a segment: the CTA's tasks j0 .. j1-1 of one unit ----
-    const int unit = (int)(seg / tpu), j0 = (int)(seg % tpu);
-    const int j1 = (int)min((long long)tpu, (long long)j0 + (c1 - seg));
-    seg += j1 - j0;
-    int lo = 0, hi = n_runs_all - 1;
-    while (lo < hi) {
-      const int m = (lo + hi + 1) >> 1;
-      if (sh.first[m] <= unit) lo = m; else hi = m - 1;
+  if (n_units == 0) return;
+  // ---- the copy stream: a slot = one group of K blocks of a unit, M::kSlots groups ahead ----
+  const uint32_t ring = M::kRing + (uint32_t)warp * M::kSlots * M::kSlot, full = M::kBarFull + (uint32_t)warp * M::kSlots * 8;
+  int q_left = n_units, q_g = 0, q_sub = c0 / upr, q_j = c0 % upr;
+  uint32_t q_slot = 0;
+  const uint32_t unit_b = (uint32_t)KB * M::kSub;
+  const uint8_t* q_ptr;  // the slice's first K block of the unit at hand: the units of an expert follow one another
+  auto q_pass = [&]() {
+    const uint32_t e = lds32(M::kSubs + q_sub * 8) & 0xFFFFu;
+    q_ptr = im.data + ((size_t)e * upr + q_j) * unit_b + (uint32_t)kb0 * M::kSub;
+  };
+  q_pass();
+  auto issue = [&]() {
+    if (q_left > 0) {
+      if (lane == 0) {
+        const uint32_t bar = full + q_slot * 8;
+        const uint32_t bytes = min(M::kGroup, nk - q_g * M::kGroup) * M::kSub;  // > 0: groups without K blocks are stepped over
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                         ring + q_slot * M::kSlot), "l"(q_ptr + q_g * M::kSlot), "r"(bytes), "r"(bar)
+                     : "memory");
+      }
+      q_slot = q_slot + 1 == M::kSlots ? 0 : q_slot + 1;
+      if (M::kGroups > 1 && q_g + 1 < M::kGroups && (q_g + 1) * M::kGroup < nk) {
+        q_g++;
+      } else {
+        q_g = 0;
+        q_left--;
+        q_j++;
+        q_ptr += unit_b;
+        if (q_j == upr) {
+          q_j = 0;
+          q_sub++;
+          if (q_left > 0) q_pass();
+        }
+      }
     }
-    const bool routed = lo < n_routed;
-    Run run = routed ? p.runs[lo] : p.runs[kMaxExperts];
-    run.first += unit - sh.first[lo];
-    const Image& im = routed ? p.img : p.img_sh;
-    const size_t mt_b = (size_t)im.n_kblocks * tile_b;
-    const uint8_t* const ebase = im.data + (size_t)run.expert * im.n_mtiles * mt_b + (size_t)kb0 * tile_b;
-    const uint32_t lut = (routed ? kTab0 : (UP && lane >= 16 && im.dual_book ? kTab1 : kTab0 + 128)) + lane * 4;
-    // this lane's row of task j: offset of its codes in the first K block of the warp's slice
-    auto row_off = [&](int j) -> size_t {
-      if (UP) return (size_t)(j >> 2) * mt_b + ((lane < 16 ? 0 : 48) + (j & 3) * 16 + lane) * 16;  // gate rows 0..63, up rows 64..127
-      return (size_t)(j >> 1) * mt_b + ((j & 1) * 64 + (warp & 1) * 32 + lane) * 16;
-    };
-    auto fetch = [&](int s, int j, int i) {  // item (task j, K block i of the slice) into slot s
-      if (kb0 + i < KB) {
-        const uint8_t* pc = ebase + row_off(j) + (size_t)i * tile_b;
-        const size_t r16 = row_off(j) - (size_t)(UP ? j >> 2 : j >> 1) * mt_b;  // row * 16
-        cw[2 * s] = __ldg((const uint4*)pc);
-        cw[2 * s + 1] = __ldg((const uint4*)(pc + 2048));
-        const uint8_t* pm = pc - r16 + kCodeBytes + (r16 >> 4) * kMetaRow;
-        if (FMT == kQ4CP) {
-          sw[s].x = __ldg((const uint32_t*)pm);
-        } else if (FMT == kQ4K) {
-          const uint2 u = __ldg((const uint2*)pm);
-          sw[s].x = u.x;
-          sw[s].y = u.y;
+  };
+  for (uint32_t s = 0; s < M::kSlots; s++) issue();
+  if (!UP) pdl_wait();
+
+  bool dead = false, lost = false;  // a wait for the team, for the warp's own copies gave up
+  uint32_t c_slot = 0, c_ph = 0;
+  int sub = c0 / upr, j = c0 % upr, cnt = 0, first = 0;
+  bool fresh = true;
+  uint32_t bv[KPW][4], bw[KPW][4];          // activations: lane (g, t) holds row g >> 1, half g & 1, elements 8t .. 8t+7 of every K block
+  float xs[KPW][2];             // GGUF: sums of the activations of row t, halves 0 and 1
+  const uint32_t m0 = (g & 1) ? 0u : 0xFFFFFFFFu, m1 = ~m0;
+  const uint32_t lut_a = (uint32_t)lane * 4, lut_b = lut_a + (UP && im.dual_book ? 128u : 0u);
+  const uint32_t lane_src = (uint32_t)(lane >> 4) * kHalfBytes + (uint32_t)(lane & 15) * 16;
+  const uint32_t part0 = M::kPart + (uint32_t)(team * p.slices) * (kSubRows * kRows * 4);
+  constexpr uint32_t kPartBuf = kWarps * kSubRows * kRows * 4;
+  const uint32_t bar_sum = M::kBarSum + team * kRed * 8, bar_free = M::kBarFree + team * kRed * 8;
+  // adds the slices of unit n (its number in this team's share) in slice order and writes its results
+  auto finish = [&](int n, int uj, int ucnt, int ufirst) {
+    const uint32_t b = n & (kRed - 1);
+    mbar_wait(bar_sum + b * 8, (n / kRed) & 1, dead, p.status, 22);
+    float tot[kRows] = {0.f, 0.f, 0.f, 0.f};
+    const uint32_t a = part0 + b * kPartBuf + lane * 16;
+#pragma unroll 4
+    for (int s = 0; s < p.slices; s++) {
+      const uint4 v = lds128(a + s * (kSubRows * kRows * 4));
+      tot[0] += __uint_as_float(v.x);
+      tot[1] += __uint_as_float(v.y);
+      tot[2] += __uint_as_float(v.z);
+      tot[3] += __uint_as_float(v.w);
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar_free + b * 8);
+#pragma unroll
+    for (int r = 0; r < kRows; r++) {
+      if (r < ucnt) {
+        if (UP) {
+          const float up = __shfl_down_sync(0xffffffffu, tot[r], 16);
+          if (lane < 16)
+            p.hid[(size_t)(ufirst + r) * p.mid + uj * 16 + lane] = __float2half_rn(sat_f16(silu_f32(tot[r]) * up));
         } else {
-          sw[s] = __ldg((const uint4*)pm);
+          p.out[(size_t)(ufirst + r) * (upr * kSubRows) + uj * kSubRows + lane] = tot[r];
         }
       }
-    };
-    const int nseg = (j1 - j0) * kpw;
-    // the first four items go out before anything else: they are in flight while the tables
-    // are built and the activations staged
-    int pj = j0, pi = 0;  // the fetch stream's position
-#pragma unroll
-    for (int s = 0; s < kKpw; s++) {
-      if (s < nseg) fetch(s, pj, pi);
-      if (++pi == kpw) { pi = 0; pj++; }
     }
-    // activations of the unit (the previous segment's reads of xs ended before its last barrier)
-    bool staged = false;
-    if (UP) {
-      const int tok = p.tokidx[run.first];
-      if (tok != cur_tok) {
-        for (int c = threadIdx.x; c < p.K / 8; c += kGemvThreads) {
-          const uint4 u = __ldg((const uint4*)(p.x + (size_t)tok * p.K) + c);
-          const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-          uint4 o;
-          o.x = pack_half2_sat(__uint_as_float(w[0] << 16), __uint_as_float(w[0] & 0xFFFF0000u));
-          o.y = pack_half2_sat(__uint_as_float(w[1] << 16), __uint_as_float(w[1] & 0xFFFF0000u));
-          o.z = pack_half2_sat(__uint_as_float(w[2] << 16), __uint_as_float(w[2] & 0xFFFF0000u));
-          o.w = pack_half2_sat(__uint_as_float(w[3] << 16), __uint_as_float(w[3] & 0xFFFF0000u));
-          ((uint4*)xs)[c] = o;
+  };
+  // one K block (number i of the slice) of a unit: 32 rows x 64 columns
+  auto item = [&](int i, uint32_t s0, float (&acc)[2][2]) {
+    uint32_t m[2][4];
+    ldsm4(s0 + lane_src, m[0]);
+    ldsm4(s0 + lane_src + 256, m[1]);
+    float k[2][2][4];  // constants of the lane's rows: factors of the two halves' sums (and of the activations' sums)
+    if (FMT == kQ4K) {
+      // a lane turns one row's constants into floats, all lanes pick up theirs
+      const uint32_t sa = M::kScratch + warp * 512;
+      const uint2 v = lds64(s0 + kSubCodes + lane * 8);
+      const float2 dd = __half22float2(*(const __half2*)&v.x);
+      // {sc0, m0, sc1, m1} as fp16 1024 + value, then exactly the values
+      const uint32_t u0 = __byte_perm(v.y, 0x64646464u, 0x4240), u1 = __byte_perm(v.y, 0x64646464u, 0x4341);
+      const __half2 k1024 = __float2half2_rn(1024.f);
+      const float2 sc = __half22float2(__hsub2(*(const __half2*)&u0, k1024)), mn = __half22float2(__hsub2(*(const __half2*)&u1, k1024));
+      const float ds = dd.x * 16777216.f;  // the codes stand as code * 2^-24
+      __syncwarp();
+      asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(sa + lane * 16), "f"(ds * sc.x), "f"(ds * sc.y), "f"(-dd.y * mn.x), "f"(-dd.y * mn.y) : "memory");
+      __syncwarp();
+#pragma unroll
+      for (int b = 0; b < 2; b++)
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+          const uint4 w = lds128(sa + (uint32_t)(b * 16 + r * 8 + g) * 16);
+          k[b][r][0] = __uint_as_float(w.x); k[b][r][1] = __uint_as_float(w.y); k[b][r][2] = __uint_as_float(w.z); k[b][r][3] = __uint_as_float(w.w);
         }
-        cur_tok = tok;
-        staged = true;
-      }
-    } else {
-      for (int c = threadIdx.x; c < p.K / 8; c += kGemvThreads)
-        ((uint4*)xs)[c] = ((const uint4*)(p.hid + (size_t)run.first * p.mid))[c];  // written by the previous kernel: plain loads
-      staged = true;
     }
-    if (staged) {
-      __syncthreads();
-      if (FMT != kQ4CP) {
-        for (int g = threadIdx.x; g < p.K / 32; g += kGemvThreads) {
-          float t = 0.f;
-          for (int i = 0; i < 32; i++) t += __half2float(xs[g * 32 + i]);
-          xsum[g] = t;
+    uint32_t f[2][4];
+#pragma unroll
+    for (int b = 0; b < 2; b++)
+#pragma unroll
+      for (int r = 0; r < 2; r++) {
+        const uint32_t ma = s0 + kSubCodes + (uint32_t)(b * 16 + r * 8 + g) * meta_row_bytes(FMT);
+        if (FMT == kQ4CP) {
+          const uint32_t v = lds32(ma);
+          const float2 s = __half22float2(*(const __half2*)&v);
+          k[b][r][0] = s.x; k[b][r][1] = s.y;
+        } else if (FMT == kQ51) {
+          const uint4 v = lds128(ma);
+          const float2 e0 = __half22float2(*(const __half2*)&v.x), e1 = __half22float2(*(const __half2*)&v.z);
+          k[b][r][0] = e0.x * 16777216.f; k[b][r][1] = e1.x * 16777216.f; k[b][r][2] = e0.y; k[b][r][3] = e1.y;
+          // this lane's eight fifth bits of the row's two halves to bits 0..3 and 16..19
+          f[b][r] = v.y >> (4 * t);
+          f[b][2 + r] = v.w >> (4 * t);
         }
-        __syncthreads();
       }
-    }
-
-    int cj = j0, ci = 0;  // the compute stream's position
-    float acc = 0.f;
-    for (int n0 = 0; n0 < nseg; n0 += kKpw) {
 #pragma unroll
-      for (int s = 0; s < kKpw; s++) {
-        if (n0 + s < nseg) {
-          if (kb0 + ci < KB) {
-            const uint32_t xa = xs_addr + (uint32_t)((kb0 + ci) >> ash) * (kTileK * 2);
-            if (FMT == kQ4CP) {
-              const float d0 = chunk_dot(cw[2 * s], lut, xa), d1 = chunk_dot(cw[2 * s + 1], lut, xa + 64);
-              acc += half_bits_to_f32((uint16_t)(sw[s].x & 0xFFFFu)) * d0 + half_bits_to_f32((uint16_t)(sw[s].x >> 16)) * d1;
-            } else if (FMT == kQ4K) {
-              // metadata {fp16 d, fp16 dmin, u8 sc0, u8 m0, u8 sc1, u8 m1}
-              const float d0 = chunk_dot(cw[2 * s], lut, xa), d1 = chunk_dot(cw[2 * s + 1], lut, xa + 64);
-              const float dd = half_bits_to_f32((uint16_t)(sw[s].x & 0xFFFFu)), dm = half_bits_to_f32((uint16_t)(sw[s].x >> 16));
-              const float x0 = xsum[2 * ((kb0 + ci) >> ash)], x1 = xsum[2 * ((kb0 + ci) >> ash) + 1];
-              acc += (dd * (float)(sw[s].y & 0xFFu)) * d0 - (dm * (float)((sw[s].y >> 8) & 0xFFu)) * x0;
-              acc += (dd * (float)((sw[s].y >> 16) & 0xFFu)) * d1 - (dm * (float)(sw[s].y >> 24)) * x1;
-            } else {
-              // metadata [2]{fp16 d, fp16 m, u32 fifth bits}
-              const float d0 = chunk_dot5(cw[2 * s], sw[s].y, lut, xa), d1 = chunk_dot5(cw[2 * s + 1], sw[s].w, lut, xa + 64);
-              const float x0 = xsum[2 * ((kb0 + ci) >> ash)], x1 = xsum[2 * ((kb0 + ci) >> ash) + 1];
-              acc += half_bits_to_f32((uint16_t)(sw[s].x & 0xFFFFu)) * d0 + half_bits_to_f32((uint16_t)(sw[s].x >> 16)) * x0;
-              acc += half_bits_to_f32((uint16_t)(sw[s].z & 0xFFFFu)) * d1 + half_bits_to_f32((uint16_t)(sw[s].z >> 16)) * x1;
-            }
-          }
-          // the slot just consumed receives the item four further down the stream
-          if (n0 + s + kKpw < nseg) fetch(s, pj, pi);
-          if (++pi == kpw) { pi = 0; pj++; }
-          if (++ci == kpw) {
-            // ---- end of a task: the K slices meet in shared memory; one warp per row group
-            // adds them in slice order ----
-            red[buf][warp][lane] = acc;
-            __syncthreads();
-            if (UP) {
-              if (warp == 0) {
-                float tot = 0.f;
+    for (int b = 0; b < 2; b++) {
+      float c[4], c16[4];
 #pragma unroll
-                for (int w = 0; w < kGemvWarps; w++) tot += red[buf][w][lane];
-                const float up = __shfl_down_sync(0xffffffffu, tot, 16);
-                if (lane < 16)
-                  p.hid[(size_t)run.first * p.mid + cj * 16 + lane] =
-                      __float2half_rn(sat_f16(silu_f32(tot) * up));
-              }
-            } else {
-              if (warp < 2) {
-                float tot = 0.f;
+      for (int q = 0; q < 4; q++) {
+        uint32_t a[4];
 #pragma unroll
-                for (int w = 0; w < kGemvWarps / 2; w++) tot += red[buf][2 * w + warp][lane];
-                p.out[(size_t)run.first * out_rows + cj * 64 + warp * 32 + lane] = tot;
-              }
-            }
-            buf ^= 1;
-            acc = 0.f;
-            ci = 0;
-            cj++;
+        for (int h = 0; h < 4; h++) {
+          if (FMT == kQ4CP) {
+            a[h] = lut32<M::kLut>(__byte_perm(m[b][h], b ? lut_b : lut_a, 0x5504 | (q << 4)));
+          } else if (FMT == kQ4K) {
+            // codes q and q + 4 of the word as the fp16 pair code * 2^-24, for odd q 16 times that (denormal numbers: exact, also in the products)
+            a[h] = (q & 2 ? m[b][h] >> 8 : m[b][h]) & (q & 1 ? 0x00F000F0u : 0x000F000Fu);
+          } else {
+            // the two codes of byte q as the fp16 pair code * 2^-24
+            a[h] = __byte_perm(m[b][h], m[b][h] >> 4, q | (4 + q) << 8) & 0x000F000Fu;
+            a[h] |= (f[b][h] << (4 - q)) & 0x00100010u;
           }
         }
+        float* cc = FMT == kQ4K && (q & 1) ? c16 : c;
+        if (q == 0 || (FMT == kQ4K && q == 1)) mma16816_first(cc, a[0], a[1], a[2], a[3], bv[i][q], bw[i][q]);
+        else mma16816(cc, a[0], a[1], a[2], a[3], bv[i][q], bw[i][q]);
       }
+      if (FMT == kQ4K) {
+#pragma unroll
+        for (int h = 0; h < 4; h++) c[h] = fmaf(c16[h], 0.0625f, c[h]);
+      }
+#pragma unroll
+      for (int r = 0; r < 2; r++) {
+        acc[b][r] = fmaf(k[b][r][1], c[2 * r + 1], fmaf(k[b][r][0], c[2 * r], acc[b][r]));
+        if (FMT != kQ4CP) acc[b][r] = fmaf(k[b][r][3], xs[i][1], fmaf(k[b][r][2], xs[i][0], acc[b][r]));
+      }
+    }
+  };
+  int pj = 0, pcnt = 0, pfirst = 0, turn = 0;
+  for (int n = 0; n <= n_units; n++) {
+   if (n < n_units) {
+    if (fresh) {
+      fresh = false;
+      const uint2 e = lds64(M::kSubs + sub * 8);
+      cnt = (int)(e.x >> 16);
+      first = (int)e.y;
+      const int tok = g >> 1;
+      const bool live = tok < cnt;
+      const size_t row = live ? (UP ? (size_t)p.tokidx[first + tok] : (size_t)(first + tok)) : 0;
+#pragma unroll
+      for (int i = 0; i < KPW; i++) {
+        uint4 u = make_uint4(0, 0, 0, 0);
+        if (live && i < nk) {
+          const size_t o = row * p.K + (size_t)((kb0 + i) >> ash) * kTileK + (g & 1) * 32 + t * 8;
+          u = UP ? __ldg((const uint4*)(p.x + o)) : *(const uint4*)(p.hid + o);
+        }
+        const uint32_t w0 = UP ? bf16x2_to_f16x2(u.x) : u.x, w1 = UP ? bf16x2_to_f16x2(u.y) : u.y;
+        const uint32_t w2 = UP ? bf16x2_to_f16x2(u.z) : u.z, w3 = UP ? bf16x2_to_f16x2(u.w) : u.w;
+        if (FMT == kQ4K) {  // elements q and q + 4
+          bv[i][0] = __byte_perm(w0, w2, 0x5410); bv[i][1] = __byte_perm(w0, w2, 0x7632);
+          bv[i][2] = __byte_perm(w1, w3, 0x5410); bv[i][3] = __byte_perm(w1, w3, 0x7632);
+        } else {            // elements 2q and 2q + 1
+          bv[i][0] = w0; bv[i][1] = w1; bv[i][2] = w2; bv[i][3] = w3;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          bw[i][q] = bv[i][q] & m1;
+          bv[i][q] &= m0;
+        }
+        if (FMT != kQ4CP) {
+          float c[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+          for (int q = 0; q < 4; q++)
+            mma16816(c, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u, bv[i][q], bw[i][q]);
+          xs[i][0] = c[0];
+          xs[i][1] = c[1];
+        }
+      }
+    }
+    float acc[2][2] = {{0.f, 0.f}, {0.f, 0.f}};  // [16-row block][row g, row g + 8] of row t
+#pragma unroll
+    for (int gi = 0; gi < M::kGroups; gi++) {
+      if (gi * M::kGroup < nk) {
+        mbar_wait(full + c_slot * 8, c_ph, lost, p.status, 20);
+        const uint32_t slot0 = ring + c_slot * M::kSlot;
+#pragma unroll
+        for (int ii = 0; ii < M::kGroup; ii++) {
+          const int i = gi * M::kGroup + ii;
+          if (i < nk) item(i, slot0 + ii * M::kSub, acc);
+        }
+        __syncwarp();
+        issue();  // the slot has been read
+        c_slot++;
+        if (c_slot == M::kSlots) {
+          c_slot = 0;
+          c_ph ^= 1;
+        }
+      }
+    }
+    // ---- the slice's sums of this unit ----
+    const uint32_t b = n & (kRed - 1);
+    if (n >= kRed) mbar_wait(bar_free + b * 8, ((n / kRed) & 1) ^ 1, dead, p.status, 21);
+    if (t < cnt) {
+      const uint32_t a = part0 + b * kPartBuf + (uint32_t)slice * (kSubRows * kRows * 4) + (uint32_t)g * 16 + t * 4;
+#pragma unroll
+      for (int bb = 0; bb < 2; bb++)
+#pragma unroll
+        for (int r = 0; r < 2; r++) sts32(a + (bb * 16 + r * 8) * 16, __float_as_uint(acc[bb][r]));
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar_sum + b * 8);
+   }
+    // the slices take turns at finishing the unit before this one, whose last sums have come in meanwhile
+    if (n > 0) {
+      if (turn == slice) finish(n - 1, pj, pcnt, pfirst);
+      turn = turn + 1 == p.slices ? 0 : turn + 1;
+    }
+    pj = j;
+    pcnt = cnt;
+    pfirst = first;
+    if (++j == upr) {
+      j = 0;
+      sub++;
+      fresh = true;
     }
   }
 }
 
-template <bool UP, int FMT>
+template <bool UP, int FMT, int KPW>
 cudaError_t launch_gemv(const GemvParams& p, cudaStream_t st) {
-  // the dynamic allocation must reach the end of the last table, wherever it starts
-  constexpr int kMaxSmem = UP ? kTab1 + 65536 : kTab0 + 65536;
-  const bool two = UP && p.img_sh.data && p.img_sh.dual_book;
-  const int smem = two ? kTab1 + 65536 : kTab0 + 65536;
+  constexpr int smem = Map<FMT, KPW>::kBytes;
   static bool attr_done = false;
   static int sms = 0;
   if (!attr_done) {
-    cudaError_t e = cudaFuncSetAttribute(k_gemv<UP, FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
+    cudaError_t e = cudaFuncSetAttribute(k_gemv<UP, FMT, KPW>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     int dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     attr_done = true;
   }
-  return launch_pdl(k_gemv<UP, FMT>, dim3(sms), dim3(kGemvThreads), (size_t)smem, st, p);
+  return launch_pdl(k_gemv<UP, FMT, KPW>, dim3(sms), dim3(kThreads), (size_t)smem, st, p);
+}
+
+template <bool UP, int FMT>
+cudaError_t launch_fmt(GemvParams& p, cudaStream_t st) {
+  const int KB = p.img.n_kblocks;
+  // The fewest K blocks per warp with which one team covers K, but two at least: more warps at work on a unit beat
+  // longer slices (K = 2560: 14 slices of three 85 us at T = 13, 10 of four 95); at K <= 1024 two and four are level.
+  const int kpw = KB > 48 ? 4 : KB > 32 ? 3 : 2;
+  p.slices = (KB + kpw - 1) / kpw;
+  p.teams = kWarps / p.slices;
+  if (p.teams < 1) return cudaErrorInvalidValue;
+  if (kpw == 4) return launch_gemv<UP, FMT, 4>(p, st);
+  if (kpw == 3) return launch_gemv<UP, FMT, 3>(p, st);
+  return launch_gemv<UP, FMT, 2>(p, st);
+}
+
+// CTAs for the shared expert: its share of the passes that T tokens with even routing make. (Fewer routed
+// passes than that only leave the routed CTAs idle a little earlier.)
+int shared_ctas(int T, int k, int E) {
+  const double idle = 1.0 - (double)k / E;
+  double unused = 1.0;
+  for (int i = 0; i < T; i++) unused *= idle;
+  const double routed = E * (1.0 - unused) * 1.02, shared = (T + kRows - 1) / kRows;
+  const int n = (int)(148.0 * shared / (routed + shared) + 0.5);
+  return n < 1 ? 1 : n > 74 ? 74 : n;
 }
 
 }  // namespace
 
-int gemv_max_runs() { return kGemvMaxRuns; }
-int gemv_max_k() { return kGemvMaxK; }                       // 16 K slices x 4 K blocks
-int gemv_max_mid() { return (kGemvWarps / 2) * kKpw * kTileK; }  // 8 K slices x 4 K blocks = 2048
+int gemv_max_runs() { return 192; }
+int gemv_max_k() { return kWarps * 4 * kTileK; }
+int gemv_max_mid() { return kWarps / 2 * 4 * kTileK; }
 
-cudaError_t launch_up_gemv(const Image& img, const Image* img_sh, const void* x_bf16, int d, int mid,
+cudaError_t launch_up_gemv(const Image& img, const Image* img_sh, const void* x_bf16, int T, int k, int E, int d, int mid,
                            const int32_t* tokidx, const Run* runs, const int32_t* n_runs,
-                           __half* hid16, cudaStream_t st) {
+                           __half* hid16, int32_t* status, cudaStream_t st) {
   GemvParams p{};
   p.img = img;
-  if (img_sh) p.img_sh = *img_sh;
+  if (img_sh) p.img_sh = *img_sh, p.n_sh = shared_ctas(T, k, E);
   p.runs = runs; p.n_runs = n_runs; p.K = d; p.mid = mid;
-  p.x = (const uint16_t*)x_bf16; p.tokidx = tokidx; p.hid = hid16;
-  if (img.fmt == kQ4K) return launch_gemv<true, kQ4K>(p, st);
-  if (img.fmt == kQ51) return launch_gemv<true, kQ51>(p, st);
-  return launch_gemv<true, kQ4CP>(p, st);
+  p.x = (const uint16_t*)x_bf16; p.tokidx = tokidx; p.hid = hid16; p.status = status;
+  if (img.fmt == kQ4K) return launch_fmt<true, kQ4K>(p, st);
+  if (img.fmt == kQ51) return launch_fmt<true, kQ51>(p, st);
+  return launch_fmt<true, kQ4CP>(p, st);
 }
 
-cudaError_t launch_down_gemv(const Image& img, const Image* img_sh, const __half* hid16, int d, int mid,
-                             const Run* runs, const int32_t* n_runs, float* pairs_f32, cudaStream_t st) {
+cudaError_t launch_down_gemv(const Image& img, const Image* img_sh, const __half* hid16, int T, int k, int E, int d, int mid,
+                             const Run* runs, const int32_t* n_runs, float* pairs_f32, int32_t* status, cudaStream_t st) {
   GemvParams p{};
   p.img = img;
-  if (img_sh) p.img_sh = *img_sh;
+  if (img_sh) p.img_sh = *img_sh, p.n_sh = shared_ctas(T, k, E);
   p.runs = runs; p.n_runs = n_runs; p.K = mid; p.mid = mid;
   p.hid = const_cast<__half*>(hid16);
-  p.out = pairs_f32;
-  if (img.fmt == kQ4K) return launch_gemv<false, kQ4K>(p, st);
-  if (img.fmt == kQ51) return launch_gemv<false, kQ51>(p, st);
-  return launch_gemv<false, kQ4CP>(p, st);
+  p.out = pairs_f32; p.status = status;
+  if (img.fmt == kQ4K) return launch_fmt<false, kQ4K>(p, st);
+  if (img.fmt == kQ51) return launch_fmt<false, kQ51>(p, st);
+  return launch_fmt<false, kQ4CP>(p, st);
 }
 
 }  // namespace b200moe

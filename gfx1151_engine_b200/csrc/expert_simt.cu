@@ -27,8 +27,8 @@ template <>
 struct RowMeta<kQ4CP> {
   float s;
   const float* book;
-  __device__ __forceinline__ void load(const uint8_t* meta, int r, int h, const float* bk) {
-    s = half_bits_to_f32(((const uint16_t*)meta)[r * 2 + h]);
+  __device__ __forceinline__ void load(const uint8_t* meta, int h, const float* bk) {
+    s = half_bits_to_f32(((const uint16_t*)meta)[h]);
     book = bk;
   }
   __device__ __forceinline__ float value(int nib, int) const { return __fmul_rn(book[nib], s); }
@@ -36,8 +36,8 @@ struct RowMeta<kQ4CP> {
 template <>
 struct RowMeta<kQ4K> {
   float d1, dm1;
-  __device__ __forceinline__ void load(const uint8_t* meta, int r, int h, const float*) {
-    const uint8_t* m = meta + r * 8;
+  __device__ __forceinline__ void load(const uint8_t* meta, int h, const float*) {
+    const uint8_t* m = meta;
     float d = half_bits_to_f32(*(const uint16_t*)m), dmin = half_bits_to_f32(*(const uint16_t*)(m + 2));
     d1 = __fmul_rn(d, (float)m[4 + 2 * h]);
     dm1 = __fmul_rn(dmin, (float)m[5 + 2 * h]);
@@ -50,8 +50,8 @@ template <>
 struct RowMeta<kQ51> {
   float d, m;
   uint32_t qh;
-  __device__ __forceinline__ void load(const uint8_t* meta, int r, int h, const float*) {
-    const uint8_t* p = meta + r * 16 + h * 8;
+  __device__ __forceinline__ void load(const uint8_t* meta, int h, const float*) {
+    const uint8_t* p = meta + h * 8;
     d = half_bits_to_f32(*(const uint16_t*)p);
     m = half_bits_to_f32(*(const uint16_t*)(p + 2));
     qh = *(const uint32_t*)(p + 4);
@@ -70,12 +70,12 @@ __device__ __forceinline__ void row_dot(const Image& img, int e, int mt, int r, 
   // (a two-plane image of 8-bit codes has 1 << act_shift image K blocks per activation K block)
   for (int kbi = (k0 / kTileK) << img.act_shift; kbi < ((k0 + klen) / kTileK) << img.act_shift; kbi++) {
     const int kb = kbi >> img.act_shift;
-    const uint8_t* tile = img.tile(e, mt, kbi);
+    const uint8_t *codes = img.codes(e, mt, kbi, r), *meta = img.meta(e, mt, kbi, r);
 #pragma unroll
     for (int h = 0; h < 2; h++) {
-      const uint4 c4 = *(const uint4*)(tile + h * 2048 + r * 16);
+      const uint4 c4 = *(const uint4*)(codes + h * kHalfBytes);
       RowMeta<FMT> rm;
-      rm.load(tile + kCodeBytes, r, h, book);
+      rm.load(meta, h, book);
       const uint32_t wds[4] = {c4.x, c4.y, c4.z, c4.w};
       const int xo = kb * kTileK - k0 + h * 32;
 #pragma unroll

@@ -451,14 +451,15 @@ k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ C
         // The dequantising warps fetch their packed weights into registers only one own pair ahead
         // of their use (~18 KB in flight per SM). This thread, which has time to spare, also asks for
         // both tiles of a later pair -- of this item or of the next one -- to be brought into L2
-        // with one bulk prefetch, so that the fetch finds them there. Measured: 6 % on a launch
+        // with bulk prefetches, so that the fetch finds them there. Measured: 6 % on a launch
         // whose tiles all have ~10 rows (short MMAs: the fetch latency shows), nothing on the
         // benchmark's mix; with every weight read served from L2 (a diagnostic run on one expert's
         // tiles) such a launch gains 23 %.
-        constexpr size_t w_tile_b = tile_bytes(FMT);
-        const uint8_t* w_this = img.tile(t.expert, it % img.n_mtiles, 0);
+        constexpr size_t w_sub_b = sub_bytes(FMT);
+        const size_t w_col_b = KB * w_sub_b;  // from one sub-block to the next
+        const uint8_t* w_this = img.mtile(t.expert, it % img.n_mtiles);
         const uint8_t* w_next =
-            it + (int)gridDim.x < n_items ? img.tile(t_ahead.expert, (it + (int)gridDim.x) % img.n_mtiles, 0) : nullptr;
+            it + (int)gridDim.x < n_items ? img.mtile(t_ahead.expert, (it + (int)gridDim.x) % img.n_mtiles) : nullptr;
         for (int pp = 0; pp < NP && ok; pp++, pi++) {
           if (!kNarrow && p.l2_ahead > 0) {
             int q = pp + 2 * p.l2_ahead;
@@ -467,10 +468,13 @@ k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ C
               q -= NP;
               b2 = w_next;
             }
-            if (b2 != nullptr && q < NP)
-              asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(b2 + (size_t)(2 * q) * w_tile_b),
-                           "r"((uint32_t)(min(2, KB - 2 * q) * (int)w_tile_b))
-                           : "memory");
+            if (b2 != nullptr && q < NP) {
+#pragma unroll
+              for (int s = 0; s < kTileM / kSubRows; s++)
+                asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(b2 + s * w_col_b + (size_t)(2 * q) * w_sub_b),
+                             "r"((uint32_t)(min(2, KB - 2 * q) * (int)w_sub_b))
+                             : "memory");
+            }
           }
           // slot = pi % kNBS, sph = (pi / kNBS) & 1, kept as counters (no division in the loop)
           const int nk = min(2, KB - 2 * pp);
@@ -561,29 +565,31 @@ k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ C
     // The fetch stream runs one own pair ahead of the decode. It walks (item, pair) with
     // counters, and the first tile of the NEXT item is looked up when an item is entered,
     // so that no fetch waits for the dependent read of the tile list.
-    constexpr size_t tile_b = tile_bytes(FMT);  // the launcher picks FMT from img.fmt
-    // byte offsets of this thread's reads inside a tile: its 16 code bytes of half 0 and its metadata
-    constexpr int kMetaRow = FMT == kQ4CP ? 4 : FMT == kQ4K ? 8 : 16;
-    const uint32_t off_c = (uint32_t)r * 16u, off_m = (uint32_t)kCodeBytes + (uint32_t)r * kMetaRow;
+    constexpr size_t sub_b = sub_bytes(FMT);  // the launcher picks FMT from img.fmt
+    // this thread's row: its sub-block in an m-tile (K blocks follow one another there), its 16 code bytes of
+    // half 0 and its metadata in that
+    const int pos = tile_pos(r, img.paired);
+    const uint32_t off_c = (uint32_t)code_offset(pos), off_m = (uint32_t)meta_offset(FMT, pos);
+    const size_t row0 = img.row_sub(r) + off_c;
     auto item_base = [&](int io) -> const uint8_t* {
       const int item = blockIdx.x + io * (int)gridDim.x;
       if (io >= my_items) return nullptr;
-      return img.tile(p.tiles[item / img.n_mtiles].expert, item % img.n_mtiles, 0);
+      return img.mtile(p.tiles[item / img.n_mtiles].expert, item % img.n_mtiles) + row0;
     };
     const int io_step = NP == 1 ? 2 : 1;  // a set visits every item, or every other one when an item is one pair
     int f_io = set / NP, f_pp = set % NP;
     const uint8_t* f_base = kNarrow ? nullptr : item_base(f_io);
     const uint8_t* f_next = kNarrow ? nullptr : item_base(f_io + io_step);
-    // f_tile walks with the stream: the tile of K block 2 * f_pp + kblk of the current item
-    const uint8_t* f_tile = f_base ? f_base + (size_t)(2 * f_pp + kblk) * tile_b : nullptr;
-    const size_t step_b = 4 * tile_b;  // the set's next pair is two pairs = four K blocks further
+    // f_tile walks with the stream: this row's codes in K block 2 * f_pp + kblk of the current item
+    const uint8_t* f_tile = f_base ? f_base + (size_t)(2 * f_pp + kblk) * sub_b : nullptr;
+    const size_t step_b = 4 * sub_b;  // the set's next pair is two pairs = four K blocks further
     bool f_valid = false;              // the last fetch had a K block to read (false only beyond an odd tail or the last item)
     auto fetch = [&](uint4& a, uint4& b, RowMetaTc& s2x) {
       f_valid = f_tile != nullptr && 2 * f_pp + kblk < KB;
       if (f_valid) {
-        const uint8_t* pc = f_tile + off_c;  // the metadata sits off_m - off_c bytes further
+        const uint8_t* pc = f_tile;  // the metadata sits off_m - off_c bytes further
         a = __ldg((const uint4*)pc);
-        b = __ldg((const uint4*)(pc + 2048));
+        b = __ldg((const uint4*)(pc + kHalfBytes));
         if (FMT == kQ4CP) {
           s2x.a = __ldg((const uint32_t*)(pc + (off_m - off_c)));
         } else if (FMT == kQ4K) {
@@ -603,7 +609,7 @@ k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ C
         f_io += io_step;
         f_base = f_next;
         f_next = item_base(f_io + io_step);
-        f_tile = f_base ? f_base + (size_t)(2 * f_pp + kblk) * tile_b : nullptr;
+        f_tile = f_base ? f_base + (size_t)(2 * f_pp + kblk) * sub_b : nullptr;
       }
     };
     if (!kNarrow) fetch(ca, cb, sc);
@@ -616,9 +622,9 @@ k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ C
       if (!__all_sync(0xffffffffu, mbar_wait(bars + 8 * (kBarCFull + c_stage), c_ph, abort_flag, p.status, 11))) return false;
       mine = 2 * c_pp + kblk < KB;
       if (mine) {
-        const uint8_t* pc = smem + M::kOffB1 + c_stage * (2 * (uint32_t)tile_b) + kblk * (uint32_t)tile_b + off_c;
+        const uint8_t* pc = smem + M::kOffB1 + c_stage * (8 * (uint32_t)sub_b) + (pos >> 5) * (2 * (uint32_t)sub_b) + kblk * (uint32_t)sub_b + off_c;
         ca = *(const uint4*)pc;
-        cb = *(const uint4*)(pc + 2048);
+        cb = *(const uint4*)(pc + kHalfBytes);
         const uint8_t* pm = pc + (off_m - off_c);
         if (FMT == kQ4CP) {
           sc.a = *(const uint32_t*)pm;
@@ -701,23 +707,26 @@ k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ C
       if (lane == 0) mbar_arrive(bars + 8 * (kBarAFull + aslot));
     }
   } else if (kNarrow && warp == 2) {
-    // ================= producer of packed weights (one bulk copy per pair of K blocks) ==========
+    // ================= producer of packed weights (a bulk copy per sub-block and pair of K blocks) ==========
     if (lane == 0) {
-      constexpr uint32_t w_tile_b = tile_bytes(FMT);
+      constexpr uint32_t w_sub_b = sub_bytes(FMT);
+      const size_t w_col_b = (size_t)KB * w_sub_b;  // from one sub-block to the next
       uint32_t stage = 0, ph = 0;
       bool ok = true;
       Tile t_ahead = (int)blockIdx.x < n_items ? p.tiles[blockIdx.x / img.n_mtiles] : Tile{0, 0, 0};
       for (int it = blockIdx.x; it < n_items && ok; it += gridDim.x) {
-        const uint8_t* src = img.tile(t_ahead.expert, it % img.n_mtiles, 0);
+        const uint8_t* src = img.mtile(t_ahead.expert, it % img.n_mtiles);
         if (it + (int)gridDim.x < n_items) t_ahead = p.tiles[(it + gridDim.x) / img.n_mtiles];
-        for (int pp = 0; pp < NP; pp++, src += 2 * w_tile_b) {
+        for (int pp = 0; pp < NP; pp++, src += 2 * w_sub_b) {
           ok = mbar_wait(bars + 8 * (kBarCEmpty + stage), ph ^ 1, abort_flag, p.status, 12, 64);
           if (!ok) break;
-          const uint32_t bytes = (uint32_t)min(2, KB - 2 * pp) * w_tile_b, bar = bars + 8 * (kBarCFull + stage);
-          mbar_expect_tx(bar, bytes);
-          asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                           (uint32_t)M::kOffB1 + stage * (2 * w_tile_b)), "l"(src), "r"(bytes), "r"(bar)
-                       : "memory");
+          const uint32_t bytes = (uint32_t)min(2, KB - 2 * pp) * w_sub_b, bar = bars + 8 * (kBarCFull + stage);
+          mbar_expect_tx(bar, kTileM / kSubRows * bytes);
+#pragma unroll
+          for (int s = 0; s < kTileM / kSubRows; s++)
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                             (uint32_t)M::kOffB1 + stage * (8 * w_sub_b) + s * (2 * w_sub_b)), "l"(src + s * w_col_b), "r"(bytes), "r"(bar)
+                         : "memory");
           if (++stage == (uint32_t)kNST) {
             stage = 0;
             ph ^= 1;

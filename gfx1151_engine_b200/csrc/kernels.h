@@ -122,18 +122,18 @@ cudaError_t launch_down_simt(const Image& img, const float* hid_f32, int d, int 
                              const int32_t* n_runs, int max_runs, float* pairs_f32,
                              cudaStream_t st);
 
-// ---- expert_gemv.cu (q4cp decode / verify path) ----
+// ---- expert_gemv.cu (decode / verify path) ----
 int gemv_max_runs();
 int gemv_max_k();     // largest d
 int gemv_max_mid();   // largest mid
 // img_sh: the shared expert's image (nullptr: none); its run is runs[kMaxExperts].
 // hid16: fp16 [rows][mid] hidden activations silu(gate) * up, written by the gate/up kernel and
 // read by the down kernel.
-cudaError_t launch_up_gemv(const Image& img, const Image* img_sh, const void* x_bf16, int d, int mid,
+cudaError_t launch_up_gemv(const Image& img, const Image* img_sh, const void* x_bf16, int T, int k, int E, int d, int mid,
                            const int32_t* tokidx, const Run* runs, const int32_t* n_runs,
-                           __half* hid16, cudaStream_t st);
-cudaError_t launch_down_gemv(const Image& img, const Image* img_sh, const __half* hid16, int d, int mid,
-                             const Run* runs, const int32_t* n_runs, float* pairs_f32, cudaStream_t st);
+                           __half* hid16, int32_t* status, cudaStream_t st);
+cudaError_t launch_down_gemv(const Image& img, const Image* img_sh, const __half* hid16, int T, int k, int E, int d, int mid,
+                             const Run* runs, const int32_t* n_runs, float* pairs_f32, int32_t* status, cudaStream_t st);
 
 // ---- decode.cu (q4cp decode / verify, T <= decode_max_tokens(), as one kernel) ----
 // Routing (from logits, or from the caller's ids / w when logits is null), gate/up GEMV + SwiGLU,

@@ -34,23 +34,22 @@ __global__ void k_repack_q4cp(Image img, SrcTensor a, SrcTensor b, int K, int fi
     long long t2 = t / img.n_kblocks;
     int mt = (int)(t2 % img.n_mtiles);
     int e = (int)(t2 / img.n_mtiles);
-    uint8_t* dst = const_cast<uint8_t*>(img.tile(e, mt, kb));
     const SrcTensor* s;
     if (j < 256) {
       int h = j >> 7, r = j & 127;
       long long row = src_row(img, a, b, emap ? emap[e + first_expert] : e + first_expert, mt, r, &s);
       const uint4* src = (const uint4*)(s->codes + row * (K / 2) + kb * 32 + h * 16);
-      *(uint4*)(dst + h * 2048 + r * 16) = *src;
+      *(uint4*)(img.codes(e, mt, kb, r) + h * kHalfBytes) = *src;
     } else {
       int r = j - 256;
       long long row = src_row(img, a, b, emap ? emap[e + first_expert] : e + first_expert, mt, r, &s);
       if (s->scale_group == 128) {
         // hgn v2 i4r: one fp16 scale per 128 columns serves both 32-groups of two K blocks
         const uint32_t v = *(const uint16_t*)(s->scales + row * s->scale_stride + (kb >> 1) * 2);
-        *(uint32_t*)(dst + kCodeBytes + r * 4) = v | (v << 16);
+        *(uint32_t*)img.meta(e, mt, kb, r) = v | (v << 16);
       } else {
         const uint32_t* src = (const uint32_t*)(s->scales + row * s->scale_stride + kb * 4);
-        *(uint32_t*)(dst + kCodeBytes + r * 4) = *src;
+        *(uint32_t*)img.meta(e, mt, kb, r) = *src;
       }
     }
   }
@@ -80,7 +79,6 @@ __global__ void k_repack_q4k(Image img, SrcTensor a, SrcTensor b, int K, int fir
     long long t2 = t / img.n_kblocks;
     int mt = (int)(t2 % img.n_mtiles);
     int e = (int)(t2 / img.n_mtiles);
-    uint8_t* dst = const_cast<uint8_t*>(img.tile(e, mt, kb));
     const SrcTensor* s;
     long long row = src_row(img, a, b, emap ? emap[e + first_expert] : e + first_expert, mt, r, &s);
     const uint8_t* blk = s->codes + row * row_bytes + (long long)(kb >> 2) * 144;
@@ -93,12 +91,12 @@ __global__ void k_repack_q4k(Image img, SrcTensor a, SrcTensor b, int K, int fir
       lo[q] = (uint8_t)((c0 & 15) | ((c1 & 15) << 4));
       hi[q] = (uint8_t)((c0 >> 4) | ((c1 >> 4) << 4));
     }
-    *(uint4*)(dst + r * 16) = *(uint4*)lo;
-    *(uint4*)(dst + 2048 + r * 16) = *(uint4*)hi;
+    *(uint4*)img.codes(e, mt, kb, r) = *(uint4*)lo;
+    *(uint4*)(img.codes(e, mt, kb, r) + kHalfBytes) = *(uint4*)hi;
     uint8_t s0, m0, s1, m1;
     k4_scale_min(2 * sub, blk + 4, s0, m0);
     k4_scale_min(2 * sub + 1, blk + 4, s1, m1);
-    uint8_t* meta = dst + kCodeBytes + r * 8;
+    uint8_t* meta = img.meta(e, mt, kb, r);
     meta[0] = blk[0];
     meta[1] = blk[1];
     meta[2] = blk[2];
@@ -126,7 +124,6 @@ __global__ void k_repack_q51(Image img, SrcTensor a, SrcTensor b, int K, int fir
     long long t2 = t / img.n_kblocks;
     int mt = (int)(t2 % img.n_mtiles);
     int e = (int)(t2 / img.n_mtiles);
-    uint8_t* dst = const_cast<uint8_t*>(img.tile(e, mt, kb));
     const SrcTensor* s;
     long long row = src_row(img, a, b, emap ? emap[e + first_expert] : e + first_expert, mt, r, &s);
     const uint8_t* blk = s->codes + row * row_bytes + (long long)(kb * 2 + h) * 24;
@@ -137,8 +134,8 @@ __global__ void k_repack_q51(Image img, SrcTensor a, SrcTensor b, int K, int fir
       out[q] = (uint8_t)((qs[2 * q] & 15) | ((qs[2 * q + 1] & 15) << 4));
       out[q + 8] = (uint8_t)((qs[2 * q] >> 4) | ((qs[2 * q + 1] >> 4) << 4));
     }
-    *(uint4*)(dst + h * 2048 + r * 16) = *(uint4*)out;
-    uint8_t* meta = dst + kCodeBytes + r * 16 + h * 8;
+    *(uint4*)(img.codes(e, mt, kb, r) + h * kHalfBytes) = *(uint4*)out;
+    uint8_t* meta = img.meta(e, mt, kb, r) + h * 8;
 #pragma unroll
     for (int q = 0; q < 4; q++) meta[q] = blk[q];
     // the image keeps the block's element order (code byte i = elements 2i, 2i+1), and bit j of the
@@ -165,7 +162,6 @@ __global__ void k_repack_q5k(Image img, SrcTensor a, SrcTensor b, int K, int fir
     long long t2 = t / img.n_kblocks;
     int mt = (int)(t2 % img.n_mtiles);
     int e = (int)(t2 / img.n_mtiles);
-    uint8_t* dst = const_cast<uint8_t*>(img.tile(e, mt, kb));
     const SrcTensor* s;
     long long row = src_row(img, a, b, emap ? emap[e + first_expert] : e + first_expert, mt, r, &s);
     const uint8_t* blk = s->codes + row * row_bytes + (long long)(kb >> 2) * 176;
@@ -181,12 +177,12 @@ __global__ void k_repack_q5k(Image img, SrcTensor a, SrcTensor b, int K, int fir
     }
 #pragma unroll
     for (int l = 0; l < 32; l++) fifth |= (uint32_t)((qh[l] >> (2 * sub + h)) & 1) << l;
-    *(uint4*)(dst + h * 2048 + r * 16) = *(uint4*)out;
+    *(uint4*)(img.codes(e, mt, kb, r) + h * kHalfBytes) = *(uint4*)out;
     uint8_t sc, mn;
     k4_scale_min(2 * sub + h, blk + 4, sc, mn);
     const float d = half_bits_to_f32((uint16_t)(blk[0] | (blk[1] << 8)));
     const float dmin = half_bits_to_f32((uint16_t)(blk[2] | (blk[3] << 8)));
-    uint8_t* meta = dst + kCodeBytes + r * 16 + h * 8;
+    uint8_t* meta = img.meta(e, mt, kb, r) + h * 8;
     *(__half*)meta = __float2half_rn(__fmul_rn(d, (float)sc));
     *(__half*)(meta + 2) = __float2half_rn(-__fmul_rn(dmin, (float)mn));
     *(uint32_t*)(meta + 4) = fifth_bits_split(fifth);
@@ -213,7 +209,6 @@ __global__ void k_repack_iq4(Image img, SrcTensor a, SrcTensor b, int K, int fir
     long long t2 = t / img.n_kblocks;
     int mt = (int)(t2 % img.n_mtiles);
     int e = (int)(t2 / img.n_mtiles);
-    uint8_t* dst = const_cast<uint8_t*>(img.tile(e, mt, kb));
     const SrcTensor* s;
     long long row = src_row(img, a, b, emap ? emap[e + first_expert] : e + first_expert, mt, r, &s);
     const int blk32 = kb * 2 + h;  // 32-element block of the row
@@ -240,8 +235,8 @@ __global__ void k_repack_iq4(Image img, SrcTensor a, SrcTensor b, int K, int fir
       out[q] = (uint8_t)((qs[2 * q] & 15) | ((qs[2 * q + 1] & 15) << 4));
       out[q + 8] = (uint8_t)((qs[2 * q] >> 4) | ((qs[2 * q + 1] >> 4) << 4));
     }
-    *(uint4*)(dst + h * 2048 + r * 16) = *(uint4*)out;
-    ((__half*)(dst + kCodeBytes))[r * 2 + h] = __float2half_rn(scale);
+    *(uint4*)(img.codes(e, mt, kb, r) + h * kHalfBytes) = *(uint4*)out;
+    ((__half*)img.meta(e, mt, kb, r))[h] = __float2half_rn(scale);
   }
 }
 
@@ -262,7 +257,6 @@ __global__ void k_repack_q80(Image img, SrcTensor a, SrcTensor b, int K, int fir
     int mt = (int)(t2 % img.n_mtiles);
     int e = (int)(t2 / img.n_mtiles);
     const int kb = kbi >> 1, plane = kbi & 1;  // plane 0: high nibbles, 1: low nibbles
-    uint8_t* dst = const_cast<uint8_t*>(img.tile(e, mt, kbi));
     const SrcTensor* s;
     long long row = src_row(img, a, b, emap ? emap[e + first_expert] : e + first_expert, mt, r, &s);
     const uint8_t* blk = s->codes + row * row_bytes + (long long)(kb * 2 + h) * 34;
@@ -273,9 +267,9 @@ __global__ void k_repack_q80(Image img, SrcTensor a, SrcTensor b, int K, int fir
       const int u0 = (int)qs[2 * q] + 128, u1 = (int)qs[2 * q + 1] + 128;
       out[q] = plane ? (uint8_t)((u0 & 15) | ((u1 & 15) << 4)) : (uint8_t)((u0 >> 4) | ((u1 >> 4) << 4));
     }
-    *(uint4*)(dst + h * 2048 + r * 16) = *(uint4*)out;
+    *(uint4*)(img.codes(e, mt, kbi, r) + h * kHalfBytes) = *(uint4*)out;
     const float d = half_bits_to_f32((uint16_t)(blk[0] | (blk[1] << 8)));
-    uint8_t* meta = dst + kCodeBytes + r * 16 + h * 8;
+    uint8_t* meta = img.meta(e, mt, kbi, r) + h * 8;
     *(__half*)meta = __float2half_rn(plane ? d : __fmul_rn(d, 16.f));
     *(__half*)(meta + 2) = __float2half_rn(plane ? 0.f : __fmul_rn(d, -128.f));
     *(uint32_t*)(meta + 4) = 0u;
@@ -309,31 +303,29 @@ __global__ void k_dequant_rows(Image img, int expert, int row0, int nrows, int m
     if (img.act_shift) {
       // Q8_0 in two planes: put the code together again and multiply once, as the reference
       // does (y = d * q, src/gguf.h:352-359)
-      const uint8_t* hi = img.tile(expert, mt, 2 * kb);
-      const uint8_t* lo = img.tile(expert, mt, 2 * kb + 1);
-      const uint8_t bh = hi[h * 2048 + r * 16 + j / 2], bl = lo[h * 2048 + r * 16 + j / 2];
+      const int at = h * kHalfBytes + j / 2;
+      const uint8_t bh = img.codes(expert, mt, 2 * kb, r)[at], bl = img.codes(expert, mt, 2 * kb + 1, r)[at];
       const int q = 16 * ((j & 1) ? (bh >> 4) : (bh & 15)) + ((j & 1) ? (bl >> 4) : (bl & 15)) - 128;
-      const float d = half_bits_to_f32(*(const uint16_t*)(lo + kCodeBytes + r * 16 + h * 8));
+      const float d = half_bits_to_f32(*(const uint16_t*)(img.meta(expert, mt, 2 * kb + 1, r) + h * 8));
       out[i] = __fmul_rn(d, (float)q);
       continue;
     }
-    const uint8_t* tile = img.tile(expert, mt, kb);
-    uint8_t byte = tile[h * 2048 + r * 16 + j / 2];
+    uint8_t byte = img.codes(expert, mt, kb, r)[h * kHalfBytes + j / 2];
     int nib = (j & 1) ? (byte >> 4) : (byte & 15);
-    const uint8_t* meta = tile + kCodeBytes;
+    const uint8_t* meta = img.meta(expert, mt, kb, r);
     float v;
     if (img.fmt == kQ4CP) {
-      float s = half_bits_to_f32(((const uint16_t*)meta)[r * 2 + h]);
+      float s = half_bits_to_f32(((const uint16_t*)meta)[h]);
       v = __fmul_rn(img.book[(r >= 64 ? 16 : 0) + nib], s);
     } else if (img.fmt == kQ4K) {
-      const uint8_t* m = meta + r * 8;
+      const uint8_t* m = meta;
       float d = half_bits_to_f32(*(const uint16_t*)m);
       float dmin = half_bits_to_f32(*(const uint16_t*)(m + 2));
       float d1 = __fmul_rn(d, (float)m[4 + 2 * h]);
       float dm1 = __fmul_rn(dmin, (float)m[5 + 2 * h]);
       v = __fsub_rn(__fmul_rn(d1, (float)nib), dm1);
     } else {
-      const uint8_t* m = meta + r * 16 + h * 8;
+      const uint8_t* m = meta + h * 8;
       float d = half_bits_to_f32(*(const uint16_t*)m);
       float mn = half_bits_to_f32(*(const uint16_t*)(m + 2));
       uint32_t qh = *(const uint32_t*)(m + 4);
