@@ -317,6 +317,8 @@ int b200moe_create(const b200moe_config* cfg, b200moe_handle* out) {
   A(&h->status_dev, 4);
   h->rb.status = h->status_dev;
   if (e == cudaSuccess) e = cudaMemset(h->status_dev, 0, 16);
+  A(&h->rb.ready, 1);
+  if (e == cudaSuccess) e = cudaMemset(h->rb.ready, 0, sizeof(int32_t));
   A(&h->grid_bar, 2);
   if (e == cudaSuccess) e = cudaMemset(h->grid_bar, 0, 16);
   if (getenv("B200MOE_DECODE_TRACE")) {
@@ -691,10 +693,16 @@ int b200moe_route(b200moe_handle h, const int32_t* topids_dev, const float* topw
   return B200MOE_OK;
 }
 
-// logits != nullptr: the router has not run yet (the fused small-T routing kernel runs it).
+static bool fused_decode(const b200moe_config& c) {
+  static const bool env = getenv("B200MOE_FUSED_DECODE") != nullptr && atoi(getenv("B200MOE_FUSED_DECODE")) != 0;
+  return env || c.decode_impl == B200MOE_DECODE_FUSED;
+}
+
+// logits != nullptr: the router has not run yet (the fused small-T routing kernel runs it; with router_w it first
+// puts near-ties of these logits, its own buffer then, into the reference's arithmetic).
 static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const int32_t* ids,
                         const float* w, int stride, void* out, cudaStream_t st,
-                        bool router_timed = false, const float* logits = nullptr) {
+                        bool router_timed = false, const float* logits = nullptr, const uint16_t* router_w = nullptr) {
   const b200moe_config& c = h->cfg;
   LayerWeights& L = h->layers[layer];
   const int k = c.topk, E = c.experts, d = c.d_model, mid = c.d_mid;
@@ -712,8 +720,7 @@ static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const
   // once for all its rows): opt-in with decode_impl = B200MOE_DECODE_FUSED in the configuration or B200MOE_FUSED_DECODE=1. Measured slower than the
   // separate kernels (whose launches overlap through programmatic dependent launch), so they
   // stay the default.
-  static const bool fused_env = getenv("B200MOE_FUSED_DECODE") != nullptr && atoi(getenv("B200MOE_FUSED_DECODE")) != 0;
-  const bool fused = fused_env || c.decode_impl == B200MOE_DECODE_FUSED;
+  const bool fused = fused_decode(c);
   if (L.i4r && (c.gemm_impl == B200MOE_GEMM_SIMT || !h->tc))
     return fail(h, B200MOE_ERR_UNSUPPORTED, "forward: hgn v2 i4r layers run on the tensor-core path only");
   if (fused && !L.i4r && c.gemm_impl == B200MOE_GEMM_AUTO && T <= h->decode_max && T <= decode_max_tokens() &&
@@ -738,15 +745,20 @@ static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const
   const bool split = few && T > 16 && T * k * 2 >= min_saved * (2 * kTcNarrowN + 1), narrow = few && !split;
   const bool sh_narrow = few && (long long)(T / kTcNarrowN) * (mid / 64) <= kSharedNarrowItems;
   const TileCut cut{narrow ? kTcNarrowN : h->tile_cap, sh_narrow ? kTcNarrowN : h->tile_cap, split ? kTcNarrowN : 0, min_saved};
+  // (the shared expert's images are q4cp: it can ride along only with q4cp routed experts)
+  const bool gemv = simt && c.gemm_impl == B200MOE_GEMM_AUTO &&
+                    (!shared || (L.gu.fmt == kQ4CP && L.dn.fmt == kQ4CP)) &&
+                    T * k + (shared ? T : 0) <= h->dec_rows && std::min(E, T * k) + 1 <= gemv_max_runs() &&
+                    (d << L.gu.act_shift) <= gemv_max_k() && (mid << L.dn.act_shift) <= gemv_max_mid() && d % 32 == 0 &&
+                    mid % 32 == 0;
   const uint16_t* gate_w = nullptr;  // set: the shared expert's gate is still to be computed
-  static const bool slow_router = getenv("B200MOE_EXACT_ROUTER") != nullptr;  // A/B: the general routing body for every call
-  if (logits && !slow_router && T <= decode_max_tokens() && T * k <= 128 && d % 8 == 0 && (!shared || ((uintptr_t)x & 15) == 0)) {
-    // decode / verify: the compact router (ids from the logits' order, general body only on a near-tie)
-    CU_TRY(h, launch_route_fast(h->rb, logits, T, k, E, x, shared ? L.sh_gate_w : nullptr, d, cut.routed, st));
-    n++;
-  } else if (T * k <= route_small_max_pairs() && T <= 16) {
-    CU_TRY(h, launch_route_small(h->rb, logits, ids, w, stride, T, k, E, x, shared ? L.sh_gate_w : nullptr,
-                                 d, cut.routed, st));
+  static const bool slow_router = getenv("B200MOE_EXACT_ROUTER") != nullptr;  // A/B: the general routing body for every token
+  const bool in_block = route_block_supported(T, k);
+  RouteIn route{logits, ids, w, stride, router_w, (const uint16_t*)x, shared ? L.sh_gate_w : nullptr, T, E, k, d, cut.routed, slow_router, h->rb};
+  if (gemv && in_block) {
+    // (the gate/up kernel routes)
+  } else if (in_block) {
+    CU_TRY(h, launch_route_block(route, st));
     n++;
   } else {
     if (logits) {
@@ -768,23 +780,17 @@ static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const
   const int pairs = T * k;
   if (simt && c.gemm_impl != B200MOE_GEMM_SIMT && T > h->decode_max)
     return fail(h, B200MOE_ERR_BAD_ARG, "forward: T exceeds the GEMV path's workspace");
-  // (the shared expert's images are q4cp: it can ride along only with q4cp routed experts)
-  const bool gemv = simt && c.gemm_impl == B200MOE_GEMM_AUTO &&
-                    (!shared || (L.gu.fmt == kQ4CP && L.dn.fmt == kQ4CP)) &&
-                    pairs + (shared ? T : 0) <= h->dec_rows && std::min(E, pairs) + 1 <= gemv_max_runs() &&
-                    (d << L.gu.act_shift) <= gemv_max_k() && (mid << L.dn.act_shift) <= gemv_max_mid() && d % 32 == 0 &&
-                    mid % 32 == 0;
   if (gemv) {
     // decode / verify: persistent dequant GEMV, routed and shared expert in one launch each
     if (ev) CU_TRY(h, cudaEventRecord(ev[2], st));
     CU_TRY(h, launch_up_gemv(L.gu, shared ? &L.sh_gu : nullptr, x, T, k, E, d, mid, h->rb.tokidx, h->rb.runs,
-                             h->rb.n_runs, (__half*)h->hid, h->status_dev, st));
+                             h->rb.n_runs, (__half*)h->hid, h->status_dev, in_block ? &route : nullptr, st));
     if (ev) CU_TRY(h, cudaEventRecord(ev[3], st));
     CU_TRY(h, launch_down_gemv(L.dn, shared ? &L.sh_dn : nullptr, (const __half*)h->hid, T, k, E, d, mid,
-                               h->rb.runs, h->rb.n_runs, (float*)h->pairs, h->status_dev, st));
+                               h->rb.runs, h->rb.n_runs, (float*)h->pairs, h->status_dev, in_block ? h->rb.ready : nullptr, st));
     if (ev) CU_TRY(h, cudaEventRecord(ev[4], st));
     CU_TRY(h, launch_combine_f32((const float*)h->pairs, h->rb.pw, h->rb.pairids, T, k, d,
-                                 shared ? pairs : -1, out, st, h->hc_w4, h->hc_state));
+                                 shared ? pairs : -1, out, st, h->hc_w4, h->hc_state, in_block ? h->rb.ready : nullptr));
     n += 3;
   } else if (simt) {
     const int max_runs = std::min(E, pairs);
@@ -950,6 +956,16 @@ int b200moe_forward_hidden(b200moe_handle h, int layer, const void* x_bf16_dev, 
   if (!x_bf16_dev || !out_bf16_dev || T < 0 || T > h->cfg.max_tokens)
     return fail(h, B200MOE_ERR_BAD_ARG, "forward_hidden: bad argument (null pointer or T out of range)");
   if (T == 0) return B200MOE_OK;
+  const b200moe_config& c = h->cfg;
+  LayerWeights& L = h->layers[layer];
+  if (L.router_w && route_block_supported(T, c.topk) && !fused_decode(c)) {
+    // few tokens: the routing kernel itself looks for near-ties (router_logits: two kernels and a memset more)
+    cudaStream_t st = (cudaStream_t)stream;
+    CU_TRY(h, launch_router_dots(x_bf16_dev, L.router_w, T, c.experts, c.d_model, h->router_logits, st));
+    h->launches++;
+    if (h->prof) CU_TRY(h, cudaEventRecord(h->prof_ev[(size_t)h->prof_head * kProfEvents], st));
+    return forward_impl(h, layer, x_bf16_dev, T, h->rb.topids, h->rb.topw, kIdStride, out_bf16_dev, st, h->prof, h->router_logits, L.router_w);
+  }
   if (int s = b200moe_router_logits(h, layer, x_bf16_dev, T, h->router_logits, stream)) return s;
   return b200moe_forward(h, layer, x_bf16_dev, T, h->router_logits, out_bf16_dev, stream);
 }

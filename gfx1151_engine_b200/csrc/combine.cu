@@ -142,11 +142,12 @@ k_combine(const TP* __restrict__ pairs, const float* __restrict__ pw,
 __global__ void __launch_bounds__(128)
 k_combine_small(const float* __restrict__ pairs, const float* __restrict__ pw,
                 const int32_t* __restrict__ pairids, int k, int d, int shared_row0,
-                __nv_bfloat16* __restrict__ out, HcWriteBack hc) {
+                __nv_bfloat16* __restrict__ out, HcWriteBack hc, int32_t* ready) {
   const int t = blockIdx.x;
   const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
   pdl_trigger();
   pdl_wait();
+  if (ready && (t | blockIdx.y | threadIdx.x) == 0) *ready = 0;  // the lists are about to be free for the next call
   if (c >= d) return;
   const int n = k + (shared_row0 >= 0 ? 1 : 0);
   float4 v[kMaxTopK + 1];
@@ -250,11 +251,11 @@ k_scatter_f16(const uint16_t* __restrict__ x, const int32_t* __restrict__ pairid
 
 cudaError_t launch_combine_f32(const float* pairs, const float* pw, const int32_t* pairids, int T,
                                int k, int d, int shared_row0, void* out_bf16, cudaStream_t st,
-                               const float* hc_w4, void* hc_state) {
+                               const float* hc_w4, void* hc_state, int32_t* ready) {
   const HcWriteBack hc{hc_w4, (uint16_t*)hc_state};
   if (T <= 64 && d % 4 == 0)
     return launch_pdl(k_combine_small, dim3(T, (d / 4 + 127) / 128), dim3(128), 0, st, pairs, pw, pairids, k, d, shared_row0,
-                      (__nv_bfloat16*)out_bf16, hc);
+                      (__nv_bfloat16*)out_bf16, hc, ready);
   else
     return launch_pdl(k_combine<float>, dim3(T, (d + 2047) / 2048), dim3(256), 0, st, pairs, pw, pairids, k, d, shared_row0,
                       (__nv_bfloat16*)out_bf16, hc, nullptr);

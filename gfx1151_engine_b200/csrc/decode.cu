@@ -1033,84 +1033,12 @@ k_decode(const DecParams p) {
 }
 
 
-// The same routing as a kernel of its own, for the decode path that keeps the GEMVs and the
-// combine as separate kernels: 512 threads select and bucket, 512 threads form the shared
-// expert's gate. Writes what k_route_small writes.
-struct RouteFastParams {
-  const float* logits;
-  const uint16_t* x;
-  const uint16_t* gate_w;  // null: no shared expert
-  int T, E, k, d, tile_cap;
-  RouteBuffers rb;
-};
-
-__global__ void __launch_bounds__(kDecThreads, 1)
-k_route_fast(const RouteFastParams q) {
-  extern __shared__ __align__(16) uint8_t rsm[];
-  FastScratch& fs = *(FastScratch*)rsm;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int T = q.T, P = q.T * q.k, d = q.d;
-  DecParams p{};  // the fields the routing pieces read
-  p.logits = q.logits; p.x = q.x; p.gate_w = q.gate_w; p.T = q.T; p.E = q.E; p.k = q.k; p.d = q.d; p.tile_cap = q.tile_cap;
-  p.status = q.rb.status;
-  pdl_trigger();
-  pdl_wait();  // inputs may come from the previous kernel; the buffers written here may still be read by it
-  if (warp < 16) {
-    RouteSmallOut out, none;
-    out.topids = q.rb.topids; out.topw = q.rb.topw; out.tokidx = q.rb.tokidx; out.pw = q.rb.pw;
-    out.pairids = q.rb.pairids; out.eoff = q.rb.eoff; out.runs = q.rb.runs; out.shared_slot = kMaxExperts;
-    out.n_runs = q.rb.n_runs; out.tiles = q.rb.tiles; out.tiles_sh = q.rb.tiles_sh; out.n_tiles = q.rb.n_tiles;
-    if (route_fast_select(p, fs, out)) {
-      // (loc and glob are the same arrays here: the placement writes each result twice, harmlessly)
-      route_fast_place(p, fs, out, out);
-    } else {
-      RouteOuts ro;
-      ro.loc = out;
-      ro.glob = none;
-      route_exact(p, (RouteSmallScratch<kDecMaxT>*)(rsm + sizeof(FastScratch)), &ro, q.rb.status);
-    }
-  } else if (q.gate_w) {
-    const int gtid = tid - 512, gw = warp - 16;
-#pragma unroll 1
-    for (int t = 0; t < T; t++) {
-      double a = 0;
-      const uint4* xv = (const uint4*)(q.x + (size_t)t * d);
-      const uint4* gv = (const uint4*)q.gate_w;
-#pragma unroll 1
-      for (int c = gtid; c < d / 8; c += 512) {
-        const uint4 xa = xv[c], ga = __ldg(gv + c);
-        const uint32_t xw[4] = {xa.x, xa.y, xa.z, xa.w}, gq[4] = {ga.x, ga.y, ga.z, ga.w};
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-          a += (double)__uint_as_float(gq[i] << 16) * (double)__uint_as_float(xw[i] << 16);
-          a += (double)__uint_as_float(gq[i] & 0xFFFF0000u) * (double)__uint_as_float(xw[i] & 0xFFFF0000u);
-        }
-      }
-#pragma unroll
-      for (int o = 16; o; o >>= 1)
-        a += __hiloint2double(__shfl_xor_sync(0xffffffffu, __double2hiint(a), o),
-                              __shfl_xor_sync(0xffffffffu, __double2loint(a), o));
-      if (lane == 0) fs.gpart[t][gw] = a;
-    }
-  }
-  __syncthreads();
-  if (q.gate_w && tid < T) {
-    double tot = 0;
-#pragma unroll 1
-    for (int w2 = 0; w2 < 16; w2++) tot += fs.gpart[tid][w2];
-    const float gate = sigmoid_f32((float)tot);
-    q.rb.sgate[tid] = gate;
-    q.rb.tokidx[P + tid] = tid;
-    q.rb.pw[P + tid] = gate;
-  }
-}
-
 }  // namespace
 
 int decode_max_tokens() { return kDecMaxT; }
 
 bool decode_supported(const Image& gu, const Image& dn, const Image* sh_gu, const Image* sh_dn, int T, int k, int E, int d, int mid) {
-  if (T < 1 || T > kDecMaxT || T * k > kDecMaxPairs || T * k > route_small_max_pairs() || E > kMaxExperts) return false;
+  if (T < 1 || T > kDecMaxT || T * k > kDecMaxPairs || T * k > kSmallPairs || E > kMaxExperts) return false;
   if (gu.fmt != kQ4CP || dn.fmt != kQ4CP || gu.dual_book) return false;
   if (sh_gu && (sh_gu->fmt != kQ4CP || !sh_dn || sh_dn->fmt != kQ4CP)) return false;
   return d % 128 == 0 && mid % 64 == 0;
@@ -1143,27 +1071,10 @@ cudaError_t launch_decode(const Image& gu, const Image& dn, const Image* sh_gu, 
   p.logits = logits; p.ids = ids; p.w = w; p.stride = stride;
   p.x = (const uint16_t*)x_bf16; p.gate_w = gate_w;
   p.T = T; p.E = E; p.k = k; p.d = d; p.mid = mid;
-  p.tile_cap = route_small_max_pairs();  // (nothing reads this kernel's work list)
+  p.tile_cap = kSmallPairs;  // (nothing reads this kernel's work list)
   p.hid = hid16; p.out = (uint16_t*)out_bf16; p.hc_w4 = hc_w4; p.hc_state = (uint16_t*)hc_state;
   p.rb = rb; p.bar = bar; p.status = status; p.trace = trace;
   return launch_pdl(k_decode, dim3(sms), dim3(kDecThreads), (size_t)smem, st, p);
-}
-
-
-// Routing stage of a decode call (logits given, T <= decode_max_tokens(), T*k <= 128) in one launch;
-// same outputs as launch_route_small.
-cudaError_t launch_route_fast(const RouteBuffers& rb, const float* logits, int T, int k, int E, const void* x_bf16,
-                              const uint16_t* gate_w_bf16, int d, int tile_cap, cudaStream_t st) {
-  static bool attr_done = false;
-  const int smem = (int)(sizeof(FastScratch) + sizeof(RouteSmallScratch<kDecMaxT>));
-  if (!attr_done) {
-    cudaError_t e = cudaFuncSetAttribute(k_route_fast, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    attr_done = true;
-  }
-  RouteFastParams q{};
-  q.logits = logits; q.x = (const uint16_t*)x_bf16; q.gate_w = gate_w_bf16; q.T = T; q.E = E; q.k = k; q.d = d; q.tile_cap = tile_cap; q.rb = rb;
-  return launch_pdl(k_route_fast, dim3(1), dim3(kDecThreads), (size_t)smem, st, q);
 }
 
 }  // namespace b200moe

@@ -29,6 +29,7 @@
 // 120 / 80, T = 13 288 / 177 (gate/up 4.85 TB/s); Q4_K / Q5_1 T = 5 128 / 88 (gate/up 5.0 TB/s, down 4.0: the
 // fifth bits); 64 experts of 2048 x 512, 16 tokens (2.2 rows an expert) 90 / 33.
 #include "kernels.h"
+#include "route_block.cuh"
 
 namespace b200moe {
 
@@ -36,15 +37,15 @@ namespace {
 
 constexpr int kWarps = 16;            // compute warps of a CTA
 constexpr int kThreads = kWarps * 32;
-constexpr int kRows = 4;              // rows of an expert that one pass over its weights serves
-constexpr int kRed = 4;               // partial-sum buffers of a team
-constexpr int kMaxSubs = 448;         // passes: every expert's rows in fours
+constexpr int kMaxSubs = 448;         // passes over an expert's weights
 constexpr uint32_t kOffLow = 2048;    // the dynamic allocation must start at or below this (its absolute shared address)
 
 // Shared memory map, absolute shared addresses.
 // KPW: K blocks of a slice, at most.
 template <int FMT, int KPW>
 struct Map {
+  static constexpr int kRows = FMT == kQ4CP ? 8 : 4;  // rows of an expert that one pass over its weights serves
+  static constexpr int kRed = FMT == kQ4CP ? 2 : 4;   // partial-sum buffers of a team
   static constexpr int kGroup = KPW == 4 ? 2 : KPW;   // K blocks per ring slot
   static constexpr int kGroups = KPW / kGroup;        // slots per unit
   static constexpr uint32_t kLut = kOffLow;  // kQ4CP: 256 lines of {32 lanes x 4 B, first book}{32 x 4 B, second book}
@@ -52,13 +53,14 @@ struct Map {
   static constexpr uint32_t kSub = (uint32_t)sub_bytes(FMT), kSlot = kGroup * kSub;
   static constexpr uint32_t kSlots = KPW == 3 ? 2 : 3;  // per warp
   static constexpr uint32_t kScr = FMT == kQ4K ? 512 : 0;  // per warp: the rows' constants as floats
-  static constexpr uint32_t kPart = kRing + kWarps * kSlots * kSlot;          // partial sums [kRed][warp][32 rows][4]
+  static constexpr uint32_t kPart = kRing + kWarps * kSlots * kSlot;          // partial sums [kRed][warp][rows in fours][32 weight rows][4]
   static constexpr uint32_t kBar = kPart + kRed * kWarps * kSubRows * kRows * 4;
   static constexpr uint32_t kBarFull = kBar;                                  // [warp][slot]
   static constexpr uint32_t kBarSum = kBarFull + kWarps * kSlots * 8;         // [team][kRed]: the slices' sums are there
   static constexpr uint32_t kBarFree = kBarSum + kWarps * kRed * 8;           // [team][kRed]: they have been taken
   static constexpr uint32_t kSubs = kBarFree + kWarps * kRed * 8;             // int2 [kMaxSubs]
-  static constexpr uint32_t kScratch = kSubs + kMaxSubs * 8;
+  static constexpr uint32_t kRowTok = kSubs + kMaxSubs * 8;                   // the token of every routed row, where this kernel routes
+  static constexpr uint32_t kScratch = kRowTok + kSmallPairs;
   static constexpr uint32_t kEnd = kScratch + kWarps * kScr;
   static constexpr int kBytes = (int)(kEnd - 1024);
 };
@@ -77,6 +79,9 @@ struct GemvParams {
   __half* hid;           // gate/up writes, down reads: fp16 [rows][mid] = silu(gate) * up
   float* out;            // down: pairs fp32 [rows][d]
   int32_t* status;
+  RouteIn route;         // gate/up, fused: the routing is done here (runs, n_runs, tokidx are not read)
+  int fused;
+  int32_t* ready;        // down: set once the lists are there (null: they were before the gate/up kernel started)
 };
 
 __device__ __forceinline__ uint32_t lds32(uint32_t a) {
@@ -161,6 +166,7 @@ template <bool UP, int FMT, int KPW>
 __global__ void __launch_bounds__(kThreads, 1)
 k_gemv(const GemvParams p) {
   using M = Map<FMT, KPW>;
+  constexpr int kRows = M::kRows, kRed = M::kRed;
   extern __shared__ __align__(16) uint8_t gsm[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   {
@@ -190,17 +196,65 @@ k_gemv(const GemvParams p) {
       for (int c = 0; c < 16; c++) sts32(dst + c * 256, hi16 | __shfl_sync(0xffffffffu, mine, c));
     }
   }
-  if (UP) pdl_wait();
-  pdl_trigger();
-  // ---- passes: every expert's rows in fours ----
-  // (the down kernel reads the run list before its wait: the routing kernel was complete before any CTA of the
-  // gate/up kernel triggered)
-  __shared__ int s_cnt[kWarps];
   int n_subs;
-  {
-    const int n_runs = sh ? 1 : min(p.n_runs[0], kThreads);
+  auto put_pass = [&](int i, int expert, int first, int count) {
+    if (i < kMaxSubs) {
+      sts32(M::kSubs + i * 8, (uint32_t)expert | (uint32_t)count << 16);
+      sts32(M::kSubs + i * 8 + 4, (uint32_t)first);
+    }
+  };
+  uint8_t* const smem = gsm - (uint32_t)__cvta_generic_to_shared(gsm);  // smem + A is the generic pointer of absolute shared address A
+  uint8_t* const row_token = smem + M::kRowTok;
+  if (UP) pdl_wait();
+  if (UP && p.fused) {
+    // ---- routing (route_block.cuh), by every CTA of the routed experts for itself; the first of them leaves the
+    // lists for the kernels behind. Its scratch is the place of the partial sums, which come later ----
+    static_assert(kRouteBlockBytes <= kRed * kWarps * kSubRows * kRows * 4, "the routing's scratch");
+    if (sh) {
+      n_subs = (p.route.T + kRows - 1) / kRows;
+      if (tid < n_subs) put_pass(tid, 0, p.route.T * p.route.k + tid * kRows, min(kRows, p.route.T - tid * kRows));
+    } else {
+      n_subs = route_block(p.route, *(RouteBlock*)(smem + M::kPart), (int)blockIdx.x == p.n_sh, kRows, row_token,
+                           [&](int expert, int first, int count, int at) {
+                             for (int i = 0; i * kRows < count; i++) put_pass(at + i, expert, first + i * kRows, min(kRows, count - i * kRows));
+                           });
+      n_subs = min(n_subs, kMaxSubs);
+    }
+    __syncthreads();
+    if ((int)blockIdx.x == p.n_sh && tid == 0) {
+      __threadfence();
+      asm volatile("st.release.gpu.global.b32 [%0], 1;" ::"l"(p.route.rb.ready) : "memory");
+    }
+    pdl_trigger();  // (behind the flag: the down kernel starts when every CTA has come here)
+  } else {
+    pdl_trigger();
+    // ---- passes: every expert's rows, kRows at a time ----
+    // The down kernel reads the run list before its wait: the routing kernel was complete before any CTA of the
+    // gate/up kernel triggered, or, where that kernel routes, the flag tells.
+    __shared__ int s_cnt[kWarps];
+    if (!UP && p.ready) {
+      if (tid == 0) {
+        unsigned long long t0 = 0, now;
+        int v;
+        for (;;) {
+          asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p.ready) : "memory");
+          if (v) break;
+          asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
+          if (t0 == 0) t0 = now;
+          if (now - t0 > 2000000000ull) {
+            if (p.status && atomicCAS(p.status, 0, 8) == 0) p.status[1] = 23;
+            break;
+          }
+        }
+      }
+      __syncthreads();
+    }
+    const int n_runs = sh ? 1 : min(__ldcg(p.n_runs), kThreads);
     Run run{0, 0, 0};
-    if (tid < n_runs) run = sh ? p.runs[kMaxExperts] : p.runs[tid];
+    if (tid < n_runs) {
+      const int32_t* r = (const int32_t*)(p.runs + (sh ? kMaxExperts : tid));
+      run = Run{__ldcg(r), __ldcg(r + 1), __ldcg(r + 2)};
+    }
     const int c = (run.count + kRows - 1) / kRows;
     int incl = c;
 #pragma unroll
@@ -218,17 +272,12 @@ k_gemv(const GemvParams p) {
       n_subs += v;
     }
     n_subs = min(n_subs, kMaxSubs);
-    for (int i = 0; i < c; i++)
-      if (before + i < kMaxSubs) {
-        sts32(M::kSubs + (before + i) * 8, (uint32_t)run.expert | (uint32_t)min(kRows, run.count - i * kRows) << 16);
-        sts32(M::kSubs + (before + i) * 8 + 4, (uint32_t)(run.first + i * kRows));
-      }
+    for (int i = 0; i < c; i++) put_pass(before + i, run.expert, run.first + i * kRows, min(kRows, run.count - i * kRows));
     __syncthreads();
   }
   // ---- this team's share: units c0 .. c1-1 of all passes. A unit = one sub-block column, 32 tile rows over the whole K ----
   const int KB = im.n_kblocks, ash = im.act_shift;
   const int slice = warp % p.slices, team = warp / p.slices;
-  if (team >= p.teams) return;
   const int kb0 = slice * KPW, nk = min(KPW, KB - kb0);
   const int upr = im.n_mtiles * 4;  // units of a pass
   int c0, n_units;
@@ -240,7 +289,7 @@ k_gemv(const GemvParams p) {
     c0 = ti * base + min(ti, rem);
     n_units = base + (ti < rem ? 1 : 0);
   }
-  if (n_units == 0) return;
+  if (team >= p.teams) n_units = 0;
   // ---- the copy stream: a slot = one group of K blocks of a unit, M::kSlots groups ahead ----
   const uint32_t ring = M::kRing + (uint32_t)warp * M::kSlots * M::kSlot, full = M::kBarFull + (uint32_t)warp * M::kSlots * 8;
   int q_left = n_units, q_g = 0, q_sub = c0 / upr, q_j = c0 % upr;
@@ -251,7 +300,7 @@ k_gemv(const GemvParams p) {
     const uint32_t e = lds32(M::kSubs + q_sub * 8) & 0xFFFFu;
     q_ptr = im.data + ((size_t)e * upr + q_j) * unit_b + (uint32_t)kb0 * M::kSub;
   };
-  q_pass();
+  if (n_units > 0) q_pass();
   auto issue = [&]() {
     if (q_left > 0) {
       if (lane == 0) {
@@ -280,14 +329,20 @@ k_gemv(const GemvParams p) {
   };
   for (uint32_t s = 0; s < M::kSlots; s++) issue();
   if (!UP) pdl_wait();
+  if (UP && p.fused && sh && p.route.gate_w) {
+    gate_block(p.route, blockIdx.x, p.n_sh, tid, (double*)(smem + M::kPart), [] { __syncthreads(); });
+    __syncthreads();  // (its scratch is the place of the partial sums)
+  }
+  if (n_units == 0) return;
 
   bool dead = false, lost = false;  // a wait for the team, for the warp's own copies gave up
   uint32_t c_slot = 0, c_ph = 0;
   int sub = c0 / upr, j = c0 % upr, cnt = 0, first = 0;
   bool fresh = true;
-  uint32_t bv[KPW][4], bw[KPW][4];          // activations: lane (g, t) holds row g >> 1, half g & 1, elements 8t .. 8t+7 of every K block
+  // Activations of the slice, B operands. kQ4CP: lane (g, t) holds row g, elements 8t .. 8t+7 of both halves of every
+  // K block. Else row g >> 1, half g & 1, in bv for half 0 and in bw for half 1, zeros in the other.
+  uint32_t bv[KPW][4], bw[KPW][4];
   float xs[KPW][2];             // GGUF: sums of the activations of row t, halves 0 and 1
-  const uint32_t m0 = (g & 1) ? 0u : 0xFFFFFFFFu, m1 = ~m0;
   const uint32_t lut_a = (uint32_t)lane * 4, lut_b = lut_a + (UP && im.dual_book ? 128u : 0u);
   const uint32_t lane_src = (uint32_t)(lane >> 4) * kHalfBytes + (uint32_t)(lane & 15) * 16;
   const uint32_t part0 = M::kPart + (uint32_t)(team * p.slices) * (kSubRows * kRows * 4);
@@ -297,15 +352,21 @@ k_gemv(const GemvParams p) {
   auto finish = [&](int n, int uj, int ucnt, int ufirst) {
     const uint32_t b = n & (kRed - 1);
     mbar_wait(bar_sum + b * 8, (n / kRed) & 1, dead, p.status, 22);
-    float tot[kRows] = {0.f, 0.f, 0.f, 0.f};
+    float tot[kRows];
     const uint32_t a = part0 + b * kPartBuf + lane * 16;
+#pragma unroll
+    for (int pl = 0; pl < kRows; pl += 4) {
+      tot[pl] = tot[pl + 1] = tot[pl + 2] = tot[pl + 3] = 0.f;
+      if (pl < ucnt) {
 #pragma unroll 4
-    for (int s = 0; s < p.slices; s++) {
-      const uint4 v = lds128(a + s * (kSubRows * kRows * 4));
-      tot[0] += __uint_as_float(v.x);
-      tot[1] += __uint_as_float(v.y);
-      tot[2] += __uint_as_float(v.z);
-      tot[3] += __uint_as_float(v.w);
+        for (int s = 0; s < p.slices; s++) {
+          const uint4 v = lds128(a + s * (kSubRows * kRows * 4) + pl * (kSubRows * 4));
+          tot[pl] += __uint_as_float(v.x);
+          tot[pl + 1] += __uint_as_float(v.y);
+          tot[pl + 2] += __uint_as_float(v.z);
+          tot[pl + 3] += __uint_as_float(v.w);
+        }
+      }
     }
     __syncwarp();
     if (lane == 0) mbar_arrive(bar_free + b * 8);
@@ -322,8 +383,9 @@ k_gemv(const GemvParams p) {
       }
     }
   };
+  constexpr int kAcc = kRows / 4;  // activation rows of a lane: t, or 2t and 2t + 1
   // one K block (number i of the slice) of a unit: 32 rows x 64 columns
-  auto item = [&](int i, uint32_t s0, float (&acc)[2][2]) {
+  auto item = [&](int i, uint32_t s0, float (&acc)[2][2][kAcc]) {
     uint32_t m[2][4];
     ldsm4(s0 + lane_src, m[0]);
     ldsm4(s0 + lane_src + 256, m[1]);
@@ -370,35 +432,55 @@ k_gemv(const GemvParams p) {
       }
 #pragma unroll
     for (int b = 0; b < 2; b++) {
-      float c[4], c16[4];
+      if (FMT == kQ4CP) {
 #pragma unroll
-      for (int q = 0; q < 4; q++) {
-        uint32_t a[4];
+        for (int h = 0; h < 2; h++) {
+          // the half's products: K slots 2t, 2t+1 are the codes of byte 2q, slots 2t+8, 2t+9 those of byte 2q+1
+          float c[4];
 #pragma unroll
-        for (int h = 0; h < 4; h++) {
-          if (FMT == kQ4CP) {
-            a[h] = lut32<M::kLut>(__byte_perm(m[b][h], b ? lut_b : lut_a, 0x5504 | (q << 4)));
-          } else if (FMT == kQ4K) {
-            // codes q and q + 4 of the word as the fp16 pair code * 2^-24, for odd q 16 times that (denormal numbers: exact, also in the products)
-            a[h] = (q & 2 ? m[b][h] >> 8 : m[b][h]) & (q & 1 ? 0x00F000F0u : 0x000F000Fu);
-          } else {
-            // the two codes of byte q as the fp16 pair code * 2^-24
-            a[h] = __byte_perm(m[b][h], m[b][h] >> 4, q | (4 + q) << 8) & 0x000F000Fu;
-            a[h] |= (f[b][h] << (4 - q)) & 0x00100010u;
+          for (int q = 0; q < 2; q++) {
+            uint32_t a[4];
+#pragma unroll
+            for (int i4 = 0; i4 < 4; i4++)
+              a[i4] = lut32<M::kLut>(__byte_perm(m[b][2 * h + (i4 & 1)], b ? lut_b : lut_a, 0x5504 | (2 * q + (i4 >> 1)) << 4));
+            const uint32_t b0 = h ? bw[i][2 * q] : bv[i][2 * q], b1 = h ? bw[i][2 * q + 1] : bv[i][2 * q + 1];
+            if (q == 0) mma16816_first(c, a[0], a[1], a[2], a[3], b0, b1);
+            else mma16816(c, a[0], a[1], a[2], a[3], b0, b1);
           }
+#pragma unroll
+          for (int r = 0; r < 2; r++)
+#pragma unroll
+            for (int w = 0; w < kAcc; w++) acc[b][r][w] = fmaf(k[b][r][h], c[2 * r + w], acc[b][r][w]);
         }
-        float* cc = FMT == kQ4K && (q & 1) ? c16 : c;
-        if (q == 0 || (FMT == kQ4K && q == 1)) mma16816_first(cc, a[0], a[1], a[2], a[3], bv[i][q], bw[i][q]);
-        else mma16816(cc, a[0], a[1], a[2], a[3], bv[i][q], bw[i][q]);
-      }
-      if (FMT == kQ4K) {
+      } else {
+        float c[4], c16[4];
 #pragma unroll
-        for (int h = 0; h < 4; h++) c[h] = fmaf(c16[h], 0.0625f, c[h]);
-      }
+        for (int q = 0; q < 4; q++) {
+          uint32_t a[4];
 #pragma unroll
-      for (int r = 0; r < 2; r++) {
-        acc[b][r] = fmaf(k[b][r][1], c[2 * r + 1], fmaf(k[b][r][0], c[2 * r], acc[b][r]));
-        if (FMT != kQ4CP) acc[b][r] = fmaf(k[b][r][3], xs[i][1], fmaf(k[b][r][2], xs[i][0], acc[b][r]));
+          for (int h = 0; h < 4; h++) {
+            if (FMT == kQ4K) {
+              // codes q and q + 4 of the word as the fp16 pair code * 2^-24, for odd q 16 times that (denormal numbers: exact, also in the products)
+              a[h] = (q & 2 ? m[b][h] >> 8 : m[b][h]) & (q & 1 ? 0x00F000F0u : 0x000F000Fu);
+            } else {
+              // the two codes of byte q as the fp16 pair code * 2^-24
+              a[h] = __byte_perm(m[b][h], m[b][h] >> 4, q | (4 + q) << 8) & 0x000F000Fu;
+              a[h] |= (f[b][h] << (4 - q)) & 0x00100010u;
+            }
+          }
+          float* cc = FMT == kQ4K && (q & 1) ? c16 : c;
+          if (q == 0 || (FMT == kQ4K && q == 1)) mma16816_first(cc, a[0], a[1], a[2], a[3], bv[i][q], bw[i][q]);
+          else mma16816(cc, a[0], a[1], a[2], a[3], bv[i][q], bw[i][q]);
+        }
+        if (FMT == kQ4K) {
+#pragma unroll
+          for (int h = 0; h < 4; h++) c[h] = fmaf(c16[h], 0.0625f, c[h]);
+        }
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+          acc[b][r][0] = fmaf(k[b][r][1], c[2 * r + 1], fmaf(k[b][r][0], c[2 * r], acc[b][r][0]));
+          acc[b][r][0] = fmaf(k[b][r][3], xs[i][1], fmaf(k[b][r][2], xs[i][0], acc[b][r][0]));
+        }
       }
     }
   };
@@ -410,40 +492,50 @@ k_gemv(const GemvParams p) {
       const uint2 e = lds64(M::kSubs + sub * 8);
       cnt = (int)(e.x >> 16);
       first = (int)e.y;
-      const int tok = g >> 1;
-      const bool live = tok < cnt;
-      const size_t row = live ? (UP ? (size_t)p.tokidx[first + tok] : (size_t)(first + tok)) : 0;
-#pragma unroll
-      for (int i = 0; i < KPW; i++) {
+      const int at = FMT == kQ4CP ? g : g >> 1;
+      const bool live = at < cnt;
+      size_t row = first + at;
+      if (UP && live) row = !p.fused ? p.tokidx[row] : sh ? row - p.route.T * p.route.k : row_token[row];
+      if (!live) row = 0;
+      auto load8 = [&](int i, int h, uint32_t* v) {
         uint4 u = make_uint4(0, 0, 0, 0);
         if (live && i < nk) {
-          const size_t o = row * p.K + (size_t)((kb0 + i) >> ash) * kTileK + (g & 1) * 32 + t * 8;
+          const size_t o = row * p.K + (size_t)((kb0 + i) >> ash) * kTileK + h * 32 + t * 8;
           u = UP ? __ldg((const uint4*)(p.x + o)) : *(const uint4*)(p.hid + o);
         }
-        const uint32_t w0 = UP ? bf16x2_to_f16x2(u.x) : u.x, w1 = UP ? bf16x2_to_f16x2(u.y) : u.y;
-        const uint32_t w2 = UP ? bf16x2_to_f16x2(u.z) : u.z, w3 = UP ? bf16x2_to_f16x2(u.w) : u.w;
-        if (FMT == kQ4K) {  // elements q and q + 4
-          bv[i][0] = __byte_perm(w0, w2, 0x5410); bv[i][1] = __byte_perm(w0, w2, 0x7632);
-          bv[i][2] = __byte_perm(w1, w3, 0x5410); bv[i][3] = __byte_perm(w1, w3, 0x7632);
-        } else {            // elements 2q and 2q + 1
-          bv[i][0] = w0; bv[i][1] = w1; bv[i][2] = w2; bv[i][3] = w3;
-        }
+        v[0] = UP ? bf16x2_to_f16x2(u.x) : u.x;
+        v[1] = UP ? bf16x2_to_f16x2(u.y) : u.y;
+        v[2] = UP ? bf16x2_to_f16x2(u.z) : u.z;
+        v[3] = UP ? bf16x2_to_f16x2(u.w) : u.w;
+      };
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-          bw[i][q] = bv[i][q] & m1;
-          bv[i][q] &= m0;
-        }
-        if (FMT != kQ4CP) {
+      for (int i = 0; i < KPW; i++) {
+        if (FMT == kQ4CP) {
+          load8(i, 0, bv[i]);
+          load8(i, 1, bw[i]);
+        } else {
+          uint32_t v[4];
+          load8(i, g & 1, v);
+          if (FMT == kQ4K) {  // pairs of elements q and q + 4
+            const uint32_t w0 = v[0], w1 = v[1];
+            v[0] = __byte_perm(w0, v[2], 0x5410);
+            v[1] = __byte_perm(w0, v[2], 0x7632);
+            v[2] = __byte_perm(w1, v[3], 0x5410);
+            v[3] = __byte_perm(w1, v[3], 0x7632);
+          }
           float c[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-          for (int q = 0; q < 4; q++)
+          for (int q = 0; q < 4; q++) {
+            bv[i][q] = (g & 1) ? 0u : v[q];
+            bw[i][q] = (g & 1) ? v[q] : 0u;
             mma16816(c, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u, bv[i][q], bw[i][q]);
+          }
           xs[i][0] = c[0];
           xs[i][1] = c[1];
         }
       }
     }
-    float acc[2][2] = {{0.f, 0.f}, {0.f, 0.f}};  // [16-row block][row g, row g + 8] of row t
+    float acc[2][2][kAcc] = {};  // [16-row block][weight row g, g + 8][activation rows of the lane]
 #pragma unroll
     for (int gi = 0; gi < M::kGroups; gi++) {
       if (gi * M::kGroup < nk) {
@@ -466,12 +558,15 @@ k_gemv(const GemvParams p) {
     // ---- the slice's sums of this unit ----
     const uint32_t b = n & (kRed - 1);
     if (n >= kRed) mbar_wait(bar_free + b * 8, ((n / kRed) & 1) ^ 1, dead, p.status, 21);
-    if (t < cnt) {
-      const uint32_t a = part0 + b * kPartBuf + (uint32_t)slice * (kSubRows * kRows * 4) + (uint32_t)g * 16 + t * 4;
+    if (t * kAcc < cnt) {
+      const uint32_t a = part0 + b * kPartBuf + (uint32_t)slice * (kSubRows * kRows * 4) + (uint32_t)((t * kAcc) >> 2) * (kSubRows * 16) +
+                         (uint32_t)g * 16 + ((t * kAcc) & 3) * 4;
 #pragma unroll
       for (int bb = 0; bb < 2; bb++)
 #pragma unroll
-        for (int r = 0; r < 2; r++) sts32(a + (bb * 16 + r * 8) * 16, __float_as_uint(acc[bb][r]));
+        for (int r = 0; r < 2; r++)
+#pragma unroll
+          for (int w = 0; w < kAcc; w++) sts32(a + (bb * 16 + r * 8) * 16 + w * 4, __float_as_uint(acc[bb][r][w]));
     }
     __syncwarp();
     if (lane == 0) mbar_arrive(bar_sum + b * 8);
@@ -524,11 +619,11 @@ cudaError_t launch_fmt(GemvParams& p, cudaStream_t st) {
 
 // CTAs for the shared expert: its share of the passes that T tokens with even routing make. (Fewer routed
 // passes than that only leave the routed CTAs idle a little earlier.)
-int shared_ctas(int T, int k, int E) {
+int shared_ctas(int T, int k, int E, int rows) {
   const double idle = 1.0 - (double)k / E;
   double unused = 1.0;
   for (int i = 0; i < T; i++) unused *= idle;
-  const double routed = E * (1.0 - unused) * 1.02, shared = (T + kRows - 1) / kRows;
+  const double routed = E * (1.0 - unused) * 1.02, shared = (T + rows - 1) / rows;
   const int n = (int)(148.0 * shared / (routed + shared) + 0.5);
   return n < 1 ? 1 : n > 74 ? 74 : n;
 }
@@ -541,25 +636,27 @@ int gemv_max_mid() { return kWarps / 2 * 4 * kTileK; }
 
 cudaError_t launch_up_gemv(const Image& img, const Image* img_sh, const void* x_bf16, int T, int k, int E, int d, int mid,
                            const int32_t* tokidx, const Run* runs, const int32_t* n_runs,
-                           __half* hid16, int32_t* status, cudaStream_t st) {
+                           __half* hid16, int32_t* status, const RouteIn* route, cudaStream_t st) {
   GemvParams p{};
   p.img = img;
-  if (img_sh) p.img_sh = *img_sh, p.n_sh = shared_ctas(T, k, E);
+  if (img_sh) p.img_sh = *img_sh, p.n_sh = shared_ctas(T, k, E, Map<kQ4CP, 4>::kRows);
   p.runs = runs; p.n_runs = n_runs; p.K = d; p.mid = mid;
   p.x = (const uint16_t*)x_bf16; p.tokidx = tokidx; p.hid = hid16; p.status = status;
+  if (route) p.route = *route, p.fused = 1;
   if (img.fmt == kQ4K) return launch_fmt<true, kQ4K>(p, st);
   if (img.fmt == kQ51) return launch_fmt<true, kQ51>(p, st);
   return launch_fmt<true, kQ4CP>(p, st);
 }
 
 cudaError_t launch_down_gemv(const Image& img, const Image* img_sh, const __half* hid16, int T, int k, int E, int d, int mid,
-                             const Run* runs, const int32_t* n_runs, float* pairs_f32, int32_t* status, cudaStream_t st) {
+                             const Run* runs, const int32_t* n_runs, float* pairs_f32, int32_t* status, int32_t* ready,
+                             cudaStream_t st) {
   GemvParams p{};
   p.img = img;
-  if (img_sh) p.img_sh = *img_sh, p.n_sh = shared_ctas(T, k, E);
+  if (img_sh) p.img_sh = *img_sh, p.n_sh = shared_ctas(T, k, E, Map<kQ4CP, 4>::kRows);
   p.runs = runs; p.n_runs = n_runs; p.K = mid; p.mid = mid;
   p.hid = const_cast<__half*>(hid16);
-  p.out = pairs_f32; p.status = status;
+  p.out = pairs_f32; p.status = status; p.ready = ready;
   if (img.fmt == kQ4K) return launch_fmt<false, kQ4K>(p, st);
   if (img.fmt == kQ51) return launch_fmt<false, kQ51>(p, st);
   return launch_fmt<false, kQ4CP>(p, st);

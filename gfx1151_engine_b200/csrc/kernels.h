@@ -82,6 +82,7 @@ struct RouteBuffers {
   Tile* tiles_sh;    // work list of the shared expert (all T tokens)
   int32_t* n_tiles;  // [3]: tiles, tiles_sh, tiles_narrow
   float* sgate;      // [T] sigmoid gate of the shared expert
+  int32_t* ready;    // 1 from the gate/up GEMV's own routing to the combine: the lists above are there
   int32_t* status;   // the handle's status word (may be null): {4, id} when an expert id outside [0, E) was dropped
 };
 cudaError_t launch_router_topk(const float* logits, int T, int E, int k, int32_t* ids, float* w,
@@ -94,13 +95,23 @@ struct TileCut {
 };
 cudaError_t launch_route(const RouteBuffers& rb, const int32_t* ids, const float* w, int stride,
                          int T, int k, int E, const TileCut& cut, cudaStream_t st, int* launches);
-// Whole routing stage in one launch for T*k <= route_small_max_pairs(): logits != nullptr runs
-// the router too (ids/w ignored), gate_w_bf16 != nullptr adds the shared expert's gate. tile_cap: most rows
-// of one tile; all go on tiles.
-int route_small_max_pairs();
-cudaError_t launch_route_small(const RouteBuffers& rb, const float* logits, const int32_t* ids,
-                               const float* w, int stride, int T, int k, int E, const void* x_bf16,
-                               const uint16_t* gate_w_bf16, int d, int tile_cap, cudaStream_t st);
+// Routing of a decode call (route_block_supported; route_block.cuh).
+struct RouteIn {
+  const float* logits;     // [T][E], or null: the caller's ids / w
+  const int32_t* ids;
+  const float* w;
+  int stride;
+  const uint16_t* router;  // bf16 [E][d]: the logits are double tree sums of x and that weight, those that decide a near-tie are
+                           // put into the reference's arithmetic first. Null: the logits are final
+  const uint16_t* x;       // bf16 [T][d], 16-byte aligned
+  const uint16_t* gate_w;  // the shared expert's gate, or null
+  int T, E, k, d;
+  int tile_cap;            // most rows of one tile; all tiles go on rb.tiles
+  int exact;               // every token in the general body
+  RouteBuffers rb;
+};
+bool route_block_supported(int T, int k);
+cudaError_t launch_route_block(const RouteIn& q, cudaStream_t st);  // the whole routing stage in one launch
 cudaError_t launch_shared_gate(const void* x_bf16, const uint16_t* gate_w_bf16, int T, int d,
                                int k, const RouteBuffers& rb, cudaStream_t st);
 cudaError_t launch_apply_placement(int32_t* ids, int stride, int T, int k, int E, const int32_t* place,
@@ -129,11 +140,12 @@ int gemv_max_mid();   // largest mid
 // img_sh: the shared expert's image (nullptr: none); its run is runs[kMaxExperts].
 // hid16: fp16 [rows][mid] hidden activations silu(gate) * up, written by the gate/up kernel and
 // read by the down kernel.
+// route: the gate/up kernel does the routing, too (T*k <= 256; the lists above are then its results).
 cudaError_t launch_up_gemv(const Image& img, const Image* img_sh, const void* x_bf16, int T, int k, int E, int d, int mid,
                            const int32_t* tokidx, const Run* runs, const int32_t* n_runs,
-                           __half* hid16, int32_t* status, cudaStream_t st);
+                           __half* hid16, int32_t* status, const RouteIn* route, cudaStream_t st);
 cudaError_t launch_down_gemv(const Image& img, const Image* img_sh, const __half* hid16, int T, int k, int E, int d, int mid,
-                             const Run* runs, const int32_t* n_runs, float* pairs_f32, int32_t* status, cudaStream_t st);
+                             const Run* runs, const int32_t* n_runs, float* pairs_f32, int32_t* status, int32_t* ready, cudaStream_t st);
 
 // ---- decode.cu (q4cp decode / verify, T <= decode_max_tokens(), as one kernel) ----
 // Routing (from logits, or from the caller's ids / w when logits is null), gate/up GEMV + SwiGLU,
@@ -149,11 +161,6 @@ cudaError_t launch_decode(const Image& gu, const Image& dn, const Image* sh_gu, 
                           int E, int k, int d, int mid, __half* hid16, void* out_bf16, const float* hc_w4, void* hc_state,
                           const RouteBuffers& rb, unsigned long long* bar, int32_t* status, cudaStream_t st,
                           unsigned long long* trace = nullptr);  // trace: debug, [SMs][8] phase time stamps of the last launch
-
-// The routing stage alone with the decode kernel's compact router (logits given, T <= decode_max_tokens(),
-// T*k <= 128, x 16-byte aligned when gate_w_bf16 is given); same outputs as launch_route_small.
-cudaError_t launch_route_fast(const RouteBuffers& rb, const float* logits, int T, int k, int E, const void* x_bf16,
-                              const uint16_t* gate_w_bf16, int d, int tile_cap, cudaStream_t st);
 
 // Bounded wait (2 s) until n <= 32 flags written by other GPUs have reached `expected`; a
 // timeout sets status {3, flag index}.
@@ -180,9 +187,10 @@ cudaError_t launch_router_pairs(const void* x_bf16, const void* w_bf16, const in
 // ---- combine.cu ----
 // hc_w4 / hc_state non-null: add the result into the four branches of the bf16 state
 // [T][4][d] with gates 2*sigmoid(w4[t][b]/4) instead of storing out_bf16.
+// ready non-null: the flag is taken back (T <= 64).
 cudaError_t launch_combine_f32(const float* pairs, const float* pw, const int32_t* pairids, int T,
                                int k, int d, int shared_row0, void* out_bf16, cudaStream_t st,
-                               const float* hc_w4 = nullptr, void* hc_state = nullptr);
+                               const float* hc_w4 = nullptr, void* hc_state = nullptr, int32_t* ready = nullptr);
 cudaError_t launch_combine_f16(const __half* pairs, const float* pw, const int32_t* pairids, int T,
                                int k, int d, int shared_row0, void* out_bf16, cudaStream_t st,
                                const float* hc_w4 = nullptr, void* hc_state = nullptr);

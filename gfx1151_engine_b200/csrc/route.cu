@@ -13,7 +13,7 @@
 // Everything here is integer/bookkeeping work and deterministic: no atomics on global
 // memory, no dependence on block scheduling order.
 #include "kernels.h"
-#include "route_small.cuh"
+#include "route_block.cuh"
 
 namespace b200moe {
 
@@ -30,9 +30,10 @@ __device__ __forceinline__ double shfl_double(double v, int src) {
   return __hiloint2double(hi, lo);
 }
 
-// Router for one token by one warp, E <= 512: lane holds experts lane, lane+32, ...
+// Router for one token by one warp, E <= 512: lane holds experts lane, lane+32, ... The reference's arithmetic, out
+// of line: only tokens whose ids the logits' order does not decide come here.
 // sp: this warp's scratch row of kMaxExperts floats in shared memory.
-__device__ __forceinline__ void router_one_token(const float* __restrict__ lg, int E, int k, int lane,
+__device__ __noinline__ void router_one_token(const float* __restrict__ lg, int E, int k, int lane,
                                                  float* sp, int32_t* __restrict__ ids_row,
                                                  float* __restrict__ w_row, int stride) {
   float v[16];
@@ -143,23 +144,36 @@ k_router_topk(const float* __restrict__ logits, int T, int E, int k, int32_t* __
   pdl_trigger();
   pdl_wait();
   if (t >= T) return;
-  router_one_token(logits + (size_t)t * E, E, k, lane, s_p[warp], ids + (size_t)t * stride,
-                   w + (size_t)t * stride, stride);
+  // The ids from the logits' order where that decides them (route_block.cuh), which saves E double exponentials and
+  // divisions and k rounds of arg-max: 16384 tokens x 512 experts XX us, before that XX.
+  float vr, wv;
+  int id;
+  const int C = warp_leaders(logits + (size_t)t * E, E, k, lane, s_p[warp], vr, id);
+  if (C > 0 && warp_topk(C, vr, k, lane, wv)) {
+    for (int i = lane; i < stride; i += 32) {  // zeros behind the k
+      ids[(size_t)t * stride + i] = i < k ? id : 0;
+      w[(size_t)t * stride + i] = i < k ? wv : 0.f;
+    }
+  } else {
+    __syncwarp();
+    router_one_token(logits + (size_t)t * E, E, k, lane, s_p[warp], ids + (size_t)t * stride, w + (size_t)t * stride, stride);
+  }
 }
 
-// Decode / verify (T*k <= 256): the whole routing stage in ONE block (route_small.cuh).
-__global__ void __launch_bounds__(kMaxExperts, 1)
-k_route_small(const float* __restrict__ logits, const int32_t* __restrict__ ids_in,
-              const float* __restrict__ w_in, int stride_in, int T, int E, int k, int tile_cap, RouteBuffers rb,
-              const uint16_t* __restrict__ x, const uint16_t* __restrict__ gw, int d) {
-  __shared__ RouteSmallScratch<16> sc;
+// Decode / verify (T <= 16, T*k <= 256): the whole routing stage in one block (route_block.cuh). Warps 0..15 route,
+// warps 16..31 form the shared expert's gates.
+__global__ void __launch_bounds__(1024)
+k_route_block(const RouteIn q) {
+  extern __shared__ __align__(16) uint8_t rsm[];
+  __shared__ uint8_t row_token[kSmallPairs];
+  __shared__ double gpart[16 * 16];
   pdl_trigger();
   pdl_wait();  // inputs may come from the previous kernel; the buffers written here may still be read by it
-  RouteSmallOut o;
-  o.topids = rb.topids; o.topw = rb.topw; o.tokidx = rb.tokidx; o.pw = rb.pw; o.pairids = rb.pairids;
-  o.eoff = rb.eoff; o.runs = rb.runs; o.shared_slot = kMaxExperts; o.n_runs = rb.n_runs; o.tiles = rb.tiles;
-  o.tiles_sh = rb.tiles_sh; o.n_tiles = rb.n_tiles; o.sgate = rb.sgate;
-  route_small_body<16>(logits, ids_in, w_in, stride_in, T, E, k, tile_cap, x, gw, d, sc, o, RouteSmallOut{}, rb.status);
+  if (threadIdx.x < 512) {
+    route_block(q, *(RouteBlock*)rsm, true, 16, row_token, [](int, int, int, int) {});
+  } else if (q.gate_w) {
+    gate_block(q, 0, 1, threadIdx.x - 512, gpart, [] { asm volatile("bar.sync 2, 512;" ::: "memory"); });
+  }
 }
 
 __global__ void __launch_bounds__(kChunk)
@@ -380,6 +394,13 @@ cudaError_t launch_router_topk(const float* logits, int T, int E, int k, int32_t
                     k, ids, w, stride);
 }
 
+bool route_block_supported(int T, int k) { return T <= 16 && T * k <= kSmallPairs; }
+
+cudaError_t launch_route_block(const RouteIn& q, cudaStream_t st) {
+  static_assert(kRouteBlockBytes <= 48 * 1024, "opt-in size");
+  return launch_pdl(k_route_block, dim3(1), dim3(1024), (size_t)kRouteBlockBytes, st, q);
+}
+
 cudaError_t launch_route(const RouteBuffers& rb, const int32_t* ids, const float* w, int stride,
                          int T, int k, int E, const TileCut& cut, cudaStream_t st, int* launches) {
   const int pairs = T * k;
@@ -577,13 +598,6 @@ cudaError_t launch_ep_merge_tails(__half* x_recv, const int32_t* segs, int n_seg
   return cudaGetLastError();
 }
 
-cudaError_t launch_route_small(const RouteBuffers& rb, const float* logits, const int32_t* ids,
-                               const float* w, int stride, int T, int k, int E, const void* x_bf16,
-                               const uint16_t* gate_w_bf16, int d, int tile_cap, cudaStream_t st) {
-  return launch_pdl(k_route_small, dim3(1), dim3(kMaxExperts), 0, st, logits, ids, w, stride, T, E, k, tile_cap, rb,
-                    (const uint16_t*)x_bf16, gate_w_bf16, d);
-}
-
 // Waits until every one of n flags (written by peer GPUs' copy engines behind their data)
 // has reached `expected`. Bounded: after 2 s the kernel records status {3, index of the
 // missing flag} and returns, so that the context stays usable and the host sees the timeout.
@@ -613,7 +627,6 @@ cudaError_t launch_wait_flags(const int32_t* flags, int n, int32_t expected, int
   return cudaGetLastError();
 }
 
-int route_small_max_pairs() { return kSmallPairs; }
 int route_chunk() { return kChunk; }
 
 }  // namespace b200moe

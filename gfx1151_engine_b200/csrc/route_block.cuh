@@ -1,0 +1,333 @@
+// route_block.cuh -- the whole routing stage of a decode / verify call (T <= 16, T*k <= 256) by the 512 threads of
+// one block: router top-k (a warp per token), stable bucketing of the pairs by expert, offsets, run and tile
+// lists. Used by k_route_block (route.cu) and by the gate/up GEMV (expert_gemv.cu), whose blocks each repeat it for
+// themselves: that costs every block 2 us, but no launch, and no lists that travel through memory.
+//   * Selection. "Largest probability, ties to the lowest id" is "largest logit, ties to the lowest id" unless two
+//     different logits round to one float probability (exp and the division by the sum are monotone): the ids come
+//     from the logits' order. Where two of a token's k+1 largest are closer than 1e-6, or a logit is not finite, that
+//     token takes the general body instead (route_small.cuh: the reference's arithmetic to the letter, out of
+//     line, since its 5000 instructions would be fetched cold by every call).
+//   * Weights: double exponentials of the k selected logits over their sum in rank order; the sum over all experts
+//     cancels and is not formed.
+//   * With a router weight the logits are double tree sums (k_router_dots) and the warp first does what
+//     k_router_flag / k_router_pairs do for longer calls: where two of the leaders are closer than 5e-7 of the
+//     magnitude, all that can be in or next to the top-k are formed again in the reference's arithmetic.
+//   * Bucketing: a thread per pair, ranks inside a warp by match, over warps and experts by prefix sums.
+#pragma once
+#include "kernels.h"
+#include "route_small.cuh"
+#include "router_exact.cuh"
+
+namespace b200moe {
+
+constexpr int kPairWarps = kSmallPairs / 32;
+
+struct alignas(16) RouteBlock {
+  int key[kSmallPairs];      // expert of pair t*k + s; kMaxExperts: dropped
+  float w[kSmallPairs];
+  uint16_t before[kPairWarps][kMaxExperts + 8];  // pairs of an expert: per warp, then in the warps before; [kMaxExperts]: dropped pairs
+  int start[kMaxExperts + 1];
+  int wsum[16], wmore[16];
+  int fallback[16];
+  int xid[kIdStride];        // the general body's answer for one token
+  float xw[kIdStride];
+  float row[kMaxExperts];    // a near-tied token's logits
+  float cand[16][128];       // per warp
+};
+// scratch behind it: the general body's, or the products of 16 warps' exact logits one warp at a time
+constexpr int kRouteBlockBytes = (int)(sizeof(RouteBlock) + sizeof(RouteSmallScratch<3>));
+static_assert(sizeof(RouteSmallScratch<3>) >= 256 * sizeof(double) && sizeof(RouteBlock) % 16 == 0, "scratch");
+
+__device__ __forceinline__ double shfl_f64(double v, int src) {
+  return __hiloint2double(__shfl_sync(0xffffffffu, __double2hiint(v), src), __shfl_sync(0xffffffffu, __double2loint(v), src));
+}
+
+// The k+1 largest of E <= 512 logits in order (value descending, id ascending), by one warp: lane i gets the i-th.
+// s: 128 floats of the warp. Returns how many candidates there were, at least min(k+1, E); 0: a logit is not finite, or more than 32.
+__device__ __forceinline__ int warp_leaders(const float* lg, int E, int k, int lane, float* s, float& vr, int& id) {
+  float v[16];
+  float lm = -INFINITY;  // the lane's largest
+  bool odd = false;
+#pragma unroll
+  for (int j = 0; j < 16; j++) {
+    const int e = j * 32 + lane;
+    v[j] = e < E ? lg[e] : -INFINITY;
+    odd |= e < E && !(fabsf(v[j]) <= 3.0e38f);
+    lm = fmaxf(lm, v[j]);
+  }
+  if (__any_sync(0xffffffffu, odd)) return 0;
+  // the (k+1)-th largest of the lanes' maxima is a lower bound of the (k+1)-th largest logit
+  int rank = 0;
+#pragma unroll
+  for (int i = 0; i < 32; i++) {
+    const float o = __shfl_sync(0xffffffffu, lm, i);
+    rank += (o > lm) || (o == lm && i < lane);
+  }
+  const float bound = __shfl_sync(0xffffffffu, lm, __ffs(__ballot_sync(0xffffffffu, rank == k)) - 1);
+  float *cv = s, *sv = s + 64;
+  int *ci = (int*)s + 32, *si = (int*)s + 96;
+  int C = 0;
+#pragma unroll
+  for (int j = 0; j < 16; j++) {
+    const bool c = j * 32 + lane < E && v[j] >= bound;
+    const unsigned bal = __ballot_sync(0xffffffffu, c);
+    const int pos = C + __popc(bal & ((1u << lane) - 1u));
+    if (c && pos < 32) {
+      cv[pos] = v[j];
+      ci[pos] = j * 32 + lane;
+    }
+    C += __popc(bal);
+  }
+  if (C > 32) return 0;
+  __syncwarp();
+  if (lane < C) {
+    const float mv = cv[lane];
+    const int mi = ci[lane];
+    int r = 0;
+    for (int i = 0; i < C; i++) r += (cv[i] > mv) || (cv[i] == mv && ci[i] < mi);
+    sv[r] = mv;
+    si[r] = mi;
+  }
+  __syncwarp();
+  vr = lane < C ? sv[lane] : -INFINITY;
+  id = lane < C ? si[lane] : 0;
+  __syncwarp();
+  return C;
+}
+
+// Top-k ids and weights from the order of the logits: lane r < k gets the r-th. False where that does not decide.
+__device__ __forceinline__ bool warp_topk(int C, float vr, int k, int lane, float& wv) {
+  const float vn = __shfl_down_sync(0xffffffffu, vr, 1), mx = __shfl_sync(0xffffffffu, vr, 0);
+  // neighbours in the order closer than 1e-6: their probabilities might round to one float
+  if (__any_sync(0xffffffffu, lane < k && lane + 1 < C && !(vr - vn > 1e-6f * fmaxf(1.f, fabsf(vr)))) || C < k) return false;
+  const double e = lane < k ? exp((double)vr - (double)mx) : 0.0;
+  double kept = 0;
+#pragma unroll 1
+  for (int r = 0; r < k; r++) kept += shfl_f64(e, r);  // rank order, as the reference adds
+  wv = lane < k ? (float)(e / kept) : 0.f;
+  return true;
+}
+
+// k_router_pairs' arithmetic for one token's logits that are not below `floor`, by one warp. (In the block's own copy:
+// other blocks read the same logits at the same time and have to come to the same answer.)
+static __device__ __noinline__ void warp_refine(const RouteIn& q, int t, int lane, float floor, float* row, double* prod) {
+  for (int e0 = 0; e0 < q.E; e0 += 32) {
+    unsigned m = __ballot_sync(0xffffffffu, e0 + lane < q.E && row[e0 + lane] >= floor);
+    for (; m; m &= m - 1) {
+      const int e = e0 + __ffs(m) - 1;
+      const float v = exact_logit(q.x + (size_t)t * q.d, q.router + (size_t)e * q.d, q.d, prod, lane);
+      if (lane == 0) row[e] = v;
+    }
+  }
+}
+
+static __device__ __noinline__ void token_exact(const RouteIn& q, int t, const float* logits, RouteBlock& sc) {
+  RouteSmallOut o;
+  o.topids = sc.xid;
+  o.topw = sc.xw;
+  route_small_body<3, 2>(logits, nullptr, nullptr, 0, 1, q.E, q.k, q.tile_cap, nullptr, nullptr, q.d,
+                         *(RouteSmallScratch<3>*)(&sc + 1), o, RouteSmallOut{}, nullptr);
+  rs_sync();
+  if (threadIdx.x < q.k) {
+    sc.key[t * q.k + threadIdx.x] = sc.xid[threadIdx.x];
+    sc.w[t * q.k + threadIdx.x] = sc.xw[threadIdx.x];
+  }
+  rs_sync();
+}
+
+// Threads 0..511 of a block, sc and the scratch behind it in shared memory. write: leave everything in q.rb, too.
+// row_token (shared memory, [T*k]): the token of every permuted row. Calls emit(expert, first, count, at) for
+// every non-empty expert from one thread; at: passes of `rows` rows of the experts before. Returns their number.
+template <typename Emit>
+__device__ __forceinline__ int route_block(const RouteIn& q, RouteBlock& sc, bool write, int rows, uint8_t* row_token, Emit emit) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int T = q.T, E = q.E, k = q.k, P = T * k;
+  for (int i = tid; i < (int)sizeof(sc.before) / 4; i += 512) ((uint32_t*)sc.before)[i] = 0;
+  if (q.logits) {
+    if (warp < T) {
+      const float* lg = q.logits + (size_t)warp * E;
+      float vr, wv = 0.f;
+      int id;
+      int C = warp_leaders(lg, E, k, lane, sc.cand[warp], vr, id);
+      if (q.router && C > 0) {
+        const float margin = 5e-7f * fmaxf(1.f, fabsf(__shfl_sync(0xffffffffu, vr, 0)));
+        const float vn = __shfl_down_sync(0xffffffffu, vr, 1), kth = __shfl_sync(0xffffffffu, vr, min(k, E) - 1);
+        if (__any_sync(0xffffffffu, lane < k && lane + 1 < C && vr - vn < margin)) C = -1;
+        if (lane == 0) sc.cand[warp][0] = kth - 2.f * margin;
+      }
+      const bool ok = C > 0 && !q.exact && warp_topk(C, vr, k, lane, wv);
+      if (ok && lane < k) {
+        sc.key[warp * k + lane] = id;
+        sc.w[warp * k + lane] = wv;
+      }
+      if (lane == 0) sc.fallback[warp] = C < 0 ? 2 : !ok;
+    }
+    rs_sync();
+    // tokens that their logits' order does not decide, one after the other (rare; uniform for the block)
+    for (int t = 0; t < T; t++) {
+      const int f = sc.fallback[t];
+      if (f == 0) continue;
+      const float* lg = q.logits + (size_t)t * E;
+      if (f == 2) {
+        if (tid < E) sc.row[tid] = lg[tid];
+        rs_sync();
+        if (warp == 0) warp_refine(q, t, lane, sc.cand[t][0], sc.row, (double*)(&sc + 1));
+        rs_sync();
+        lg = sc.row;
+      }
+      token_exact(q, t, lg, sc);
+    }
+  } else {
+    for (int p = tid; p < P; p += 512) {
+      // a caller-supplied id outside [0, E) must never index anything: the pair is dropped (it sorts behind
+      // every expert) and the status word records it
+      int id = q.ids[(size_t)(p / k) * q.stride + p % k];
+      if ((unsigned)id >= (unsigned)E) {
+        if (write && q.rb.status && atomicCAS(q.rb.status, 0, kStatusBadId) == 0) q.rb.status[1] = id;
+        id = kMaxExperts;
+      }
+      sc.key[p] = id;
+      sc.w[p] = q.w[(size_t)(p / k) * q.stride + p % k];
+    }
+    rs_sync();
+  }
+  // ---- bucketing ----
+  const bool live = tid < P;
+  const int key = live ? sc.key[tid] : -1, pt = live ? tid / k : 0;
+  unsigned same = 0;
+  if (warp < kPairWarps) {
+    same = __match_any_sync(0xffffffffu, key);
+    if (live && lane == __ffs(same) - 1) sc.before[warp][key] = (uint16_t)__popc(same);
+  }
+  if (write && q.logits)
+    for (int i = tid; i < T * kIdStride; i += 512) {
+      const int t = i / kIdStride, s = i % kIdStride;
+      q.rb.topids[i] = s < k ? sc.key[t * k + s] : 0;
+      q.rb.topw[i] = s < k ? sc.w[t * k + s] : 0.f;
+    }
+  rs_sync();
+  // a thread per expert (the first one also for the dropped pairs): its pairs before each warp's, its count
+  int cnt = 0;
+#pragma unroll
+  for (int v = 0; v < kPairWarps; v++) {
+    const int n = sc.before[v][tid];
+    sc.before[v][tid] = (uint16_t)cnt;
+    cnt += n;
+  }
+  if (tid == 0) {
+    int c = 0;
+    for (int v = 0; v < kPairWarps; v++) {
+      const int n = sc.before[v][kMaxExperts];
+      sc.before[v][kMaxExperts] = (uint16_t)c;
+      c += n;
+    }
+  }
+  // Ids may repeat within a token (a caller's, or the selection's on non-finite logits), so an expert can have
+  // up to T*k rows: the first tile_cap of them stand at the expert's place among the non-empty ones, the tiles
+  // cut from the rest behind all of those.
+  const int more = cnt > q.tile_cap ? (cnt - 1) / q.tile_cap : 0, passes = (cnt + rows - 1) / rows;
+  int a = cnt | (cnt > 0) << 16, b = more | passes << 16;  // sums of counts and of non-empty experts; of further tiles and of passes
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, a, o), v = __shfl_up_sync(0xffffffffu, b, o);
+    if (lane >= o) {
+      a += u;
+      b += v;
+    }
+  }
+  if (lane == 31) {
+    sc.wsum[warp] = a;
+    sc.wmore[warp] = b;
+  }
+  rs_sync();
+  int all = 0, all_more = 0;
+#pragma unroll
+  for (int w2 = 0; w2 < 16; w2++) {
+    const int u = sc.wsum[w2], v = sc.wmore[w2];
+    if (w2 < warp) {
+      a += u;
+      b += v;
+    }
+    all += u;
+    all_more += v;
+  }
+  const int n_rows = all & 0xffff, n_active = all >> 16;
+  const int first = (a & 0xffff) - cnt, at = (a >> 16) - 1;
+  sc.start[tid] = first;
+  if (cnt > 0) emit(tid, first, cnt, (b >> 16) - passes);
+  if (tid == 0) sc.start[kMaxExperts] = n_rows;
+  if (write) {
+    if (tid < E) q.rb.eoff[tid] = first;
+    if (cnt > 0) {
+      q.rb.runs[at] = Run{tid, first, cnt};
+      q.rb.tiles[at] = Tile{tid, first, min(cnt, q.tile_cap)};
+      for (int j = 1; j <= more; j++)
+        q.rb.tiles[n_active + ((b & 0xffff) - more) + j - 1] = Tile{tid, first + j * q.tile_cap, min(cnt - j * q.tile_cap, q.tile_cap)};
+    }
+    if (tid == 0) {
+      q.rb.eoff[E] = n_rows;  // pairs actually placed
+      q.rb.n_runs[0] = n_active;
+      q.rb.n_runs[1] = 1;
+      q.rb.runs[kMaxExperts] = Run{0, P, T};
+      q.rb.n_tiles[0] = n_active + (all_more & 0xffff);
+      q.rb.n_tiles[1] = 1;
+      q.rb.tiles_sh[0] = Tile{0, P, T};
+    }
+  }
+  rs_sync();
+  if (live) {
+    const int row = sc.start[key] + sc.before[warp][key] + __popc(same & ((1u << lane) - 1u));
+    row_token[row] = (uint8_t)pt;
+    if (write) {
+      // slot of the pair in the token's reduce order: ascending expert id; equal ids (a caller's duplicate, or
+      // two dropped pairs) keep their slot order, so every slot is written
+      int rank = 0;
+#pragma unroll 4
+      for (int p = pt * k; p < pt * k + k; p++) rank += (sc.key[p] < key) || (sc.key[p] == key && p < tid);
+      q.rb.tokidx[row] = pt;
+      q.rb.pw[row] = sc.w[tid];
+      q.rb.pairids[(size_t)pt * k + rank] = key == kMaxExperts ? -1 : row;  // the combine skips negative rows
+    }
+  }
+  return all_more >> 16;
+}
+
+// Scalar sigmoid gate of the shared expert (src/ref.cpp:623-626) of the tokens t0, t0 + step, ...: d-long dot products
+// in double by 512 threads (tid: their number), gpart: [16][16] doubles of shared memory, sync: their barrier.
+template <typename Sync>
+__device__ __forceinline__ void gate_block(const RouteIn& q, int t0, int step, int tid, double* gpart, Sync sync) {
+  const int lane = tid & 31, T = q.T, d = q.d, P = q.T * q.k;
+#pragma unroll 1
+  for (int t = t0; t < T; t += step) {
+    double a = 0;
+    const uint4* xv = (const uint4*)(q.x + (size_t)t * d);
+    const uint4* gv = (const uint4*)q.gate_w;
+#pragma unroll 1
+    for (int c = tid; c < d / 8; c += 512) {
+      const uint4 xa = xv[c], ga = __ldg(gv + c);
+      const uint32_t xw[4] = {xa.x, xa.y, xa.z, xa.w}, gq[4] = {ga.x, ga.y, ga.z, ga.w};
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        a += (double)__uint_as_float(gq[i] << 16) * (double)__uint_as_float(xw[i] << 16);
+        a += (double)__uint_as_float(gq[i] & 0xFFFF0000u) * (double)__uint_as_float(xw[i] & 0xFFFF0000u);
+      }
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1)
+      a += __hiloint2double(__shfl_xor_sync(0xffffffffu, __double2hiint(a), o),
+                            __shfl_xor_sync(0xffffffffu, __double2loint(a), o));
+    if (lane == 0) gpart[t * 16 + (tid >> 5)] = a;
+  }
+  sync();
+  if (tid < T && tid >= t0 && (tid - t0) % step == 0) {
+    double tot = 0;
+#pragma unroll 1
+    for (int w2 = 0; w2 < 16; w2++) tot += gpart[tid * 16 + w2];
+    const float gate = sigmoid_f32((float)tot);
+    q.rb.sgate[tid] = gate;
+    q.rb.tokidx[P + tid] = tid;
+    q.rb.pw[P + tid] = gate;
+  }
+}
+
+}  // namespace b200moe

@@ -25,6 +25,7 @@
 // Every wait on an mbarrier is bounded; a timeout sets the status word and the CTA leaves
 // after releasing its tensor memory.
 #include "kernels.h"
+#include "router_exact.cuh"
 
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -230,18 +231,21 @@ k_router_gemm(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
 }
 
 // ---- logits in double --------------------------------------------------------------------
-// A block takes 8 tokens x 8 experts: the tokens' activations are staged in shared memory,
-// warp w owns expert 8*chunk + w and adds the eight dot products side by side in double (one
+// A block takes kExTok tokens x 8 experts: the tokens' activations are staged in shared memory,
+// warp w owns expert 8*chunk + w and adds the tokens' dot products side by side in double (one
 // fused multiply-add per term: the product of two bf16 values is exact in double, so the
 // fused form rounds exactly like multiply-then-add). Tokens 0 .. n-1.
-constexpr int kExTok = 8, kExExp = 8;
+constexpr int kExExp = 8;
 
+template <int kExTok>
 __global__ void __launch_bounds__(256)
 k_router_dots(const uint16_t* __restrict__ x, const uint16_t* __restrict__ w, int n, int E, int d,
               float* __restrict__ logits) {
   extern __shared__ __align__(16) uint16_t ex_x[];  // [kExTok][d] bf16 bits
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_groups = (n + kExTok - 1) / kExTok, n_chunks = (E + kExExp - 1) / kExExp;
+  pdl_trigger();
+  pdl_wait();
   for (long long job = blockIdx.x; job < (long long)n_groups * n_chunks; job += gridDim.x) {
     const int grp = (int)(job / n_chunks), chunk = (int)(job % n_chunks);
     __syncthreads();  // the previous job's reads of the staged rows are over
@@ -304,55 +308,8 @@ k_router_pairs(const uint16_t* __restrict__ x, const uint16_t* __restrict__ w, c
     const int t = pairs[i] / E, e = pairs[i] % E;
     const uint16_t* xr = x + (size_t)t * d;
     const uint16_t* wr = w + (size_t)e * d;
-    double acc = 0, mag = 0;
-    for (int c = lane * 8; c < d; c += 256) {
-      const uint4 xv = *(const uint4*)(xr + c), wv = __ldg((const uint4*)(wr + c));
-      const uint16_t* xb = (const uint16_t*)&xv;
-      const uint16_t* wb = (const uint16_t*)&wv;
-#pragma unroll
-      for (int j = 0; j < 8; j++) {
-        const double pd = (double)bf16_bits_to_f32(wb[j]) * (double)bf16_bits_to_f32(xb[j]);  // exact
-        acc += pd;
-        mag += fabs(pd);
-      }
-    }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-      acc += __hiloint2double(__shfl_xor_sync(0xffffffffu, __double2hiint(acc), o),
-                              __shfl_xor_sync(0xffffffffu, __double2loint(acc), o));
-      mag += __hiloint2double(__shfl_xor_sync(0xffffffffu, __double2hiint(mag), o),
-                              __shfl_xor_sync(0xffffffffu, __double2loint(mag), o));
-    }
-    acc = __hiloint2double(__shfl_sync(0xffffffffu, __double2hiint(acc), 0), __shfl_sync(0xffffffffu, __double2loint(acc), 0));
-    mag = __hiloint2double(__shfl_sync(0xffffffffu, __double2hiint(mag), 0), __shfl_sync(0xffffffffu, __double2loint(mag), 0));
-    // |index-order sum - true sum| <= gamma(d-1) * sum|p|, |this tree sum - true sum| <=
-    // gamma(d/32 + 5) * sum|p| (d/32 additions per lane, five shuffle levels), gamma(n) ~ n * 2^-53;
-    // `mag` is within the same tiny factor of sum|p|: 1 % of slack covers both second-order terms
-    const double delta = 1.01 * (double)(d + d / 32 + 8) * 1.1102230246251565e-16 * mag;
-    if ((float)(acc - delta) != (float)(acc + delta)) {  // warp-uniform
-      // replay of the reference's order: the lanes form the (exact) products of 256 elements at a
-      // time, lane 0 adds them in index order -- the chain of dependent additions is all that is
-      // left on one thread
-      acc = 0;
-      double* sp = s_prod[threadIdx.x >> 5];
-      for (int c0 = 0; c0 < d; c0 += 256) {
-        const int c = c0 + lane * 8;
-        if (c < d) {
-          const uint4 xv = *(const uint4*)(xr + c), wv = __ldg((const uint4*)(wr + c));
-          const uint16_t* xb = (const uint16_t*)&xv;
-          const uint16_t* wb = (const uint16_t*)&wv;
-#pragma unroll
-          for (int j = 0; j < 8; j++) sp[lane * 8 + j] = (double)bf16_bits_to_f32(wb[j]) * (double)bf16_bits_to_f32(xb[j]);
-        }
-        __syncwarp();
-        if (lane == 0) {
-          const int n = min(256, d - c0);
-          for (int j = 0; j < n; j++) acc += sp[j];
-        }
-        __syncwarp();
-      }
-    }
-    if (lane == 0) logits[(size_t)t * E + e] = (float)acc;
+    const float v = exact_logit(xr, wr, d, s_prod[threadIdx.x >> 5], lane);
+    if (lane == 0) logits[(size_t)t * E + e] = v;
   }
 }
 
@@ -467,20 +424,31 @@ cudaError_t launch_router_flag(const float* logits, int T, int E, int k, float r
   return cudaGetLastError();
 }
 
-cudaError_t launch_router_dots(const void* x_bf16, const void* w_bf16, int T, int E, int d, float* logits,
-                               cudaStream_t st) {
-  const size_t smem = (size_t)kExTok * d * 2;
+template <int TOK>
+static cudaError_t launch_dots(const uint16_t* x, const uint16_t* w, int T, int E, int d, float* logits, cudaStream_t st) {
+  const size_t smem = (size_t)TOK * d * 2;
   static size_t smem_set = 0;
   if (smem > smem_set) {
-    cudaError_t e = cudaFuncSetAttribute(k_router_dots, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(k_router_dots<TOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     smem_set = smem;
   }
-  long long jobs = (long long)((T + kExTok - 1) / kExTok) * ((E + kExExp - 1) / kExExp);
+  long long jobs = (long long)((T + TOK - 1) / TOK) * ((E + kExExp - 1) / kExExp);
   int blocks = (int)(jobs < 148 * 3 ? jobs : 148 * 3);
   if (blocks < 1) blocks = 1;
-  k_router_dots<<<blocks, 256, smem, st>>>((const uint16_t*)x_bf16, (const uint16_t*)w_bf16, T, E, d, logits);
-  return cudaGetLastError();
+  return launch_pdl(k_router_dots<TOK>, dim3(blocks), dim3(256), smem, st, x, w, T, E, d, logits);
+}
+
+cudaError_t launch_router_dots(const void* x_bf16, const void* w_bf16, int T, int E, int d, float* logits,
+                               cudaStream_t st) {
+  // As many tokens beside one another as still give every SM a block: 16 tokens x 64 experts in eights were
+  // 16 blocks and 15 us.
+  const long long chunks = (E + kExExp - 1) / kExExp;
+  const uint16_t *x = (const uint16_t*)x_bf16, *w = (const uint16_t*)w_bf16;
+  if ((T + 7) / 8 * chunks >= 148) return launch_dots<8>(x, w, T, E, d, logits, st);
+  if ((T + 3) / 4 * chunks >= 148) return launch_dots<4>(x, w, T, E, d, logits, st);
+  if ((T + 1) / 2 * chunks >= 148) return launch_dots<2>(x, w, T, E, d, logits, st);
+  return launch_dots<1>(x, w, T, E, d, logits, st);
 }
 
 cudaError_t launch_router_pairs(const void* x_bf16, const void* w_bf16, const int32_t* pairs, const int32_t* count,
