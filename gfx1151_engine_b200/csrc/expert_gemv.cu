@@ -164,7 +164,7 @@ __device__ __forceinline__ uint32_t bf16x2_to_f16x2(uint32_t w) {
 
 template <bool UP, int FMT, int KPW>
 __global__ void __launch_bounds__(kThreads, 1)
-k_gemv(const GemvParams p) {
+k_gemv(const __grid_constant__ GemvParams p) {
   using M = Map<FMT, KPW>;
   constexpr int kRows = M::kRows, kRed = M::kRed;
   extern __shared__ __align__(16) uint8_t gsm[];
@@ -624,8 +624,8 @@ int shared_ctas(int T, int k, int E, int rows) {
   double unused = 1.0;
   for (int i = 0; i < T; i++) unused *= idle;
   const double routed = E * (1.0 - unused) * 1.02, shared = (T + rows - 1) / rows;
-  const int n = (int)(148.0 * shared / (routed + shared) + 0.5);
-  return n < 1 ? 1 : n > 74 ? 74 : n;
+  const int n = (int)(148.0 * shared / (routed + shared)) + 1;  // rounded up: a CTA less would be the one that all wait for
+  return n > 74 ? 74 : n;
 }
 
 }  // namespace

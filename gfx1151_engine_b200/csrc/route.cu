@@ -14,6 +14,7 @@
 // memory, no dependence on block scheduling order.
 #include "kernels.h"
 #include "route_block.cuh"
+#include "tc.h"
 
 namespace b200moe {
 
@@ -163,7 +164,7 @@ k_router_topk(const float* __restrict__ logits, int T, int E, int k, int32_t* __
 // Decode / verify (T <= 16, T*k <= 256): the whole routing stage in one block (route_block.cuh). Warps 0..15 route,
 // warps 16..31 form the shared expert's gates.
 __global__ void __launch_bounds__(1024)
-k_route_block(const RouteIn q) {
+k_route_block(const __grid_constant__ RouteIn q) {
   extern __shared__ __align__(16) uint8_t rsm[];
   __shared__ uint8_t row_token[kSmallPairs];
   __shared__ double gpart[16 * 16];
@@ -201,7 +202,8 @@ __global__ void __launch_bounds__(kMaxExperts)
 k_route_scan(int32_t* __restrict__ blockcnt, int nblk, int E, int pairs, int T, TileCut cut,
              int32_t* __restrict__ eoff, Run* __restrict__ runs, int32_t* __restrict__ n_runs,
              Tile* __restrict__ tiles, Tile* __restrict__ tiles_narrow, Tile* __restrict__ tiles_sh, int32_t* __restrict__ n_tiles) {
-  __shared__ __align__(16) int s_a[kMaxExperts];
+  __shared__ __align__(4) uint16_t s_bin[kMaxExperts / 32][kTcTileN + 8];  // ragged tiles of a size: per warp, then in the warps before
+  __shared__ int s_gt[256], s_gw[8];                          // larger ones, of all
   __shared__ unsigned long long s_w[kMaxExperts / 32];
   __shared__ int s_wc[kMaxExperts / 32], s_saved[kMaxExperts / 32];
   const int e = threadIdx.x, lane = e & 31, warp = e >> 5;
@@ -211,21 +213,16 @@ k_route_scan(int32_t* __restrict__ blockcnt, int nblk, int E, int pairs, int T, 
   if (e < E) {
     // exclusive prefix down this expert's column of the chunk counts; the loads of sixteen
     // rows are issued together so that the walk does not pay one memory latency per chunk
-    int b = 0;
-    for (; b + 16 <= nblk; b += 16) {
+    for (int b = 0; b < nblk; b += 16) {
       int c[16];
 #pragma unroll
-      for (int i = 0; i < 16; i++) c[i] = blockcnt[(size_t)(b + i) * E + e];
+      for (int i = 0; i < 16; i++) c[i] = b + i < nblk ? blockcnt[(size_t)(b + i) * E + e] : 0;
 #pragma unroll
-      for (int i = 0; i < 16; i++) {
-        blockcnt[(size_t)(b + i) * E + e] = cnt;
-        cnt += c[i];
-      }
-    }
-    for (; b < nblk; b++) {
-      const int c = blockcnt[(size_t)b * E + e];
-      blockcnt[(size_t)b * E + e] = cnt;
-      cnt += c;
+      for (int i = 0; i < 16; i++)
+        if (b + i < nblk) {
+          blockcnt[(size_t)(b + i) * E + e] = cnt;
+          cnt += c[i];
+        }
     }
   }
   // three inclusive scans side by side: counts (low 32 bits) and non-empty flags, full tiles
@@ -256,8 +253,40 @@ k_route_scan(int32_t* __restrict__ blockcnt, int nblk, int E, int pairs, int T, 
     s_w[warp] = ab;
     s_wc[warp] = c;
   }
-  s_a[e] = part;
-  const int wide_parts = __syncthreads_count(part > cut.narrow);
+  for (int i = e; i < (int)sizeof(s_bin) / 4; i += kMaxExperts) ((uint32_t*)s_bin)[i] = 0;
+  __syncthreads();
+  const unsigned same = __match_any_sync(0xffffffffu, part);
+  if (lane == __ffs(same) - 1) s_bin[warp][part] = (uint16_t)__popc(same);
+  __syncthreads();
+  // rank of the ragged tile among all ragged tiles: larger first, ties to the lower id (a loop over the 512 sizes took
+  // most of this kernel's 17 us on a short prompt)
+  const int bin = 255 - e;
+  int above = 0;
+  if (e < 256) {
+    int tot = 0;
+    if (bin <= kTcTileN)
+#pragma unroll
+      for (int w = 0; w < kMaxExperts / 32; w++) {
+        const int n = s_bin[w][bin];
+        s_bin[w][bin] = (uint16_t)tot;
+        tot += n;
+      }
+    above = tot;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, above, o);
+      if (lane >= o) above += v;
+    }
+    if (lane == 31) s_gw[warp] = above;
+    above -= tot;
+  }
+  __syncthreads();
+  if (e < 256) {
+    for (int w = 0; w < warp; w++) above += s_gw[w];
+    s_gt[bin] = above;
+  }
+  __syncthreads();
+  const int nparts = s_gt[0], wide_parts = s_gt[cut.narrow], rank = s_gt[part] + s_bin[warp][part] + __popc(same & ((1u << lane) - 1u));
   unsigned long long ab_all = 0;
   int c_all = 0;
 #pragma unroll
@@ -288,15 +317,6 @@ k_route_scan(int32_t* __restrict__ blockcnt, int nblk, int E, int pairs, int T, 
   };
   const int full0 = c - nfull;
   for (int j = 0; j < nfull; j++) put(full0 + j, Tile{e, first + j * tile_cap, tile_cap});
-  // rank of the ragged tile among all ragged tiles: larger first, ties to the lower id
-  int rank = 0, nparts = 0;
-#pragma unroll 4
-  for (int o = 0; o < kMaxExperts; o += 4) {
-    const int4 q = *(const int4*)(s_a + o);
-    nparts += (q.x > 0) + (q.y > 0) + (q.z > 0) + (q.w > 0);
-    rank += (q.x > part || (q.x == part && o < e)) + (q.y > part || (q.y == part && o + 1 < e)) +
-            (q.z > part || (q.z == part && o + 2 < e)) + (q.w > part || (q.w == part && o + 3 < e));
-  }
   if (part > 0) put(total_full + rank, Tile{e, first + nfull * tile_cap, part});
   // tiles of the shared expert: all T tokens in token order, rows behind the routed ones
   const int nsh = (T + cut.shared - 1) / cut.shared;
