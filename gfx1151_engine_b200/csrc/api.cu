@@ -52,6 +52,16 @@ constexpr long long kMinSavedWork = 2ll * 148 * 4096 * 128 / 3;
 // blocks: they fill SMs beside the routed ones, so that more and shorter items end earlier. Wide / narrow: 144
 // items (768 tokens, mid 768) 288 / 282 us, 384 (1536, mid 1024) 871 / 868, 576 (2304, mid 1024) 906 / 937.
 constexpr int kSharedNarrowItems = 384;
+// Experts of such a call with no more rows than one pass of the decode GEMV serves (8, 4 in the GGUF formats) take the
+// GEMV, which decodes a 128 x 64 block of weights in 250 cycles against 330 to 400, and the tensor-core launches run
+// beside it with the rest. That costs two more launches, 10 to 15 us, and gains 0.09 us per million weights of a
+// projection: the line lies at 160 million in such experts, which only the device can count (k_route_scan). It is
+// not asked where the average is above 5/4 of those rows: even routing then leaves less than a third of the experts there.
+// Without / with, us, cold L2, even routing and skews 0.5 and 1: 512 experts of 4096 x 1024, 24 tokens 423 / 351,
+// 269 / 239, 148 / 155; 100 tokens 892 / 698, 496 / 427, 208 / 204; 400 tokens 1026 / 916, 872 / 751, 339 / 317; 51
+// tokens in Q4_K / Q5_1 733 / 587, 409 / 353, 181 / 179; 512 of 2560 x 640 + shared, 51 tokens 310 / 267, 193 / 181, 101 / 112;
+// 500 tokens 476 / 463, 425 / 390, 202 / 204; 64 of 2048 x 512, 64 tokens 71 / 87 (all below the line: without).
+constexpr long long kMinFewWork = 160000000;
 
 struct b200moe_ctx {
   b200moe_config cfg{};
@@ -744,7 +754,12 @@ static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const
   // (no expert saves more than two tiles in 2 * 64 + 1 rows; the small routing writes one list)
   const bool split = few && T > 16 && T * k * 2 >= min_saved * (2 * kTcNarrowN + 1), narrow = few && !split;
   const bool sh_narrow = few && (long long)(T / kTcNarrowN) * (mid / 64) <= kSharedNarrowItems;
-  const TileCut cut{narrow ? kTcNarrowN : h->tile_cap, sh_narrow ? kTcNarrowN : h->tile_cap, split ? kTcNarrowN : 0, min_saved};
+  const int min_few = (int)((kMinFewWork + (long long)d * mid - 1) / ((long long)d * mid));
+  const int pass_rows = std::min(gemv_rows(L.gu.fmt), gemv_rows(L.dn.fmt));
+  const bool mixed = T > 16 && !simt && !L.i4r && c.gemm_impl == B200MOE_GEMM_AUTO && 4 * T * k <= 5 * pass_rows * E && few &&
+                     std::min(E, T * k) >= min_few && (d << L.gu.act_shift) <= gemv_max_k() && (mid << L.dn.act_shift) <= gemv_max_mid();
+  const TileCut cut{narrow ? kTcNarrowN : h->tile_cap, sh_narrow ? kTcNarrowN : h->tile_cap, split ? kTcNarrowN : 0, min_saved,
+                    mixed ? pass_rows : 0, min_few};
   // (the shared expert's images are q4cp: it can ride along only with q4cp routed experts)
   const bool gemv = simt && c.gemm_impl == B200MOE_GEMM_AUTO &&
                     (!shared || (L.gu.fmt == kQ4CP && L.dn.fmt == kQ4CP)) &&
@@ -787,7 +802,7 @@ static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const
                              h->rb.n_runs, (__half*)h->hid, h->status_dev, in_block ? &route : nullptr, st));
     if (ev) CU_TRY(h, cudaEventRecord(ev[3], st));
     CU_TRY(h, launch_down_gemv(L.dn, shared ? &L.sh_dn : nullptr, (const __half*)h->hid, T, k, E, d, mid,
-                               h->rb.runs, h->rb.n_runs, (float*)h->pairs, h->status_dev, in_block ? h->rb.ready : nullptr, st));
+                               h->rb.runs, h->rb.n_runs, h->pairs, false, h->status_dev, in_block ? h->rb.ready : nullptr, st));
     if (ev) CU_TRY(h, cudaEventRecord(ev[4], st));
     CU_TRY(h, launch_combine_f32((const float*)h->pairs, h->rb.pw, h->rb.pairids, T, k, d,
                                  shared ? pairs : -1, out, st, h->hc_w4, h->hc_state, in_block ? h->rb.ready : nullptr));
@@ -823,7 +838,7 @@ static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const
     auto stage_tc = [&](auto launch, const Image& img, const Image* sh, __half* out16) -> cudaError_t {
       const Tile* first = split ? h->rb.tiles_narrow : h->rb.tiles;
       cudaError_t e = launch(h->tc, img, first, h->rb.n_tiles + (split ? 2 : 0), split ? h->max_tiles_narrow : h->max_tiles,
-                             out16, h->status_dev, st, TcLaunch{few, false});
+                             out16, h->status_dev, st, TcLaunch{few, mixed});  // (mixed: beside the GEMV in front)
       if (e == cudaSuccess && sh)
         e = launch(h->tc, *sh, h->rb.tiles_sh, h->rb.n_tiles + 1, h->max_tiles_sh, out16, h->status_dev, st,
                    TcLaunch{sh_narrow, true});
@@ -858,8 +873,18 @@ static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const
     CU_TRY(h, launch_scatter_f16(x, T, k, d, shared ? pairs : -1, h->x_sorted, gate_w, h->rb, st));
     n++;
     if (ev) CU_TRY(h, cudaEventRecord(ev[2], st));
+    if (mixed) {
+      CU_TRY(h, launch_up_gemv(L.gu, nullptr, x, T, k, E, d, mid, h->rb.tokidx, h->rb.runs, h->rb.n_runs, (__half*)h->hid, h->status_dev,
+                               nullptr, st));
+      n++;
+    }
     CU_TRY(h, stage_tc(launch_up_tc, L.gu, shared ? &L.sh_gu : nullptr, (__half*)h->hid));
     if (ev) CU_TRY(h, cudaEventRecord(ev[3], st));
+    if (mixed) {
+      CU_TRY(h, launch_down_gemv(L.dn, nullptr, (const __half*)h->hid, T, k, E, d, mid, h->rb.runs, h->rb.n_runs, h->pairs, true,
+                                 h->status_dev, nullptr, st));
+      n++;
+    }
     CU_TRY(h, stage_tc(launch_down_tc, L.dn, shared ? &L.sh_dn : nullptr, (__half*)h->pairs));
     if (ev) CU_TRY(h, cudaEventRecord(ev[4], st));
     CU_TRY(h, launch_combine_f16((const __half*)h->pairs, h->rb.pw, h->rb.pairids, T, k, d,

@@ -146,21 +146,25 @@ k_combine_small(const float* __restrict__ pairs, const float* __restrict__ pw,
   const int t = blockIdx.x;
   const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
   pdl_trigger();
-  pdl_wait();
-  if (ready && (t | blockIdx.y | threadIdx.x) == 0) *ready = 0;  // the lists are about to be free for the next call
-  if (c >= d) return;
   const int n = k + (shared_row0 >= 0 ? 1 : 0);
   float4 v[kMaxTopK + 1];
+  int row[kMaxTopK + 1];
   float w[kMaxTopK + 1];
+  // The lists come from a kernel before the one in front, where that one routes (ready): the down GEMV has waited
+  // for it before it let this kernel start, so that they can be read ahead of the wait.
+  if (!ready) pdl_wait();
 #pragma unroll
-  for (int s = 0; s < kMaxTopK + 1; s++) {
+  for (int s = 0; s < kMaxTopK + 1; s++)
     if (s < n) {
-      const int row = s < k ? pairids[(size_t)t * k + s] : shared_row0 + t;
-      const bool live = row >= 0;  // negative: a pair the bucketing dropped (expert id outside [0, E))
-      w[s] = live ? pw[row] : 0.f;
-      v[s] = live ? *(const float4*)(pairs + (size_t)row * d + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+      row[s] = s < k ? pairids[(size_t)t * k + s] : shared_row0 + t;
+      w[s] = row[s] >= 0 ? pw[row[s]] : 0.f;  // negative: a pair the bucketing dropped (expert id outside [0, E))
     }
-  }
+  if (ready) pdl_wait();
+  if (ready && (t | blockIdx.y | threadIdx.x) == 0) *ready = 0;  // the lists are about to be free for the next call
+  if (c >= d) return;
+#pragma unroll
+  for (int s = 0; s < kMaxTopK + 1; s++)
+    if (s < n) v[s] = row[s] >= 0 ? *(const float4*)(pairs + (size_t)row[s] * d + c) : make_float4(0.f, 0.f, 0.f, 0.f);
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
   for (int s = 0; s < kMaxTopK + 1; s++) {

@@ -37,7 +37,7 @@ namespace {
 
 constexpr int kWarps = 16;            // compute warps of a CTA
 constexpr int kThreads = kWarps * 32;
-constexpr int kMaxSubs = 448;         // passes over an expert's weights
+constexpr int kMaxSubs = 640;         // passes over an expert's weights
 constexpr uint32_t kOffLow = 2048;    // the dynamic allocation must start at or below this (its absolute shared address)
 
 // Shared memory map, absolute shared addresses.
@@ -77,7 +77,8 @@ struct GemvParams {
   const uint16_t* x;     // gate/up: bf16 [T][d]
   const int32_t* tokidx;
   __half* hid;           // gate/up writes, down reads: fp16 [rows][mid] = silu(gate) * up
-  float* out;            // down: pairs fp32 [rows][d]
+  float* out;            // down: pairs fp32 [rows][d], or null:
+  __half* out16;         // the same in fp16
   int32_t* status;
   RouteIn route;         // gate/up, fused: the routing is done here (runs, n_runs, tokidx are not read)
   int fused;
@@ -205,7 +206,56 @@ k_gemv(const __grid_constant__ GemvParams p) {
   };
   uint8_t* const smem = gsm - (uint32_t)__cvta_generic_to_shared(gsm);  // smem + A is the generic pointer of absolute shared address A
   uint8_t* const row_token = smem + M::kRowTok;
+  const int KB = im.n_kblocks, ash = im.act_shift;
+  const int slice = warp % p.slices, team = warp / p.slices;
+  const int kb0 = slice * KPW, nk = min(KPW, KB - kb0);
+  // Activations of the slice, B operands. kQ4CP: lane (g, t) holds row g, elements 8t .. 8t+7 of both halves of every
+  // K block. Else row g >> 1, half g & 1, in bv for half 0 and in bw for half 1, zeros in the other.
+  uint32_t bv[KPW][4], bw[KPW][4];
+  float xs[KPW][2];             // GGUF: sums of the activations of row t, halves 0 and 1
+  auto load_rows = [&](bool live, size_t row) {
+    auto load8 = [&](int i, int h, uint32_t* v) {
+      uint4 u = make_uint4(0, 0, 0, 0);
+      if (live && i < nk) {
+        const size_t o = row * p.K + (size_t)((kb0 + i) >> ash) * kTileK + h * 32 + t * 8;
+        u = UP ? __ldg((const uint4*)(p.x + o)) : *(const uint4*)(p.hid + o);
+      }
+      v[0] = UP ? bf16x2_to_f16x2(u.x) : u.x;
+      v[1] = UP ? bf16x2_to_f16x2(u.y) : u.y;
+      v[2] = UP ? bf16x2_to_f16x2(u.z) : u.z;
+      v[3] = UP ? bf16x2_to_f16x2(u.w) : u.w;
+    };
+#pragma unroll
+    for (int i = 0; i < KPW; i++) {
+      if (FMT == kQ4CP) {
+        load8(i, 0, bv[i]);
+        load8(i, 1, bw[i]);
+      } else {
+        uint32_t v[4];
+        load8(i, g & 1, v);
+        if (FMT == kQ4K) {  // pairs of elements q and q + 4
+          const uint32_t w0 = v[0], w1 = v[1];
+          v[0] = __byte_perm(w0, v[2], 0x5410);
+          v[1] = __byte_perm(w0, v[2], 0x7632);
+          v[2] = __byte_perm(w1, v[3], 0x5410);
+          v[3] = __byte_perm(w1, v[3], 0x7632);
+        }
+        float c[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          bv[i][q] = (g & 1) ? 0u : v[q];
+          bw[i][q] = (g & 1) ? v[q] : 0u;
+          mma16816(c, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u, bv[i][q], bw[i][q]);
+        }
+        xs[i][0] = c[0];
+        xs[i][1] = c[1];
+      }
+    }
+  };
   if (UP) pdl_wait();
+  // One token: its activations serve every pass, and travel while the routing runs.
+  const bool one = UP && p.fused && p.route.T == 1;
+  if (one) load_rows((FMT == kQ4CP ? g : g >> 1) == 0, 0);
   if (UP && p.fused) {
     // ---- routing (route_block.cuh), by every CTA of the routed experts for itself; the first of them leaves the
     // lists for the kernels behind. Its scratch is the place of the partial sums, which come later ----
@@ -227,7 +277,7 @@ k_gemv(const __grid_constant__ GemvParams p) {
     }
     pdl_trigger();  // (behind the flag: the down kernel starts when every CTA has come here)
   } else {
-    pdl_trigger();
+    if (UP) pdl_trigger();
     // ---- passes: every expert's rows, kRows at a time ----
     // The down kernel reads the run list before its wait: the routing kernel was complete before any CTA of the
     // gate/up kernel triggered, or, where that kernel routes, the flag tells.
@@ -276,9 +326,6 @@ k_gemv(const __grid_constant__ GemvParams p) {
     __syncthreads();
   }
   // ---- this team's share: units c0 .. c1-1 of all passes. A unit = one sub-block column, 32 tile rows over the whole K ----
-  const int KB = im.n_kblocks, ash = im.act_shift;
-  const int slice = warp % p.slices, team = warp / p.slices;
-  const int kb0 = slice * KPW, nk = min(KPW, KB - kb0);
   const int upr = im.n_mtiles * 4;  // units of a pass
   int c0, n_units;
   {
@@ -328,7 +375,12 @@ k_gemv(const __grid_constant__ GemvParams p) {
     }
   };
   for (uint32_t s = 0; s < M::kSlots; s++) issue();
-  if (!UP) pdl_wait();
+  if (!UP) {
+    // The launch behind comes behind this wait: the combine of a decode call reads its lists before its own wait, and
+    // a tensor-core launch may run beside this one.
+    pdl_wait();
+    pdl_trigger();
+  }
   if (UP && p.fused && sh && p.route.gate_w) {
     gate_block(p.route, blockIdx.x, p.n_sh, tid, (double*)(smem + M::kPart), [] { __syncthreads(); });
     __syncthreads();  // (its scratch is the place of the partial sums)
@@ -339,10 +391,6 @@ k_gemv(const __grid_constant__ GemvParams p) {
   uint32_t c_slot = 0, c_ph = 0;
   int sub = c0 / upr, j = c0 % upr, cnt = 0, first = 0;
   bool fresh = true;
-  // Activations of the slice, B operands. kQ4CP: lane (g, t) holds row g, elements 8t .. 8t+7 of both halves of every
-  // K block. Else row g >> 1, half g & 1, in bv for half 0 and in bw for half 1, zeros in the other.
-  uint32_t bv[KPW][4], bw[KPW][4];
-  float xs[KPW][2];             // GGUF: sums of the activations of row t, halves 0 and 1
   const uint32_t lut_a = (uint32_t)lane * 4, lut_b = lut_a + (UP && im.dual_book ? 128u : 0u);
   const uint32_t lane_src = (uint32_t)(lane >> 4) * kHalfBytes + (uint32_t)(lane & 15) * 16;
   const uint32_t part0 = M::kPart + (uint32_t)(team * p.slices) * (kSubRows * kRows * 4);
@@ -378,7 +426,9 @@ k_gemv(const __grid_constant__ GemvParams p) {
           if (lane < 16)
             p.hid[(size_t)(ufirst + r) * p.mid + uj * 16 + lane] = __float2half_rn(sat_f16(silu_f32(tot[r]) * up));
         } else {
-          p.out[(size_t)(ufirst + r) * (upr * kSubRows) + uj * kSubRows + lane] = tot[r];
+          const size_t o = (size_t)(ufirst + r) * (upr * kSubRows) + uj * kSubRows + lane;
+          if (p.out) p.out[o] = tot[r];
+          else p.out16[o] = __float2half_rn(sat_f16(tot[r]));
         }
       }
     }
@@ -497,43 +547,7 @@ k_gemv(const __grid_constant__ GemvParams p) {
       size_t row = first + at;
       if (UP && live) row = !p.fused ? p.tokidx[row] : sh ? row - p.route.T * p.route.k : row_token[row];
       if (!live) row = 0;
-      auto load8 = [&](int i, int h, uint32_t* v) {
-        uint4 u = make_uint4(0, 0, 0, 0);
-        if (live && i < nk) {
-          const size_t o = row * p.K + (size_t)((kb0 + i) >> ash) * kTileK + h * 32 + t * 8;
-          u = UP ? __ldg((const uint4*)(p.x + o)) : *(const uint4*)(p.hid + o);
-        }
-        v[0] = UP ? bf16x2_to_f16x2(u.x) : u.x;
-        v[1] = UP ? bf16x2_to_f16x2(u.y) : u.y;
-        v[2] = UP ? bf16x2_to_f16x2(u.z) : u.z;
-        v[3] = UP ? bf16x2_to_f16x2(u.w) : u.w;
-      };
-#pragma unroll
-      for (int i = 0; i < KPW; i++) {
-        if (FMT == kQ4CP) {
-          load8(i, 0, bv[i]);
-          load8(i, 1, bw[i]);
-        } else {
-          uint32_t v[4];
-          load8(i, g & 1, v);
-          if (FMT == kQ4K) {  // pairs of elements q and q + 4
-            const uint32_t w0 = v[0], w1 = v[1];
-            v[0] = __byte_perm(w0, v[2], 0x5410);
-            v[1] = __byte_perm(w0, v[2], 0x7632);
-            v[2] = __byte_perm(w1, v[3], 0x5410);
-            v[3] = __byte_perm(w1, v[3], 0x7632);
-          }
-          float c[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-          for (int q = 0; q < 4; q++) {
-            bv[i][q] = (g & 1) ? 0u : v[q];
-            bw[i][q] = (g & 1) ? v[q] : 0u;
-            mma16816(c, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u, bv[i][q], bw[i][q]);
-          }
-          xs[i][0] = c[0];
-          xs[i][1] = c[1];
-        }
-      }
+      if (!one) load_rows(live, row);
     }
     float acc[2][2][kAcc] = {};  // [16-row block][weight row g, g + 8][activation rows of the lane]
 #pragma unroll
@@ -631,6 +645,7 @@ int shared_ctas(int T, int k, int E, int rows) {
 }  // namespace
 
 int gemv_max_runs() { return 192; }
+int gemv_rows(int fmt) { return fmt == kQ4CP ? Map<kQ4CP, 4>::kRows : Map<kQ4K, 4>::kRows; }
 int gemv_max_k() { return kWarps * 4 * kTileK; }
 int gemv_max_mid() { return kWarps / 2 * 4 * kTileK; }
 
@@ -649,14 +664,15 @@ cudaError_t launch_up_gemv(const Image& img, const Image* img_sh, const void* x_
 }
 
 cudaError_t launch_down_gemv(const Image& img, const Image* img_sh, const __half* hid16, int T, int k, int E, int d, int mid,
-                             const Run* runs, const int32_t* n_runs, float* pairs_f32, int32_t* status, int32_t* ready,
-                             cudaStream_t st) {
+                             const Run* runs, const int32_t* n_runs, void* pairs, bool pairs_f16, int32_t* status,
+                             int32_t* ready, cudaStream_t st) {
   GemvParams p{};
   p.img = img;
   if (img_sh) p.img_sh = *img_sh, p.n_sh = shared_ctas(T, k, E, Map<kQ4CP, 4>::kRows);
   p.runs = runs; p.n_runs = n_runs; p.K = mid; p.mid = mid;
   p.hid = const_cast<__half*>(hid16);
-  p.out = pairs_f32; p.status = status; p.ready = ready;
+  if (pairs_f16) p.out16 = (__half*)pairs; else p.out = (float*)pairs;
+  p.status = status; p.ready = ready;
   if (img.fmt == kQ4K) return launch_fmt<false, kQ4K>(p, st);
   if (img.fmt == kQ51) return launch_fmt<false, kQ51>(p, st);
   return launch_fmt<false, kQ4CP>(p, st);

@@ -92,6 +92,8 @@ cudaError_t launch_router_topk(const float* logits, int T, int E, int k, int32_t
 // `routed` rows make at least min_saved fewer of them than tiles of `narrow` rows; else all rows are cut to that.
 struct TileCut {
   int routed, shared, narrow = 0, min_saved = 0;
+  // > 0: if at least min_few experts have rows, but no more than gemv_rows, those get no tiles; runs / n_runs[0] list them and no others.
+  int gemv_rows = 0, min_few = 0;
 };
 cudaError_t launch_route(const RouteBuffers& rb, const int32_t* ids, const float* w, int stride,
                          int T, int k, int E, const TileCut& cut, cudaStream_t st, int* launches);
@@ -135,6 +137,7 @@ cudaError_t launch_down_simt(const Image& img, const float* hid_f32, int d, int 
 
 // ---- expert_gemv.cu (decode / verify path) ----
 int gemv_max_runs();
+int gemv_rows(int fmt);  // rows of an expert that one pass over its weights serves
 int gemv_max_k();     // largest d
 int gemv_max_mid();   // largest mid
 // img_sh: the shared expert's image (nullptr: none); its run is runs[kMaxExperts].
@@ -145,7 +148,8 @@ cudaError_t launch_up_gemv(const Image& img, const Image* img_sh, const void* x_
                            const int32_t* tokidx, const Run* runs, const int32_t* n_runs,
                            __half* hid16, int32_t* status, const RouteIn* route, cudaStream_t st);
 cudaError_t launch_down_gemv(const Image& img, const Image* img_sh, const __half* hid16, int T, int k, int E, int d, int mid,
-                             const Run* runs, const int32_t* n_runs, float* pairs_f32, int32_t* status, int32_t* ready, cudaStream_t st);
+                             const Run* runs, const int32_t* n_runs, void* pairs, bool pairs_f16, int32_t* status, int32_t* ready,
+                             cudaStream_t st);
 
 // ---- decode.cu (q4cp decode / verify, T <= decode_max_tokens(), as one kernel) ----
 // Routing (from logits, or from the caller's ids / w when logits is null), gate/up GEMV + SwiGLU,

@@ -237,8 +237,11 @@ k_route_scan(int32_t* __restrict__ blockcnt, int nblk, int E, int pairs, int T, 
     for (int w = 0; w < kMaxExperts / 32; w++) all += s_saved[w];
     if (all < cut.min_saved) tile_cap = cut.narrow;
   }
-  const int nfull = cnt / tile_cap, part = cnt % tile_cap;
-  unsigned long long ab = (unsigned long long)(uint32_t)cnt | (unsigned long long)(cnt > 0) << 32;
+  // experts with few rows to the decode GEMV, where there are enough of them
+  const bool by_gemv = cut.gemv_rows > 0 && __syncthreads_count(cnt > 0 && cnt <= cut.gemv_rows) >= cut.min_few && cnt <= cut.gemv_rows;
+  const bool listed = cnt > 0 && (by_gemv || cut.gemv_rows == 0);
+  const int nfull = by_gemv ? 0 : cnt / tile_cap, part = by_gemv ? 0 : cnt % tile_cap;
+  unsigned long long ab = (unsigned long long)(uint32_t)cnt | (unsigned long long)listed << 32;
   int c = nfull;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -308,7 +311,7 @@ k_route_scan(int32_t* __restrict__ blockcnt, int nblk, int E, int pairs, int T, 
     n_runs[1] = 1;  // the shared expert's run, kept at runs[kMaxExperts]
     runs[kMaxExperts] = Run{0, pairs, T};
   }
-  if (cnt > 0) runs[(int)(ab >> 32) - 1] = Run{e, first, cnt};
+  if (listed) runs[(int)(ab >> 32) - 1] = Run{e, first, cnt};
   // full tiles first, then the ragged ones from large to small: those with more than cut.narrow rows on tiles
   const int n_wide = tile_cap > cut.narrow ? total_full + wide_parts : 0;
   auto put = [&](int i, const Tile& t) {

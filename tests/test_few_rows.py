@@ -1,0 +1,83 @@
+"""Calls of more than 16 tokens with few rows per expert on a large layer: experts with as many rows as one pass of the
+decode GEMV serves (8, 4 in the GGUF formats) take that, the others the tensor-core kernels beside it -- if the
+former are enough: 123 experts of 2560 x 512. Against the oracle on both sides of either line, and captured in a graph."""
+import numpy as np
+import pytest
+
+import oracle
+from gfx1151_engine_b200 import synth
+from helpers import assert_output_close, bf16_out_to_f32, bf16_tensor
+from test_gpu_parity import bits, make_op, run_layer
+
+pytestmark = pytest.mark.gpu
+E = 128
+
+# tokens, top-k, rows of the 128 experts
+CASES = {
+    "some above": (40, 8, [9, 20, 12, 30, 10] + [8] * 15 + [7] + [2] * 5 + [1] * 102),          # 123 of at most 8 rows
+    "one expert short": (40, 8, [9] * 6 + [8] * 18 + [2] * 18 + [1] * 86),                    # 122: all on the tensor cores
+    "at most 4": (48, 4, [30, 5, 6] + [4] * 5 + [2] * 11 + [1] * 109),                        # 125 of at most 4 rows
+    "all": (32, 4, [1] * 128),
+    "popular": (200, 4, [200, 200, 150, 65, 17] + [4] * 15 + [1] * 108),                      # wide tiles and narrow ones too
+}
+
+
+def routed_to(T, topk, counts):
+    """Logits that give expert e counts[e] rows (sum T * topk, no token twice to one expert), spread over the tokens."""
+    left = np.array(counts)
+    assert left.sum() == T * topk and left.max() <= T
+    lg = np.zeros((T, E), np.float32)
+    for t in range(T):
+        take = np.argsort(-left, kind="stable")[:topk]
+        left[take] -= 1
+        lg[t, take] = 8.0 + 0.25 * np.arange(topk)
+    assert (left == 0).all()
+    return lg
+
+
+@pytest.fixture(scope="module", params=["q4cp", "gguf"])
+def layer(request):
+    spec = synth.LayerSpec(experts=E, topk=8, d=2560, mid=512, shared=request.param == "q4cp", fmt=request.param)
+    return spec, synth.make_layer(spec, seed=95)
+
+
+@pytest.mark.parametrize("case", CASES)
+def test_against_oracle(cuda, layer, case):
+    T, topk, rows = CASES[case]
+    spec = synth.LayerSpec(**dict(vars(layer[0]), topk=topk))
+    counts = np.array(rows)[np.random.default_rng(T).permutation(E)]
+    logits = routed_to(T, topk, counts)
+    xb = synth.make_x(synth.rng_for(95, 9), T, spec.d)
+    op = make_op(cuda, spec, T, layer=layer[1])
+    y = run_layer(cuda, op, spec, xb, logits)
+    n = min(T, 48)
+    y_o, ids_o, _ = oracle.moe_forward(spec, layer[1], synth.bf16_bits_to_f32(xb[:n]), logits=logits[:n])
+    assert np.array_equal(op.get_routing(T)[0][:n, :topk], ids_o[:, :topk])
+    assert np.isfinite(y).all()
+    assert_output_close(y[:n], y_o, case)
+    assert np.array_equal(bits(run_layer(cuda, op, spec, xb, logits)), bits(y))
+    op.close()
+
+
+def test_captured_call_replays_with_new_inputs(cuda, layer):
+    torch = cuda
+    spec = layer[0]
+    T = 40
+    op = make_op(torch, spec, T, layer=layer[1])
+    xs = [synth.make_x(synth.rng_for(96, i), T, spec.d) for i in range(2)]
+    lgs = [routed_to(T, 8, CASES["some above"][2]), synth.make_logits(synth.rng_for(96, 11), T, E)]
+    want = [run_layer(torch, op, spec, x, lg) for x, lg in zip(xs, lgs)]
+    x, lg = bf16_tensor(torch, xs[0], (T, spec.d)), torch.from_numpy(lgs[0]).cuda()
+    out = torch.empty((T, spec.d), dtype=torch.bfloat16, device="cuda")
+    st = torch.cuda.Stream()
+    st.wait_stream(torch.cuda.current_stream())
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=st):
+        op.moe_b(0, x, lg, out, stream=st.cuda_stream)
+    for i in (1, 0):
+        x.copy_(bf16_tensor(torch, xs[i], (T, spec.d)))
+        lg.copy_(torch.from_numpy(lgs[i]))
+        g.replay()
+        torch.cuda.synchronize()
+        assert np.array_equal(bits(bf16_out_to_f32(torch, out)), bits(want[i]))
+    op.close()
