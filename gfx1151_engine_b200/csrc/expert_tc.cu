@@ -450,18 +450,19 @@ k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ C
         const uint32_t bytes = (n_pad <= 16 ? 16 : n_pad <= 64 ? 64 : n_pad <= 128 ? 128 : kTcTileN) * 128;
         // The dequantising warps fetch their packed weights into registers only one own pair ahead
         // of their use (~18 KB in flight per SM). This thread, which has time to spare, also asks for
-        // both tiles of a later pair -- of this item or of the next one -- to be brought into L2
-        // with bulk prefetches, so that the fetch finds them there. Measured: 6 % on a launch
-        // whose tiles all have ~10 rows (short MMAs: the fetch latency shows), nothing on the
-        // benchmark's mix; with every weight read served from L2 (a diagnostic run on one expert's
-        // tiles) such a launch gains 23 %.
+        // the tiles of two later pairs -- of this item or of the next one -- to be brought into L2
+        // with four bulk prefetches, so that the fetch finds them there. Measured: 6 % on a launch
+        // whose tiles all have ~10 rows (short MMAs: the fetch latency shows); with every weight read
+        // served from L2 (a diagnostic run on one expert's tiles) such a launch gains 23 %. One pair at a time
+        // is twice the instructions of this thread: 2048 tokens on i4r experts 751 us against 723, 4096 of
+        // 4096 x 1024 from host buffers 2372 / 2320, 16384 tokens 5040 / 5010; four pairs are level with two.
         constexpr size_t w_sub_b = sub_bytes(FMT);
         const size_t w_col_b = KB * w_sub_b;  // from one sub-block to the next
         const uint8_t* w_this = img.mtile(t.expert, it % img.n_mtiles);
         const uint8_t* w_next =
             it + (int)gridDim.x < n_items ? img.mtile(t_ahead.expert, (it + (int)gridDim.x) % img.n_mtiles) : nullptr;
         for (int pp = 0; pp < NP && ok; pp++, pi++) {
-          if (!kNarrow && p.l2_ahead > 0) {
+          if (!kNarrow && p.l2_ahead > 0 && (pp & 1) == 0) {  // two pairs at a time: they lie side by side in a sub-block
             int q = pp + 2 * p.l2_ahead;
             const uint8_t* b2 = w_this;
             if (q >= NP) {
@@ -472,7 +473,7 @@ k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ C
 #pragma unroll
               for (int s = 0; s < kTileM / kSubRows; s++)
                 asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(b2 + s * w_col_b + (size_t)(2 * q) * w_sub_b),
-                             "r"((uint32_t)(min(2, KB - 2 * q) * (int)w_sub_b))
+                             "r"((uint32_t)(min(4, KB - 2 * q) * (int)w_sub_b))
                              : "memory");
             }
           }
