@@ -73,45 +73,85 @@ k_rot_in(const uint16_t* __restrict__ x, const float* __restrict__ pre, const in
   }
 }
 
-__device__ __forceinline__ void load4(const __half* p, float (&v)[4]) {
-  const uint2 u = *(const uint2*)p;
-  const float2 a = __half22float2(*(const __half2*)&u.x), b = __half22float2(*(const __half2*)&u.y);
-  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+__device__ __forceinline__ void load8(const __half* p, float* v) {
+  const uint4 u = *(const uint4*)p;
+  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const float2 f = __half22float2(*(const __half2*)&w[i]);
+    v[2 * i] = f.x;
+    v[2 * i + 1] = f.y;
+  }
+}
+
+// The same transform by eight lanes: lane l holds elements 8l .. 8l+7 and 64+8l .. 64+8l+7, so index bits 0-2 and 6 are
+// butterflies inside the lane and bits 3-5 lane shuffles: 12 a vector and warp, against 20 with a vector per warp.
+__device__ __forceinline__ void fwht128_8(float (&v)[16], int lane) {
+#pragma unroll
+  for (int b = 1; b < 16; b <<= 1)
+#pragma unroll
+    for (int i = 0; i < 16; i++)
+      if (!(i & b)) {
+        const float p = v[i], q = v[i | b];
+        v[i] = p + q;
+        v[i | b] = p - q;
+      }
+#pragma unroll
+  for (int bit = 1; bit < 8; bit <<= 1) {
+    const float sign = (lane & bit) ? -1.f : 1.f;
+#pragma unroll
+    for (int i = 0; i < 16; i++) v[i] = fmaf(sign, v[i], __shfl_xor_sync(0xffffffffu, v[i], bit));
+  }
 }
 
 // hr[row][b*128 ..] = fp16( Hn( suh_dn * silu(g) * u ) ) with g = svh_gu * Hn(z[row][b*128 ..]),
-// u = svh_gu[mid + ..] * Hn(z[row][mid + b*128 ..]); one warp per (row, block of mid)
-// (k_i4r_mid of the reference, src/gpu/parts/28_kernels_hgn_v2.inc:98-143).
+// u = svh_gu[mid + ..] * Hn(z[row][mid + b*128 ..]) (k_i4r_mid of the reference,
+// src/gpu/parts/28_kernels_hgn_v2.inc:98-143). Eight lanes per (row, block b = blockIdx.y of mid), whose planes stay in
+// registers. With a warp per vector, 60 shuffles and 64-bit index arithmetic bounded it, not its 6 bytes a hidden
+// value: 20480 rows of 640 took 45 us (78 MB: 12 us at the copy bandwidth); a 2048-token call gained 2 us with this alone.
 __global__ void __launch_bounds__(256)
 k_i4r_mid(const __half* __restrict__ z, const float* __restrict__ svh_gu, const float* __restrict__ suh_dn,
-          long long rows, int mid, __half* __restrict__ hr) {
+          int rows, int mid, __half* __restrict__ hr) {
   const int lane = threadIdx.x & 31;
-  const int nb = mid >> 7;
+  const int c = blockIdx.y * 128 + (lane & 7) * 8;
+  float sg[16], su[16], sd[16];
+#pragma unroll
+  for (int i = 0; i < 16; i++) {
+    const int e = c + (i & 7) + (i >> 3) * 64;
+    sg[i] = svh_gu[e];
+    su[i] = svh_gu[mid + e];
+    sd[i] = suh_dn[e];
+  }
   pdl_trigger();
   pdl_wait();
-  const long long total = rows * nb;
-  for (long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < total;
-       w += (long long)gridDim.x * (blockDim.x >> 5)) {
-    const long long row = w / nb;
-    const int c = (int)(w % nb) * 128 + lane * 4;
-    float g[4], u[4];
-    load4(z + row * 2 * mid + c, g);
-    load4(z + row * 2 * mid + mid + c, u);
-    fwht128(g, lane);
-    fwht128(u, lane);
-    const float4 sg = *(const float4*)(svh_gu + c), su = *(const float4*)(svh_gu + mid + c), sd = *(const float4*)(suh_dn + c);
-    const float sgv[4] = {sg.x, sg.y, sg.z, sg.w}, suv[4] = {su.x, su.y, su.z, su.w}, sdv[4] = {sd.x, sd.y, sd.z, sd.w};
-    float h[4];
+  // (whole warps stay in the loop: the shuffles take all lanes)
+  for (int r0 = (blockIdx.x * 8 + (threadIdx.x >> 5)) * 4; r0 < rows; r0 += gridDim.x * 32) {
+    const int row = r0 + (lane >> 3);
+    const bool live = row < rows;
+    float g[16], u[16];
+    const __half* zr = z + (size_t)(live ? row : r0) * 2 * mid + c;
+    load8(zr, g);
+    load8(zr + 64, g + 8);
+    load8(zr + mid, u);
+    load8(zr + mid + 64, u + 8);
+    fwht128_8(g, lane);
+    fwht128_8(u, lane);
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const float gv = g[j] * kRs128 * sgv[j], uv = u[j] * kRs128 * suv[j];
-      h[j] = silu_f32(gv) * uv * sdv[j];
+    for (int i = 0; i < 16; i++) {
+      const float gv = g[i] * kRs128 * sg[i], uv = u[i] * kRs128 * su[i];
+      g[i] = silu_f32(gv) * uv * sd[i];
     }
-    fwht128(h, lane);
-    uint2 o;
-    o.x = pack_f16x2_sat(h[0] * kRs128, h[1] * kRs128);
-    o.y = pack_f16x2_sat(h[2] * kRs128, h[3] * kRs128);
-    *(uint2*)(hr + row * mid + c) = o;
+    fwht128_8(g, lane);
+    if (!live) continue;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      uint4 o;
+      o.x = pack_f16x2_sat(g[8 * h] * kRs128, g[8 * h + 1] * kRs128);
+      o.y = pack_f16x2_sat(g[8 * h + 2] * kRs128, g[8 * h + 3] * kRs128);
+      o.z = pack_f16x2_sat(g[8 * h + 4] * kRs128, g[8 * h + 5] * kRs128);
+      o.w = pack_f16x2_sat(g[8 * h + 6] * kRs128, g[8 * h + 7] * kRs128);
+      *(uint4*)(hr + (size_t)row * mid + c + h * 64) = o;
+    }
   }
 }
 
@@ -132,11 +172,11 @@ cudaError_t launch_rot_in(const void* x_bf16, const float* pre, const int32_t* p
 
 cudaError_t launch_i4r_mid(const __half* z, const float* svh_gu, const float* suh_dn, int rows, int mid, __half* hr,
                            cudaStream_t st) {
-  long long warps = (long long)rows * (mid >> 7);
-  long long blocks = (warps + 7) / 8;
-  if (blocks > 148 * 16) blocks = 148 * 16;
-  if (blocks < 1) blocks = 1;
-  return launch_pdl(k_i4r_mid, dim3((unsigned)blocks), dim3(256), 0, st, z, svh_gu, suh_dn, (long long)rows, mid, hr);
+  const int nb = mid >> 7, per_wave = 148 * 4;  // blocks of 32 rows a wave takes (registers: two a SM, two waves)
+  int gx = (rows + 31) / 32;
+  if ((long long)gx * nb > per_wave) gx = (per_wave + nb - 1) / nb;
+  if (gx < 1) gx = 1;
+  return launch_pdl(k_i4r_mid, dim3((unsigned)gx, (unsigned)nb), dim3(256), 0, st, z, svh_gu, suh_dn, rows, mid, hr);
 }
 
 cudaError_t launch_f16_to_f32(const void* src_f16_dev, float* dst, int n, cudaStream_t st) {
