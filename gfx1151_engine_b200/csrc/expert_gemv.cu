@@ -9,15 +9,15 @@
 // on 512 code bytes, of which 16 were table lookups and 16 the activations, and stood at 2.7 TB/s. Here:
 //   * mma.m16n8k16 forms the products (exact) and sums (fp32). Its A operand is 16 weight rows: ldmatrix deals the
 //     packed codes of a row out to the four lanes of a quad, 8 codes each, a code BYTE becomes an fp16 pair. Scales
-//     stay in fp32: the K slots of the two 32-groups of a K block meet their activations in DIFFERENT columns of B
-//     (a column = a row of activations x a half), zeros elsewhere, so that a column is one group's unscaled sum.
-//     Eight columns = up to four rows of an expert in one pass over its weights.
+//     stay in fp32: no sum runs over two 32-groups. q4cp takes one group per instruction and up to EIGHT rows of an
+//     expert in the columns of B; the GGUF formats, whose constants cost more per row, put the two groups of a K block
+//     into different columns (zeros elsewhere) and serve FOUR rows per pass over the weights.
 //   * B never moves: a warp owns at most four K blocks (its slice) of all the rows its team works on, and the
-//     activations of a slice are 4 registers per K block and lane (8 with the zeros).
+//     activations of a slice are 8 registers per K block and lane.
 //   * q4cp: a code byte is decoded by one lookup in a 256-entry half2 table replicated per lane in shared memory
 //     (no bank conflicts; a line is 256 bytes, so the address is one byte permute): 32 of the 48 wavefronts per
 //     32 x 64 block, the load pipe is 76 % busy with them. GGUF: the codes are masked into fp16 bit patterns,
-//     code * 2^-24 (denormal, exact), no lookup; 2^24 goes into the fp32 constants.
+//     code * 2^-24 (denormal, exact), no lookup; 2^24 goes into the fp32 constants. Issue slots bound those.
 //   * Weights come by bulk copies into a ring of three slots of two K blocks per warp (110 KB in flight per SM), one
 //     copy and one wait per slot; the image keeps a slice's K blocks together (common.cuh).
 //   * A unit of work = 32 rows (16 hidden outputs: gate and up rows meet in one warp) over the whole K. The slices
@@ -25,9 +25,14 @@
 //     that nobody waits at a barrier. A row's sums depend on nothing but its slice cut, a function of the shape.
 //   * Persistent; units are cut into equal contiguous shares per team. The shared expert has CTAs of its own, so
 //     that a CTA needs one image's tables.
-// us of the two kernels, the multiply-add form / this one, 4096 x 1024 with shared expert: T = 1 35 / 26, T = 5
-// 120 / 80, T = 13 288 / 177 (gate/up 4.85 TB/s); Q4_K / Q5_1 T = 5 128 / 88 (gate/up 5.0 TB/s, down 4.0: the
-// fifth bits); 64 experts of 2048 x 512, 16 tokens (2.2 rows an expert) 90 / 33.
+//   * The gate/up kernel does the routing of a decode call itself (route_block.cuh), every CTA for itself; the last
+//     CTA leaves the lists for the kernels behind, the shared expert's CTAs form its gates.
+//   * Longer calls with few rows per expert come here with a run list of k_route_scan instead (api.cu, kMinFewWork).
+// us of the two kernels, the multiply-add form / this one, 4096 x 1024 with shared expert: T = 1 35 / 28, T = 5
+// 120 / 84, T = 13 288 / 191 (gate/up 4.65 TB/s); Q4_K / Q5_1 T = 5 128 / 92 (gate/up 4.6 TB/s, down 4.0: the
+// fifth bits); 64 experts of 2048 x 512, 16 tokens (2.2 rows an expert) 90 / 38. (Four q4cp rows per pass: 26 / 80 / 177 and
+// 33; but of the 211 experts of a 77-token prompt one pass of eight serves 191, one of four 171.) One call, T = 1, from the end of the
+// kernel in front: routing 4.3 us, first copies and activations 3, gate/up 11, hand-over 2, down 6, combine 5.
 #include "kernels.h"
 #include "route_block.cuh"
 
@@ -257,21 +262,21 @@ k_gemv(const __grid_constant__ GemvParams p) {
   const bool one = UP && p.fused && p.route.T == 1;
   if (one) load_rows((FMT == kQ4CP ? g : g >> 1) == 0, 0);
   if (UP && p.fused) {
-    // ---- routing (route_block.cuh), by every CTA of the routed experts for itself; the first of them leaves the
-    // lists for the kernels behind. Its scratch is the place of the partial sums, which come later ----
+    // ---- routing (route_block.cuh), by every CTA of the routed experts for itself; the last one, whose share is
+    // never the larger, leaves the lists and weights for the kernels behind. Its scratch is the place of the partial sums, which come later ----
     static_assert(kRouteBlockBytes <= kRed * kWarps * kSubRows * kRows * 4, "the routing's scratch");
     if (sh) {
       n_subs = (p.route.T + kRows - 1) / kRows;
       if (tid < n_subs) put_pass(tid, 0, p.route.T * p.route.k + tid * kRows, min(kRows, p.route.T - tid * kRows));
     } else {
-      n_subs = route_block(p.route, *(RouteBlock*)(smem + M::kPart), (int)blockIdx.x == p.n_sh, kRows, row_token,
+      n_subs = route_block(p.route, *(RouteBlock*)(smem + M::kPart), blockIdx.x == gridDim.x - 1, kRows, row_token,
                            [&](int expert, int first, int count, int at) {
                              for (int i = 0; i * kRows < count; i++) put_pass(at + i, expert, first + i * kRows, min(kRows, count - i * kRows));
                            });
       n_subs = min(n_subs, kMaxSubs);
     }
     __syncthreads();
-    if ((int)blockIdx.x == p.n_sh && tid == 0) {
+    if (blockIdx.x == gridDim.x - 1 && tid == 0) {
       __threadfence();
       asm volatile("st.release.gpu.global.b32 [%0], 1;" ::"l"(p.route.rb.ready) : "memory");
     }

@@ -146,11 +146,12 @@ k_router_topk(const float* __restrict__ logits, int T, int E, int k, int32_t* __
   pdl_wait();
   if (t >= T) return;
   // The ids from the logits' order where that decides them (route_block.cuh), which saves E double exponentials and
-  // divisions and k rounds of arg-max: 16384 tokens x 512 experts XX us, before that XX.
+  // divisions and k rounds of arg-max: 16384 tokens x 512 experts 24 us (33.6 MB: 5 us at the copy bandwidth), with them 63;
+  // 77 tokens 5 us and 11.
   float vr, wv;
   int id;
   const int C = warp_leaders(logits + (size_t)t * E, E, k, lane, s_p[warp], vr, id);
-  if (C > 0 && warp_topk(C, vr, k, lane, wv)) {
+  if (C > 0 && warp_topk(C, vr, k, lane, true, wv)) {
     for (int i = lane; i < stride; i += 32) {  // zeros behind the k
       ids[(size_t)t * stride + i] = i < k ? id : 0;
       w[(size_t)t * stride + i] = i < k ? wv : 0.f;

@@ -1,7 +1,9 @@
 // route_block.cuh -- the whole routing stage of a decode / verify call (T <= 16, T*k <= 256) by the 512 threads of
 // one block: router top-k (a warp per token), stable bucketing of the pairs by expert, offsets, run and tile
 // lists. Used by k_route_block (route.cu) and by the gate/up GEMV (expert_gemv.cu), whose blocks each repeat it for
-// themselves: that costs every block 2 us, but no launch, and no lists that travel through memory.
+// themselves: 4.3 us of every block at T = 1, 5.8 at T = 13 (a chain of latencies: loads of the logits, shuffles, five
+// barriers), against a launch of its own, 6.3 us at T = 1 and 12.7 at T = 5 (one block for all tokens in double
+// arithmetic: 15 us for 16 tokens of 64 experts), and lists that travelled through memory.
 //   * Selection. "Largest probability, ties to the lowest id" is "largest logit, ties to the lowest id" unless two
 //     different logits round to one float probability (exp and the division by the sum are monotone): the ids come
 //     from the logits' order. Where two of a token's k+1 largest are closer than 1e-6, or a logit is not finite, that
@@ -95,11 +97,13 @@ __device__ __forceinline__ int warp_leaders(const float* lg, int E, int k, int l
   return C;
 }
 
-// Top-k ids and weights from the order of the logits: lane r < k gets the r-th. False where that does not decide.
-__device__ __forceinline__ bool warp_topk(int C, float vr, int k, int lane, float& wv) {
+// Top-k ids and weights from the order of the logits: lane r < k gets the r-th (weights only if asked for). False where
+// that does not decide.
+__device__ __forceinline__ bool warp_topk(int C, float vr, int k, int lane, bool weights, float& wv) {
   const float vn = __shfl_down_sync(0xffffffffu, vr, 1), mx = __shfl_sync(0xffffffffu, vr, 0);
   // neighbours in the order closer than 1e-6: their probabilities might round to one float
   if (__any_sync(0xffffffffu, lane < k && lane + 1 < C && !(vr - vn > 1e-6f * fmaxf(1.f, fabsf(vr)))) || C < k) return false;
+  if (!weights) return true;
   const double e = lane < k ? exp((double)vr - (double)mx) : 0.0;
   double kept = 0;
 #pragma unroll 1
@@ -155,7 +159,7 @@ __device__ __forceinline__ int route_block(const RouteIn& q, RouteBlock& sc, boo
         if (__any_sync(0xffffffffu, lane < k && lane + 1 < C && vr - vn < margin)) C = -1;
         if (lane == 0) sc.cand[warp][0] = kth - 2.f * margin;
       }
-      const bool ok = C > 0 && !q.exact && warp_topk(C, vr, k, lane, wv);
+      const bool ok = C > 0 && !q.exact && warp_topk(C, vr, k, lane, write, wv);
       if (ok && lane < k) {
         sc.key[warp * k + lane] = id;
         sc.w[warp * k + lane] = wv;

@@ -1,7 +1,8 @@
 // route_small.cuh -- the whole routing stage for a few tokens (T*k <= 256) as a device function
 // run by 512 threads of one block: shared expert's sigmoid gate, router top-k, stable bucketing
-// by rank counting, expert offsets, run and tile lists. Used by k_route_small (route.cu) and by
-// the fused decode kernel (decode.cu), where every block repeats it for itself.
+// by rank counting, expert offsets, run and tile lists. Used by
+// route_block.cuh for single tokens and by the fused decode kernel (decode.cu) for all of a call's, where their logits' order
+// does not decide.
 // Arithmetic and tie rule: see route.cu.
 #pragma once
 #include "kernels.h"
@@ -57,7 +58,7 @@ struct RouteSmallOut {
 // more warps, which do not take part)
 __device__ __forceinline__ void rs_sync() { asm volatile("bar.sync 1, 512;" ::: "memory"); }
 
-// Run by threads 0..511 of a block (tid = threadIdx.x < 512). Inputs as k_route_small's; tile_cap: most rows
+// Run by threads 0..511 of a block (tid = threadIdx.x < 512). tile_cap: most rows
 // of one tile (T, at most 16, is below it).
 // GU: 16-byte pieces of the shared expert's gate product a lane loads before it uses any (a
 // register-hungry prefetch: 8 where the body has the whole SM's registers, 2 inside a larger kernel).

@@ -52,7 +52,7 @@ enum {
 
 /* How decode / verify calls (T <= decode_max_tokens) of q4cp layers run. */
 enum {
-  B200MOE_DECODE_AUTO = 0,   /* routing, gate/up GEMV, down GEMV, combine as four kernels chained by programmatic dependent launch */
+  B200MOE_DECODE_AUTO = 0,   /* gate/up GEMV (with the routing), down GEMV, combine as three kernels chained by programmatic dependent launch */
   B200MOE_DECODE_FUSED = 1   /* T <= 8: ONE kernel for the whole call; every expert is read once for all the rows that use it
                                 (the reference's expert dedup, src/gpu/parts/26_kernels_moe_gguf.inc:749-793), bit-identical to T = 1 */
 };
