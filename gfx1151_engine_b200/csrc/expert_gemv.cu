@@ -18,8 +18,8 @@
 //     (no bank conflicts; a line is 256 bytes, so the address is one byte permute): 32 of the 48 wavefronts per
 //     32 x 64 block, the load pipe is 76 % busy with them. GGUF: the codes are masked into fp16 bit patterns,
 //     code * 2^-24 (denormal, exact), no lookup; 2^24 goes into the fp32 constants. Issue slots bound those.
-//   * Weights come by bulk copies into a ring of three slots of two K blocks per warp (110 KB in flight per SM), one
-//     copy and one wait per slot; the image keeps a slice's K blocks together (common.cuh).
+//   * Weights come by bulk copies into a ring of two or three slots of two K blocks per warp (74 to 123 KB in flight per
+//     SM), one copy and one wait per slot; the image keeps a slice's K blocks together (common.cuh).
 //   * A unit of work = 32 rows (16 hidden outputs: gate and up rows meet in one warp) over the whole K. The slices
 //     leave their sums in shared memory and go on; they take turns at adding up the unit BEFORE, in slice order, so
 //     that nobody waits at a barrier. A row's sums depend on nothing but its slice cut, a function of the shape.
@@ -50,13 +50,16 @@ constexpr uint32_t kOffLow = 2048;    // the dynamic allocation must start at or
 template <int FMT, int KPW>
 struct Map {
   static constexpr int kRows = FMT == kQ4CP ? 8 : 4;  // rows of an expert that one pass over its weights serves
-  static constexpr int kRed = FMT == kQ4CP ? 2 : 4;   // partial-sum buffers of a team
+  // Partial-sum buffers of a team, and ring slots per warp. Shared memory holds four and two or two and three for q4cp
+  // (four and three without the table): four let the slices drift further apart, 31.1 against 32.1 us at T = 1, 195.4 / 196.6
+  // at T = 13; slices of three K blocks keep two and two.
+  static constexpr int kRed = FMT == kQ4CP && KPW == 3 ? 2 : 4;
   static constexpr int kGroup = KPW == 4 ? 2 : KPW;   // K blocks per ring slot
   static constexpr int kGroups = KPW / kGroup;        // slots per unit
   static constexpr uint32_t kLut = kOffLow;  // kQ4CP: 256 lines of {32 lanes x 4 B, first book}{32 x 4 B, second book}
   static constexpr uint32_t kRing = kLut + (FMT == kQ4CP ? 65536u : 0u);
   static constexpr uint32_t kSub = (uint32_t)sub_bytes(FMT), kSlot = kGroup * kSub;
-  static constexpr uint32_t kSlots = KPW == 3 ? 2 : 3;  // per warp
+  static constexpr uint32_t kSlots = KPW == 3 || FMT == kQ4CP ? 2 : 3;
   static constexpr uint32_t kScr = FMT == kQ4K ? 512 : 0;  // per warp: the rows' constants as floats
   static constexpr uint32_t kPart = kRing + kWarps * kSlots * kSlot;          // partial sums [kRed][warp][rows in fours][32 weight rows][4]
   static constexpr uint32_t kBar = kPart + kRed * kWarps * kSubRows * kRows * 4;
