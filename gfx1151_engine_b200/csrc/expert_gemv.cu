@@ -261,9 +261,9 @@ k_gemv(const __grid_constant__ GemvParams p) {
     }
   };
   if (UP) pdl_wait();
-  // One token: its activations serve every pass, and travel while the routing runs.
+  // One token: its activations serve every row of every pass (a caller's ids may repeat), and travel while the routing runs.
   const bool one = UP && p.fused && p.route.T == 1;
-  if (one) load_rows((FMT == kQ4CP ? g : g >> 1) == 0, 0);
+  if (one) load_rows(true, 0);
   if (UP && p.fused) {
     // ---- routing (route_block.cuh), by every CTA of the routed experts for itself; the last one, whose share is
     // never the larger, leaves the lists and weights for the kernels behind. Its scratch is the place of the partial sums, which come later ----

@@ -1,0 +1,41 @@
+"""Decode GEMV with more rows of an expert than one pass over its weights serves (8, 4 in the GGUF formats): ids that
+repeat within a token."""
+import numpy as np
+import pytest
+
+import oracle
+from gfx1151_engine_b200 import synth
+from helpers import assert_output_close, bf16_out_to_f32, bf16_tensor
+from test_gpu_parity import make_op
+
+pytestmark = pytest.mark.gpu
+
+
+def expert_outputs(spec, layer, x):
+    """[experts][T][d]: every expert's output for every token, weight 1."""
+    one = synth.LayerSpec(**dict(vars(spec), topk=1, shared=False))
+    logits = np.full((spec.experts, len(x), spec.experts), -50.0, np.float32)
+    for e in range(spec.experts):
+        logits[e, :, e] = 50.0
+    return np.stack([oracle.moe_forward(one, layer, x, logits=logits[e])[0] for e in range(spec.experts)])
+
+
+@pytest.mark.parametrize("T", [1, 2, 5])
+@pytest.mark.parametrize("fmt", ["q4cp", "gguf"])
+def test_repeated_ids(cuda, fmt, T):
+    torch = cuda
+    spec = synth.LayerSpec(experts=16, topk=16, d=512, mid=128, fmt=fmt)
+    layer = synth.make_layer(spec, seed=96)
+    xb = synth.make_x(synth.rng_for(96, 9), T, spec.d)
+    y_e = expert_outputs(spec, layer, synth.bf16_bits_to_f32(xb))
+    w = synth.rng_for(96, 1).uniform(0.5, 1.5, size=(T, 16)).astype(np.float32)
+    w /= w.sum(axis=1, keepdims=True)
+    op = make_op(torch, spec, 16, layer=layer)
+    for row in ([3] * 16, [3] * 9 + [5] * 5 + [0, 7], [2, 9, 2, 11, 4, 9, 0, 1, 3, 5, 6, 7, 8, 10, 12, 13]):
+        ids = np.stack([np.roll(row, t) for t in range(T)]).astype(np.int32)
+        out = torch.full((T, spec.d), float("nan"), dtype=torch.bfloat16, device="cuda")
+        op.moe_q4w_run(0, bf16_tensor(torch, xb, (T, spec.d)), torch.from_numpy(ids).cuda(), torch.from_numpy(w).cuda(), out)
+        op.synchronize()
+        want = sum(w[:, s, None] * y_e[ids[:, s], np.arange(T)] for s in range(16))
+        assert_output_close(bf16_out_to_f32(torch, out), want, "%s T=%d %r" % (fmt, T, row))
+    op.close()
