@@ -798,15 +798,16 @@ static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const
   if (gemv) {
     // decode / verify: persistent dequant GEMV, routed and shared expert in one launch each
     if (ev) CU_TRY(h, cudaEventRecord(ev[2], st));
-    CU_TRY(h, launch_up_gemv(L.gu, shared ? &L.sh_gu : nullptr, x, T, k, E, d, mid, h->rb.tokidx, h->rb.runs,
-                             h->rb.n_runs, (__half*)h->hid, h->status_dev, in_block ? &route : nullptr, st));
+    CU_TRY(h, launch_up_gemv(L.gu, shared ? &L.sh_gu : nullptr, x, T, k, E, d, mid, h->rb.tokidx, h->rb.runs, h->rb.n_runs,
+                             gemv_passes(L.gu.fmt, T, k, E), (__half*)h->hid, h->status_dev, in_block ? &route : nullptr, &n, st));
     if (ev) CU_TRY(h, cudaEventRecord(ev[3], st));
     CU_TRY(h, launch_down_gemv(L.dn, shared ? &L.sh_dn : nullptr, (const __half*)h->hid, T, k, E, d, mid,
-                               h->rb.runs, h->rb.n_runs, h->pairs, false, h->status_dev, in_block ? h->rb.ready : nullptr, st));
+                               h->rb.runs, h->rb.n_runs, gemv_passes(L.dn.fmt, T, k, E), h->pairs, false, h->status_dev,
+                               in_block ? h->rb.ready : nullptr, &n, st));
     if (ev) CU_TRY(h, cudaEventRecord(ev[4], st));
     CU_TRY(h, launch_combine_f32((const float*)h->pairs, h->rb.pw, h->rb.pairids, T, k, d,
                                  shared ? pairs : -1, out, st, h->hc_w4, h->hc_state, in_block ? h->rb.ready : nullptr));
-    n += 3;
+    n++;
   } else if (simt) {
     const int max_runs = std::min(E, pairs);
     if (ev) CU_TRY(h, cudaEventRecord(ev[2], st));
@@ -874,16 +875,14 @@ static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const
     n++;
     if (ev) CU_TRY(h, cudaEventRecord(ev[2], st));
     if (mixed) {
-      CU_TRY(h, launch_up_gemv(L.gu, nullptr, x, T, k, E, d, mid, h->rb.tokidx, h->rb.runs, h->rb.n_runs, (__half*)h->hid, h->status_dev,
-                               nullptr, st));
-      n++;
+      CU_TRY(h, launch_up_gemv(L.gu, nullptr, x, T, k, E, d, mid, h->rb.tokidx, h->rb.runs, h->rb.n_runs, std::min(E, pairs),
+                               (__half*)h->hid, h->status_dev, nullptr, &n, st));  // (a pass each)
     }
     CU_TRY(h, stage_tc(launch_up_tc, L.gu, shared ? &L.sh_gu : nullptr, (__half*)h->hid));
     if (ev) CU_TRY(h, cudaEventRecord(ev[3], st));
     if (mixed) {
-      CU_TRY(h, launch_down_gemv(L.dn, nullptr, (const __half*)h->hid, T, k, E, d, mid, h->rb.runs, h->rb.n_runs, h->pairs, true,
-                                 h->status_dev, nullptr, st));
-      n++;
+      CU_TRY(h, launch_down_gemv(L.dn, nullptr, (const __half*)h->hid, T, k, E, d, mid, h->rb.runs, h->rb.n_runs,
+                                 std::min(E, pairs), h->pairs, true, h->status_dev, nullptr, &n, st));
     }
     CU_TRY(h, stage_tc(launch_down_tc, L.dn, shared ? &L.sh_dn : nullptr, (__half*)h->pairs));
     if (ev) CU_TRY(h, cudaEventRecord(ev[4], st));

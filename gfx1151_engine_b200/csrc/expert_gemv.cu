@@ -36,13 +36,15 @@
 #include "kernels.h"
 #include "route_block.cuh"
 
+#include <algorithm>
+
 namespace b200moe {
 
 namespace {
 
 constexpr int kWarps = 16;            // compute warps of a CTA
 constexpr int kThreads = kWarps * 32;
-constexpr int kMaxSubs = 640;         // passes over an expert's weights
+constexpr int kMaxSubs = 640;         // passes over an expert's weights that a launch takes
 constexpr uint32_t kOffLow = 2048;    // the dynamic allocation must start at or below this (its absolute shared address)
 
 // Shared memory map, absolute shared addresses.
@@ -79,6 +81,7 @@ struct GemvParams {
   const Run* runs;       // routed runs [n_runs[0]]; the shared run sits at runs[kMaxExperts]
   const int32_t* n_runs;
   int n_sh;              // CTAs 0 .. n_sh-1 work on the shared expert, the others on the routed ones
+  int pass0;             // first pass of this launch, of the routed experts and of the shared one alike
   int K;                 // d (gate/up) or mid (down)
   int mid;
   int slices, teams;     // warps that share a unit's K blocks; units in work at a time
@@ -207,7 +210,8 @@ k_gemv(const __grid_constant__ GemvParams p) {
   }
   int n_subs;
   auto put_pass = [&](int i, int expert, int first, int count) {
-    if (i < kMaxSubs) {
+    i -= p.pass0;
+    if ((unsigned)i < (unsigned)kMaxSubs) {
       sts32(M::kSubs + i * 8, (uint32_t)expert | (uint32_t)count << 16);
       sts32(M::kSubs + i * 8 + 4, (uint32_t)first);
     }
@@ -267,6 +271,7 @@ k_gemv(const __grid_constant__ GemvParams p) {
   if (UP && p.fused) {
     // ---- routing (route_block.cuh), by every CTA of the routed experts for itself; the last one, whose share is
     // never the larger, leaves the lists and weights for the kernels behind. Its scratch is the place of the partial sums, which come later ----
+    static_assert(kSmallPairs <= kMaxSubs, "a call that is routed here fits one launch");
     static_assert(kRouteBlockBytes <= kRed * kWarps * kSubRows * kRows * 4, "the routing's scratch");
     if (sh) {
       n_subs = (p.route.T + kRows - 1) / kRows;
@@ -276,7 +281,6 @@ k_gemv(const __grid_constant__ GemvParams p) {
                            [&](int expert, int first, int count, int at) {
                              for (int i = 0; i * kRows < count; i++) put_pass(at + i, expert, first + i * kRows, min(kRows, count - i * kRows));
                            });
-      n_subs = min(n_subs, kMaxSubs);
     }
     __syncthreads();
     if (blockIdx.x == gridDim.x - 1 && tid == 0) {
@@ -329,7 +333,7 @@ k_gemv(const __grid_constant__ GemvParams p) {
       if (w < warp) before += v;
       n_subs += v;
     }
-    n_subs = min(n_subs, kMaxSubs);
+    n_subs = min(max(n_subs - p.pass0, 0), kMaxSubs);
     for (int i = 0; i < c; i++) put_pass(before + i, run.expert, run.first + i * kRows, min(kRows, run.count - i * kRows));
     __syncthreads();
   }
@@ -625,8 +629,9 @@ cudaError_t launch_gemv(const GemvParams& p, cudaStream_t st) {
   return launch_pdl(k_gemv<UP, FMT, KPW>, dim3(sms), dim3(kThreads), (size_t)smem, st, p);
 }
 
+// One launch for the passes pass0 .. pass0 + kMaxSubs - 1.
 template <bool UP, int FMT>
-cudaError_t launch_fmt(GemvParams& p, cudaStream_t st) {
+cudaError_t launch_one(GemvParams& p, cudaStream_t st) {
   const int KB = p.img.n_kblocks;
   // The fewest K blocks per warp with which one team covers K, but two at least: more warps at work on a unit beat
   // longer slices (K = 2560: 14 slices of three 85 us at T = 13, 10 of four 95); at K <= 1024 two and four are level.
@@ -637,6 +642,18 @@ cudaError_t launch_fmt(GemvParams& p, cudaStream_t st) {
   if (kpw == 4) return launch_gemv<UP, FMT, 4>(p, st);
   if (kpw == 3) return launch_gemv<UP, FMT, 3>(p, st);
   return launch_gemv<UP, FMT, 2>(p, st);
+}
+
+// Passes that the host cannot count take as many launches as could be needed (a call of up to 16 tokens: one). Each
+// waits for the one before; those beyond the last pass end at once.
+template <bool UP, int FMT>
+cudaError_t launch_fmt(GemvParams& p, int T, int max_passes, int* launches, cudaStream_t st) {
+  if (p.n_sh > 0) max_passes = std::max(max_passes, (T + Map<FMT, 4>::kRows - 1) / Map<FMT, 4>::kRows);
+  for (p.pass0 = 0; p.pass0 == 0 || p.pass0 < max_passes; p.pass0 += kMaxSubs) {
+    if (cudaError_t e = launch_one<UP, FMT>(p, st)) return e;
+    ++*launches;
+  }
+  return cudaSuccess;
 }
 
 // CTAs for the shared expert: its share of the passes that T tokens with even routing make. (Fewer routed
@@ -654,26 +671,30 @@ int shared_ctas(int T, int k, int E, int rows) {
 
 int gemv_max_runs() { return 192; }
 int gemv_rows(int fmt) { return fmt == kQ4CP ? Map<kQ4CP, 4>::kRows : Map<kQ4K, 4>::kRows; }
+int gemv_passes(int fmt, int T, int k, int E) {
+  const int rows = gemv_rows(fmt), runs = T * k < E ? T * k : E;
+  return (T * k + runs * (rows - 1)) / rows;
+}
 int gemv_max_k() { return kWarps * 4 * kTileK; }
 int gemv_max_mid() { return kWarps / 2 * 4 * kTileK; }
 
 cudaError_t launch_up_gemv(const Image& img, const Image* img_sh, const void* x_bf16, int T, int k, int E, int d, int mid,
                            const int32_t* tokidx, const Run* runs, const int32_t* n_runs,
-                           __half* hid16, int32_t* status, const RouteIn* route, cudaStream_t st) {
+                           int max_passes, __half* hid16, int32_t* status, const RouteIn* route, int* launches, cudaStream_t st) {
   GemvParams p{};
   p.img = img;
   if (img_sh) p.img_sh = *img_sh, p.n_sh = shared_ctas(T, k, E, Map<kQ4CP, 4>::kRows);
   p.runs = runs; p.n_runs = n_runs; p.K = d; p.mid = mid;
   p.x = (const uint16_t*)x_bf16; p.tokidx = tokidx; p.hid = hid16; p.status = status;
   if (route) p.route = *route, p.fused = 1;
-  if (img.fmt == kQ4K) return launch_fmt<true, kQ4K>(p, st);
-  if (img.fmt == kQ51) return launch_fmt<true, kQ51>(p, st);
-  return launch_fmt<true, kQ4CP>(p, st);
+  if (img.fmt == kQ4K) return launch_fmt<true, kQ4K>(p, T, max_passes, launches, st);
+  if (img.fmt == kQ51) return launch_fmt<true, kQ51>(p, T, max_passes, launches, st);
+  return launch_fmt<true, kQ4CP>(p, T, max_passes, launches, st);
 }
 
 cudaError_t launch_down_gemv(const Image& img, const Image* img_sh, const __half* hid16, int T, int k, int E, int d, int mid,
-                             const Run* runs, const int32_t* n_runs, void* pairs, bool pairs_f16, int32_t* status,
-                             int32_t* ready, cudaStream_t st) {
+                             const Run* runs, const int32_t* n_runs, int max_passes, void* pairs, bool pairs_f16, int32_t* status,
+                             int32_t* ready, int* launches, cudaStream_t st) {
   GemvParams p{};
   p.img = img;
   if (img_sh) p.img_sh = *img_sh, p.n_sh = shared_ctas(T, k, E, Map<kQ4CP, 4>::kRows);
@@ -681,9 +702,9 @@ cudaError_t launch_down_gemv(const Image& img, const Image* img_sh, const __half
   p.hid = const_cast<__half*>(hid16);
   if (pairs_f16) p.out16 = (__half*)pairs; else p.out = (float*)pairs;
   p.status = status; p.ready = ready;
-  if (img.fmt == kQ4K) return launch_fmt<false, kQ4K>(p, st);
-  if (img.fmt == kQ51) return launch_fmt<false, kQ51>(p, st);
-  return launch_fmt<false, kQ4CP>(p, st);
+  if (img.fmt == kQ4K) return launch_fmt<false, kQ4K>(p, T, max_passes, launches, st);
+  if (img.fmt == kQ51) return launch_fmt<false, kQ51>(p, T, max_passes, launches, st);
+  return launch_fmt<false, kQ4CP>(p, T, max_passes, launches, st);
 }
 
 }  // namespace b200moe

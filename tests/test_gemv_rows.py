@@ -1,12 +1,12 @@
 """Decode GEMV with more rows of an expert than one pass over its weights serves (8, 4 in the GGUF formats): ids that
-repeat within a token."""
+repeat within a token, and calls of more than 16 tokens where decode_max_tokens takes them there."""
 import numpy as np
 import pytest
 
 import oracle
 from gfx1151_engine_b200 import synth
 from helpers import assert_output_close, bf16_out_to_f32, bf16_tensor
-from test_gpu_parity import make_op
+from test_gpu_parity import bits, make_op, run_layer
 
 pytestmark = pytest.mark.gpu
 
@@ -38,4 +38,23 @@ def test_repeated_ids(cuda, fmt, T):
         op.synchronize()
         want = sum(w[:, s, None] * y_e[ids[:, s], np.arange(T)] for s in range(16))
         assert_output_close(bf16_out_to_f32(torch, out), want, "%s T=%d %r" % (fmt, T, row))
+    op.close()
+
+
+# one launch per GEMM holds 640 passes: (T * 8 + 24 * (rows - 1)) / rows at most
+@pytest.mark.parametrize("fmt,T", [("gguf", 40), ("gguf", 311), ("gguf", 330), ("gguf", 700), ("q4cp", 622), ("q4cp", 640), ("q4cp", 1300)])
+def test_decode_max_tokens_above_16(cuda, fmt, T):
+    torch = cuda
+    spec = synth.LayerSpec(experts=24, topk=8, d=256, mid=64, fmt=fmt, shared=fmt == "q4cp")
+    layer = synth.make_layer(spec, seed=97)
+    xb = synth.make_x(synth.rng_for(97, 9), T, spec.d)
+    logits = synth.make_logits(synth.rng_for(97, T), T, spec.experts)
+    y_o, ids_o, _ = oracle.moe_forward(spec, layer, synth.bf16_bits_to_f32(xb), logits=logits)
+    op = make_op(torch, spec, T, layer=layer, decode_max_tokens=T)
+    y = run_layer(torch, op, spec, xb, logits)
+    assert np.array_equal(op.get_routing(T)[0][:, :8], ids_o[:, :8])
+    assert_output_close(y, y_o, "%s T=%d" % (fmt, T))
+    # the fp32 sums of this path, to the bit those of calls of 16
+    for t in (0, (T - 16) // 2, T - 16):
+        assert np.array_equal(bits(run_layer(torch, op, spec, xb[t:t + 16], logits[t:t + 16])), bits(y[t:t + 16])), t
     op.close()
