@@ -219,9 +219,9 @@ __device__ __forceinline__ void wait_shared_ge(const int32_t* ctr, int target, D
 // top-k ids and order from the logits themselves (exp and the division by the sum are
 // monotone, so "largest probability, ties to the lowest id" is "largest logit, ties to the
 // lowest id" unless two different logits round to one float probability) and is a few hundred
-// instructions. Where two logits of a token's k+1 largest are closer than 1e-6 -- the only case in
-// which their probabilities could round to the same float -- or a logit is not finite, the block
-// runs the general body instead, so the ids are the reference's in every case. The weights
+// instructions. Where two logits of a token's k+1 largest are closer than 1e-6, the k-th is more than
+// kMaxSpread below the largest -- else their probabilities could round to the same float -- or a logit is not
+// finite, the block runs the general body instead, so the ids are the reference's in every case. The weights
 // p_i / sum of the selected p come from float exponentials: within ~2e-7 of the reference's
 // (its own rounding of p to float is 6e-8); the sum over all experts cancels and is not formed.
 struct FastScratch {
@@ -328,8 +328,9 @@ __device__ __forceinline__ bool route_fast_select(const DecParams& p, FastScratc
     const float vr = (lane <= k && lane < C) ? fs.sel_v[t][lane] : -INFINITY;
     const int id = (lane < k && lane < C) ? fs.sel_id[t][lane] : 0;
     const float vn = __shfl_down_sync(0xffffffffu, vr, 1);
-    // neighbours in the order closer than 1e-6: their probabilities might round to one float
-    const bool close = lane < k && lane + 1 < C && !(vr - vn > 1e-6f * fmaxf(1.f, fabsf(vr)));
+    // neighbours in the order closer than 1e-6, or a probability that is no normal float: two might round to one float
+    const bool close = (lane < k && lane + 1 < C && !(vr - vn > 1e-6f * fmaxf(1.f, fabsf(vr)))) ||
+                       (lane == k - 1 && !(fs.mx[t] - vr <= kMaxSpread));
     if (__any_sync(0xffffffffu, close) || C < k) {
       if (lane == 0) fs.fallback = 1;
     }

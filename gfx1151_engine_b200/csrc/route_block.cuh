@@ -6,7 +6,8 @@
 // arithmetic: 15 us for 16 tokens of 64 experts), and lists that travelled through memory.
 //   * Selection. "Largest probability, ties to the lowest id" is "largest logit, ties to the lowest id" unless two
 //     different logits round to one float probability (exp and the division by the sum are monotone): the ids come
-//     from the logits' order. Where two of a token's k+1 largest are closer than 1e-6, or a logit is not finite, that
+//     from the logits' order. Where two of a token's k+1 largest are closer than 1e-6, the k-th is so far below the
+//     largest that its probability might not be a normal float (kMaxSpread), or a logit is not finite, that
 //     token takes the general body instead (route_small.cuh: the reference's arithmetic to the letter, out of
 //     line, since its 5000 instructions would be fetched cold by every call).
 //   * Weights: double exponentials of the k selected logits over their sum in rank order; the sum over all experts
@@ -100,9 +101,11 @@ __device__ __forceinline__ int warp_leaders(const float* lg, int E, int k, int l
 // Top-k ids and weights from the order of the logits: lane r < k gets the r-th (weights only if asked for). False where
 // that does not decide.
 __device__ __forceinline__ bool warp_topk(int C, float vr, int k, int lane, bool weights, float& wv) {
-  const float vn = __shfl_down_sync(0xffffffffu, vr, 1), mx = __shfl_sync(0xffffffffu, vr, 0);
+  const float vn = __shfl_down_sync(0xffffffffu, vr, 1), mx = __shfl_sync(0xffffffffu, vr, 0), vk = __shfl_sync(0xffffffffu, vr, k - 1);
   // neighbours in the order closer than 1e-6: their probabilities might round to one float
-  if (__any_sync(0xffffffffu, lane < k && lane + 1 < C && !(vr - vn > 1e-6f * fmaxf(1.f, fabsf(vr)))) || C < k) return false;
+  if (__any_sync(0xffffffffu, lane < k && lane + 1 < C && !(vr - vn > 1e-6f * fmaxf(1.f, fabsf(vr)))) || C < k ||
+      !(mx - vk <= kMaxSpread))
+    return false;
   if (!weights) return true;
   const double e = lane < k ? exp((double)vr - (double)mx) : 0.0;
   double kept = 0;

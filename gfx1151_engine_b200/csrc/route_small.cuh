@@ -17,6 +17,11 @@ constexpr int kStatusBadId = 4;       // status word {4, offending id}: reported
 // and the shared expert's sigmoid gate. Same results as the general kernels below.
 constexpr int kSmallPairs = 256;
 
+// Selection by the logits' order (route_block.cuh, decode.cu): the k-th may lie so far below the largest. Its probability is
+// then at least exp(-80) / kMaxExperts = 3.5e-38, above the smallest normal float (1.2e-38), so that logits 1e-6 apart
+// are several of its steps apart.
+constexpr float kMaxSpread = 80.f;
+
 // Shared-memory scratch of the routing body; NROW = most tokens it is used for (at least 3:
 // the single-token selection keeps its candidate list in rows 1 and 2).
 template <int NROW>
