@@ -45,8 +45,43 @@ __device__ __forceinline__ double shfl_f64(double v, int src) {
   return __hiloint2double(__shfl_sync(0xffffffffu, __double2hiint(v), src), __shfl_sync(0xffffffffu, __double2loint(v), src));
 }
 
+// The same by n rounds of arg-max, n <= 32: for the rare token with more candidates than warp_leaders ranks (a few residues
+// mod 32 hold most of its leaders, or many logits are equal). Value and id.
+static __device__ __noinline__ float2 warp_leaders_rounds(const float* lg, int E, int n, int lane) {
+  float v[16], last = INFINITY;
+  int last_id = -1;
+  float2 mine = make_float2(-INFINITY, 0.f);
+#pragma unroll
+  for (int j = 0; j < 16; j++) v[j] = j * 32 + lane < E ? lg[j * 32 + lane] : -INFINITY;
+  for (int r = 0; r < n; r++) {
+    float bv = -INFINITY;
+    int bi = kMaxExperts;  // none
+#pragma unroll
+    for (int j = 0; j < 16; j++) {
+      const int e = j * 32 + lane;
+      if (e < E && (v[j] < last || (v[j] == last && e > last_id)) && (v[j] > bv || bi == kMaxExperts)) {
+        bv = v[j];
+        bi = e;
+      }
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+      const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
+      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+      if (ov > bv || (ov == bv && oi < bi)) {
+        bv = ov;
+        bi = oi;
+      }
+    }
+    last = bv;
+    last_id = bi;
+    if (lane == r) mine = make_float2(bv, __int_as_float(bi));
+  }
+  return mine;
+}
+
 // The k+1 largest of E <= 512 logits in order (value descending, id ascending), by one warp: lane i gets the i-th.
-// s: 128 floats of the warp. Returns how many candidates there were, at least min(k+1, E); 0: a logit is not finite, or more than 32.
+// s: 128 floats of the warp. Returns how many lanes have one, at least min(k+1, E); 0: a logit is not finite.
 __device__ __forceinline__ int warp_leaders(const float* lg, int E, int k, int lane, float* s, float& vr, int& id) {
   float v[16];
   float lm = -INFINITY;  // the lane's largest
@@ -81,7 +116,12 @@ __device__ __forceinline__ int warp_leaders(const float* lg, int E, int k, int l
     }
     C += __popc(bal);
   }
-  if (C > 32) return 0;
+  if (C > 32) {
+    const float2 mine = warp_leaders_rounds(lg, E, min(k + 1, E), lane);
+    vr = mine.x;
+    id = __float_as_int(mine.y);
+    return min(k + 1, E);
+  }
   __syncwarp();
   if (lane < C) {
     const float mv = cv[lane];

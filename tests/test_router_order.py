@@ -1,11 +1,12 @@
 """Top-k selection where the order of the logits alone does not give the reference's ids: probabilities that are
-denormal or zero floats."""
+denormal or zero floats, many leaders in few residues mod 32."""
 import numpy as np
 import pytest
 
 import gfx1151_engine_b200 as pkg
 import oracle
 from gfx1151_engine_b200 import synth
+from helpers import assert_output_close, bf16_out_to_f32, bf16_tensor, dev_bytes
 from test_gpu_parity import make_op, run_layer
 
 pytestmark = pytest.mark.gpu
@@ -49,3 +50,34 @@ def test_widely_spread_logits(cuda, T, E, k, decode_impl):
         if T > 1:
             logits[T // 2, 7:7 + k // 2] = lead - 0.5 - np.arange(k // 2)
         check_ids(cuda, spec, layer, logits, decode_impl=decode_impl)
+
+
+@pytest.mark.parametrize("T", [1, 5, 16])
+def test_near_tie_among_many_leaders(cuda, T):
+    """Hidden states, T <= 16: 48 leaders in three residues mod 32. Expert 40's logit stands on a rounding boundary: added
+    in index order it is 1, as expert 8's, which then goes first; added as a tree it is the next larger float."""
+    torch = cuda
+    spec = synth.LayerSpec(experts=512, topk=3, d=128, mid=64, router=True)
+    layer = synth.make_layer(spec, seed=99)
+    w = np.zeros((512, 128), np.float32)
+    w[:, 0] = -(1.0 + np.arange(512)) / 512
+    lead = [e for e in range(512) if e % 32 in (8, 9, 10)]
+    w[lead, 0] = (128.0 + np.arange(len(lead))) / 256
+    w[10, 0], w[9, 0], w[8, 0] = 1.5, 1.25, 1.0
+    w[40] = 2.0 ** -54
+    w[40, :2] = 1.0, 2.0 ** -24
+    layer["router_w"] = synth.f32_to_bf16_bits(w)
+    assert np.array_equal(synth.bf16_bits_to_f32(layer["router_w"])[lead], w[lead])
+    x = np.ones((T, 128), np.float32) * (2.0 ** (np.arange(T) % 3)).astype(np.float32)[:, None]
+    x[T // 2, 127] = 1.5
+    xb = synth.f32_to_bf16_bits(x)
+    y_o, ids_o, _ = oracle.moe_forward(spec, layer, x)
+    assert ids_o[0, :3].tolist() == [10, 9, 8]
+    op = make_op(torch, spec, T, layer=layer)
+    op.load_router(0, dev_bytes(torch, layer["router_w"]))
+    out = torch.full((T, spec.d), float("nan"), dtype=torch.bfloat16, device="cuda")
+    op.moe_hidden(0, bf16_tensor(torch, xb, (T, spec.d)), out)
+    op.synchronize()
+    assert np.array_equal(op.get_routing(T)[0][:, :3], ids_o[:, :3])
+    assert_output_close(bf16_out_to_f32(torch, out), y_o, "T=%d" % T)
+    op.close()
