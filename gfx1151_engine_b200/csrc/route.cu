@@ -24,122 +24,10 @@ constexpr int kRouterWarps = 8;
 
 constexpr int kChunk = 512;  // pairs handled by one block (a thread per pair) of the bucketing kernels
 
-__device__ __forceinline__ double shfl_double(double v, int src) {
-  int lo = __double2loint(v), hi = __double2hiint(v);
-  lo = __shfl_sync(0xffffffffu, lo, src);
-  hi = __shfl_sync(0xffffffffu, hi, src);
-  return __hiloint2double(hi, lo);
-}
-
-// Router for one token by one warp, E <= 512: lane holds experts lane, lane+32, ... The reference's arithmetic, out
-// of line: only tokens whose ids the logits' order does not decide come here.
-// sp: this warp's scratch row of kMaxExperts floats in shared memory.
-__device__ __noinline__ void router_one_token(const float* __restrict__ lg, int E, int k, int lane,
-                                                 float* sp, int32_t* __restrict__ ids_row,
-                                                 float* __restrict__ w_row, int stride) {
-  float v[16];
-  float mx = -INFINITY;
-#pragma unroll
-  for (int j = 0; j < 16; j++) {
-    int e = j * 32 + lane;
-    v[j] = e < E ? lg[e] : -INFINITY;
-    mx = fmaxf(mx, v[j]);
-  }
-#pragma unroll
-  for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  const double dmx = (double)mx;
-#pragma unroll
-  for (int j = 0; j < 16; j++) {
-    int e = j * 32 + lane;
-    float p = e < E ? (float)exp((double)v[j] - dmx) : 0.f;
-    if (e < E) sp[e] = p;
-    v[j] = p;
-  }
-  __syncwarp();
-  // Sum of the exponentials, as the reference takes it: in double, in index order. All terms
-  // are floats in (0, 1]: when the smallest non-zero one's last mantissa bit still fits a
-  // double that holds the total, every partial sum of ANY order is exact, so the tree sum has
-  // the very same bits and the E dependent additions are only needed otherwise.
-  double se = 0;
-  float mn = 2.f;
-#pragma unroll
-  for (int j = 0; j < 16; j++)
-    if (j * 32 + lane < E) {
-      se += (double)v[j];
-      if (v[j] > 0.f) mn = fminf(mn, v[j]);
-    }
-#pragma unroll
-  for (int o = 16; o; o >>= 1) {
-    se += __hiloint2double(__shfl_xor_sync(0xffffffffu, __double2hiint(se), o),
-                           __shfl_xor_sync(0xffffffffu, __double2loint(se), o));
-    mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-  }
-  se = shfl_double(se, 0);  // (inexact sums may differ between lanes in the last bit: take one)
-  {
-    const int e_min = (int)((__float_as_uint(mn) >> 23) & 0xFF) - 127;
-    const int bits_total = (int)((__double2hiint(se) >> 20) & 0x7FF) - 1023 + 2;  // generous by one bit
-    const bool exact = mn >= 1.17549435e-38f && bits_total - (e_min - 23) <= 53;
-    if (!exact) {  // warp-uniform: mn and se are the same in every lane
-      se = 0;
-      if (lane == 0)
-        for (int i = 0; i < E; i++) se += (double)sp[i];  // index order, as the reference sums
-      se = shfl_double(se, 0);
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < 16; j++) {
-    int e = j * 32 + lane;
-    v[j] = e < E ? (float)((double)v[j] / se) : -1.f;
-  }
-  int my_id = 0;
-  float my_p = 0.f;
-  double kept = 0;
-  for (int r = 0; r < k; r++) {
-    // The search starts from an id inside [0, E) (the reference's GPU router starts at `lane`,
-    // src/gpu/parts/20_kernels_gemv.inc:1517): with a non-finite logit every probability is NaN, no
-    // comparison below is ever true, and the ids written are then still valid expert numbers
-    // (with NaN weights, so the token's output is NaN) instead of an out-of-range value.
-    float bv = -1.f;
-    int bi = min(lane, E - 1);
-#pragma unroll
-    for (int j = 0; j < 16; j++)
-      if (v[j] > bv) {
-        bv = v[j];
-        bi = j * 32 + lane;
-      }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-      float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-      int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-      if (ov > bv || (ov == bv && oi < bi)) {
-        bv = ov;
-        bi = oi;
-      }
-    }
-    bi = __shfl_sync(0xffffffffu, bi, 0);  // (NaN probabilities: the lanes may disagree; take lane 0's)
-    bv = __shfl_sync(0xffffffffu, bv, 0);
-    if (bv < 0.f) bv = __int_as_float(0x7fc00000);  // nothing was selectable: the weight is NaN, as in the reference
-#pragma unroll
-    for (int j = 0; j < 16; j++)
-      if (j == (bi >> 5) && lane == (bi & 31)) v[j] = -1.f;
-    if (lane == r) {
-      my_id = bi;
-      my_p = bv;
-    }
-    kept += (double)bv;
-  }
-  for (int i = lane; i < stride; i += 32) {
-    // lanes >= k hold zeros; stride > 32 is padded with zeros as well
-    bool valid = i < k && i < 32;
-    ids_row[i] = valid ? my_id : 0;
-    w_row[i] = valid ? (float)((double)my_p / kept) : 0.f;
-  }
-}
-
 __global__ void __launch_bounds__(kRouterWarps * 32)
 k_router_topk(const float* __restrict__ logits, int T, int E, int k, int32_t* __restrict__ ids,
               float* __restrict__ w, int stride) {
-  __shared__ float s_p[kRouterWarps][kMaxExperts];
+  __shared__ float s_c[kRouterWarps][128];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t = blockIdx.x * kRouterWarps + warp;
   pdl_trigger();
@@ -150,15 +38,18 @@ k_router_topk(const float* __restrict__ logits, int T, int E, int k, int32_t* __
   // 77 tokens 5 us and 11.
   float vr, wv;
   int id;
-  const int C = warp_leaders(logits + (size_t)t * E, E, k, lane, s_p[warp], vr, id);
+  const int C = warp_leaders(logits + (size_t)t * E, E, k, lane, s_c[warp], vr, id);
   if (C > 0 && warp_topk(C, vr, k, lane, true, wv)) {
     for (int i = lane; i < stride; i += 32) {  // zeros behind the k
       ids[(size_t)t * stride + i] = i < k ? id : 0;
       w[(size_t)t * stride + i] = i < k ? wv : 0.f;
     }
   } else {
-    __syncwarp();
-    router_one_token(logits + (size_t)t * E, E, k, lane, s_p[warp], ids + (size_t)t * stride, w + (size_t)t * stride, stride);
+    const float2 r = router_one_token(logits + (size_t)t * E, E, k, lane);
+    for (int i = lane; i < stride; i += 32) {
+      ids[(size_t)t * stride + i] = i < k ? __float_as_int(r.y) : 0;
+      w[(size_t)t * stride + i] = i < k ? r.x : 0.f;
+    }
   }
 }
 

@@ -6,10 +6,10 @@
 // arithmetic: 15 us for 16 tokens of 64 experts), and lists that travelled through memory.
 //   * Selection. "Largest probability, ties to the lowest id" is "largest logit, ties to the lowest id" unless two
 //     different logits round to one float probability (exp and the division by the sum are monotone): the ids come
-//     from the logits' order. Where two of a token's k+1 largest are closer than 1e-6, the k-th is so far below the
-//     largest that its probability might not be a normal float (kMaxSpread), or a logit is not finite, that
-//     token takes the general body instead (route_small.cuh: the reference's arithmetic to the letter, out of
-//     line, since its 5000 instructions would be fetched cold by every call).
+//     from the logits' order. Where two of a token's k+1 largest differ by less than 1e-6 (equal ones have equal probabilities),
+//     the k-th is so far below the largest that its probability might not be a normal float (kMaxSpread), or a logit is NaN or
+//     +inf, the token's warp takes the general body instead (router_one_token: the reference's arithmetic to the letter, out of
+//     line, so that calls without such tokens do not fetch it).
 //   * Weights: double exponentials of the k selected logits over their sum in rank order; the sum over all experts
 //     cancels and is not formed.
 //   * With a router weight the logits are double tree sums (k_router_dots) and the warp first does what
@@ -31,19 +31,12 @@ struct alignas(16) RouteBlock {
   uint16_t before[kPairWarps][kMaxExperts + 8];  // pairs of an expert: per warp, then in the warps before; [kMaxExperts]: dropped pairs
   int start[kMaxExperts + 1];
   int wsum[16], wmore[16];
-  int fallback[16];
-  int xid[kIdStride];        // the general body's answer for one token
-  float xw[kIdStride];
+  int tied[16];              // a token's logits are to be refined first
   float row[kMaxExperts];    // a near-tied token's logits
+  double prod[256];          // products of one of them
   float cand[16][128];       // per warp
 };
-// scratch behind it: the general body's, or the products of 16 warps' exact logits one warp at a time
-constexpr int kRouteBlockBytes = (int)(sizeof(RouteBlock) + sizeof(RouteSmallScratch<3>));
-static_assert(sizeof(RouteSmallScratch<3>) >= 256 * sizeof(double) && sizeof(RouteBlock) % 16 == 0, "scratch");
-
-__device__ __forceinline__ double shfl_f64(double v, int src) {
-  return __hiloint2double(__shfl_sync(0xffffffffu, __double2hiint(v), src), __shfl_sync(0xffffffffu, __double2loint(v), src));
-}
+constexpr int kRouteBlockBytes = (int)sizeof(RouteBlock);
 
 // The same by n rounds of arg-max, n <= 32: for the rare token with more candidates than warp_leaders ranks (a few residues
 // mod 32 hold most of its leaders, or many logits are equal). Value and id.
@@ -81,7 +74,7 @@ static __device__ __noinline__ float2 warp_leaders_rounds(const float* lg, int E
 }
 
 // The k+1 largest of E <= 512 logits in order (value descending, id ascending), by one warp: lane i gets the i-th.
-// s: 128 floats of the warp. Returns how many lanes have one, at least min(k+1, E); 0: a logit is not finite.
+// s: 128 floats of the warp. Returns how many lanes have one, at least min(k+1, E); 0: a logit is NaN or +inf.
 __device__ __forceinline__ int warp_leaders(const float* lg, int E, int k, int lane, float* s, float& vr, int& id) {
   float v[16];
   float lm = -INFINITY;  // the lane's largest
@@ -90,7 +83,7 @@ __device__ __forceinline__ int warp_leaders(const float* lg, int E, int k, int l
   for (int j = 0; j < 16; j++) {
     const int e = j * 32 + lane;
     v[j] = e < E ? lg[e] : -INFINITY;
-    odd |= e < E && !(fabsf(v[j]) <= 3.0e38f);
+    odd |= e < E && !(v[j] <= 3.0e38f);  // (-inf, a masked expert, has its place in the order)
     lm = fmaxf(lm, v[j]);
   }
   if (__any_sync(0xffffffffu, odd)) return 0;
@@ -142,8 +135,8 @@ __device__ __forceinline__ int warp_leaders(const float* lg, int E, int k, int l
 // that does not decide.
 __device__ __forceinline__ bool warp_topk(int C, float vr, int k, int lane, bool weights, float& wv) {
   const float vn = __shfl_down_sync(0xffffffffu, vr, 1), mx = __shfl_sync(0xffffffffu, vr, 0), vk = __shfl_sync(0xffffffffu, vr, k - 1);
-  // neighbours in the order closer than 1e-6: their probabilities might round to one float
-  if (__any_sync(0xffffffffu, lane < k && lane + 1 < C && !(vr - vn > 1e-6f * fmaxf(1.f, fabsf(vr)))) || C < k ||
+  // neighbours in the order closer than 1e-6, but not equal: their probabilities might round to one float
+  if (__any_sync(0xffffffffu, lane < k && lane + 1 < C && vr != vn && !(vr - vn > 1e-6f * fmaxf(1.f, fabsf(vr)))) || C < k ||
       !(mx - vk <= kMaxSpread))
     return false;
   if (!weights) return true;
@@ -168,20 +161,6 @@ static __device__ __noinline__ void warp_refine(const RouteIn& q, int t, int lan
   }
 }
 
-static __device__ __noinline__ void token_exact(const RouteIn& q, int t, const float* logits, RouteBlock& sc) {
-  RouteSmallOut o;
-  o.topids = sc.xid;
-  o.topw = sc.xw;
-  route_small_body<3, 2>(logits, nullptr, nullptr, 0, 1, q.E, q.k, q.tile_cap, nullptr, nullptr, q.d,
-                         *(RouteSmallScratch<3>*)(&sc + 1), o, RouteSmallOut{}, nullptr);
-  rs_sync();
-  if (threadIdx.x < q.k) {
-    sc.key[t * q.k + threadIdx.x] = sc.xid[threadIdx.x];
-    sc.w[t * q.k + threadIdx.x] = sc.xw[threadIdx.x];
-  }
-  rs_sync();
-}
-
 // Threads 0..511 of a block, sc and the scratch behind it in shared memory. write: leave everything in q.rb, too.
 // row_token (shared memory, [T*k]): the token of every permuted row. Calls emit(expert, first, count, at) for
 // every non-empty expert from one thread; at: passes of `rows` rows of the experts before. Returns their number.
@@ -202,27 +181,33 @@ __device__ __forceinline__ int route_block(const RouteIn& q, RouteBlock& sc, boo
         if (__any_sync(0xffffffffu, lane < k && lane + 1 < C && vr - vn < margin)) C = -1;
         if (lane == 0) sc.cand[warp][0] = kth - 2.f * margin;
       }
-      const bool ok = C > 0 && !q.exact && warp_topk(C, vr, k, lane, write, wv);
-      if (ok && lane < k) {
+      if (C >= 0 && (C == 0 || q.exact || !warp_topk(C, vr, k, lane, write, wv))) {
+        const float2 r = router_one_token(lg, E, k, lane);
+        wv = r.x;
+        id = __float_as_int(r.y);
+      }
+      if (lane < k) {
         sc.key[warp * k + lane] = id;
         sc.w[warp * k + lane] = wv;
       }
-      if (lane == 0) sc.fallback[warp] = C < 0 ? 2 : !ok;
+      if (lane == 0) sc.tied[warp] = C < 0;
     }
     rs_sync();
-    // tokens that their logits' order does not decide, one after the other (rare; uniform for the block)
+    // tokens with near-ties to refine, one after the other (rare; uniform for the block)
     for (int t = 0; t < T; t++) {
-      const int f = sc.fallback[t];
-      if (f == 0) continue;
-      const float* lg = q.logits + (size_t)t * E;
-      if (f == 2) {
-        if (tid < E) sc.row[tid] = lg[tid];
-        rs_sync();
-        if (warp == 0) warp_refine(q, t, lane, sc.cand[t][0], sc.row, (double*)(&sc + 1));
-        rs_sync();
-        lg = sc.row;
+      if (!sc.tied[t]) continue;
+      if (tid < E) sc.row[tid] = q.logits[(size_t)t * E + tid];
+      rs_sync();
+      if (warp == 0) {
+        warp_refine(q, t, lane, sc.cand[t][0], sc.row, sc.prod);
+        __syncwarp();
+        const float2 r = router_one_token(sc.row, E, k, lane);
+        if (lane < k) {
+          sc.key[t * k + lane] = __float_as_int(r.y);
+          sc.w[t * k + lane] = r.x;
+        }
       }
-      token_exact(q, t, lg, sc);
+      rs_sync();
     }
   } else {
     for (int p = tid; p < P; p += 512) {

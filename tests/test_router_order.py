@@ -1,5 +1,5 @@
 """Top-k selection where the order of the logits alone does not give the reference's ids: probabilities that are
-denormal or zero floats, many leaders in few residues mod 32."""
+denormal or zero floats, many leaders in few residues mod 32, equal and masked (-inf) logits."""
 import numpy as np
 import pytest
 
@@ -81,3 +81,24 @@ def test_near_tie_among_many_leaders(cuda, T):
     assert np.array_equal(op.get_routing(T)[0][:, :3], ids_o[:, :3])
     assert_output_close(bf16_out_to_f32(torch, out), y_o, "T=%d" % T)
     op.close()
+
+
+def tied(kind, T, E):
+    lg = synth.make_logits(synth.rng_for(97, T), T, E)
+    if kind == "bf16":
+        return synth.bf16_bits_to_f32(synth.f32_to_bf16_bits(lg))
+    if kind == "eighths":
+        return np.round(lg * 8).astype(np.float32) / 8
+    if kind == "masked":      # half of the experts
+        return np.where(np.arange(E) % 2 == np.arange(T)[:, None] % 2, lg, -np.inf).astype(np.float32)
+    if kind == "few left":    # as many as are selected, one more, one less
+        left = 8 + np.arange(T)[:, None] % 3 - 1
+        return np.where(np.arange(E) * 5 % E < left, lg, -np.inf).astype(np.float32)
+    return np.full((T, E), 0.25, np.float32)
+
+
+@pytest.mark.parametrize("kind", ["bf16", "eighths", "masked", "few left", "equal"])
+@pytest.mark.parametrize("T,E,k", [(1, 64, 8), (16, 64, 8), (16, 512, 16), (7, 12, 8), (77, 512, 8)])
+def test_equal_and_masked_logits(cuda, T, E, k, kind):
+    spec = synth.LayerSpec(experts=E, topk=k, d=128, mid=64)
+    check_ids(cuda, spec, synth.make_layer(spec, seed=98), tied(kind, T, E))
