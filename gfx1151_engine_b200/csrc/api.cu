@@ -708,11 +708,23 @@ static bool fused_decode(const b200moe_config& c) {
   return env || c.decode_impl == B200MOE_DECODE_FUSED;
 }
 
+// Experts of so many tokens' call that fill one pass of the decode GEMV or less may go there (kMinFewWork): how many of
+// them it takes. 0: no call of this size does that.
+static int few_row_experts(b200moe_handle h, const LayerWeights& L, int T) {
+  const b200moe_config& c = h->cfg;
+  const int k = c.topk, E = c.experts, d = c.d_model, mid = c.d_mid, rows = std::min(gemv_rows(L.gu.fmt), gemv_rows(L.dn.fmt));
+  const int least = (int)((kMinFewWork + (long long)d * mid - 1) / ((long long)d * mid));
+  return T > 16 && T > h->decode_max && !L.i4r && c.gemm_impl == B200MOE_GEMM_AUTO && 4 * T * k <= 5 * rows * E && T * k <= kFewRows * E &&
+                 std::min(E, T * k) >= least && (d << L.gu.act_shift) <= gemv_max_k() && (mid << L.dn.act_shift) <= gemv_max_mid()
+             ? least : 0;
+}
+
 // logits != nullptr: the router has not run yet (the fused small-T routing kernel runs it; with router_w it first
 // puts near-ties of these logits, its own buffer then, into the reference's arithmetic).
+// range: the tokens are a part of a longer call that few_row_experts keeps off the GEMV, and stay off it, too.
 static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const int32_t* ids,
                         const float* w, int stride, void* out, cudaStream_t st,
-                        bool router_timed = false, const float* logits = nullptr, const uint16_t* router_w = nullptr) {
+                        bool router_timed = false, const float* logits = nullptr, const uint16_t* router_w = nullptr, bool range = false) {
   const b200moe_config& c = h->cfg;
   LayerWeights& L = h->layers[layer];
   const int k = c.topk, E = c.experts, d = c.d_model, mid = c.d_mid;
@@ -754,12 +766,10 @@ static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const
   // (no expert saves more than two tiles in 2 * 64 + 1 rows; the small routing writes one list)
   const bool split = few && T > 16 && T * k * 2 >= min_saved * (2 * kTcNarrowN + 1), narrow = few && !split;
   const bool sh_narrow = few && (long long)(T / kTcNarrowN) * (mid / 64) <= kSharedNarrowItems;
-  const int min_few = (int)((kMinFewWork + (long long)d * mid - 1) / ((long long)d * mid));
-  const int pass_rows = std::min(gemv_rows(L.gu.fmt), gemv_rows(L.dn.fmt));
-  const bool mixed = T > 16 && !simt && !L.i4r && c.gemm_impl == B200MOE_GEMM_AUTO && 4 * T * k <= 5 * pass_rows * E && few &&
-                     std::min(E, T * k) >= min_few && (d << L.gu.act_shift) <= gemv_max_k() && (mid << L.dn.act_shift) <= gemv_max_mid();
+  const int min_few = range ? 0 : few_row_experts(h, L, T);
+  const bool mixed = min_few > 0;
   const TileCut cut{narrow ? kTcNarrowN : h->tile_cap, sh_narrow ? kTcNarrowN : h->tile_cap, split ? kTcNarrowN : 0, min_saved,
-                    mixed ? pass_rows : 0, min_few};
+                    mixed ? std::min(gemv_rows(L.gu.fmt), gemv_rows(L.dn.fmt)) : 0, min_few};
   // (the shared expert's images are q4cp: it can ride along only with q4cp routed experts)
   const bool gemv = simt && c.gemm_impl == B200MOE_GEMM_AUTO &&
                     (!shared || (L.gu.fmt == kQ4CP && L.dn.fmt == kQ4CP)) &&
@@ -899,8 +909,8 @@ static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const
   return B200MOE_OK;
 }
 
-int b200moe_forward(b200moe_handle h, int layer, const void* x_bf16_dev, int T,
-                    const float* logits_dev, void* out_bf16_dev, void* stream) {
+static int forward_logits(b200moe_handle h, int layer, const void* x_bf16_dev, int T, const float* logits_dev,
+                          void* out_bf16_dev, void* stream, bool range) {
   if (int s = check_layer(h, layer)) return s;
   if (!x_bf16_dev || !logits_dev || !out_bf16_dev || T < 0 || T > h->cfg.max_tokens)
     return fail(h, B200MOE_ERR_BAD_ARG, "forward: bad argument (null pointer or T out of range)");
@@ -908,7 +918,12 @@ int b200moe_forward(b200moe_handle h, int layer, const void* x_bf16_dev, int T,
   cudaStream_t st = (cudaStream_t)stream;
   if (h->prof) CU_TRY(h, cudaEventRecord(h->prof_ev[(size_t)h->prof_head * kProfEvents], st));
   return forward_impl(h, layer, x_bf16_dev, T, h->rb.topids, h->rb.topw, kIdStride, out_bf16_dev, st,
-                      h->prof, logits_dev);
+                      h->prof, logits_dev, nullptr, range);
+}
+
+int b200moe_forward(b200moe_handle h, int layer, const void* x_bf16_dev, int T,
+                    const float* logits_dev, void* out_bf16_dev, void* stream) {
+  return forward_logits(h, layer, x_bf16_dev, T, logits_dev, out_bf16_dev, stream, false);
 }
 
 int b200moe_forward_hc(b200moe_handle h, int layer, const void* x_bf16_dev, int T, const float* logits_dev,
@@ -1015,12 +1030,14 @@ int b200moe_forward_host(b200moe_handle h, int layer, const void* x_bf16_host, i
   cudaStream_t st = (cudaStream_t)stream;
   const int d = h->cfg.d_model, E = h->cfg.experts;
   // Large chunks are cut into up to four token ranges (of unequal size, see below): the copy of range c+1 to the device
-  // and the copy of range c-1 back run on their own streams while range c computes. A
-  // token's result does not depend on which other tokens share its call, so the output is
-  // the same as for one call. B200MOE_HOST_CHUNKS overrides the number of ranges.
+  // and the copy of range c-1 back run on their own streams while range c computes. The output is
+  // the same as for one call: on the tensor-core path a token's result does not depend on which other tokens share
+  // its call, and calls of which the decode path or the few-row experts' GEMV would take the whole or a range
+  // are not cut, or their ranges stay off it. B200MOE_HOST_CHUNKS overrides the number of ranges.
   static const int forced = getenv("B200MOE_HOST_CHUNKS") ? atoi(getenv("B200MOE_HOST_CHUNKS")) : 0;
   int C = forced > 0 ? forced : (T >= 8192 ? 4 : T >= 2048 ? 2 : 1);
   C = std::min(C, (int)b200moe_ctx::kHostChunks);
+  if (few_row_experts(h, h->layers[layer], T) > 0 || (T > h->decode_max && T / (C == 4 ? 8 : C) <= h->decode_max)) C = 1;
   if (C > 1 && !h->s_in) {
     CU_TRY(h, cudaStreamCreateWithFlags(&h->s_in, cudaStreamNonBlocking));
     CU_TRY(h, cudaStreamCreateWithFlags(&h->s_out, cudaStreamNonBlocking));
@@ -1075,8 +1092,8 @@ int b200moe_forward_host(b200moe_handle h, int layer, const void* x_bf16_host, i
       const int a = off[c], n = off[c + 1] - a;
       if (n <= 0) continue;
       CU_TRY(h, cudaStreamWaitEvent(st, h->ev_in[c], 0));
-      if (int s = b200moe_forward(h, layer, (uint8_t*)h->x_stage + (size_t)a * d * 2, n, h->logits_stage + (size_t)a * E,
-                                  (uint8_t*)h->out_stage + (size_t)a * d * 2, stream))
+      if (int s = forward_logits(h, layer, (uint8_t*)h->x_stage + (size_t)a * d * 2, n, h->logits_stage + (size_t)a * E,
+                                 (uint8_t*)h->out_stage + (size_t)a * d * 2, stream, true))
         return s;
       CU_TRY(h, cudaEventRecord(h->ev_done[c], st));
       CU_TRY(h, cudaStreamWaitEvent(h->s_out, h->ev_done[c], 0));

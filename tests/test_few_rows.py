@@ -81,3 +81,31 @@ def test_captured_call_replays_with_new_inputs(cuda, layer):
         torch.cuda.synchronize()
         assert np.array_equal(bits(bf16_out_to_f32(torch, out)), bits(want[i]))
     op.close()
+
+
+@pytest.mark.parametrize("T,popular,decode_max", [(2560, 0, 0), (2048, 10, 0), (2560, 0, 1300)])
+def test_host_call_equals_device_call(cuda, T, popular, decode_max):
+    """moe_b_host cuts a call into two ranges, in which every expert has few rows; in the whole call none has, or ten
+    have more than one pass of the GEMV serves; or a range is no longer than decode_max_tokens. The bytes are those of one
+    call."""
+    torch = cuda
+    spec = synth.LayerSpec(experts=512, topk=2, d=1024, mid=320)
+    op = make_op(torch, spec, T, layer=synth.make_layer(spec, seed=94), decode_max_tokens=decode_max)
+    n = T // 2
+    left = np.array([6] * popular + [(2 * n - 6 * popular) // (512 - popular)] * (512 - popular))
+    left[512 - (2 * n - left.sum()):] += 1
+    lg = np.zeros((n, 512), np.float32)
+    for t in range(n):
+        take = np.argsort(-left, kind="stable")[:2]
+        left[take] -= 1
+        lg[t, take] = 8.0, 8.5
+    assert (left == 0).all()
+    x = bf16_tensor(torch, synth.make_x(synth.rng_for(94, 9), T, spec.d), (T, spec.d))
+    logits = torch.from_numpy(np.concatenate([lg, lg])).cuda()
+    out = torch.empty_like(x)
+    op.moe_b(0, x, logits, out)
+    op.synchronize()
+    host = torch.empty((T, spec.d), dtype=torch.bfloat16).pin_memory()
+    op.moe_b_host(0, x.cpu().pin_memory(), logits.cpu().pin_memory(), host, T)
+    assert torch.equal(host.view(torch.int16), out.cpu().view(torch.int16))
+    op.close()
