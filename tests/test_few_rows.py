@@ -1,9 +1,11 @@
 """Calls of more than 16 tokens with few rows per expert on a large layer: experts with as many rows as one pass of the
 decode GEMV serves (8, 4 in the GGUF formats) take that, the others the tensor-core kernels beside it -- if the
-former are enough: 123 experts of 2560 x 512. Against the oracle on both sides of either line, and captured in a graph."""
+former are enough: 123 experts of 2560 x 512. Against the oracle on both sides of either line, in every weight format and
+through the other entry points, captured in a graph, and what the other tokens of a call may change."""
 import numpy as np
 import pytest
 
+import gfx1151_engine_b200 as pkg
 import oracle
 from gfx1151_engine_b200 import synth
 from helpers import assert_output_close, bf16_out_to_f32, bf16_tensor
@@ -109,3 +111,73 @@ def test_host_call_equals_device_call(cuda, T, popular, decode_max):
     op.moe_b_host(0, x.cpu().pin_memory(), logits.cpu().pin_memory(), host, T)
     assert torch.equal(host.view(torch.int16), out.cpu().view(torch.int16))
     op.close()
+
+
+@pytest.mark.parametrize("gu,dn,d,mid", [(pkg.GGML_Q5_K, pkg.GGML_Q5_1, 2560, 512), (pkg.GGML_IQ4_XS, pkg.GGML_IQ4_XS, 2048, 768),
+                                         (pkg.GGML_Q8_0, pkg.GGML_Q8_0, 2048, 640), (pkg.GGML_Q4_K, pkg.GGML_IQ4_NL, 2560, 512)])
+def test_weight_formats(cuda, gu, dn, d, mid):
+    """125 of 128 experts have at most four rows."""
+    T, topk, rows = CASES["at most 4"]
+    spec = synth.LayerSpec(experts=E, topk=topk, d=d, mid=mid, fmt="gguf", gg_gu=gu, gg_dn=dn)
+    layer = synth.make_layer(spec, seed=97)
+    logits = routed_to(T, topk, np.array(rows)[np.random.default_rng(T).permutation(E)])
+    xb = synth.make_x(synth.rng_for(97, 9), T, d)
+    y_o, _, _ = oracle.moe_forward(spec, layer, synth.bf16_bits_to_f32(xb), logits=logits)
+    op = make_op(cuda, spec, T, layer=layer)
+    assert_output_close(run_layer(cuda, op, spec, xb, logits), y_o, "%d/%d" % (gu, dn))
+    op.close()
+
+
+def test_other_entry_points(cuda, layer):
+    """moe_b_hc adds what moe_b stores; moe_q4w_run with the call's own ids gives its bytes, and with the ids of two tokens out of
+    range leaves those tokens zero and the others within the suite's bounds (the experts lose rows)."""
+    torch = cuda
+    spec = layer[0]
+    T, topk, rows = CASES["some above"]
+    logits = routed_to(T, topk, rows)
+    xb = synth.make_x(synth.rng_for(98, 9), T, spec.d)
+    op = make_op(torch, spec, T, layer=layer[1])
+    y = run_layer(torch, op, spec, xb, logits)
+    ids, w = op.get_routing(T)[:2]
+    x, lg = bf16_tensor(torch, xb, (T, spec.d)), torch.from_numpy(logits).cuda()
+    state = torch.zeros((T, 4, spec.d), dtype=torch.bfloat16, device="cuda")
+    w4 = torch.zeros((T, 4), device="cuda")     # gates of 2 * sigmoid(0) = 1
+    op.moe_b_hc(0, x, lg, w4, state)
+    op.synchronize()
+    assert np.array_equal(bits(bf16_out_to_f32(torch, state)), bits(np.repeat(y[:, None], 4, axis=1)))
+
+    def routed(i):
+        out = torch.full((T, spec.d), float("nan"), dtype=torch.bfloat16, device="cuda")
+        op.moe_q4w_run(0, x, torch.from_numpy(i).cuda(), torch.from_numpy(w).cuda(), out)
+        torch.cuda.synchronize()
+        return bf16_out_to_f32(torch, out)
+    assert np.array_equal(bits(routed(ids)), bits(y))
+    bad = ids.copy()
+    bad[[3, 29]] = E + 1
+    z = routed(bad)
+    with pytest.raises(pkg.B200MoeError):
+        op.synchronize()
+    keep = np.setdiff1d(np.arange(T), [3, 29])
+    assert_output_close(z[keep], y[keep], "others")
+    if not spec.shared:
+        assert (z[[3, 29]] == 0).all()
+    op.close()
+
+
+def test_neighbours(cuda, layer):
+    """Whether an expert's rows take the GEMV depends on the other tokens of the call: a token's output may differ by rounding
+    between calls (the suite's bounds), with GEMM_TC it does not."""
+    spec = layer[0]
+    T = 40
+    xb = synth.make_x(synth.rng_for(99, 9), T, spec.d)
+    a = routed_to(T, 8, CASES["some above"][2])
+    b = a.copy()
+    b[20:] = 0.0
+    b[20:, :8] = 8.0 + 0.25 * np.arange(8)    # popular experts: fewer than 123 are left for the GEMV
+    for impl in (pkg.GEMM_AUTO, pkg.GEMM_TC):
+        op = make_op(cuda, spec, T, layer=layer[1], impl=impl)
+        ya, yb = run_layer(cuda, op, spec, xb, a)[:20], run_layer(cuda, op, spec, xb, b)[:20]
+        assert_output_close(ya, yb, "impl %d" % impl)
+        if impl == pkg.GEMM_TC:
+            assert np.array_equal(bits(ya), bits(yb))
+        op.close()
