@@ -11,7 +11,7 @@
 //
 // A decode call moves ~78 MB of 4-bit weights once and does almost no arithmetic, so what
 // counts is how little of the call is NOT spent streaming weights:
-//   * one launch instead of four: no launch gaps, no re-reading of routing tables from global
+//   * one launch instead of three: no launch gaps, no re-reading of routing tables from global
 //     memory, the code-book tables are built once per phase;
 //   * every block repeats the routing of the few tokens for itself in shared memory (512
 //     threads, route_small.cuh), so no block waits for another one before it knows its experts;
@@ -20,7 +20,8 @@
 //     bytes in flight), two slots in flight while the third is consumed;
 //   * a lane owns a weight row (a warp's read is 512 contiguous bytes of the tiled image), the
 //     32 warps of a block split K; code byte -> half2 pair by one lookup in a lane-replicated
-//     table whose address is one byte permute; exact products, fp32 sums (as expert_gemv.cu);
+//     table whose address is one byte permute; exact products, fp32 sums by multiply-adds (expert_gemv.cu sums
+//     the same products in another order: the two agree to rounding, not to the bit);
 //   * the warps of a block never meet at a block-wide barrier inside a phase: at the end of a
 //     task a warp leaves its partial sums in shared memory, bumps a counter and goes on; one
 //     warp per task (they take turns) waits for the 32 arrivals and adds the sums in a fixed order;
@@ -246,7 +247,7 @@ struct RouteOuts {
 
 // The general body, kept out of line: the fast path's instruction footprint stays small.
 __device__ __noinline__ void route_exact(const DecParams& p, RouteSmallScratch<kDecMaxT>* sc, const RouteOuts* o, int32_t* status) {
-  route_small_body<kDecMaxT, 2>(p.logits, p.ids, p.w, p.stride, p.T, p.E, p.k, p.tile_cap, p.x, nullptr, p.d, *sc, o->loc, o->glob, status);
+  route_small_body<kDecMaxT>(p.logits, p.ids, p.w, p.stride, p.T, p.E, p.k, p.tile_cap, *sc, o->loc, o->glob, status);
 }
 
 // Threads 0..511. Fills fs.key / fs.w (pair order) from the logits; returns false when the

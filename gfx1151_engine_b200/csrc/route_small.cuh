@@ -1,8 +1,6 @@
 // route_small.cuh -- the whole routing stage for a few tokens (T*k <= 256) as a device function
-// run by 512 threads of one block: shared expert's sigmoid gate, router top-k, stable bucketing
-// by rank counting, expert offsets, run and tile lists. Used by
-// route_block.cuh for single tokens and by the fused decode kernel (decode.cu) for all of a call's, where their logits' order
-// does not decide.
+// run by 512 threads of one block: router top-k, stable bucketing by rank counting, expert offsets, run and tile
+// lists. Used by the one-kernel decode (decode.cu) where the logits' order does not decide, or the caller gives the ids.
 // Arithmetic and tie rule: see route.cu.
 #pragma once
 #include "kernels.h"
@@ -12,10 +10,7 @@ namespace b200moe {
 constexpr int kBadKey = 0x7fffffff;   // sort key of a dropped pair (expert id outside [0, E))
 constexpr int kStatusBadId = 4;       // status word {4, offending id}: reported as B200MOE_ERR_BAD_ARG
 
-// Decode / verify (T*k <= 256): the whole routing stage in ONE block -- router top-k (when
-// logits are given), stable bucketing by rank counting, expert offsets, run and tile lists,
-// and the shared expert's sigmoid gate. Same results as the general kernels below.
-constexpr int kSmallPairs = 256;
+constexpr int kSmallPairs = 256;  // the most pairs of a call that one block routes (route_block.cuh, too)
 
 // Selection by the logits' order (route_block.cuh, decode.cu): the k-th may lie so far below the largest. Its probability is
 // then at least exp(-80) / kMaxExperts = 3.5e-38, above the smallest normal float (1.2e-38), so that logits 1e-6 apart
@@ -51,7 +46,6 @@ struct RouteSmallOut {
   Tile* tiles = nullptr;
   Tile* tiles_sh = nullptr;
   int32_t* n_tiles = nullptr;  // [2]
-  float* sgate = nullptr;      // [T]
 };
 #define RS_PUT(field, idx, val)                 \
   do {                                          \
@@ -65,22 +59,11 @@ __device__ __forceinline__ void rs_sync() { asm volatile("bar.sync 1, 512;" ::: 
 
 // Run by threads 0..511 of a block (tid = threadIdx.x < 512). tile_cap: most rows
 // of one tile (T, at most 16, is below it).
-// GU: 16-byte pieces of the shared expert's gate product a lane loads before it uses any (a
-// register-hungry prefetch: 8 where the body has the whole SM's registers, 2 inside a larger kernel).
-template <int NROW, int GU = 8>
+template <int NROW>
 __device__ __forceinline__ void route_small_body(
     const float* __restrict__ logits, const int32_t* __restrict__ ids_in, const float* __restrict__ w_in,
-    int stride_in, int T, int E, int k, int tile_cap, const uint16_t* __restrict__ x, const uint16_t* __restrict__ gw, int d,
-    RouteSmallScratch<NROW>& sc, const RouteSmallOut& o1, const RouteSmallOut& o2, int32_t* status,
-    unsigned long long* dbg = nullptr) {
-#define RS_STAMP(i)                                                     \
-  do {                                                                  \
-    if (dbg && threadIdx.x == 0) {                                      \
-      unsigned long long t_;                                            \
-      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_));            \
-      dbg[i] = t_;                                                      \
-    }                                                                   \
-  } while (0)
+    int stride_in, int T, int E, int k, int tile_cap,
+    RouteSmallScratch<NROW>& sc, const RouteSmallOut& o1, const RouteSmallOut& o2, int32_t* status) {
   float (*s_p)[kMaxExperts] = sc.p;
   int* s_key = sc.key;
   float* s_w = sc.w;
@@ -95,55 +78,6 @@ __device__ __forceinline__ void route_small_body(
   const int Tp = T <= 1 ? 1 : T <= 2 ? 2 : T <= 4 ? 4 : T <= 8 ? 8 : 16;
   const int W = 16 / Tp, ts = warp / W, wq = warp % W;  // token slot, warp in the token's group
   const bool tok = ts < T;
-  if (gw) {
-    // scalar sigmoid gate of the shared expert: a d-long dot product in double, 16-byte
-    // loads spread over the token's warps, partial sums added in a fixed order
-    double a = 0;
-    if (tok) {
-      const uint4* xv = (const uint4*)(x + (size_t)ts * d);
-      const uint4* gv = (const uint4*)gw;
-      // eight pieces per lane are loaded before any is used (with one warp per token the loop
-      // would otherwise pay a global-load latency per piece); the additions keep their order
-      for (int c0 = wq * 32 + lane; c0 < d / 8; c0 += W * 32 * GU) {
-        uint4 xa[GU], ga[GU];
-#pragma unroll
-        for (int u = 0; u < GU; u++) {
-          const int c = c0 + u * W * 32;
-          if (c < d / 8) {
-            xa[u] = xv[c];
-            ga[u] = __ldg(gv + c);
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < GU; u++) {
-          if (c0 + u * W * 32 < d / 8) {
-            const uint32_t xw[4] = {xa[u].x, xa[u].y, xa[u].z, xa[u].w}, gq[4] = {ga[u].x, ga[u].y, ga[u].z, ga[u].w};
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-              a += (double)__uint_as_float(gq[q] << 16) * (double)__uint_as_float(xw[q] << 16);
-              a += (double)__uint_as_float(gq[q] & 0xFFFF0000u) * (double)__uint_as_float(xw[q] & 0xFFFF0000u);
-            }
-          }
-        }
-      }
-    }
-#pragma unroll
-    for (int o = 16; o; o >>= 1)
-      a += __hiloint2double(__shfl_xor_sync(0xffffffffu, __double2hiint(a), o),
-                            __shfl_xor_sync(0xffffffffu, __double2loint(a), o));
-    if (lane == 0) s_part[warp] = a;
-    rs_sync();
-    if (tok && wq == 0 && lane == 0) {
-      double tot = 0;
-      for (int w2 = 0; w2 < W; w2++) tot += s_part[ts * W + w2];
-      const float gate = sigmoid_f32((float)tot);
-      RS_PUT(sgate, ts, gate);
-      RS_PUT(tokidx, P + ts, ts);
-      RS_PUT(pw, P + ts, gate);
-    }
-    rs_sync();  // s_part is reused by the router
-  RS_STAMP(0);
-  }
   if (logits) {
     // Router: the token's W warps share its exponentials, divisions and the selection, so
     // that a single token is spread over the whole block instead of one warp. Same arithmetic
@@ -162,7 +96,6 @@ __device__ __forceinline__ void route_small_body(
     for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     if (lane == 0) s_bv[0][warp] = mx;
     rs_sync();
-  RS_STAMP(1);
     for (int w2 = 0; w2 < W; w2++) mx = fmaxf(mx, s_bv[0][ts * W + w2]);
     const double dmx = (double)mx;
 #pragma unroll
@@ -174,7 +107,6 @@ __device__ __forceinline__ void route_small_body(
       }
     }
     rs_sync();
-  RS_STAMP(2);
     // Sum of the exponentials, as the reference takes it: in double, in index order. All terms
     // are floats in (0, 1]: when the smallest non-zero one is at least 2^(B - 30), B = bits of
     // the total's integer part, every partial sum of ANY order is a multiple of one grid that
@@ -201,7 +133,6 @@ __device__ __forceinline__ void route_small_body(
       }
     }
     rs_sync();
-  RS_STAMP(3);
     if (tok && wq == 0 && lane == 0) {
       double se = 0;
       float mn = 2.f;
@@ -220,7 +151,6 @@ __device__ __forceinline__ void route_small_body(
       s_se[ts] = se;
     }
     rs_sync();
-  RS_STAMP(4);
     const double se = tok ? s_se[ts] : 1.0;
 #pragma unroll
     for (int j = 0; j < 16; j++) {
@@ -368,7 +298,6 @@ __device__ __forceinline__ void route_small_body(
     }
   }
   rs_sync();
-  RS_STAMP(5);
   // pair p -> row = number of pairs ordered before it by (expert, p)
   int n_bad = 0;
   if (tid < P) {
@@ -410,7 +339,6 @@ __device__ __forceinline__ void route_small_body(
   }
   if (lane == 0) s_wcnt[warp] = __popc(active) | more_warp << 16;
   rs_sync();
-  RS_STAMP(6);
   int at = __popc(active & ((1u << lane) - 1u)) | (more_upto - more) << 16, all = 0;
   for (int w2 = 0; w2 < 16; w2++) {
     if (w2 < warp) at += s_wcnt[w2];
@@ -436,7 +364,6 @@ __device__ __forceinline__ void route_small_body(
   }
 }
 #undef RS_PUT
-#undef RS_STAMP
 
 
 }  // namespace b200moe
