@@ -61,6 +61,8 @@ constexpr int kSharedNarrowItems = 384;
 // 269 / 239, 148 / 155; 100 tokens 892 / 698, 496 / 427, 208 / 204; 400 tokens 1026 / 916, 872 / 751, 339 / 317; 51
 // tokens in Q4_K / Q5_1 733 / 587, 409 / 353, 181 / 179; 512 of 2560 x 640 + shared, 51 tokens 310 / 267, 193 / 181, 101 / 112;
 // 500 tokens 476 / 463, 425 / 390, 202 / 204; 64 of 2048 x 512, 64 tokens 71 / 87 (all below the line: without).
+// The two round differently (fp32 scales and sums by slices against fp16 weights), so that an output of such a call depends on the
+// other tokens by rounding; calls that must not have GEMM_TC.
 constexpr long long kMinFewWork = 160000000;
 
 struct b200moe_ctx {
@@ -708,8 +710,8 @@ static bool fused_decode(const b200moe_config& c) {
   return env || c.decode_impl == B200MOE_DECODE_FUSED;
 }
 
-// Experts of so many tokens' call that fill one pass of the decode GEMV or less may go there (kMinFewWork): how many of
-// them it takes. 0: no call of this size does that.
+// How many experts with no more rows than one pass of the decode GEMV serves it takes for a call of T tokens to send them
+// there (kMinFewWork). 0: no call of this size does.
 static int few_row_experts(b200moe_handle h, const LayerWeights& L, int T) {
   const b200moe_config& c = h->cfg;
   const int k = c.topk, E = c.experts, d = c.d_model, mid = c.d_mid, rows = std::min(gemv_rows(L.gu.fmt), gemv_rows(L.dn.fmt));
@@ -777,7 +779,7 @@ static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const
                     (d << L.gu.act_shift) <= gemv_max_k() && (mid << L.dn.act_shift) <= gemv_max_mid() && d % 32 == 0 &&
                     mid % 32 == 0;
   const uint16_t* gate_w = nullptr;  // set: the shared expert's gate is still to be computed
-  static const bool slow_router = getenv("B200MOE_EXACT_ROUTER") != nullptr;  // A/B: the general routing body for every token
+  static const bool slow_router = getenv("B200MOE_EXACT_ROUTER") != nullptr;  // A/B: the general routing body for every token of a call of up to 16
   const bool in_block = route_block_supported(T, k);
   RouteIn route{logits, ids, w, stride, router_w, (const uint16_t*)x, shared ? L.sh_gate_w : nullptr, T, E, k, d, cut.routed, slow_router, h->rb};
   if (gemv && in_block) {

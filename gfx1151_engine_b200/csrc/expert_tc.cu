@@ -454,8 +454,11 @@ k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ C
         // with four bulk prefetches, so that the fetch finds them there. Measured: 6 % on a launch
         // whose tiles all have ~10 rows (short MMAs: the fetch latency shows); with every weight read
         // served from L2 (a diagnostic run on one expert's tiles) such a launch gains 23 %. One pair at a time
-        // is twice the instructions of this thread: 2048 tokens on i4r experts 751 us against 723, 4096 of
-        // 4096 x 1024 from host buffers 2372 / 2320, 16384 tokens 5040 / 5010; four pairs are level with two.
+        // is twice the instructions of this thread: 2048 tokens on i4r experts 751 us against 723 (with the SwiGLU step of
+        // eight lanes a vector in both), 4096 of 4096 x 1024 from host buffers 2372 / 2320, 16384 tokens level;
+        // four pairs are level with two. With an odd number of pairs the next item's first one is never asked for. Asking
+        // for it costs more than it gives: 128 experts of 1792 x 896, 4096 tokens 425 us; 437 where every pair is followed
+        // exactly, 428 with one more request per item.
         constexpr size_t w_sub_b = sub_bytes(FMT);
         const size_t w_col_b = KB * w_sub_b;  // from one sub-block to the next
         const uint8_t* w_this = img.mtile(t.expert, it % img.n_mtiles);

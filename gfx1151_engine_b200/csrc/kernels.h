@@ -9,12 +9,12 @@
 
 namespace b200moe {
 
-// Programmatic dependent launch for the decode chain (route -> gate/up -> down -> combine):
+// Programmatic dependent launch for the decode chain (gate/up with the routing -> down -> combine):
 // the next kernel of the stream may start its prologue (code-book tables, index setup) while
 // this one drains. A kernel launched this way must call pdl_wait() before it touches anything
 // an earlier kernel of the stream wrote (or still reads); pdl_trigger() lets its own successor
 // start early. (One exception: k_expert_tc launches with TcLaunch::beside rely on the wait of the
-// k_expert_tc launch in front of them, which triggers behind it.) B200MOE_NO_PDL=1 in the environment turns the attribute off (plain launches).
+// k_expert_tc or k_gemv launch in front of them, which triggers behind it.) B200MOE_NO_PDL=1 in the environment turns the attribute off (plain launches).
 // launch_opt(false, ...) is a plain launch of the same kernel.
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -108,7 +108,8 @@ __device__ __forceinline__ void fwht128_8(float (&v)[16], int lane) {
 // u = svh_gu[mid + ..] * Hn(z[row][mid + b*128 ..]) (k_i4r_mid of the reference,
 // src/gpu/parts/28_kernels_hgn_v2.inc:98-143). Eight lanes per (row, block b = blockIdx.y of mid), whose planes stay in
 // registers. With a warp per vector, 60 shuffles and 64-bit index arithmetic bounded it, not its 6 bytes a hidden
-// value: 20480 rows of 640 took 45 us (78 MB: 12 us at the copy bandwidth); a 2048-token call gained 2 us with this alone.
+// value: 20480 rows of 640 took 45 us (78 MB: 12 us at the copy bandwidth). Of a whole 2048-token call (724 us) the
+// gain is below what two runs differ by.
 __global__ void __launch_bounds__(256)
 k_i4r_mid(const __half* __restrict__ z, const float* __restrict__ svh_gu, const float* __restrict__ suh_dn,
           int rows, int mid, __half* __restrict__ hr) {

@@ -43,9 +43,13 @@ enum {
 /* GGUF tensor type ids accepted by b200moe_load_gguf (values of ggml / src/gguf.h:36-41). */
 enum { B200MOE_GGML_Q5_1 = 7, B200MOE_GGML_Q8_0 = 8, B200MOE_GGML_Q4_K = 12, B200MOE_GGML_Q5_K = 13, B200MOE_GGML_IQ4_NL = 20, B200MOE_GGML_IQ4_XS = 23 };
 
-/* Which expert GEMM implementation forward uses for T > decode_max_tokens. */
+/* Which expert GEMM implementation forward uses for T > decode_max_tokens.
+ * Row invariance (a token's bytes do not depend on the other tokens of the call, tools/ktest.cu:920-923 of the reference):
+ * with AUTO among calls of T <= decode_max_tokens, and among longer ones whose layer and size keep every expert on the grouped
+ * GEMM; not where short calls of large layers send experts with few rows to the GEMV kernels, since the rows
+ * of all tokens decide which (the difference is rounding, a bf16 step). With SIMT and TC always. */
 enum {
-  B200MOE_GEMM_AUTO = 0,   /* tcgen05 grouped GEMM */
+  B200MOE_GEMM_AUTO = 0,   /* tcgen05 grouped GEMM; experts with few rows of a short call through the decode path's GEMV */
   B200MOE_GEMM_SIMT = 1,   /* fp32 CUDA-core kernels (the decode path, at any T); for A/B checks */
   B200MOE_GEMM_TC = 2      /* tcgen05 grouped GEMM even for T <= decode_max_tokens */
 };
@@ -54,7 +58,7 @@ enum {
 enum {
   B200MOE_DECODE_AUTO = 0,   /* gate/up GEMV (with the routing), down GEMV, combine as three kernels chained by programmatic dependent launch */
   B200MOE_DECODE_FUSED = 1   /* T <= 8: ONE kernel for the whole call; every expert is read once for all the rows that use it
-                                (the reference's expert dedup, src/gpu/parts/26_kernels_moe_gguf.inc:749-793), bit-identical to T = 1 */
+                                (the reference's expert dedup, src/gpu/parts/26_kernels_moe_gguf.inc:749-793), bit-identical to its own T = 1 (to rounding, not to the bit, to AUTO) */
 };
 
 typedef struct {

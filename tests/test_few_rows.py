@@ -180,4 +180,5 @@ def test_neighbours(cuda, layer):
         assert_output_close(ya, yb, "impl %d" % impl)
         if impl == pkg.GEMM_TC:
             assert np.array_equal(bits(ya), bits(yb))
+            assert np.array_equal(bits(run_layer(cuda, op, spec, xb[:7], a[:7])), bits(ya[:7]))
         op.close()
