@@ -45,9 +45,10 @@ enum { B200MOE_GGML_Q5_1 = 7, B200MOE_GGML_Q8_0 = 8, B200MOE_GGML_Q4_K = 12, B20
 
 /* Which expert GEMM implementation forward uses for T > decode_max_tokens.
  * Row invariance (a token's bytes do not depend on the other tokens of the call, tools/ktest.cu:920-923 of the reference):
- * with AUTO among calls of T <= decode_max_tokens, and among longer ones whose layer and size keep every expert on the grouped
- * GEMM; not where short calls of large layers send experts with few rows to the GEMV kernels, since the rows
- * of all tokens decide which (the difference is rounding, a bf16 step). With SIMT and TC always. */
+ * with AUTO among calls of T <= decode_max_tokens that can reach at most 191 experts (min(experts, T * topk); the others run on the
+ * fp32 kernels), and among longer ones whose layer and size keep every expert on the grouped GEMM; not where short
+ * calls of large layers send experts with few rows to the GEMV kernels, since the rows of all tokens decide
+ * which (the difference is rounding, a bf16 step). With SIMT and TC always. */
 enum {
   B200MOE_GEMM_AUTO = 0,   /* tcgen05 grouped GEMM; experts with few rows of a short call through the decode path's GEMV */
   B200MOE_GEMM_SIMT = 1,   /* fp32 CUDA-core kernels (the decode path, at any T); for A/B checks */
