@@ -39,7 +39,7 @@ k_router_topk(const float* __restrict__ logits, int T, int E, int k, int32_t* __
   float vr, wv;
   int id;
   const int C = warp_leaders(logits + (size_t)t * E, E, k, lane, s_c[warp], vr, id);
-  if (C > 0 && warp_topk(C, vr, k, lane, true, wv)) {
+  if (C > 0 && warp_topk(logits + (size_t)t * E, E, C, vr, k, lane, true, wv)) {
     for (int i = lane; i < stride; i += 32) {  // zeros behind the k
       ids[(size_t)t * stride + i] = i < k ? id : 0;
       w[(size_t)t * stride + i] = i < k ? wv : 0.f;

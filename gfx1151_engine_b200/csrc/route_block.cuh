@@ -131,14 +131,22 @@ __device__ __forceinline__ int warp_leaders(const float* lg, int E, int k, int l
   return C;
 }
 
+// Several equal logits in the last places: the next smaller one is none of the leaders, and might share their probability.
+static __device__ __noinline__ bool warp_near_below(const float* lg, int E, float vk, int lane) {
+  bool near = false;
+  for (int e = lane; e < E; e += 32) near |= lg[e] < vk && !(vk - lg[e] > 1e-6f * fmaxf(1.f, fabsf(vk)));
+  return __any_sync(0xffffffffu, near);
+}
+
 // Top-k ids and weights from the order of the logits: lane r < k gets the r-th (weights only if asked for). False where
 // that does not decide.
-__device__ __forceinline__ bool warp_topk(int C, float vr, int k, int lane, bool weights, float& wv) {
+__device__ __forceinline__ bool warp_topk(const float* lg, int E, int C, float vr, int k, int lane, bool weights, float& wv) {
   const float vn = __shfl_down_sync(0xffffffffu, vr, 1), mx = __shfl_sync(0xffffffffu, vr, 0), vk = __shfl_sync(0xffffffffu, vr, k - 1);
   // neighbours in the order closer than 1e-6, but not equal: their probabilities might round to one float
   if (__any_sync(0xffffffffu, lane < k && lane + 1 < C && vr != vn && !(vr - vn > 1e-6f * fmaxf(1.f, fabsf(vr)))) || C < k ||
       !(mx - vk <= kMaxSpread))
     return false;
+  if (k < C && vk == __shfl_sync(0xffffffffu, vr, k) && warp_near_below(lg, E, vk, lane)) return false;
   if (!weights) return true;
   const double e = lane < k ? exp((double)vr - (double)mx) : 0.0;
   double kept = 0;
@@ -181,7 +189,7 @@ __device__ __forceinline__ int route_block(const RouteIn& q, RouteBlock& sc, boo
         if (__any_sync(0xffffffffu, lane < k && lane + 1 < C && vr - vn < margin)) C = -1;
         if (lane == 0) sc.cand[warp][0] = kth - 2.f * margin;
       }
-      if (C >= 0 && (C == 0 || q.exact || !warp_topk(C, vr, k, lane, write, wv))) {
+      if (C >= 0 && (C == 0 || q.exact || !warp_topk(lg, E, C, vr, k, lane, write, wv))) {
         const float2 r = router_one_token(lg, E, k, lane);
         wv = r.x;
         id = __float_as_int(r.y);

@@ -94,10 +94,12 @@ def tied(kind, T, E):
     if kind == "few left":    # as many as are selected, one more, one less
         left = 8 + np.arange(T)[:, None] % 3 - 1
         return np.where(np.arange(E) * 5 % E < left, lg, -np.inf).astype(np.float32)
+    if kind == "adjacent":    # a few floats apart: their probabilities share one
+        return (np.float32(0.44) + np.float32(2.0) ** -25 * (np.arange(E) * 7 % 11 + np.arange(T)[:, None] % 5)).astype(np.float32)
     return np.full((T, E), 0.25, np.float32)
 
 
-@pytest.mark.parametrize("kind", ["bf16", "eighths", "masked", "few left", "equal"])
+@pytest.mark.parametrize("kind", ["bf16", "eighths", "masked", "few left", "adjacent", "equal"])
 @pytest.mark.parametrize("T,E,k", [(1, 64, 8), (16, 64, 8), (16, 512, 16), (7, 12, 8), (77, 512, 8)])
 def test_equal_and_masked_logits(cuda, T, E, k, kind):
     spec = synth.LayerSpec(experts=E, topk=k, d=128, mid=64)
