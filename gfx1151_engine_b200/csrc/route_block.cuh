@@ -31,9 +31,10 @@ struct alignas(16) RouteBlock {
   uint16_t before[kPairWarps][kMaxExperts + 8];  // pairs of an expert: per warp, then in the warps before; [kMaxExperts]: dropped pairs
   int start[kMaxExperts + 1];
   int wsum[16], wmore[16];
-  int tied[16];              // a token's logits are to be refined first
-  float row[kMaxExperts];    // a near-tied token's logits
-  double prod[256];          // products of one of them
+  float floor[16];           // a token's logits from here on are to be refined first (+inf: none)
+  int unsure;
+  float row[4][kMaxExperts];  // near-tied tokens' logits
+  double prod[256];           // products of one of them
   float cand[16][128];       // per warp
 };
 constexpr int kRouteBlockBytes = (int)sizeof(RouteBlock);
@@ -156,16 +157,74 @@ __device__ __forceinline__ bool warp_topk(const float* lg, int E, int C, float v
   return true;
 }
 
-// k_router_pairs' arithmetic for one token's logits that are not below `floor`, by one warp. (In the block's own copy:
-// other blocks read the same logits at the same time and have to come to the same answer.)
-static __device__ __noinline__ void warp_refine(const RouteIn& q, int t, int lane, float floor, float* row, double* prod) {
-  for (int e0 = 0; e0 < q.E; e0 += 32) {
-    unsigned m = __ballot_sync(0xffffffffu, e0 + lane < q.E && row[e0 + lane] >= floor);
-    for (; m; m &= m - 1) {
-      const int e = e0 + __ffs(m) - 1;
-      const float v = exact_logit(q.x + (size_t)t * q.d, q.router + (size_t)e * q.d, q.d, prod, lane);
-      if (lane == 0) row[e] = v;
+// ids and weights of one token whose logits are final: lane r < k gets the r-th.
+__device__ __forceinline__ void warp_select(const float* lg, int C, int E, int k, int lane, bool exact, bool weights, float vr, int& id, float& wv) {
+  if (C == 0 || exact || !warp_topk(lg, E, C, vr, k, lane, weights, wv)) {
+    const float2 r = router_one_token(lg, E, k, lane);
+    wv = r.x;
+    id = __float_as_int(r.y);
+  }
+}
+
+// The near-tied tokens of a call (bits of `left`): k_router_pairs' arithmetic for their logits from sc.floor on, then their
+// selection. Four tokens at a time in the block's own copy (other blocks read the same logits at the same time and have to
+// come to the same answer), the (token, expert) pairs dealt out to the 16 warps. One warp and one token at a time took 950 us
+// for 16 tokens of 512 experts whose router rows are equal in pairs.
+static __device__ __noinline__ void refine_tied(const RouteIn& q, RouteBlock& sc, unsigned left, bool write) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, E = q.E, k = q.k, d = q.d;
+  while (left) {
+    int tok[4], n = 0;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      tok[i] = __ffs(left) - 1;
+      n += left != 0;
+      left &= left - 1;
+      if (i < n && tid < E) sc.row[i][tid] = q.logits[(size_t)tok[i] * E + tid];
     }
+    if (tid == 0) sc.unsure = 0;
+    rs_sync();
+    int at = 0;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      if (i >= n) break;
+      const float* lg = q.logits + (size_t)tok[i] * E;
+      const uint16_t* x = q.x + (size_t)tok[i] * d;
+      const float floor = sc.floor[tok[i]];
+      for (int e0 = 0; e0 < E; e0 += 32)
+        for (unsigned m = __ballot_sync(0xffffffffu, e0 + lane < E && lg[min(e0 + lane, E - 1)] >= floor); m; m &= m - 1)
+          if ((at++ & 15) == warp) {
+            const int e = e0 + __ffs(m) - 1;
+            const float v = exact_logit(x, q.router + (size_t)e * d, d, nullptr, lane);
+            if (lane == 0) {
+              sc.row[i][e] = v;
+              if (v != v) sc.unsure = 1;
+            }
+          }
+    }
+    rs_sync();
+    if (sc.unsure) {  // sums on a rounding boundary: replayed one after the other
+      if (warp == 0)
+        for (int i = 0; i < n; i++)
+          for (int e0 = 0; e0 < E; e0 += 32)
+            for (unsigned m = __ballot_sync(0xffffffffu, e0 + lane < E && sc.row[i][e0 + lane] != sc.row[i][e0 + lane]); m; m &= m - 1) {
+              const int e = e0 + __ffs(m) - 1, t = i == 0 ? tok[0] : i == 1 ? tok[1] : i == 2 ? tok[2] : tok[3];
+              const float v = exact_logit(q.x + (size_t)t * d, q.router + (size_t)e * d, d, sc.prod, lane);
+              if (lane == 0) sc.row[i][e] = v;
+            }
+      rs_sync();
+    }
+    if (warp < n) {
+      const int t = warp == 0 ? tok[0] : warp == 1 ? tok[1] : warp == 2 ? tok[2] : tok[3];
+      float vr, wv = 0.f;
+      int id;
+      const int C = warp_leaders(sc.row[warp], E, k, lane, sc.cand[warp], vr, id);
+      warp_select(sc.row[warp], C, E, k, lane, q.exact, write, vr, id, wv);
+      if (lane < k) {
+        sc.key[t * k + lane] = id;
+        sc.w[t * k + lane] = wv;
+      }
+    }
+    rs_sync();
   }
 }
 
@@ -182,40 +241,28 @@ __device__ __forceinline__ int route_block(const RouteIn& q, RouteBlock& sc, boo
       const float* lg = q.logits + (size_t)warp * E;
       float vr, wv = 0.f;
       int id;
-      int C = warp_leaders(lg, E, k, lane, sc.cand[warp], vr, id);
+      const int C = warp_leaders(lg, E, k, lane, sc.cand[warp], vr, id);
+      float floor = INFINITY;
       if (q.router && C > 0) {
-        const float margin = 5e-7f * fmaxf(1.f, fabsf(__shfl_sync(0xffffffffu, vr, 0)));
+        // (Leaders that are all exactly 0 -- a token or a router of zeros -- stay: an index-order sum that differs from
+        // the tree's is too close to 0 for its probability to differ, and equal ones go to the lowest id.)
+        const float top = __shfl_sync(0xffffffffu, vr, 0), margin = 5e-7f * fmaxf(1.f, fabsf(top));
         const float vn = __shfl_down_sync(0xffffffffu, vr, 1), kth = __shfl_sync(0xffffffffu, vr, min(k, E) - 1);
-        if (__any_sync(0xffffffffu, lane < k && lane + 1 < C && vr - vn < margin)) C = -1;
-        if (lane == 0) sc.cand[warp][0] = kth - 2.f * margin;
+        if (__any_sync(0xffffffffu, lane < k && lane + 1 < C && vr - vn < margin) && (top != 0.f || kth != 0.f)) floor = kth - 2.f * margin;
       }
-      if (C >= 0 && (C == 0 || q.exact || !warp_topk(lg, E, C, vr, k, lane, write, wv))) {
-        const float2 r = router_one_token(lg, E, k, lane);
-        wv = r.x;
-        id = __float_as_int(r.y);
-      }
-      if (lane < k) {
-        sc.key[warp * k + lane] = id;
-        sc.w[warp * k + lane] = wv;
-      }
-      if (lane == 0) sc.tied[warp] = C < 0;
-    }
-    rs_sync();
-    // tokens with near-ties to refine, one after the other (rare; uniform for the block)
-    for (int t = 0; t < T; t++) {
-      if (!sc.tied[t]) continue;
-      if (tid < E) sc.row[tid] = q.logits[(size_t)t * E + tid];
-      rs_sync();
-      if (warp == 0) {
-        warp_refine(q, t, lane, sc.cand[t][0], sc.row, sc.prod);
-        __syncwarp();
-        const float2 r = router_one_token(sc.row, E, k, lane);
+      if (floor == INFINITY) {
+        warp_select(lg, C, E, k, lane, q.exact, write, vr, id, wv);
         if (lane < k) {
-          sc.key[t * k + lane] = __float_as_int(r.y);
-          sc.w[t * k + lane] = r.x;
+          sc.key[warp * k + lane] = id;
+          sc.w[warp * k + lane] = wv;
         }
       }
-      rs_sync();
+      if (lane == 0) sc.floor[warp] = floor;
+    }
+    rs_sync();
+    if (q.router) {
+      const unsigned tied = __ballot_sync(0xffffffffu, lane < T && sc.floor[lane & 15] < INFINITY);
+      if (tied) refine_tied(q, sc, tied, write);  // (uniform for the block)
     }
   } else {
     for (int p = tid; p < P; p += 512) {

@@ -6,9 +6,10 @@
 
 namespace b200moe {
 
-// sp: 256 doubles of shared memory of this warp. The result is in every lane.
+// sp: 256 doubles of shared memory of this warp, or null: NaN where they would be needed. The result is in every lane.
 __device__ __forceinline__ float exact_logit(const uint16_t* __restrict__ xr, const uint16_t* __restrict__ wr, int d, double* sp, int lane) {
   double acc = 0, mag = 0;
+#pragma unroll 4
   for (int c = lane * 8; c < d; c += 256) {
     const uint4 xv = *(const uint4*)(xr + c), wv = __ldg((const uint4*)(wr + c));
     const uint16_t* xb = (const uint16_t*)&xv;
@@ -34,6 +35,7 @@ __device__ __forceinline__ float exact_logit(const uint16_t* __restrict__ xr, co
   // `mag` is within the same tiny factor of sum|p|: 1 % of slack covers both second-order terms
   const double delta = 1.01 * (double)(d + d / 32 + 8) * 1.1102230246251565e-16 * mag;
   if ((float)(acc - delta) != (float)(acc + delta)) {  // warp-uniform
+    if (sp == nullptr) return __int_as_float(0x7fc00000);
     // replay of the reference's order: the lanes form the (exact) products of 256 elements at a
     // time, lane 0 adds them in index order -- the chain of dependent additions is all that is
     // left on one thread

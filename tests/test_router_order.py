@@ -104,3 +104,36 @@ def tied(kind, T, E):
 def test_equal_and_masked_logits(cuda, T, E, k, kind):
     spec = synth.LayerSpec(experts=E, topk=k, d=128, mid=64)
     check_ids(cuda, spec, synth.make_layer(spec, seed=98), tied(kind, T, E))
+
+
+@pytest.mark.parametrize("kind", ["zero rows", "zero router", "pairs", "all equal", "near"])
+@pytest.mark.parametrize("T,E,k", [(1, 64, 8), (5, 64, 8), (16, 64, 8), (16, 512, 16), (3, 20, 16)])
+def test_equal_logits_from_hidden_states(cuda, T, E, k, kind):
+    """Rows of zeros (padding), equal rows of the router, and rows that differ in one small element: logits a few floats apart."""
+    torch = cuda
+    spec = synth.LayerSpec(experts=E, topk=k, d=256, mid=64, router=True)
+    layer = synth.make_layer(spec, seed=100)
+    x = synth.bf16_bits_to_f32(synth.make_x(synth.rng_for(100, T), T, spec.d)).copy()
+    w = synth.bf16_bits_to_f32(layer["router_w"]).copy()
+    if kind == "zero rows":
+        x[::2] = 0
+    if kind == "zero router":
+        w[:] = 0
+    if kind == "pairs":
+        w[1::2] = w[::2]
+    if kind in ("all equal", "near"):
+        w[:] = w[3]
+    if kind == "near":
+        x[:, 17] = 1.0
+        w[:, 17] = np.float32(2.0) ** -26 * (np.arange(E) * 7 % 11)
+    layer["router_w"] = synth.f32_to_bf16_bits(w)
+    xb = synth.f32_to_bf16_bits(x)
+    ids_o, _ = want_ids(oracle.router_logits(layer["router_w"], x), k)
+    op = make_op(torch, spec, T, layer=layer)
+    op.load_router(0, dev_bytes(torch, layer["router_w"]))
+    out = torch.full((T, spec.d), float("nan"), dtype=torch.bfloat16, device="cuda")
+    op.moe_hidden(0, bf16_tensor(torch, xb, (T, spec.d)), out)
+    op.synchronize()
+    assert np.array_equal(op.get_routing(T)[0][:, :k], ids_o)
+    assert torch.isfinite(out).all()
+    op.close()
