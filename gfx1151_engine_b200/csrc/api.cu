@@ -33,34 +33,38 @@ struct LayerWeights {
 
 }  // namespace
 
-// Calls with few rows per expert, at most this many on average: what decides there is the decoding of the
-// weights, once per tile, and the GEMM kernels' narrow form (tiles of 64 rows) hides the latency of the
-// weights. Measured wide / narrow, even routing: 77 tokens on 512 experts of 4096 x 1024 (1.5 rows) 903 / 798 us,
-// 614 tokens (12 rows) 1183 / 1061, 500 tokens on 512 of 2560 x 640 550 / 494. Longer calls run the wide form alone
-// (2048 tokens of 2560 x 640, 40 rows: 748 / 802).
+// Which form of the grouped GEMM takes which tiles. The form for few rows (expert_few.cu, tiles of at most 64 rows) decodes
+// a block of weights in 255 to 350 cycles (10 to 60 rows), the wide one (expert_tc.cu, up to 192 rows) in 380 to 600. So tiles
+// of at most 64 rows take the first and larger ones the second, on two lists that run side by side; whether both lists
+// are worth their launches only the device can tell, from the rows of all experts (TileCut, k_route_scan). us of a call with
+// a cold L2, wide form alone / both lists: 512 experts of 4096 x 1024, even routing: 614 tokens 1152 / 814, 1200 1236 /
+// 931, 2048 1306 / 1091, 3200 1478 / 1373, 4096 1616 / 1625, 8192 2274 / 2245; the benchmark's skew: 614 402 / 343,
+// 2048 775 / 705, 4096 1308 / 1221, 8192 2304 / 2201, Q4_K / Q5_1 8192 2379 / 2264; 512 of 2560 x 640, 2048 tokens even 640
+// / 542, skewed 415 / 398, 4096 even 788 / 789, skewed 665 / 645; i4r 2048 tokens 706 / 572. Layers below this many weights of a projection
+// do not win the second list's launches back (64 of 2048 x 512, 1000 tokens 107 / 115, skewed 116 / 128).
+constexpr long long kBothLists = 500000000;
+// What the second list costs: launches, set-up and last items of two GEMM stages, in cycles of every SM. 5000 / 15000 /
+// 30000: 64 of 2048 x 512, 200 tokens, skewed 87 / 71 / 71 us, 400 tokens 95 / 87 / 87; 512 of 2560 x 640 + shared, 300 tokens, skewed 211 / 199 / 213.
+constexpr long long kSecondListCycles = 15000;
+// At most this many rows per expert on average: tiles of 64 rows in any layer, with a second list where the host cannot rule out that
+// it pays (no expert saves more than two tiles in 2 * 64 + 1 rows).
 constexpr int kFewRows = 12;
-// In such a call the popular experts of a skewed routing have hundreds of rows all the same, and decoding their
-// weights once per 64 of them costs more than the narrow form gives (614 tokens, the benchmark's skew, 4096 x
-// 1024: wide 419, narrow 476). So tiles of more than 64 rows go on a list of their own, which the wide form runs
-// beside the narrow one: 407. Which experts those are only the device knows; the host bounds what they can
-// save, and k_route_scan counts it. The second launch costs its set-up and its last items, which nothing
-// fills: measured by the tiles saved x K per SM, in tiles of 4096 columns: 0.4 lose 5 %, 1.0 1 to 6 %, 1.5 +1 to -5 %, 2.0 even,
-// 2.7 gain 3 %, 3.9 7 %, 9 15 %. The line lies at 2 of them on each of 148 SMs: saved * (mid / 64 * d + d / 128 * mid) =
-// 2 * 148 * 4096, as saved * d * mid. (An empty second list costs 0 to 3 us of the call.)
-constexpr long long kMinSavedWork = 2ll * 148 * 4096 * 128 / 3;
+// Smaller layers: all tiles in the form for few rows, on one list, up to so many rows per expert and tokens (a popular
+// expert then makes 8 tiles at most). 64 of 2048 x 512, wide / few: 200 tokens 79 / 71, skewed 81 / 71; 400 tokens 85 / 77,
+// 89 / 87.
+constexpr int kOneListRows = 48, kOneListTokens = 512;
 // The shared expert's rows stay in narrow tiles while its gate/up GEMM has at most this many of them times row
 // blocks: they fill SMs beside the routed ones, so that more and shorter items end earlier. Wide / narrow: 144
 // items (768 tokens, mid 768) 288 / 282 us, 384 (1536, mid 1024) 871 / 868, 576 (2304, mid 1024) 906 / 937.
 constexpr int kSharedNarrowItems = 384;
-// Experts of such a call with no more rows than one pass of the decode GEMV serves (8, 4 in the GGUF formats) take the
-// GEMV, which decodes a 128 x 64 block of weights in 250 cycles against 330 to 400, and the tensor-core launches run
-// beside it with the rest. That costs two more launches, 10 to 15 us, and gains 0.09 us per million weights of a
-// projection: the line lies at 160 million in such experts, which only the device can count (k_route_scan). It is
-// not asked where the average is above 5/4 of those rows: even routing then leaves less than a third of the experts there.
-// Without / with, us, cold L2, even routing and skews 0.5 and 1: 512 experts of 4096 x 1024, 24 tokens 423 / 351,
-// 269 / 239, 148 / 155; 100 tokens 892 / 698, 496 / 427, 208 / 204; 400 tokens 1026 / 916, 872 / 751, 339 / 317; 51
-// tokens in Q4_K / Q5_1 733 / 587, 409 / 353, 181 / 179; 512 of 2560 x 640 + shared, 51 tokens 310 / 267, 193 / 181, 101 / 112;
-// 500 tokens 476 / 463, 425 / 390, 202 / 204; 64 of 2048 x 512, 64 tokens 71 / 87 (all below the line: without).
+// Experts of a call of the first kind (kFewRows) with no more rows than one pass of the decode GEMV serves (8, 4 in the GGUF
+// formats) take the GEMV, with the tensor-core launches beside it for the rest. That costs two more launches, 10 to 15 us, and is
+// done where the GEMV's share is worth them: 160 million weights of a projection in such experts, which only the device can
+// count (k_route_scan). It is not asked where the average is above 5/4 of those rows: even routing then leaves less
+// than a third of the experts there. Without / with, us, cold L2: 512 experts of 4096 x 1024, 24 tokens 321 / 325 and (skew 1)
+// 124 / 132, 77 with a shared expert 634 / 640 and (0.5) 370 / 388, 400 tokens 792 / 824; Q4_K / Q5_1, 24 tokens 363 / 349, 77 710
+// / 695, 200 (0.5) 572 / 577; 512 of 2560 x 640 + shared, 500 tokens 378 / 398 and (0.5) 347 / 372. So it is no longer the
+// faster form for q4cp; it stays for its precision: the GEMV multiplies exact weights in fp32, the tensor cores weights rounded to fp16.
 // The two round differently (fp32 scales and sums by slices against fp16 weights), so that an output of such a call depends on the
 // other tokens by rounding; calls that must not have GEMM_TC.
 constexpr long long kMinFewWork = 160000000;
@@ -290,8 +294,8 @@ int b200moe_create(const b200moe_config* cfg, b200moe_handle* out) {
   const size_t pairs = (size_t)Tm * k;
   const size_t rows = pairs + (c.has_shared ? Tm : 0);
   h->max_rows = (int)rows;
-  // (calls with few rows per expert cut them into narrow tiles, most calls the shared expert's)
-  h->max_tiles_narrow = (int)(std::min(pairs, (size_t)kFewRows * E) / kTcNarrowN) + E + 1;
+  // (many calls cut all rows into narrow tiles)
+  h->max_tiles_narrow = (int)(pairs / kTcNarrowN) + E + 1;
   h->max_tiles = std::max((int)(pairs / h->tile_cap) + E + 1, h->max_tiles_narrow);
   h->max_tiles_sh = Tm / kTcNarrowN + 1;
   const size_t dec_rows = (size_t)std::min(Tm, h->decode_max) * (k + (c.has_shared ? 1 : 0));
@@ -764,13 +768,14 @@ static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const
   const bool simt = !L.i4r && (c.gemm_impl == B200MOE_GEMM_SIMT ||
                                 (c.gemm_impl == B200MOE_GEMM_AUTO && T <= h->decode_max));
   const bool few = T * k <= kFewRows * E;
-  const int min_saved = (int)(kMinSavedWork / ((long long)d * mid));
-  // (no expert saves more than two tiles in 2 * 64 + 1 rows; the small routing writes one list)
-  const bool split = few && T > 16 && T * k * 2 >= min_saved * (2 * kTcNarrowN + 1), narrow = few && !split;
+  const int second = (int)(kSecondListCycles * 148 * 8192 / (3ll * d * mid));  // per tile: 3 * d * mid weights, 8192 a block
+  const bool split = T > 16 && (few ? kTileCostFew * 2ll * T * k > (2 * kTcNarrowN + 1ll) * second
+                                    : (long long)E * d * mid >= kBothLists);
+  const bool narrow = !split && (few || (T <= kOneListTokens && T * k <= kOneListRows * E));
   const bool sh_narrow = few && (long long)(T / kTcNarrowN) * (mid / 64) <= kSharedNarrowItems;
   const int min_few = range ? 0 : few_row_experts(h, L, T);
   const bool mixed = min_few > 0;
-  const TileCut cut{narrow ? kTcNarrowN : h->tile_cap, sh_narrow ? kTcNarrowN : h->tile_cap, split ? kTcNarrowN : 0, min_saved,
+  const TileCut cut{narrow ? kTcNarrowN : h->tile_cap, sh_narrow ? kTcNarrowN : h->tile_cap, split ? kTcNarrowN : 0, second,
                     mixed ? std::min(gemv_rows(L.gu.fmt), gemv_rows(L.dn.fmt)) : 0, min_few};
   // (the shared expert's images are q4cp: it can ride along only with q4cp routed experts)
   const bool gemv = simt && c.gemm_impl == B200MOE_GEMM_AUTO &&
@@ -851,7 +856,7 @@ static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const
     auto stage_tc = [&](auto launch, const Image& img, const Image* sh, __half* out16) -> cudaError_t {
       const Tile* first = split ? h->rb.tiles_narrow : h->rb.tiles;
       cudaError_t e = launch(h->tc, img, first, h->rb.n_tiles + (split ? 2 : 0), split ? h->max_tiles_narrow : h->max_tiles,
-                             out16, h->status_dev, st, TcLaunch{few, mixed});  // (mixed: beside the GEMV in front)
+                             out16, h->status_dev, st, TcLaunch{narrow || split, mixed});  // (mixed: beside the GEMV in front)
       if (e == cudaSuccess && sh)
         e = launch(h->tc, *sh, h->rb.tiles_sh, h->rb.n_tiles + 1, h->max_tiles_sh, out16, h->status_dev, st,
                    TcLaunch{sh_narrow, true});

@@ -12,19 +12,17 @@
 //   warp 0      producer of activation tiles: TMA tensor copies (128-byte swizzle, box of
 //               16/64/128/192 rows), one per K block, into a ring of 3 pair-slots in shared
 //               memory; the same thread asks for the packed weight tiles of a later pair to be
-//               brought into L2 (one bulk prefetch per pair; wide form)
+//               brought into L2 (one bulk prefetch per pair)
 //   warp 1      issues tcgen05.mma (A from tensor memory, B from shared memory): eight per
 //               pair behind ONE barrier wait and ONE commit; owns the tensor-memory allocation
-//   warp 2      narrow form (tiles of at most 64 rows, see Map): producer of packed weights, one
-//               bulk copy per pair into a ring of 8 stages in shared memory
 //   warp 3      relay: folds "activations of the pair have landed" into the barrier the MMA
 //               warp waits on, so that warp polls a single barrier
 //   warps 4-19  dequantise: two sets of eight warps alternate pairs (set s owns tensor-memory
-//               slot s); thread = one weight row of one K block. Packed codes come, in the wide
-//               form, straight from global memory (a warp's 32 rows are 512 contiguous bytes) into
+//               slot s); thread = one weight row of one K block. Packed codes come
+//               straight from global memory (a warp's 32 rows are 512 contiguous bytes) into
 //               ONE set of registers, refilled for the next own pair as soon as the decode has used
 //               them up, through a pointer that walks with the stream (the tile list is read one
-//               item ahead, never on the critical path), in the narrow form from warp 2's ring;
+//               item ahead, never on the critical path);
 //               each code byte indexes a 256-entry half2
 //               pair table replicated per lane in shared memory (bank-conflict free, the
 //               address is one byte permute); one half2 multiply by the group scale; the
@@ -42,30 +40,16 @@
 // debugging code unless it is compiled in.
 // Every wait on an mbarrier is bounded; when one gives up the CTA records a status
 // word, stops issuing work, and leaves after releasing its tensor memory.
-#include "tc.h"
-
-#include "kernels.h"
-
-#include <cuda.h>
-#include <cudaTypedefs.h>
+#include "tc_dev.cuh"
 
 #include <cstdio>
-#include <cstdlib>
 
 namespace b200moe {
-
-struct TcPlan {
-  CUtensorMap x[4], h[4];  // activation / hidden maps with boxes of 16, 64, 128, 192 rows
-  int sms = 148;
-  int margin = 0;
-  long long* trace = nullptr;  // debug timeline of CTA 0 (environment B200MOE_TC_TRACE=<file>)
-};
 
 namespace {
 
 constexpr int kNS = 2;    // tensor-memory A slots; a slot holds a pair of K blocks (64 columns)
 constexpr int kNBSMax = 3;
-constexpr int kNST = 8;                  // narrow tiles: stages of packed weights, a pair of K blocks each
 constexpr int kThreads = 768;           // 24 warps: 4 service, 16 dequantising, 4 epilogue
 constexpr int kAccCols = kTcTileN;       // columns per accumulator
 constexpr int kTmemA = 2 * kAccCols;     // first column of the A slots
@@ -79,29 +63,20 @@ static_assert(kTmemA + kNS * 64 <= 512, "tensor memory: two accumulators and the
 // boundary, so that a lookup address is ONE byte permute:
 //   bytes { lane*4 (+128), code byte, table >> 16, 0 }.
 // The first activation slot fits below the table, the other two above it.
-//
-// TN is the most rows a tile of the launch has. 192 (wide form): the activation slots take all
-// there is. 64 (narrow form: tiles with few rows, whose MMAs are short, so that the packed weights
-// decide): all three slots lie below the table and the space above it is a ring of kNST pairs of
-// weight tiles (74 to 98 KB in flight per SM), which warp 2 fills with bulk copies. The dequantising
-// warps' register fetch of the wide form reaches one pair ahead, which is less than a load from L2
-// takes: on a 77-token prompt (1 to 3 rows per expert) 40 % of their time went into that wait.
-template <int TN>
 struct Map {
-  static constexpr int kBStage = TN * 128;             // bytes of one K block of activations: rows x 64 halfs
+  static constexpr int kBStage = kTcTileN * 128;       // bytes of one K block of activations: rows x 64 halfs
   static constexpr int kNBS = 3;                       // activation ring depth, in pairs of K blocks
   static constexpr int kOffLow = 2048;                 // the dynamic allocation must start at or below this
   static constexpr int kOffBar = 2048;                 // barriers and flags (1 KB)
   static constexpr int kOffU = 3072;                   // epilogue exchange + output tile (12 KB)
   static constexpr int kOffB0 = 15360;                 // activation slot 0 (1 KB aligned)
   static constexpr int kOffLut = 65536;                // 256 lines of 256 B
-  static constexpr int kOffB1 = 131072;                // wide: activation slots 1, 2; narrow: weight stages
-  static constexpr int kSmemEnd = TN == kTcTileN ? kOffB1 + 2 * 2 * kBStage : kOffB1 + kNST * 2 * tile_bytes(kQ51);
+  static constexpr int kOffB1 = 131072;                // activation slots 1, 2
+  static constexpr int kSmemEnd = kOffB1 + 2 * 2 * kBStage;
   static constexpr int kSmemBytes = kSmemEnd - 1024;   // dynamic bytes requested
-  static_assert(kOffB0 + (TN == kTcTileN ? 1 : kNBS) * 2 * kBStage <= kOffLut, "activation slots overlap the table");
+  static_assert(kOffB0 + 2 * kBStage <= kOffLut, "activation slots overlap the table");
   static_assert(kSmemEnd <= 233472, "shared memory map exceeds the SM");
   __host__ __device__ static constexpr uint32_t slot(uint32_t s) {
-    if (TN != kTcTileN) return (uint32_t)(kOffB0 + s * 2 * kBStage);
     return s == 0 ? (uint32_t)kOffB0 : (uint32_t)(kOffB1 + (s - 1) * 2 * kBStage);
   }
 };
@@ -112,163 +87,8 @@ constexpr int kBarAFull = 0,                   // [tensor-memory slot]: A of a p
               kBarDone = kBarBFull + kNBSMax,  // [activation slot]: all MMAs of a pair have completed
               kBarAccFull = kBarDone + kNBSMax,
               kBarAccEmpty = kBarAccFull + 2,
-              kBarCFull = kBarAccEmpty + 2,    // [weight stage] (narrow): a pair's packed tiles have landed
-              kBarCEmpty = kBarCFull + kNST,   // [weight stage]: the set's eight warps hold them in registers
-              kNumBars = kBarCEmpty + kNST;
+              kNumBars = kBarAccEmpty + 2;
 static_assert(kNumBars * 8 + 16 + 32 <= 1024, "barrier block too small");
-
-constexpr long long kWaitLimitNs = 2000000000ll;  // 2 s: far beyond any legitimate wait
-
-// ---- PTX wrappers ------------------------------------------------------------------
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity), "r"(20000u)  // suspend-time hint (ns): sleep in hardware, not in a poll loop
-      : "memory");
-  return ok != 0;
-}
-// One lane of a converged warp. Code around it stays warp-uniform, which lets the compiler
-// keep descriptors and addresses in uniform registers instead of converting per instruction.
-__device__ __forceinline__ bool elect_one() {
-  uint32_t pred;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "elect.sync _|p, 0xffffffff;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(pred));
-  return pred != 0;
-}
-__device__ __forceinline__ unsigned long long now_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-  return t;
-}
-
-// Bounded wait. Returns false when the CTA is aborting (this wait or another one gave up).
-// `nap_ns` > 0 makes the waiting warp sleep between polls: warps that poll in a tight loop
-// take issue slots from the warp that shares their scheduler, and the thread that issues
-// the MMAs must not be slowed down by waiters.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
-                                          int32_t* status, int where, unsigned nap_ns = 0) {
-  if (mbar_try(bar, parity)) return true;
-  const unsigned long long t0 = now_ns();
-  for (uint32_t spin = 1;; spin++) {
-    if (nap_ns) __nanosleep(nap_ns);
-    if (mbar_try(bar, parity)) return true;
-    if ((spin & 255u) == 0) {
-      if (*abort_flag) return false;
-      if (now_ns() - t0 > (unsigned long long)kWaitLimitNs) {
-        *abort_flag = 1;
-        if (atomicCAS(status, 0, 1) == 0) status[1] = where;
-        return false;
-      }
-    }
-  }
-}
-
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y,
-                                            uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-      "l"(map), "r"(x), "r"(y), "r"(bar)
-      : "memory");
-}
-
-__device__ __forceinline__ void tc_fence_before() {
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void tc_fence_after() {
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void tc_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
-               : "memory");
-}
-// D[tmem] (+)= A[tmem] * B[smem descriptor]; fp16 operands, fp32 accumulate.
-__device__ __forceinline__ void tc_mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
-                                          uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-__device__ __forceinline__ void tc_st32(uint32_t taddr, const uint32_t* v) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-      "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" ::"r"(taddr),
-      "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
-      "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]),
-      "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]),
-      "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]),
-      "r"(v[30]), "r"(v[31])
-      : "memory");
-}
-__device__ __forceinline__ void tc_wait_st() {
-  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t* v) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
-        "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
-        "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]),
-        "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]),
-        "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-      : "r"(taddr)
-      : "memory");
-}
-__device__ __forceinline__ void tc_wait_ld() {
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-// Shared-memory matrix descriptor of a K-major fp16 tile stored as rows of 128 bytes with
-// the 128-byte swizzle (what the TMA tensor copy writes): 8-row groups are 1024 bytes
-// apart, descriptor version 1 (Blackwell), layout type 2 = 128-byte swizzle.
-__device__ __forceinline__ uint64_t b_descriptor(uint32_t smem_addr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((smem_addr & 0x3FFFFu) >> 4);
-  d |= (uint64_t)1 << 16;            // leading-dimension offset (unused for swizzled K-major)
-  d |= (uint64_t)(1024 >> 4) << 32;  // stride between 8-row groups
-  d |= (uint64_t)1 << 46;            // descriptor version
-  d |= (uint64_t)2 << 61;            // 128-byte swizzle
-  return d;
-}
-
-// Instruction descriptor: D fp32, A/B fp16, both K-major, M = 128, N = n.
-__device__ __forceinline__ uint32_t instr_desc(int n) {
-  return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-}
-
-// finite values saturate to the fp16 range (as on the GEMV path), NaN stays NaN
-// fp32 -> fp16, finite values saturating to the fp16 range, NaN staying NaN: one conversion
-__device__ __forceinline__ __half f16_sat(float v) {
-  unsigned short h;
-  asm("cvt.rn.satfinite.f16.f32 %0, %1;" : "=h"(h) : "f"(v));
-  return __ushort_as_half(h);
-}
 
 struct KParams {
   Image img;
@@ -299,55 +119,7 @@ constexpr int kTraceSlots = 512;
   } while (0)
 #endif
 
-// Per (row, K block) metadata of the source format, as loaded by a dequantising thread.
-struct RowMetaTc {
-  uint32_t a, b, c, d;
-};
-
-// Two fp16 weights from one code byte's table entry `pair` (the two codes as fp16 numbers
-// for the GGUF formats, the two code-book values for q4cp) and the group's constants.
-template <int FMT>
-struct GroupDecode {};
-template <>
-struct GroupDecode<kQ4CP> {  // w = f16(book) * f16(scale)
-  __half2 s2;
-  __device__ __forceinline__ void init(const RowMetaTc& m, int h) {
-    const uint32_t v = __byte_perm(m.a, 0u, h ? 0x3232u : 0x1010u);  // the half's fp16 scale in both lanes
-    s2 = *(const __half2*)&v;
-  }
-  __device__ __forceinline__ __half2 weight(uint32_t pair, int) const { return __hmul2(*(__half2*)&pair, s2); }
-};
-template <>
-struct GroupDecode<kQ4K> {  // w = (d*sc)*q - (dmin*m), the packed form of src/gguf.h:423-432
-  __half2 a2, nb2;
-  __device__ __forceinline__ void init(const RowMetaTc& m, int h) {
-    const float d = half_bits_to_f32((uint16_t)(m.a & 0xFFFFu)), dmin = half_bits_to_f32((uint16_t)(m.a >> 16));
-    const float sc = (float)((m.b >> (16 * h)) & 0xFFu), mn = (float)((m.b >> (16 * h + 8)) & 0xFFu);
-    a2 = __float2half2_rn(d * sc);
-    nb2 = __float2half2_rn(-(dmin * mn));
-  }
-  __device__ __forceinline__ __half2 weight(uint32_t pair, int) const { return __hfma2(*(__half2*)&pair, a2, nb2); }
-};
-template <>
-struct GroupDecode<kQ51> {  // w = d*(q + 16*fifth bit) + m, src/gguf.h:360-374
-  __half2 d2, m2;
-  uint32_t qh;
-  __device__ __forceinline__ void init(const RowMetaTc& m, int h) {
-    const uint32_t dm = h ? m.c : m.a;
-    qh = h ? m.d : m.b;
-    d2 = __half2half2(__ushort_as_half((unsigned short)(dm & 0xFFFFu)));
-    m2 = __half2half2(__ushort_as_half((unsigned short)(dm >> 16)));
-  }
-  // byte i of the group holds elements 2i, 2i+1; their fifth bits are bits i, 16 + i of qh:
-  // shifted to bits 14 and 30 they read as the fp16 pair (2.0 or 0, 2.0 or 0)
-  __device__ __forceinline__ __half2 weight(uint32_t pair, int i) const {
-    const uint32_t u = (i <= 14 ? (qh << (14 - i)) : (qh >> 1)) & 0x40004000u;
-    const __half2 q5 = __hfma2(*(const __half2*)&u, __float2half2_rn(8.f), *(const __half2*)&pair);
-    return __hfma2(q5, d2, m2);
-  }
-};
-
-template <bool UP, bool DUAL, int FMT, int TN>
+template <bool UP, bool DUAL, int FMT>
 __global__ void __launch_bounds__(kThreads, 1)
 k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ CUtensorMap map64,
             const __grid_constant__ CUtensorMap map128, const __grid_constant__ CUtensorMap map192,
@@ -357,8 +129,7 @@ k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ C
   const uint32_t dyn0 = smem_u32(smem_raw);
   uint8_t* const smem = smem_raw - dyn0;
   constexpr uint32_t sbase = 0;
-  using M = Map<TN>;
-  constexpr bool kNarrow = TN != kTcTileN;
+  using M = Map;
   constexpr int kBStage = M::kBStage, kNBS = M::kNBS, kOffLow = M::kOffLow, kOffU = M::kOffU, kOffBar = M::kOffBar,
                 kSmemEnd = M::kSmemEnd;
   {
@@ -389,10 +160,6 @@ k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ C
     for (int i = 0; i < kNBS; i++) {
       mbar_init(bars + 8 * (kBarBFull + i), 1);    // activation producer (with byte count)
       mbar_init(bars + 8 * (kBarDone + i), 1);     // one tcgen05.commit per pair
-    }
-    for (int i = 0; i < kNST; i++) {
-      mbar_init(bars + 8 * (kBarCFull + i), 1);
-      mbar_init(bars + 8 * (kBarCEmpty + i), 8);
     }
     for (int i = 0; i < 2; i++) {
       mbar_init(bars + 8 * (kBarAccFull + i), 1);
@@ -465,7 +232,7 @@ k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ C
         const uint8_t* w_next =
             it + (int)gridDim.x < n_items ? img.mtile(t_ahead.expert, (it + (int)gridDim.x) % img.n_mtiles) : nullptr;
         for (int pp = 0; pp < NP && ok; pp++, pi++) {
-          if (!kNarrow && p.l2_ahead > 0 && (pp & 1) == 0) {  // two pairs at a time: they lie side by side in a sub-block
+          if (p.l2_ahead > 0 && (pp & 1) == 0) {  // two pairs at a time: they lie side by side in a sub-block
             int q = pp + 2 * p.l2_ahead;
             const uint8_t* b2 = w_this;
             if (q >= NP) {
@@ -582,8 +349,8 @@ k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ C
     };
     const int io_step = NP == 1 ? 2 : 1;  // a set visits every item, or every other one when an item is one pair
     int f_io = set / NP, f_pp = set % NP;
-    const uint8_t* f_base = kNarrow ? nullptr : item_base(f_io);
-    const uint8_t* f_next = kNarrow ? nullptr : item_base(f_io + io_step);
+    const uint8_t* f_base = item_base(f_io);
+    const uint8_t* f_next = item_base(f_io + io_step);
     // f_tile walks with the stream: this row's codes in K block 2 * f_pp + kblk of the current item
     const uint8_t* f_tile = f_base ? f_base + (size_t)(2 * f_pp + kblk) * sub_b : nullptr;
     const size_t step_b = 4 * sub_b;  // the set's next pair is two pairs = four K blocks further
@@ -616,49 +383,15 @@ k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ C
         f_tile = f_base ? f_base + (size_t)(2 * f_pp + kblk) * sub_b : nullptr;
       }
     };
-    if (!kNarrow) fetch(ca, cb, sc);
+    fetch(ca, cb, sc);
     bool mine = f_valid;  // the codes in (ca, cb, sc) are a K block of this thread's
     bool ok = true;
-    // narrow: the pair's tiles come from the ring of weight stages
-    uint32_t c_stage = (uint32_t)set, c_ph = 0;
-    int c_pp = set % NP;
-    auto from_ring = [&]() -> bool {
-      if (!__all_sync(0xffffffffu, mbar_wait(bars + 8 * (kBarCFull + c_stage), c_ph, abort_flag, p.status, 11))) return false;
-      mine = 2 * c_pp + kblk < KB;
-      if (mine) {
-        const uint8_t* pc = smem + M::kOffB1 + c_stage * (8 * (uint32_t)sub_b) + (pos >> 5) * (2 * (uint32_t)sub_b) + kblk * (uint32_t)sub_b + off_c;
-        ca = *(const uint4*)pc;
-        cb = *(const uint4*)(pc + kHalfBytes);
-        const uint8_t* pm = pc + (off_m - off_c);
-        if (FMT == kQ4CP) {
-          sc.a = *(const uint32_t*)pm;
-        } else if (FMT == kQ4K) {
-          const uint2 u = *(const uint2*)pm;
-          sc.a = u.x;
-          sc.b = u.y;
-        } else {
-          const uint4 u = *(const uint4*)pm;
-          sc = RowMetaTc{u.x, u.y, u.z, u.w};
-        }
-      }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bars + 8 * (kBarCEmpty + c_stage));
-      c_stage += 2;
-      if (c_stage >= (uint32_t)kNST) {
-        c_stage -= kNST;
-        c_ph ^= 1;
-      }
-      for (c_pp += 2; c_pp >= NP;) c_pp -= NP;
-      return true;
-    };
-    static_assert(kNST % 2 == 0, "a set visits every other stage");
     static_assert(kNS == 2, "a set always fills the tensor-memory slot of its own index");
     const uint32_t aslot = (uint32_t)set;
     uint32_t qslot = (uint32_t)set % kNBS, qph = 0;  // (pi - kNS) % kNBS and ((pi - kNS) / kNBS) & 1, from pi == set + kNS on
     for (uint32_t pi = set; pi < total && ok; pi += 2) {
       if (lane == 0 && quarter == 0) TR(2 + kblk, pi, 0);
       uint32_t v[32];
-      if (kNarrow && !from_ring()) break;
       const bool mine_now = mine;
       if (mine_now) {
 #pragma unroll
@@ -683,10 +416,8 @@ k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ C
       // The codes are used up: the next own pair's go into the same registers (no second set, no
       // copies). They have the rest of this iteration and the wait of the next one to arrive, and
       // the producer thread's L2 prefetch has put them close.
-      if (!kNarrow) {
-        fetch(ca, cb, sc);
-        mine = f_valid;
-      }
+      fetch(ca, cb, sc);
+      mine = f_valid;
       if (lane == 0 && quarter == 0) TR(2 + kblk, pi, 1);
       if (pi >= (uint32_t)kNS) {
         // the slot is free once the MMAs of the pair that used it before (pi - kNS) have completed
@@ -709,34 +440,6 @@ k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ C
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(bars + 8 * (kBarAFull + aslot));
-    }
-  } else if (kNarrow && warp == 2) {
-    // ================= producer of packed weights (a bulk copy per sub-block and pair of K blocks) ==========
-    if (lane == 0) {
-      constexpr uint32_t w_sub_b = sub_bytes(FMT);
-      const size_t w_col_b = (size_t)KB * w_sub_b;  // from one sub-block to the next
-      uint32_t stage = 0, ph = 0;
-      bool ok = true;
-      Tile t_ahead = (int)blockIdx.x < n_items ? p.tiles[blockIdx.x / img.n_mtiles] : Tile{0, 0, 0};
-      for (int it = blockIdx.x; it < n_items && ok; it += gridDim.x) {
-        const uint8_t* src = img.mtile(t_ahead.expert, it % img.n_mtiles);
-        if (it + (int)gridDim.x < n_items) t_ahead = p.tiles[(it + gridDim.x) / img.n_mtiles];
-        for (int pp = 0; pp < NP; pp++, src += 2 * w_sub_b) {
-          ok = mbar_wait(bars + 8 * (kBarCEmpty + stage), ph ^ 1, abort_flag, p.status, 12, 64);
-          if (!ok) break;
-          const uint32_t bytes = (uint32_t)min(2, KB - 2 * pp) * w_sub_b, bar = bars + 8 * (kBarCFull + stage);
-          mbar_expect_tx(bar, kTileM / kSubRows * bytes);
-#pragma unroll
-          for (int s = 0; s < kTileM / kSubRows; s++)
-            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                             (uint32_t)M::kOffB1 + stage * (8 * w_sub_b) + s * (2 * w_sub_b)), "l"(src + s * w_col_b), "r"(bytes), "r"(bar)
-                         : "memory");
-          if (++stage == (uint32_t)kNST) {
-            stage = 0;
-            ph ^= 1;
-          }
-        }
-      }
     }
   } else if (warp == 3) {
     // ================= relay: "activations landed" folded into the A-slot barrier ==========
@@ -901,14 +604,27 @@ cudaError_t encode_2d(PFN_cuTensorMapEncodeTiled_v12000 enc, CUtensorMap* map, c
   return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
-template <bool UP, bool DUAL, int FMT, int TN>
+// Two K blocks of `box_rows` rows per copy, one behind the other.
+cudaError_t encode_pair(PFN_cuTensorMapEncodeTiled_v12000 enc, CUtensorMap* map, const void* base,
+                        long long rows, long long cols, int box_rows) {
+  cuuint64_t dims[3] = {64, (cuuint64_t)rows, (cuuint64_t)(cols / 64)};
+  cuuint64_t strides[2] = {(cuuint64_t)cols * 2, 128};
+  cuuint32_t box[3] = {64, (cuuint32_t)box_rows, 2};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(base), dims, strides,
+                   box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
+template <bool UP, bool DUAL, int FMT>
 cudaError_t launch_n(TcPlan* plan, const CUtensorMap* m, const Image& img,
                    const Tile* tiles, const int32_t* n_tiles, int max_tiles, __half* out, int out_ld,
                    int32_t* status, cudaStream_t st, const int32_t* rowmap, const int32_t* map_base, bool beside) {
-  constexpr int kSmemBytes = Map<TN>::kSmemBytes;
+  constexpr int kSmemBytes = Map::kSmemBytes;
   static bool attr_set = false;  // one flag per template instance
   if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(k_expert_tc<UP, DUAL, FMT, TN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(k_expert_tc<UP, DUAL, FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          kSmemBytes);
     if (e != cudaSuccess) return e;
     attr_set = true;
@@ -923,7 +639,7 @@ cudaError_t launch_n(TcPlan* plan, const CUtensorMap* m, const Image& img,
   // With a margin the free SMs belong to another stream's exchange kernels. The CTAs of a dependent launch
   // would take them, shared memory and registers of a whole SM each, and only wait there: no early start
   // then, neither of this launch nor (early_next) of the one behind it.
-  return launch_opt(plan->margin == 0, k_expert_tc<UP, DUAL, FMT, TN>, dim3(grid), dim3(kThreads), (size_t)kSmemBytes, st, m[0],
+  return launch_opt(plan->margin == 0, k_expert_tc<UP, DUAL, FMT>, dim3(grid), dim3(kThreads), (size_t)kSmemBytes, st, m[0],
                     m[1], m[2], m[3], p);
 }
 
@@ -931,10 +647,11 @@ template <bool UP, bool DUAL, int FMT>
 cudaError_t launch(TcPlan* plan, const CUtensorMap* m, const Image& img,
                    const Tile* tiles, const int32_t* n_tiles, int max_tiles, __half* out, int out_ld,
                    int32_t* status, cudaStream_t st, const TcLaunch& o) {
-  if (o.narrow)
-    return launch_n<UP, DUAL, FMT, kTcNarrowN>(plan, m, img, tiles, n_tiles, max_tiles, out, out_ld, status, st, o.rowmap,
-                                               o.map_base, o.beside);
-  return launch_n<UP, DUAL, FMT, kTcTileN>(plan, m, img, tiles, n_tiles, max_tiles, out, out_ld, status, st, o.rowmap,
+  if (o.narrow) {
+    if (o.rowmap != nullptr) return cudaErrorInvalidValue;
+    return launch_few(plan, UP, m == plan->h, img, tiles, n_tiles, max_tiles, out, out_ld, status, st, o.beside);
+  }
+  return launch_n<UP, DUAL, FMT>(plan, m, img, tiles, n_tiles, max_tiles, out, out_ld, status, st, o.rowmap,
                                            o.map_base, o.beside);
 }
 
@@ -957,6 +674,8 @@ cudaError_t tc_create(TcPlan** out, const __half* x_sorted, const __half* hid16,
   e = cudaSuccess;
   for (int i = 0; i < 4 && e == cudaSuccess; i++) e = encode_2d(enc, &plan->x[i], x_sorted, rows_cap, d, boxes[i]);
   for (int i = 0; i < 4 && e == cudaSuccess; i++) e = encode_2d(enc, &plan->h[i], hid16, rows_cap, mid, boxes[i]);
+  for (int i = 0; i < 3 && e == cudaSuccess; i++) e = encode_pair(enc, &plan->x2[i], x_sorted, rows_cap, d, 16 << i);
+  for (int i = 0; i < 3 && e == cudaSuccess; i++) e = encode_pair(enc, &plan->h2[i], hid16, rows_cap, mid, 16 << i);
   if (e != cudaSuccess) {
     delete plan;
     return e;

@@ -13,7 +13,7 @@ namespace b200moe {
 // the next kernel of the stream may start its prologue (code-book tables, index setup) while
 // this one drains. A kernel launched this way must call pdl_wait() before it touches anything
 // an earlier kernel of the stream wrote (or still reads); pdl_trigger() lets its own successor
-// start early. (One exception: k_expert_tc launches with TcLaunch::beside rely on the wait of the
+// start early. (One exception: k_expert_tc and k_expert_few launches with TcLaunch::beside rely on the wait of the
 // k_expert_tc or k_gemv launch in front of them, which triggers behind it.) B200MOE_NO_PDL=1 in the environment turns the attribute off (plain launches).
 // launch_opt(false, ...) is a plain launch of the same kernel.
 #ifdef __CUDACC__
@@ -88,10 +88,12 @@ struct RouteBuffers {
 cudaError_t launch_router_topk(const float* logits, int T, int E, int k, int32_t* ids, float* w,
                                int stride, cudaStream_t st);
 // How the work lists are cut: at most `routed` rows in a tile of a routed expert, `shared` in one of the shared
-// expert. Routed tiles of at most `narrow` rows go on tiles_narrow instead of tiles (0: all on tiles) if tiles of
-// `routed` rows make at least min_saved fewer of them than tiles of `narrow` rows; else all rows are cut to that.
+// expert. narrow > 0: the device chooses between tiles of `routed` rows on tiles, tiles of `narrow` rows on tiles_narrow, and
+// both lists, where the ragged tiles of at most `narrow` rows go on tiles_narrow and the others on tiles.
+// What a tile costs in the one and in the other form (cycles per 128 x 64 block of weights), and the second list's launches in that unit.
+constexpr int kTileCostWide = 380, kTileCostFew = 270;
 struct TileCut {
-  int routed, shared, narrow = 0, min_saved = 0;
+  int routed, shared, narrow = 0, second = 0;
   // > 0: if at least min_few experts have rows, but no more than gemv_rows, those get no tiles; runs / n_runs[0] list them and no others.
   int gemv_rows = 0, min_few = 0;
 };

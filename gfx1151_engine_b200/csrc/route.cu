@@ -97,7 +97,7 @@ k_route_scan(int32_t* __restrict__ blockcnt, int nblk, int E, int pairs, int T, 
   __shared__ __align__(4) uint16_t s_bin[kMaxExperts / 32][kTcTileN + 8];  // ragged tiles of a size: per warp, then in the warps before
   __shared__ int s_gt[256], s_gw[8];                          // larger ones, of all
   __shared__ unsigned long long s_w[kMaxExperts / 32];
-  __shared__ int s_wc[kMaxExperts / 32], s_saved[kMaxExperts / 32];
+  __shared__ int s_wc[kMaxExperts / 32], s_sum[3][kMaxExperts / 32];
   const int e = threadIdx.x, lane = e & 31, warp = e >> 5;
   pdl_trigger();
   pdl_wait();
@@ -117,21 +117,31 @@ k_route_scan(int32_t* __restrict__ blockcnt, int nblk, int E, int pairs, int T, 
         }
     }
   }
-  // three inclusive scans side by side: counts (low 32 bits) and non-empty flags, full tiles
-  int tile_cap = cut.routed;
-  if (cut.narrow > 0) {
-    // two lists only where the wide tiles save enough of the narrow ones
-    const int saved = __reduce_add_sync(0xffffffffu, (cnt + cut.narrow - 1) / cut.narrow - (cnt + tile_cap - 1) / tile_cap);
-    if (lane == 0) s_saved[warp] = saved;
-    __syncthreads();
-    int all = 0;
-#pragma unroll
-    for (int w = 0; w < kMaxExperts / 32; w++) all += s_saved[w];
-    if (all < cut.min_saved) tile_cap = cut.narrow;
-  }
   // experts with few rows to the decode GEMV, where there are enough of them
   const bool by_gemv = cut.gemv_rows > 0 && __syncthreads_count(cnt > 0 && cnt <= cut.gemv_rows) >= cut.min_few && cnt <= cut.gemv_rows;
+  int tile_cap = cut.routed, narrow = cut.narrow;
+  if (narrow > 0) {
+    // one list of wide tiles, one of narrow ones, or both: whichever costs least
+    const int rows = by_gemv ? 0 : cnt, part = rows % tile_cap;
+    const int n[3] = {(rows + tile_cap - 1) / tile_cap, (rows + narrow - 1) / narrow, part > 0 && part <= narrow};
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      const int sum = __reduce_add_sync(0xffffffffu, n[i]);
+      if (lane == 0) s_sum[i][warp] = sum;
+    }
+    __syncthreads();
+    int all[3] = {0, 0, 0};
+#pragma unroll
+    for (int w = 0; w < kMaxExperts / 32; w++)
+#pragma unroll
+      for (int i = 0; i < 3; i++) all[i] += s_sum[i][w];
+    const int wide = kTileCostWide * all[0], few = kTileCostFew * all[1];
+    const int both = kTileCostWide * (all[0] - all[2]) + kTileCostFew * all[2] + cut.second;
+    if (few <= wide && few <= both) tile_cap = narrow;
+    else if (wide <= both) narrow = 0;
+  }
   const bool listed = cnt > 0 && (by_gemv || cut.gemv_rows == 0);
+  // three inclusive scans side by side: counts (low 32 bits) and non-empty flags, full tiles
   const int nfull = by_gemv ? 0 : cnt / tile_cap, part = by_gemv ? 0 : cnt % tile_cap;
   unsigned long long ab = (unsigned long long)(uint32_t)cnt | (unsigned long long)listed << 32;
   int c = nfull;
@@ -181,7 +191,7 @@ k_route_scan(int32_t* __restrict__ blockcnt, int nblk, int E, int pairs, int T, 
     s_gt[bin] = above;
   }
   __syncthreads();
-  const int nparts = s_gt[0], wide_parts = s_gt[cut.narrow], rank = s_gt[part] + s_bin[warp][part] + __popc(same & ((1u << lane) - 1u));
+  const int nparts = s_gt[0], wide_parts = s_gt[narrow], rank = s_gt[part] + s_bin[warp][part] + __popc(same & ((1u << lane) - 1u));
   unsigned long long ab_all = 0;
   int c_all = 0;
 #pragma unroll
@@ -204,8 +214,8 @@ k_route_scan(int32_t* __restrict__ blockcnt, int nblk, int E, int pairs, int T, 
     runs[kMaxExperts] = Run{0, pairs, T};
   }
   if (listed) runs[(int)(ab >> 32) - 1] = Run{e, first, cnt};
-  // full tiles first, then the ragged ones from large to small: those with more than cut.narrow rows on tiles
-  const int n_wide = tile_cap > cut.narrow ? total_full + wide_parts : 0;
+  // full tiles first, then the ragged ones from large to small: those with more than `narrow` rows on tiles
+  const int n_wide = tile_cap > narrow ? total_full + wide_parts : 0;
   auto put = [&](int i, const Tile& t) {
     if (i < n_wide) tiles[i] = t;
     else tiles_narrow[i - n_wide] = t;

@@ -237,3 +237,63 @@ def test_many_non_finite_rows_in_a_short_call(cuda, E, k, T, bad, rotated):
     assert np.isnan(y[:bad]).all() and np.isfinite(y[bad:]).all()
     assert np.array_equal(bits(y[bad:]), bits(clean[bad:]))
     op.close()
+
+
+def random_blob(torch, rows, cols, fmt, seed):
+    """Random codes on the GPU: q4cp with a linear code book (fmt None), or GGUF blocks."""
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    if fmt is None:
+        stride = ((cols // 32 * 2) + 15) & ~15
+        book = torch.linspace(-1.0, 1.0, 16, device="cuda").view(torch.uint8)
+        codes = torch.randint(0, 256, (rows * cols // 2,), dtype=torch.uint8, device="cuda", generator=gen)
+        scales = torch.empty(rows * stride // 2, device="cuda").uniform_(0.005, 0.03, generator=gen).half().view(torch.uint8)
+        return torch.cat([book, codes, scales])
+    per, n, heads = {pkg.GGML_Q5_K: (256, 176, (1e-3, 5e-4)), pkg.GGML_Q5_1: (32, 24, (1e-2, -1e-1)), pkg.GGML_Q8_0: (32, 34, (2e-4,))}[fmt]
+    b = torch.randint(0, 256, (rows * cols // per, n), dtype=torch.uint8, device="cuda", generator=gen)
+    for i, h in enumerate(heads):
+        b[:, 2 * i:2 * i + 2] = torch.full((len(b), 1), h, device="cuda").half().view(torch.uint8)
+    return b.reshape(-1)
+
+
+# K blocks of gate/up and down with all remainders of a quad; rows on both sides of a box of 16 and 32, of one and two tiles
+# and of a wide tile; layers on both sides of the line for two lists
+@pytest.mark.parametrize("E,k,d,mid,types", [(96, 4, 2304, 2432, (None, None)), (384, 2, 1408, 1024, (pkg.GGML_Q8_0, pkg.GGML_Q8_0)),
+                                             (32, 4, 768, 320, (pkg.GGML_Q5_K, pkg.GGML_Q5_1)), (28, 4, 1152, 448, (None, None))])
+def test_more_than_twelve_rows(cuda, E, k, d, mid, types):
+    """Calls of more than 12 rows per expert: large layers run both forms, small ones tiles of 64 rows. Bit for bit the rows
+    of calls of 17 tokens, and the fp32 kernels' results within the roundings' bound."""
+    torch = cuda
+    counts = [193, 192, 130, 129, 128, 65, 64, 63, 49, 48, 33, 32, 31, 17, 16, 15, 1]
+    T = max(13 * E // k + 1, 320)
+    ids = torch.from_numpy(ids_of_counts(E, k, T, counts)).cuda()
+    w = torch.from_numpy(synth.rng_for(88, 1).uniform(0.2, 1.0, size=(T, 16)).astype(np.float32) / k).cuda()
+    x = bf16_tensor(torch, synth.make_x(synth.rng_for(88, 9), T, d), (T, d))
+    gu, dn = types
+
+    def make(impl):
+        op = pkg.MoeOperator(E, k, d, mid, T, gemm_impl=impl)
+        if gu is None:
+            op.load_q4cp(0, random_blob(torch, E * 2 * mid, d, gu, 1), random_blob(torch, E * d, mid, dn, 2))
+        else:
+            op.load_gguf(0, random_blob(torch, E * mid, d, gu, 1), random_blob(torch, E * mid, d, gu, 3), random_blob(torch, E * d, mid, dn, 2),
+                         type_gu=gu, type_dn=dn)
+        return op
+
+    def run(op, t0, n):
+        out = torch.full((n, d), float("nan"), dtype=torch.bfloat16, device="cuda")
+        op.moe_q4w_run(0, x[t0:t0 + n].contiguous(), ids[t0:t0 + n].contiguous(), w[t0:t0 + n].contiguous(), out)
+        op.synchronize()
+        return out
+
+    tc, simt = make(pkg.GEMM_TC), make(pkg.GEMM_SIMT)
+    for _ in range(2):
+        whole = run(tc, 0, T)
+        assert torch.isfinite(whole.float()).all()
+        for t0 in (0, 17, T - 17):
+            assert torch.equal(whole[t0:t0 + 17], run(tc, t0, 17)), t0
+    # 2-norm: both sides round to bf16 (a uniform error of 2^-9 at most: 2^-9 / sqrt(3) rms each), the tensor cores also gate, up and down
+    # weights and the hidden values to fp16 (2^-11 / sqrt(3) each): sqrt(2 * 2^-18 + 4 * 2^-22) / sqrt(3) = 1.7e-3; twice that
+    want = run(simt, 0, T).float()
+    assert (whole.float() - want).norm() <= 3.4e-3 * want.norm()
+    tc.close()
+    simt.close()
