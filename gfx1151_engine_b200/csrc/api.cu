@@ -53,6 +53,13 @@ constexpr int kFewRows = 12;
 // expert then makes 8 tiles at most). 64 of 2048 x 512, wide / few: 200 tokens 79 / 71, skewed 81 / 71; 400 tokens 85 / 77,
 // 89 / 87.
 constexpr int kOneListRows = 48, kOneListTokens = 512;
+// Experts of at least this many rows: their down weights are expanded to fp16 once per call, and whole tiles of their rows take a
+// plain fp16 GEMM on pairs of SMs (expert_dense.cu). Down stage in calls back to back (power cap), without / with, us: 16384 tokens
+// of 4096 x 1024, the benchmark's skew, 1495 / 1302 (whole call 4690 / 4570), half of it 1600 / 1520 (5000 / 4935), 8192 tokens in Q4_K /
+// Q5_1 898 / 815 (2625 / 2565), 2560 x 640, 8192 tokens 410 / 357 (1270 / 1210). Three groups of 768 rows pay the expansion back
+// (2.2 us an expert of 4096 x 1024) everywhere; 768, 1536 and 2304 differ by less than 1 %, with 4096 tokens level with none at 2304, 0.5 %
+// behind at 1536. The gate/up GEMM does not gain: 2544 / 2532 us with its expansion.
+constexpr int kPopularRows = 3 * kDenseGroup;
 // The shared expert's rows stay in narrow tiles while its gate/up GEMM has at most this many of them times row
 // blocks: they fill SMs beside the routed ones, so that more and shorter items end earlier. Wide / narrow: 144
 // items (768 tokens, mid 768) 288 / 282 us, 384 (1536, mid 1024) 871 / 868, 576 (2304, mid 1024) 906 / 937.
@@ -117,6 +124,7 @@ struct b200moe_ctx {
   bool prof = false;
   std::vector<cudaEvent_t> prof_ev;
   int prof_head = 0, prof_pending = 0;
+  int dense_cap = 0;  // experts whose expanded weights the workspaces hold
   int max_rows = 0, max_tiles = 0, max_tiles_narrow = 0, max_tiles_sh = 0;
   std::string err;
 };
@@ -319,6 +327,9 @@ int b200moe_create(const b200moe_config* cfg, b200moe_handle* out) {
   A(&h->rb.tiles_narrow, (size_t)h->max_tiles_narrow);
   A(&h->rb.tiles_sh, (size_t)h->max_tiles_sh);
   A(&h->rb.n_tiles, 3);
+  A(&h->rb.tiles_dense, pairs / kDenseRows + 1);
+  A(&h->rb.dense_experts, (size_t)kMaxExperts);
+  A(&h->rb.n_dense, 3);
   A(&h->rb.sgate, (size_t)Tm);
   A((uint8_t**)&h->hid, hid_bytes);
   A((uint8_t**)&h->pairs, pair_bytes);
@@ -344,6 +355,11 @@ int b200moe_create(const b200moe_config* cfg, b200moe_handle* out) {
   if (e == cudaSuccess) e = cudaMallocHost((void**)&h->status_host, 16);
   if (e == cudaSuccess && !simt_all)
     e = tc_create(&h->tc, h->x_sorted, (__half*)h->hid, (long long)rows, d, mid);
+  if (e == cudaSuccess && !simt_all && d % kDenseRows == 0) {
+    // expanded down weights lie where the activations were, which that stage does not use
+    h->dense_cap = (int)std::min((size_t)E, rows / mid);
+    if (h->dense_cap > 0) e = tc_set_dense(h->tc, h->x_sorted, h->dense_cap, d, mid);
+  }
   if (e == cudaSuccess && !simt_all) e = router_plan_create(&h->rplan);
   if (e != cudaSuccess) {
     std::string msg = std::string("b200moe_create: ") + cudaGetErrorString(e);
@@ -773,9 +789,11 @@ static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const
                                     : (long long)E * d * mid >= kBothLists);
   const bool narrow = !split && (few || (T <= kOneListTokens && T * k <= kOneListRows * E));
   const bool sh_narrow = few && (long long)(T / kTcNarrowN) * (mid / 64) <= kSharedNarrowItems;
+  const bool dense = !narrow && T >= kPopularRows && T > h->decode_max && h->dense_cap > 0 && !L.i4r && !L.dn.act_shift;
   const int min_few = range ? 0 : few_row_experts(h, L, T);
   const bool mixed = min_few > 0;
   const TileCut cut{narrow ? kTcNarrowN : h->tile_cap, sh_narrow ? kTcNarrowN : h->tile_cap, split ? kTcNarrowN : 0, second,
+                    dense ? kPopularRows : 0, h->dense_cap,
                     mixed ? std::min(gemv_rows(L.gu.fmt), gemv_rows(L.dn.fmt)) : 0, min_few};
   // (the shared expert's images are q4cp: it can ride along only with q4cp routed experts)
   const bool gemv = simt && c.gemm_impl == B200MOE_GEMM_AUTO &&
@@ -853,15 +871,17 @@ static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const
     if (!h->tc) return fail(h, B200MOE_ERR_UNSUPPORTED, "tensor-core path not available on this handle");
     const int rows = pairs + (shared ? T : 0);
     // One GEMM stage: its launches in one place, since those beside the first rely on being right behind it.
-    auto stage_tc = [&](auto launch, const Image& img, const Image* sh, __half* out16) -> cudaError_t {
+    auto stage_tc = [&](auto launch, const Image& img, const Image* sh, __half* out16, bool behind = false) -> cudaError_t {
+      // behind: the GEMM on expanded weights is in front of these, and has taken its rows
+      const int32_t* skip = behind ? h->rb.n_dense + 2 : nullptr;
       const Tile* first = split ? h->rb.tiles_narrow : h->rb.tiles;
       cudaError_t e = launch(h->tc, img, first, h->rb.n_tiles + (split ? 2 : 0), split ? h->max_tiles_narrow : h->max_tiles,
-                             out16, h->status_dev, st, TcLaunch{narrow || split, mixed});  // (mixed: beside the GEMV in front)
+                             out16, h->status_dev, st, TcLaunch{narrow || split, mixed || behind, nullptr, nullptr, split ? nullptr : skip});  // (mixed: beside the GEMV in front)
       if (e == cudaSuccess && sh)
         e = launch(h->tc, *sh, h->rb.tiles_sh, h->rb.n_tiles + 1, h->max_tiles_sh, out16, h->status_dev, st,
                    TcLaunch{sh_narrow, true});
       if (e == cudaSuccess && split)
-        e = launch(h->tc, img, h->rb.tiles, h->rb.n_tiles, h->max_tiles, out16, h->status_dev, st, TcLaunch{false, true});
+        e = launch(h->tc, img, h->rb.tiles, h->rb.n_tiles, h->max_tiles, out16, h->status_dev, st, TcLaunch{false, true, nullptr, nullptr, skip});
       n += 1 + (sh ? 1 : 0) + (split ? 1 : 0);
       return e;
     };
@@ -901,7 +921,12 @@ static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const
       CU_TRY(h, launch_down_gemv(L.dn, nullptr, (const __half*)h->hid, T, k, E, d, mid, h->rb.runs, h->rb.n_runs,
                                  std::min(E, pairs), h->pairs, true, h->status_dev, nullptr, &n, st));
     }
-    CU_TRY(h, stage_tc(launch_down_tc, L.dn, shared ? &L.sh_dn : nullptr, (__half*)h->pairs));
+    if (dense) {
+      CU_TRY(h, launch_expand(h->tc, L.dn, h->rb.dense_experts, h->rb.n_dense, h->x_sorted, st));
+      CU_TRY(h, launch_down_dense(h->tc, h->rb.tiles_dense, h->rb.n_dense, d, mid, (__half*)h->pairs, h->status_dev, st));
+      n += 2;
+    }
+    CU_TRY(h, stage_tc(launch_down_tc, L.dn, shared ? &L.sh_dn : nullptr, (__half*)h->pairs, dense));
     if (ev) CU_TRY(h, cudaEventRecord(ev[4], st));
     CU_TRY(h, launch_combine_f16((const __half*)h->pairs, h->rb.pw, h->rb.pairids, T, k, d,
                                  shared ? pairs : -1, out, st, h->hc_w4, h->hc_state));

@@ -103,6 +103,10 @@ struct Tile {
   int count;
 };
 
+// Rows of a tile of the GEMM on expanded weights (expert_dense.cu), and of the least that is whole tiles both there and in
+// the grouped dequant-GEMM (4 of kTcTileN).
+constexpr int kDenseRows = 256, kDenseGroup = 768;
+
 constexpr int kMaxTopK = 16;
 constexpr int kMaxExperts = 512;
 constexpr int kIdStride = 16;  // internal top-k rows are 16 wide, like the engine's

@@ -2,7 +2,7 @@
 // bit for bit, for experts with few rows, whose MMAs are so short that the decoding of the weights decides.
 //
 // One CTA per SM, 24 warps, K blocks (64 wide) in quads:
-//   warp 0      producer of activations: one tensor copy per pair of K blocks (boxes of 16, 32 or 64 rows), counted by the
+//   warp 0      producer of activations: one tensor copy per pair of K blocks (boxes of 16, 32, 48 or 64 rows), counted by the
 //               barrier that the quad's dequantising warps arrive on
 //   warp 1      sixteen tcgen05.mma per quad behind ONE barrier check, which is made (without blocking) behind the quad before
 //   warp 2      producer of packed weights: four bulk copies per quad into a ring of 4 stages (3 in the Q5_1 form)
@@ -31,8 +31,8 @@ static_assert(kTmemA + kNS * 128 <= 512, "tensor memory: two accumulators and th
 // Shared memory in absolute addresses (see Map in expert_tc.cu: the pair table on a 64 KB boundary).
 constexpr int kOffBar = 2048, kOffU = 3072, kOffX = 11264, kOffLut = 65536, kOffW = 131072, kSmemEnd = 233472;
 constexpr int kSmemBytes = kSmemEnd - 1024;  // dynamic bytes requested: the allocation starts at 1 KB
-// Activations of a pair of K blocks: 4, 8 or 16 KB by the rows of the tile's box (16, 32, 64). Two quads of 64 rows or three of
-// fewer fit below the table, but for the last pair of 64 rows, which lies behind it.
+// Activations of a pair of K blocks: 4, 8, 12 or 16 KB by the rows of the tile's box (16, 32, 48, 64). Two quads of 48 or 64 rows
+// or three of fewer fit below the table, but for the last pair of 64 rows, which lies behind it.
 constexpr int kPair64 = kRows * 256, kOffX3 = kOffLut + 65536, kOffStages = kOffX3 + kPair64;
 static_assert(kOffX + 3 * kPair64 <= kOffLut && kOffX3 == kOffW, "activations");
 constexpr uint32_t stage_bytes(int fmt) { return 16 * (uint32_t)sub_bytes(fmt); }        // four sub-blocks x four K blocks
@@ -52,11 +52,11 @@ static_assert(kNumBars * 8 + 16 + 32 <= 1024, "barrier block too small");
 // is rare); their producer then waits for all MMAs before.
 struct XSlots {
   uint32_t rows = 0, n = 0, i = 0;  // rows of the box, slots of that size, the next quad's
-  __device__ __forceinline__ static uint32_t box(int count) { return count <= 16 ? 16 : count <= 32 ? 32 : 64; }
+  __device__ __forceinline__ static uint32_t box(int count) { return (count + 15) & ~15; }
   __device__ __forceinline__ bool resize(int count) {  // true: the size is another one
     if (rows == box(count)) return false;
     rows = box(count);
-    n = rows == 64 ? 2 : 3;
+    n = rows > 32 ? 2 : 3;
     i = 0;
     return true;
   }
@@ -124,7 +124,7 @@ __device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t* v) {
 template <bool UP, bool DUAL, int FMT>
 __global__ void __launch_bounds__(kThreads, 1)
 k_expert_few(const __grid_constant__ CUtensorMap map16, const __grid_constant__ CUtensorMap map32,
-             const __grid_constant__ CUtensorMap map64, const FewParams p) {
+             const __grid_constant__ CUtensorMap map48, const __grid_constant__ CUtensorMap map64, const FewParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t dyn0 = smem_u32(smem_raw);
   uint8_t* const smem = smem_raw - dyn0;  // smem + A is the generic pointer of absolute shared address A
@@ -201,7 +201,7 @@ k_expert_few(const __grid_constant__ CUtensorMap map16, const __grid_constant__ 
       for (int it = blockIdx.x; it < n_items && ok; it += gridDim.x) {
         const Tile t = t_ahead;  // read one item ahead: its latency is off this loop's critical path
         if (it + (int)gridDim.x < n_items) t_ahead = p.tiles[(it + gridDim.x) / img.n_mtiles];
-        const CUtensorMap* map = t.count <= 16 ? &map16 : t.count <= 32 ? &map32 : &map64;
+        const CUtensorMap* map = t.count <= 16 ? &map16 : t.count <= 32 ? &map32 : t.count <= 48 ? &map48 : &map64;
         if (xs.resize(t.count) && qi > 0) ok = done(qi - 1);
         for (int qq = 0; qq < NQ && ok; qq++, qi++) {
           // (the slot's last user is done, and so is the A slot's, whose barrier takes this quad's phase then)
@@ -529,7 +529,7 @@ cudaError_t launch(const TcPlan* plan, const CUtensorMap* m, const Image& img, c
   const int grid = (int)(max_items < 1 ? 1 : max_items < usable ? max_items : usable);
   // (a margin: no early starts, as in expert_tc.cu)
   return launch_opt(plan->margin == 0, k_expert_few<UP, DUAL, FMT>, dim3(grid), dim3(kThreads), (size_t)kSmemBytes, st, m[0], m[1],
-                    m[2], p);
+                    m[2], m[3], p);
 }
 
 }  // namespace

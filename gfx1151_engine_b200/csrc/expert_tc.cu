@@ -101,6 +101,7 @@ struct KParams {
   int l2_ahead;      // weight tiles are asked into L2 this many own pairs ahead of their register fetch (0: off)
   const int32_t* rowmap;    // down kernel, may be null: tile-list row r >= map_base[0] is written to output row
   const int32_t* map_base;  // rowmap[r - map_base[0]] (rows below map_base[0], and all rows without a map: to row r)
+  const int32_t* skip;      // may be null: the first skip[0] tiles are not this launch's
   int beside;        // 1: runs beside the launch in front of it (see the wait in the set-up)
   int early_next;    // 1: the next launch of the stream may start its set-up while this one runs
 };
@@ -146,7 +147,7 @@ k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ C
   uint32_t* tmem_slot = (uint32_t*)(smem + kOffBar + kNumBars * 8 + 8);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // (a launch beside another one starts only when its list is there, see below: with none, it just keeps the order)
-  if (p.beside && p.n_tiles[0] == 0) {
+  if (p.beside && p.n_tiles[0] == (p.skip != nullptr ? p.skip[0] : 0)) {
     pdl_trigger();
     if (blockIdx.x == 0) pdl_wait();
     return;
@@ -190,7 +191,9 @@ k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ C
   // the wait to stay in front of the trigger, and nothing else between these launches.
   if (!p.beside) pdl_wait();
   if (p.early_next) pdl_trigger();
-  const int n_items = p.n_tiles[0] * img.n_mtiles;
+  const int skip = p.skip != nullptr ? p.skip[0] : 0;
+  const int n_items = (p.n_tiles[0] - skip) * img.n_mtiles;
+  const Tile* const tiles = p.tiles + skip;
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -207,10 +210,10 @@ k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ C
     if (lane == 0) {
       uint32_t pi = 0, slot = 0, sph = 0;
       bool ok = true;
-      Tile t_ahead = (int)blockIdx.x < n_items ? p.tiles[blockIdx.x / img.n_mtiles] : Tile{0, 0, 0};
+      Tile t_ahead = (int)blockIdx.x < n_items ? tiles[blockIdx.x / img.n_mtiles] : Tile{0, 0, 0};
       for (int it = blockIdx.x; it < n_items && ok; it += gridDim.x) {
         const Tile t = t_ahead;  // read one item ahead: its latency is off this loop's critical path
-        if (it + (int)gridDim.x < n_items) t_ahead = p.tiles[(it + gridDim.x) / img.n_mtiles];
+        if (it + (int)gridDim.x < n_items) t_ahead = tiles[(it + gridDim.x) / img.n_mtiles];
         const int n_pad = (t.count + 15) & ~15;
         // smallest box that covers the tile's rows: 16, 64, 128 or 192 rows of 64 halfs
         const CUtensorMap* map = n_pad <= 16 ? &map16 : n_pad <= 64 ? &map64 : n_pad <= 128 ? &map128 : &map192;
@@ -271,10 +274,10 @@ k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ C
     uint32_t pi = 0, li = 0;
     uint32_t aslot = 0, aph = 0, bslot = 0;  // pi % kNS, (pi / kNS) & 1, pi % kNBS as counters
     bool ok = true;
-    Tile t_ahead = (int)blockIdx.x < n_items ? p.tiles[blockIdx.x / img.n_mtiles] : Tile{0, 0, 0};
+    Tile t_ahead = (int)blockIdx.x < n_items ? tiles[blockIdx.x / img.n_mtiles] : Tile{0, 0, 0};
     for (int it = blockIdx.x; it < n_items && ok; it += gridDim.x, li++) {
       const Tile t = t_ahead;  // read one item ahead: its latency is off this loop's critical path
-      if (it + (int)gridDim.x < n_items) t_ahead = p.tiles[(it + gridDim.x) / img.n_mtiles];
+      if (it + (int)gridDim.x < n_items) t_ahead = tiles[(it + gridDim.x) / img.n_mtiles];
       const int n_pad = (t.count + 15) & ~15;
       const uint32_t idesc = instr_desc(n_pad);
       const uint32_t acc = li & 1, accph = (li >> 1) & 1;
@@ -345,7 +348,7 @@ k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ C
     auto item_base = [&](int io) -> const uint8_t* {
       const int item = blockIdx.x + io * (int)gridDim.x;
       if (io >= my_items) return nullptr;
-      return img.mtile(p.tiles[item / img.n_mtiles].expert, item % img.n_mtiles) + row0;
+      return img.mtile(tiles[item / img.n_mtiles].expert, item % img.n_mtiles) + row0;
     };
     const int io_step = NP == 1 ? 2 : 1;  // a set visits every item, or every other one when an item is one pair
     int f_io = set / NP, f_pp = set % NP;
@@ -479,10 +482,10 @@ k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ C
     volatile int* ep_ok = (volatile int*)(smem + kOffBar + kNumBars * 8 + 16);
     uint32_t li = 0;
     bool ok = true;
-    Tile t_ahead = (int)blockIdx.x < n_items ? p.tiles[blockIdx.x / img.n_mtiles] : Tile{0, 0, 0};
+    Tile t_ahead = (int)blockIdx.x < n_items ? tiles[blockIdx.x / img.n_mtiles] : Tile{0, 0, 0};
     for (int it = blockIdx.x; it < n_items && ok; it += gridDim.x, li++) {
       const Tile t = t_ahead;
-      if (it + (int)gridDim.x < n_items) t_ahead = p.tiles[(it + gridDim.x) / img.n_mtiles];
+      if (it + (int)gridDim.x < n_items) t_ahead = tiles[(it + gridDim.x) / img.n_mtiles];
       const int mt = it % img.n_mtiles;
       const uint32_t acc = li & 1, accph = (li >> 1) & 1;
       ok = mbar_wait(bars + 8 * (kBarAccFull + acc), accph, abort_flag, p.status, 8, 256);
@@ -620,7 +623,7 @@ cudaError_t encode_pair(PFN_cuTensorMapEncodeTiled_v12000 enc, CUtensorMap* map,
 template <bool UP, bool DUAL, int FMT>
 cudaError_t launch_n(TcPlan* plan, const CUtensorMap* m, const Image& img,
                    const Tile* tiles, const int32_t* n_tiles, int max_tiles, __half* out, int out_ld,
-                   int32_t* status, cudaStream_t st, const int32_t* rowmap, const int32_t* map_base, bool beside) {
+                   int32_t* status, cudaStream_t st, const int32_t* rowmap, const int32_t* map_base, const int32_t* skip, bool beside) {
   constexpr int kSmemBytes = Map::kSmemBytes;
   static bool attr_set = false;  // one flag per template instance
   if (!attr_set) {
@@ -631,7 +634,7 @@ cudaError_t launch_n(TcPlan* plan, const CUtensorMap* m, const Image& img,
   }
   static const int l2_ahead = getenv("B200MOE_TC_L2_AHEAD") ? atoi(getenv("B200MOE_TC_L2_AHEAD")) : 3;
   KParams p{img, tiles, n_tiles, out, out_ld, status, (UP != (getenv("B200MOE_TC_TRACE_DOWN") != nullptr)) ? plan->trace : nullptr,
-            l2_ahead, rowmap, map_base, beside ? 1 : 0, plan->margin == 0};
+            l2_ahead, rowmap, map_base, skip, beside ? 1 : 0, plan->margin == 0};
   long long max_items = (long long)max_tiles * img.n_mtiles;
   const int usable = plan->sms - plan->margin > 1 ? plan->sms - plan->margin : 1;
   int grid = (int)(max_items < usable ? max_items : usable);
@@ -648,11 +651,11 @@ cudaError_t launch(TcPlan* plan, const CUtensorMap* m, const Image& img,
                    const Tile* tiles, const int32_t* n_tiles, int max_tiles, __half* out, int out_ld,
                    int32_t* status, cudaStream_t st, const TcLaunch& o) {
   if (o.narrow) {
-    if (o.rowmap != nullptr) return cudaErrorInvalidValue;
+    if (o.rowmap != nullptr || o.skip != nullptr) return cudaErrorInvalidValue;
     return launch_few(plan, UP, m == plan->h, img, tiles, n_tiles, max_tiles, out, out_ld, status, st, o.beside);
   }
   return launch_n<UP, DUAL, FMT>(plan, m, img, tiles, n_tiles, max_tiles, out, out_ld, status, st, o.rowmap,
-                                           o.map_base, o.beside);
+                                           o.map_base, o.skip, o.beside);
 }
 
 }  // namespace
@@ -674,8 +677,8 @@ cudaError_t tc_create(TcPlan** out, const __half* x_sorted, const __half* hid16,
   e = cudaSuccess;
   for (int i = 0; i < 4 && e == cudaSuccess; i++) e = encode_2d(enc, &plan->x[i], x_sorted, rows_cap, d, boxes[i]);
   for (int i = 0; i < 4 && e == cudaSuccess; i++) e = encode_2d(enc, &plan->h[i], hid16, rows_cap, mid, boxes[i]);
-  for (int i = 0; i < 3 && e == cudaSuccess; i++) e = encode_pair(enc, &plan->x2[i], x_sorted, rows_cap, d, 16 << i);
-  for (int i = 0; i < 3 && e == cudaSuccess; i++) e = encode_pair(enc, &plan->h2[i], hid16, rows_cap, mid, 16 << i);
+  for (int i = 0; i < 4 && e == cudaSuccess; i++) e = encode_pair(enc, &plan->x2[i], x_sorted, rows_cap, d, 16 * (i + 1));
+  for (int i = 0; i < 4 && e == cudaSuccess; i++) e = encode_pair(enc, &plan->h2[i], hid16, rows_cap, mid, 16 * (i + 1));
   if (e != cudaSuccess) {
     delete plan;
     return e;
@@ -687,6 +690,16 @@ cudaError_t tc_create(TcPlan** out, const __half* x_sorted, const __half* hid16,
   }
   *out = plan;
   return cudaSuccess;
+}
+
+cudaError_t tc_set_dense(TcPlan* plan, const __half* w, int cap, int d, int mid) {
+  void* fn = nullptr;
+  cudaDriverEntryPointQueryResult qres;
+  cudaError_t e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres);
+  if (e == cudaSuccess && (!fn || qres != cudaDriverEntryPointSuccess)) e = cudaErrorNotSupported;
+  auto enc = (PFN_cuTensorMapEncodeTiled_v12000)fn;
+  if (e == cudaSuccess) e = encode_2d(enc, &plan->w_dense, w, (long long)cap * d, mid, 128);
+  return e;
 }
 
 void tc_set_sm_margin(TcPlan* plan, int sms) {

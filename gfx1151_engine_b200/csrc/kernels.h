@@ -81,6 +81,9 @@ struct RouteBuffers {
   Tile* tiles_narrow;  // a second one, of the tiles with few rows (see TileCut)
   Tile* tiles_sh;    // work list of the shared expert (all T tokens)
   int32_t* n_tiles;  // [3]: tiles, tiles_sh, tiles_narrow
+  Tile* tiles_dense;       // popular experts' tiles of kDenseRows rows for the down GEMM; their expert is the place in:
+  int32_t* dense_experts;  // the experts whose weights are expanded
+  int32_t* n_dense;        // [3]: tiles, experts, how many of `tiles` (the first) hold the same rows
   float* sgate;      // [T] sigmoid gate of the shared expert
   int32_t* ready;    // 1 from the gate/up GEMV's own routing to the combine: the lists above are there
   int32_t* status;   // the handle's status word (may be null): {4, id} when an expert id outside [0, E) was dropped
@@ -94,6 +97,8 @@ cudaError_t launch_router_topk(const float* logits, int T, int E, int k, int32_t
 constexpr int kTileCostWide = 380, kTileCostFew = 270;
 struct TileCut {
   int routed, shared, narrow = 0, second = 0;
+  // > 0: the rows of the first dense_cap experts of at least so many are on tiles_dense, too, kDenseGroup at a time.
+  int dense_rows = 0, dense_cap = 0;
   // > 0: if at least min_few experts have rows, but no more than gemv_rows, those get no tiles; runs / n_runs[0] list them and no others.
   int gemv_rows = 0, min_few = 0;
 };

@@ -93,7 +93,8 @@ k_route_count(const int32_t* __restrict__ ids, int stride, int pairs, int k, int
 __global__ void __launch_bounds__(kMaxExperts)
 k_route_scan(int32_t* __restrict__ blockcnt, int nblk, int E, int pairs, int T, TileCut cut,
              int32_t* __restrict__ eoff, Run* __restrict__ runs, int32_t* __restrict__ n_runs,
-             Tile* __restrict__ tiles, Tile* __restrict__ tiles_narrow, Tile* __restrict__ tiles_sh, int32_t* __restrict__ n_tiles) {
+             Tile* __restrict__ tiles, Tile* __restrict__ tiles_narrow, Tile* __restrict__ tiles_sh, int32_t* __restrict__ n_tiles,
+             Tile* __restrict__ tiles_dense, int32_t* __restrict__ dense_experts, int32_t* __restrict__ n_dense) {
   __shared__ __align__(4) uint16_t s_bin[kMaxExperts / 32][kTcTileN + 8];  // ragged tiles of a size: per warp, then in the warps before
   __shared__ int s_gt[256], s_gw[8];                          // larger ones, of all
   __shared__ unsigned long long s_w[kMaxExperts / 32];
@@ -140,9 +141,46 @@ k_route_scan(int32_t* __restrict__ blockcnt, int nblk, int E, int pairs, int T, 
     if (few <= wide && few <= both) tile_cap = narrow;
     else if (wide <= both) narrow = 0;
   }
+  // popular experts: what is whole tiles in both GEMMs goes to the one on expanded weights, for the down stage
+  int slot = -1, n_groups = 0, groups0 = 0, all_groups = 0;  // place among them; groups, before it, of all
+  if (cut.dense_rows > 0 && tile_cap == kTcTileN) {
+    const bool popular = cnt >= cut.dense_rows && cnt >= kDenseGroup;
+    const unsigned vote = __ballot_sync(0xffffffffu, popular);
+    __syncthreads();
+    if (lane == 0) s_sum[0][warp] = __popc(vote);
+    __syncthreads();
+    int before = __popc(vote & ((1u << lane) - 1u));
+    for (int w = 0; w < warp; w++) before += s_sum[0][w];
+    if (popular && before < cut.dense_cap) {
+      slot = before;
+      n_groups = cnt / kDenseGroup;
+      dense_experts[slot] = e;
+    }
+    groups0 = n_groups;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, groups0, o);
+      if (lane >= o) groups0 += v;
+    }
+    if (lane == 31) s_sum[1][warp] = groups0;
+    groups0 -= n_groups;
+    const int n_slots = __syncthreads_count(slot >= 0);
+    for (int w = 0; w < kMaxExperts / 32; w++) {
+      if (w < warp) groups0 += s_sum[1][w];
+      all_groups += s_sum[1][w];
+    }
+    if (e == 0) {
+      n_dense[0] = all_groups * (kDenseGroup / kDenseRows);
+      n_dense[1] = n_slots;
+      n_dense[2] = all_groups * (kDenseGroup / kTcTileN);
+    }
+  } else if (cut.dense_rows > 0 && e < 3) {
+    n_dense[e] = 0;
+  }
   const bool listed = cnt > 0 && (by_gemv || cut.gemv_rows == 0);
   // three inclusive scans side by side: counts (low 32 bits) and non-empty flags, full tiles
-  const int nfull = by_gemv ? 0 : cnt / tile_cap, part = by_gemv ? 0 : cnt % tile_cap;
+  const int in_groups = n_groups * (kDenseGroup / kTcTileN);  // full tiles that stand in front of the others
+  const int nfull = by_gemv ? 0 : cnt / tile_cap - in_groups, part = by_gemv ? 0 : cnt % tile_cap;
   unsigned long long ab = (unsigned long long)(uint32_t)cnt | (unsigned long long)listed << 32;
   int c = nfull;
 #pragma unroll
@@ -205,7 +243,7 @@ k_route_scan(int32_t* __restrict__ blockcnt, int nblk, int E, int pairs, int T, 
     ab_all += u;
     c_all += v;
   }
-  const int first = (int)(uint32_t)ab - cnt, total_full = c_all;
+  const int first = (int)(uint32_t)ab - cnt, total_full = c_all + all_groups * (kDenseGroup / kTcTileN);
   if (e < E) eoff[e] = first;
   if (e == 0) {
     eoff[E] = (int)(uint32_t)ab_all;  // pairs placed (= T*k unless ids outside [0, E) were dropped)
@@ -220,9 +258,13 @@ k_route_scan(int32_t* __restrict__ blockcnt, int nblk, int E, int pairs, int T, 
     if (i < n_wide) tiles[i] = t;
     else tiles_narrow[i - n_wide] = t;
   };
-  const int full0 = c - nfull;
-  for (int j = 0; j < nfull; j++) put(full0 + j, Tile{e, first + j * tile_cap, tile_cap});
-  if (part > 0) put(total_full + rank, Tile{e, first + nfull * tile_cap, part});
+  const int full0 = total_full - c_all + c - nfull;
+  for (int j = 0; j < in_groups; j++) put(groups0 * (kDenseGroup / kTcTileN) + j, Tile{e, first + j * tile_cap, tile_cap});
+  for (int j = 0; j < n_groups * (kDenseGroup / kDenseRows); j++)
+    tiles_dense[groups0 * (kDenseGroup / kDenseRows) + j] = Tile{slot, first + j * kDenseRows, kDenseRows};
+  const int rest = first + in_groups * tile_cap;
+  for (int j = 0; j < nfull; j++) put(full0 + j, Tile{e, rest + j * tile_cap, tile_cap});
+  if (part > 0) put(total_full + rank, Tile{e, rest + nfull * tile_cap, part});
   // tiles of the shared expert: all T tokens in token order, rows behind the routed ones
   const int nsh = (T + cut.shared - 1) / cut.shared;
   for (int j = e; j < nsh; j += kMaxExperts)
@@ -335,7 +377,7 @@ cudaError_t launch_route(const RouteBuffers& rb, const int32_t* ids, const float
   cudaError_t e = launch_pdl(k_route_count, dim3(nblk), dim3(kChunk), 0, st, ids, stride, pairs, k, E, rb.blockcnt, rb.status);
   if (e == cudaSuccess)
     e = launch_pdl(k_route_scan, dim3(1), dim3(kMaxExperts), 0, st, rb.blockcnt, nblk, E, pairs, T, cut, rb.eoff, rb.runs,
-                   rb.n_runs, rb.tiles, rb.tiles_narrow, rb.tiles_sh, rb.n_tiles);
+                   rb.n_runs, rb.tiles, rb.tiles_narrow, rb.tiles_sh, rb.n_tiles, rb.tiles_dense, rb.dense_experts, rb.n_dense);
   if (e == cudaSuccess)
     e = launch_pdl(k_route_place, dim3(nblk), dim3(kChunk), 0, st, ids, w, stride, pairs, k, E, rb.blockcnt, rb.eoff, rb.tokidx,
                    rb.pw, rb.pairids);

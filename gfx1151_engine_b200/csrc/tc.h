@@ -10,6 +10,12 @@ struct TcPlan;  // tensor maps over the activation buffers + device properties
 cudaError_t tc_create(TcPlan** plan, const __half* x_sorted, const __half* hid16,
                       long long rows_cap, int d, int mid);
 void tc_destroy(TcPlan* plan);
+// expert_dense.cu: the down GEMM of popular experts. w: where the expanded weights of `cap` experts go, [cap][d][mid] fp16.
+cudaError_t tc_set_dense(TcPlan* plan, const __half* w, int cap, int d, int mid);
+cudaError_t launch_expand(const TcPlan* plan, const Image& img, const int32_t* experts, const int32_t* n_dense, __half* out,
+                          cudaStream_t st);
+cudaError_t launch_down_dense(const TcPlan* plan, const Tile* tiles, const int32_t* n_dense, int d, int mid, __half* pairs16, int32_t* status,
+                              cudaStream_t st);
 // Leave `sms` SMs free of the persistent GEMM CTAs (for communication kernels that must run
 // at the same time).
 void tc_set_sm_margin(TcPlan* plan, int sms);
@@ -27,6 +33,7 @@ struct TcLaunch {
   // to pairs16[rowmap[r - map_base[0]]] instead of pairs16[r].
   const int32_t* rowmap = nullptr;
   const int32_t* map_base = nullptr;
+  const int32_t* skip = nullptr;  // device: so many tiles of the list, the first, are not this launch's (wide form)
 };
 
 // gate/up GEMM + SwiGLU: hid16[row][mid] = silu(W_gate x) * (W_up x) for every row of every tile.

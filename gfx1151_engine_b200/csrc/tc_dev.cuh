@@ -13,7 +13,8 @@ namespace b200moe {
 
 struct TcPlan {
   CUtensorMap x[4], h[4];    // activation / hidden maps with boxes of 16, 64, 128, 192 rows of one K block
-  CUtensorMap x2[3], h2[3];  // the same with boxes of 16, 32, 64 rows of two K blocks
+  CUtensorMap x2[4], h2[4];  // the same with boxes of 16, 32, 48, 64 rows of two K blocks
+  CUtensorMap w_dense;       // expanded down weights, boxes of 128 rows of one K block
   int sms = 148;
   int margin = 0;
   long long* trace = nullptr;  // debug timeline of CTA 0 (environment B200MOE_TC_TRACE=<file>)

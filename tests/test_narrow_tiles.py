@@ -255,16 +255,8 @@ def random_blob(torch, rows, cols, fmt, seed):
     return b.reshape(-1)
 
 
-# K blocks of gate/up and down with all remainders of a quad; rows on both sides of a box of 16 and 32, of one and two tiles
-# and of a wide tile; layers on both sides of the line for two lists
-@pytest.mark.parametrize("E,k,d,mid,types", [(96, 4, 2304, 2432, (None, None)), (384, 2, 1408, 1024, (pkg.GGML_Q8_0, pkg.GGML_Q8_0)),
-                                             (32, 4, 768, 320, (pkg.GGML_Q5_K, pkg.GGML_Q5_1)), (28, 4, 1152, 448, (None, None))])
-def test_more_than_twelve_rows(cuda, E, k, d, mid, types):
-    """Calls of more than 12 rows per expert: large layers run both forms, small ones tiles of 64 rows. Bit for bit the rows
-    of calls of 17 tokens, and the fp32 kernels' results within the roundings' bound."""
-    torch = cuda
-    counts = [193, 192, 130, 129, 128, 65, 64, 63, 49, 48, 33, 32, 31, 17, 16, 15, 1]
-    T = max(13 * E // k + 1, 320)
+def rows_agree(torch, E, k, d, mid, types, T, counts):
+    """A call's rows, bit for bit those of calls of 17 tokens, and the fp32 kernels' results within the roundings' bound."""
     ids = torch.from_numpy(ids_of_counts(E, k, T, counts)).cuda()
     w = torch.from_numpy(synth.rng_for(88, 1).uniform(0.2, 1.0, size=(T, 16)).astype(np.float32) / k).cuda()
     x = bf16_tensor(torch, synth.make_x(synth.rng_for(88, 9), T, d), (T, d))
@@ -289,7 +281,7 @@ def test_more_than_twelve_rows(cuda, E, k, d, mid, types):
     for _ in range(2):
         whole = run(tc, 0, T)
         assert torch.isfinite(whole.float()).all()
-        for t0 in (0, 17, T - 17):
+        for t0 in (0, 17, T // 2, T - 17):
             assert torch.equal(whole[t0:t0 + 17], run(tc, t0, 17)), t0
     # 2-norm: both sides round to bf16 (a uniform error of 2^-9 at most: 2^-9 / sqrt(3) rms each), the tensor cores also gate, up and down
     # weights and the hidden values to fp16 (2^-11 / sqrt(3) each): sqrt(2 * 2^-18 + 4 * 2^-22) / sqrt(3) = 1.7e-3; twice that
@@ -297,3 +289,22 @@ def test_more_than_twelve_rows(cuda, E, k, d, mid, types):
     assert (whole.float() - want).norm() <= 3.4e-3 * want.norm()
     tc.close()
     simt.close()
+
+
+# K blocks of gate/up and down with all remainders of a quad; rows on both sides of a box of 16, 32 and 48, of one and two tiles
+# and of a wide tile; layers on both sides of the line for two lists
+@pytest.mark.parametrize("E,k,d,mid,types", [(96, 4, 2304, 2432, (None, None)), (384, 2, 1408, 1024, (pkg.GGML_Q8_0, pkg.GGML_Q8_0)),
+                                             (32, 4, 768, 320, (pkg.GGML_Q5_K, pkg.GGML_Q5_1)), (28, 4, 1152, 448, (None, None))])
+def test_more_than_twelve_rows(cuda, E, k, d, mid, types):
+    """Calls of more than 12 rows per expert: large layers run both forms, small ones tiles of 64 rows."""
+    counts = [193, 192, 130, 129, 128, 65, 64, 63, 49, 48, 33, 32, 31, 17, 16, 15, 1]
+    rows_agree(cuda, E, k, d, mid, types, max(13 * E // k + 1, 320), counts)
+
+
+# one group of rows more or less than the line, a whole number of them and not; two places for three popular experts (mid > d); a
+# layer of two lists, and one K block
+@pytest.mark.parametrize("E,k,d,mid,types", [(16, 4, 512, 192, (None, None)), (16, 4, 256, 4096, (None, None)), (16, 4, 768, 64, (pkg.GGML_Q5_K, pkg.GGML_Q5_1)),
+                                             (64, 4, 2816, 2816, (None, None))])
+def test_popular_experts(cuda, E, k, d, mid, types):
+    """Experts of 2304 rows and more: the down GEMM on expanded weights."""
+    rows_agree(cuda, E, k, d, mid, types, 3200, [3200, 2304, 2303, 3071, 769])
