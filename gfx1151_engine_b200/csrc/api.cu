@@ -734,7 +734,7 @@ static bool fused_decode(const b200moe_config& c) {
 // there (kMinFewWork). 0: no call of this size does.
 static int few_row_experts(b200moe_handle h, const LayerWeights& L, int T) {
   const b200moe_config& c = h->cfg;
-  const int k = c.topk, E = c.experts, d = c.d_model, mid = c.d_mid, rows = std::min(gemv_rows(L.gu.fmt), gemv_rows(L.dn.fmt));
+  const int k = c.topk, E = c.experts, d = c.d_model, mid = c.d_mid, rows = std::min(gemv_rows(L.gu.fmt, false), gemv_rows(L.dn.fmt, false));
   const int least = (int)((kMinFewWork + (long long)d * mid - 1) / ((long long)d * mid));
   return T > 16 && T > h->decode_max && !L.i4r && c.gemm_impl == B200MOE_GEMM_AUTO && 4 * T * k <= 5 * rows * E && T * k <= kFewRows * E &&
                  std::min(E, T * k) >= least && (d << L.gu.act_shift) <= gemv_max_k() && (mid << L.dn.act_shift) <= gemv_max_mid()
@@ -794,7 +794,7 @@ static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const
   const bool mixed = min_few > 0;
   const TileCut cut{narrow ? kTcNarrowN : h->tile_cap, sh_narrow ? kTcNarrowN : h->tile_cap, split ? kTcNarrowN : 0, second,
                     dense ? kPopularRows : 0, h->dense_cap,
-                    mixed ? std::min(gemv_rows(L.gu.fmt), gemv_rows(L.dn.fmt)) : 0, min_few};
+                    mixed ? std::min(gemv_rows(L.gu.fmt, false), gemv_rows(L.dn.fmt, false)) : 0, min_few};
   // (the shared expert's images are q4cp: it can ride along only with q4cp routed experts)
   const bool gemv = simt && c.gemm_impl == B200MOE_GEMM_AUTO &&
                     (!shared || (L.gu.fmt == kQ4CP && L.dn.fmt == kQ4CP)) &&
@@ -834,10 +834,10 @@ static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const
     // decode / verify: persistent dequant GEMV, routed and shared expert in one launch each
     if (ev) CU_TRY(h, cudaEventRecord(ev[2], st));
     CU_TRY(h, launch_up_gemv(L.gu, shared ? &L.sh_gu : nullptr, x, T, k, E, d, mid, h->rb.tokidx, h->rb.runs, h->rb.n_runs,
-                             gemv_passes(L.gu.fmt, T, k, E), (__half*)h->hid, h->status_dev, in_block ? &route : nullptr, &n, st));
+                             gemv_passes(L.gu.fmt, T, k, E), true, (__half*)h->hid, h->status_dev, in_block ? &route : nullptr, &n, st));
     if (ev) CU_TRY(h, cudaEventRecord(ev[3], st));
     CU_TRY(h, launch_down_gemv(L.dn, shared ? &L.sh_dn : nullptr, (const __half*)h->hid, T, k, E, d, mid,
-                               h->rb.runs, h->rb.n_runs, gemv_passes(L.dn.fmt, T, k, E), h->pairs, false, h->status_dev,
+                               h->rb.runs, h->rb.n_runs, gemv_passes(L.dn.fmt, T, k, E), true, h->pairs, false, h->status_dev,
                                in_block ? h->rb.ready : nullptr, &n, st));
     if (ev) CU_TRY(h, cudaEventRecord(ev[4], st));
     CU_TRY(h, launch_combine_f32((const float*)h->pairs, h->rb.pw, h->rb.pairids, T, k, d,
@@ -912,14 +912,14 @@ static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const
     n++;
     if (ev) CU_TRY(h, cudaEventRecord(ev[2], st));
     if (mixed) {
-      CU_TRY(h, launch_up_gemv(L.gu, nullptr, x, T, k, E, d, mid, h->rb.tokidx, h->rb.runs, h->rb.n_runs, std::min(E, pairs),
+      CU_TRY(h, launch_up_gemv(L.gu, nullptr, x, T, k, E, d, mid, h->rb.tokidx, h->rb.runs, h->rb.n_runs, std::min(E, pairs), false,
                                (__half*)h->hid, h->status_dev, nullptr, &n, st));  // (a pass each)
     }
     CU_TRY(h, stage_tc(launch_up_tc, L.gu, shared ? &L.sh_gu : nullptr, (__half*)h->hid));
     if (ev) CU_TRY(h, cudaEventRecord(ev[3], st));
     if (mixed) {
       CU_TRY(h, launch_down_gemv(L.dn, nullptr, (const __half*)h->hid, T, k, E, d, mid, h->rb.runs, h->rb.n_runs,
-                                 std::min(E, pairs), h->pairs, true, h->status_dev, nullptr, &n, st));
+                                 std::min(E, pairs), false, h->pairs, true, h->status_dev, nullptr, &n, st));
     }
     if (dense) {
       CU_TRY(h, launch_expand(h->tc, L.dn, h->rb.dense_experts, h->rb.n_dense, h->x_sorted, st));

@@ -9,9 +9,12 @@
 // on 512 code bytes, of which 16 were table lookups and 16 the activations, and stood at 2.7 TB/s. Here:
 //   * mma.m16n8k16 forms the products (exact) and sums (fp32). Its A operand is 16 weight rows: ldmatrix deals the
 //     packed codes of a row out to the four lanes of a quad, 8 codes each, a code BYTE becomes an fp16 pair. Scales
-//     stay in fp32: no sum runs over two 32-groups. q4cp takes one group per instruction and up to EIGHT rows of an
-//     expert in the columns of B; the GGUF formats, whose constants cost more per row, put the two groups of a K block
-//     into different columns (zeros elsewhere) and serve FOUR rows per pass over the weights.
+//     stay in fp32: no sum runs over two 32-groups. The two groups of a K block stand in different columns of B (zeros
+//     elsewhere), so that a pass over the weights serves FOUR rows of an expert; for q4cp among longer calls one group per instruction
+//     and EIGHT rows. Eight cost twice the scale multiplications and partial sums (calls of T = 1 / 5 / 13 of 4096 x 1024 and of
+//     16 tokens of 64 x 2048 x 512: 31.0 / 90.1 / 204.7 and 47.1 us; four: 30.6 / 88.1 / 203.0 and 44.0), but of the 211
+//     experts of a 77-token prompt one pass of eight serves 191, one of four 171. Decode calls take four at any length, so
+//     that a token's bytes do not depend on the others of the call.
 //   * B never moves: a warp owns at most four K blocks (its slice) of all the rows its team works on, and the
 //     activations of a slice are 8 registers per K block and lane.
 //   * q4cp: a code byte is decoded by one lookup in a 256-entry half2 table replicated per lane in shared memory
@@ -30,8 +33,7 @@
 //   * Longer calls with few rows per expert come here with a run list of k_route_scan instead (api.cu, kMinFewWork).
 // us of the two kernels, the multiply-add form / this one, 4096 x 1024 with shared expert: T = 1 35 / 28, T = 5
 // 120 / 84, T = 13 288 / 191 (gate/up 4.65 TB/s); Q4_K / Q5_1 T = 5 128 / 92 (gate/up 4.6 TB/s, down 4.0: the
-// fifth bits); 64 experts of 2048 x 512, 16 tokens (2.2 rows an expert) 90 / 38. (Four q4cp rows per pass: 26 / 80 / 177 and
-// 33; but of the 211 experts of a 77-token prompt one pass of eight serves 191, one of four 171.) One call, T = 1, from the end of the
+// fifth bits); 64 experts of 2048 x 512, 16 tokens (2.2 rows an expert) 90 / 38. One call, T = 1, from the end of the
 // kernel in front: routing 4.3 us, first copies and activations 3, gate/up 11, hand-over 2, down 6, combine 5.
 #include "kernels.h"
 #include "route_block.cuh"
@@ -49,19 +51,21 @@ constexpr uint32_t kOffLow = 2048;    // the dynamic allocation must start at or
 
 // Shared memory map, absolute shared addresses.
 // KPW: K blocks of a slice, at most.
-template <int FMT, int KPW>
+// ROWS: rows of an expert that one pass over its weights serves.
+template <int FMT, int KPW, int ROWS>
 struct Map {
-  static constexpr int kRows = FMT == kQ4CP ? 8 : 4;  // rows of an expert that one pass over its weights serves
-  // Partial-sum buffers of a team, and ring slots per warp. Shared memory holds four and two or two and three for q4cp
-  // (four and three without the table): four let the slices drift further apart, 31.1 against 32.1 us at T = 1, 195.4 / 196.6
-  // at T = 13; slices of three K blocks keep two and two.
-  static constexpr int kRed = FMT == kQ4CP && KPW == 3 ? 2 : 4;
+  static_assert(ROWS == 4 || (ROWS == 8 && FMT == kQ4CP), "columns of B");
+  static constexpr int kRows = ROWS;
+  // Partial-sum buffers of a team, and ring slots per warp: what shared memory holds. For eight rows four buffers and two slots:
+  // the buffers let the slices drift further apart, 31.1 against 32.1 us at T = 1, 195.4 / 196.6 at T = 13, than two and
+  // three; slices of three K blocks keep two and two.
+  static constexpr int kRed = ROWS == 8 && KPW == 3 ? 2 : 4;
   static constexpr int kGroup = KPW == 4 ? 2 : KPW;   // K blocks per ring slot
   static constexpr int kGroups = KPW / kGroup;        // slots per unit
   static constexpr uint32_t kLut = kOffLow;  // kQ4CP: 256 lines of {32 lanes x 4 B, first book}{32 x 4 B, second book}
   static constexpr uint32_t kRing = kLut + (FMT == kQ4CP ? 65536u : 0u);
   static constexpr uint32_t kSub = (uint32_t)sub_bytes(FMT), kSlot = kGroup * kSub;
-  static constexpr uint32_t kSlots = KPW == 3 || FMT == kQ4CP ? 2 : 3;
+  static constexpr uint32_t kSlots = KPW == 3 || ROWS == 8 ? 2 : 3;
   static constexpr uint32_t kScr = FMT == kQ4K ? 512 : 0;  // per warp: the rows' constants as floats
   static constexpr uint32_t kPart = kRing + kWarps * kSlots * kSlot;          // partial sums [kRed][warp][rows in fours][32 weight rows][4]
   static constexpr uint32_t kBar = kPart + kRed * kWarps * kSubRows * kRows * 4;
@@ -174,10 +178,11 @@ __device__ __forceinline__ uint32_t bf16x2_to_f16x2(uint32_t w) {
   return *(const uint32_t*)&h;
 }
 
-template <bool UP, int FMT, int KPW>
+template <bool UP, int FMT, int KPW, int ROWS>
 __global__ void __launch_bounds__(kThreads, 1)
 k_gemv(const __grid_constant__ GemvParams p) {
-  using M = Map<FMT, KPW>;
+  using M = Map<FMT, KPW, ROWS>;
+  constexpr bool kHalves = ROWS == 4;  // the two groups of a K block in columns of their own
   constexpr int kRows = M::kRows, kRed = M::kRed;
   extern __shared__ __align__(16) uint8_t gsm[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
@@ -221,8 +226,8 @@ k_gemv(const __grid_constant__ GemvParams p) {
   const int KB = im.n_kblocks, ash = im.act_shift;
   const int slice = warp % p.slices, team = warp / p.slices;
   const int kb0 = slice * KPW, nk = min(KPW, KB - kb0);
-  // Activations of the slice, B operands. kQ4CP: lane (g, t) holds row g, elements 8t .. 8t+7 of both halves of every
-  // K block. Else row g >> 1, half g & 1, in bv for half 0 and in bw for half 1, zeros in the other.
+  // Activations of the slice, B operands. Eight rows: lane (g, t) holds row g, elements 8t .. 8t+7 of both halves of every
+  // K block. Four: row g >> 1, half g & 1, in bv for half 0 and in bw for half 1, zeros in the other.
   uint32_t bv[KPW][4], bw[KPW][4];
   float xs[KPW][2];             // GGUF: sums of the activations of row t, halves 0 and 1
   auto load_rows = [&](bool live, size_t row) {
@@ -239,7 +244,7 @@ k_gemv(const __grid_constant__ GemvParams p) {
     };
 #pragma unroll
     for (int i = 0; i < KPW; i++) {
-      if (FMT == kQ4CP) {
+      if (!kHalves) {
         load8(i, 0, bv[i]);
         load8(i, 1, bw[i]);
       } else {
@@ -257,7 +262,7 @@ k_gemv(const __grid_constant__ GemvParams p) {
         for (int q = 0; q < 4; q++) {
           bv[i][q] = (g & 1) ? 0u : v[q];
           bw[i][q] = (g & 1) ? v[q] : 0u;
-          mma16816(c, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u, bv[i][q], bw[i][q]);
+          if (FMT != kQ4CP) mma16816(c, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u, 0x3C003C00u, bv[i][q], bw[i][q]);
         }
         xs[i][0] = c[0];
         xs[i][1] = c[1];
@@ -494,7 +499,7 @@ k_gemv(const __grid_constant__ GemvParams p) {
       }
 #pragma unroll
     for (int b = 0; b < 2; b++) {
-      if (FMT == kQ4CP) {
+      if (!kHalves) {
 #pragma unroll
         for (int h = 0; h < 2; h++) {
           // the half's products: K slots 2t, 2t+1 are the codes of byte 2q, slots 2t+8, 2t+9 those of byte 2q+1
@@ -521,7 +526,9 @@ k_gemv(const __grid_constant__ GemvParams p) {
           uint32_t a[4];
 #pragma unroll
           for (int h = 0; h < 4; h++) {
-            if (FMT == kQ4K) {
+            if (FMT == kQ4CP) {
+              a[h] = lut32<M::kLut>(__byte_perm(m[b][h], b ? lut_b : lut_a, 0x5504 | q << 4));
+            } else if (FMT == kQ4K) {
               // codes q and q + 4 of the word as the fp16 pair code * 2^-24, for odd q 16 times that (denormal numbers: exact, also in the products)
               a[h] = (q & 2 ? m[b][h] >> 8 : m[b][h]) & (q & 1 ? 0x00F000F0u : 0x000F000Fu);
             } else {
@@ -541,7 +548,7 @@ k_gemv(const __grid_constant__ GemvParams p) {
 #pragma unroll
         for (int r = 0; r < 2; r++) {
           acc[b][r][0] = fmaf(k[b][r][1], c[2 * r + 1], fmaf(k[b][r][0], c[2 * r], acc[b][r][0]));
-          acc[b][r][0] = fmaf(k[b][r][3], xs[i][1], fmaf(k[b][r][2], xs[i][0], acc[b][r][0]));
+          if (FMT != kQ4CP) acc[b][r][0] = fmaf(k[b][r][3], xs[i][1], fmaf(k[b][r][2], xs[i][0], acc[b][r][0]));
         }
       }
     }
@@ -554,7 +561,7 @@ k_gemv(const __grid_constant__ GemvParams p) {
       const uint2 e = lds64(M::kSubs + sub * 8);
       cnt = (int)(e.x >> 16);
       first = (int)e.y;
-      const int at = FMT == kQ4CP ? g : g >> 1;
+      const int at = kHalves ? g >> 1 : g;
       const bool live = at < cnt;
       size_t row = first + at;
       if (UP && live) row = !p.fused ? p.tokidx[row] : sh ? row - p.route.T * p.route.k : row_token[row];
@@ -613,24 +620,24 @@ k_gemv(const __grid_constant__ GemvParams p) {
   }
 }
 
-template <bool UP, int FMT, int KPW>
+template <bool UP, int FMT, int KPW, int ROWS>
 cudaError_t launch_gemv(const GemvParams& p, cudaStream_t st) {
-  constexpr int smem = Map<FMT, KPW>::kBytes;
+  constexpr int smem = Map<FMT, KPW, ROWS>::kBytes;
   static bool attr_done = false;
   static int sms = 0;
   if (!attr_done) {
-    cudaError_t e = cudaFuncSetAttribute(k_gemv<UP, FMT, KPW>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = cudaFuncSetAttribute(k_gemv<UP, FMT, KPW, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     int dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     attr_done = true;
   }
-  return launch_pdl(k_gemv<UP, FMT, KPW>, dim3(sms), dim3(kThreads), (size_t)smem, st, p);
+  return launch_pdl(k_gemv<UP, FMT, KPW, ROWS>, dim3(sms), dim3(kThreads), (size_t)smem, st, p);
 }
 
 // One launch for the passes pass0 .. pass0 + kMaxSubs - 1.
-template <bool UP, int FMT>
+template <bool UP, int FMT, int ROWS>
 cudaError_t launch_one(GemvParams& p, cudaStream_t st) {
   const int KB = p.img.n_kblocks;
   // The fewest K blocks per warp with which one team covers K, but two at least: more warps at work on a unit beat
@@ -639,18 +646,18 @@ cudaError_t launch_one(GemvParams& p, cudaStream_t st) {
   p.slices = (KB + kpw - 1) / kpw;
   p.teams = kWarps / p.slices;
   if (p.teams < 1) return cudaErrorInvalidValue;
-  if (kpw == 4) return launch_gemv<UP, FMT, 4>(p, st);
-  if (kpw == 3) return launch_gemv<UP, FMT, 3>(p, st);
-  return launch_gemv<UP, FMT, 2>(p, st);
+  if (kpw == 4) return launch_gemv<UP, FMT, 4, ROWS>(p, st);
+  if (kpw == 3) return launch_gemv<UP, FMT, 3, ROWS>(p, st);
+  return launch_gemv<UP, FMT, 2, ROWS>(p, st);
 }
 
 // Passes that the host cannot count take as many launches as could be needed (a call of up to 16 tokens: one). Each
 // waits for the one before; those beyond the last pass end at once.
-template <bool UP, int FMT>
+template <bool UP, int FMT, int ROWS>
 cudaError_t launch_fmt(GemvParams& p, int T, int max_passes, int* launches, cudaStream_t st) {
-  if (p.n_sh > 0) max_passes = std::max(max_passes, (T + Map<FMT, 4>::kRows - 1) / Map<FMT, 4>::kRows);
+  if (p.n_sh > 0) max_passes = std::max(max_passes, (T + ROWS - 1) / ROWS);
   for (p.pass0 = 0; p.pass0 == 0 || p.pass0 < max_passes; p.pass0 += kMaxSubs) {
-    if (cudaError_t e = launch_one<UP, FMT>(p, st)) return e;
+    if (cudaError_t e = launch_one<UP, FMT, ROWS>(p, st)) return e;
     ++*launches;
   }
   return cudaSuccess;
@@ -670,9 +677,9 @@ int shared_ctas(int T, int k, int E, int rows) {
 }  // namespace
 
 int gemv_max_runs() { return 192; }
-int gemv_rows(int fmt) { return fmt == kQ4CP ? Map<kQ4CP, 4>::kRows : Map<kQ4K, 4>::kRows; }
+int gemv_rows(int fmt, bool decode) { return fmt == kQ4CP && !decode ? 8 : 4; }
 int gemv_passes(int fmt, int T, int k, int E) {
-  const int rows = gemv_rows(fmt), runs = T * k < E ? T * k : E;
+  const int rows = gemv_rows(fmt, true), runs = T * k < E ? T * k : E;
   return (T * k + runs * (rows - 1)) / rows;
 }
 int gemv_max_k() { return kWarps * 4 * kTileK; }
@@ -680,31 +687,32 @@ int gemv_max_mid() { return kWarps / 2 * 4 * kTileK; }
 
 cudaError_t launch_up_gemv(const Image& img, const Image* img_sh, const void* x_bf16, int T, int k, int E, int d, int mid,
                            const int32_t* tokidx, const Run* runs, const int32_t* n_runs,
-                           int max_passes, __half* hid16, int32_t* status, const RouteIn* route, int* launches, cudaStream_t st) {
+                           int max_passes, bool decode, __half* hid16, int32_t* status, const RouteIn* route, int* launches,
+                           cudaStream_t st) {
   GemvParams p{};
   p.img = img;
-  if (img_sh) p.img_sh = *img_sh, p.n_sh = shared_ctas(T, k, E, Map<kQ4CP, 4>::kRows);
+  if (img_sh) p.img_sh = *img_sh, p.n_sh = shared_ctas(T, k, E, gemv_rows(kQ4CP, true));
   p.runs = runs; p.n_runs = n_runs; p.K = d; p.mid = mid;
   p.x = (const uint16_t*)x_bf16; p.tokidx = tokidx; p.hid = hid16; p.status = status;
   if (route) p.route = *route, p.fused = 1;
-  if (img.fmt == kQ4K) return launch_fmt<true, kQ4K>(p, T, max_passes, launches, st);
-  if (img.fmt == kQ51) return launch_fmt<true, kQ51>(p, T, max_passes, launches, st);
-  return launch_fmt<true, kQ4CP>(p, T, max_passes, launches, st);
+  if (img.fmt == kQ4K) return launch_fmt<true, kQ4K, 4>(p, T, max_passes, launches, st);
+  if (img.fmt == kQ51) return launch_fmt<true, kQ51, 4>(p, T, max_passes, launches, st);
+  return decode ? launch_fmt<true, kQ4CP, 4>(p, T, max_passes, launches, st) : launch_fmt<true, kQ4CP, 8>(p, T, max_passes, launches, st);
 }
 
 cudaError_t launch_down_gemv(const Image& img, const Image* img_sh, const __half* hid16, int T, int k, int E, int d, int mid,
-                             const Run* runs, const int32_t* n_runs, int max_passes, void* pairs, bool pairs_f16, int32_t* status,
+                             const Run* runs, const int32_t* n_runs, int max_passes, bool decode, void* pairs, bool pairs_f16, int32_t* status,
                              int32_t* ready, int* launches, cudaStream_t st) {
   GemvParams p{};
   p.img = img;
-  if (img_sh) p.img_sh = *img_sh, p.n_sh = shared_ctas(T, k, E, Map<kQ4CP, 4>::kRows);
+  if (img_sh) p.img_sh = *img_sh, p.n_sh = shared_ctas(T, k, E, gemv_rows(kQ4CP, true));
   p.runs = runs; p.n_runs = n_runs; p.K = mid; p.mid = mid;
   p.hid = const_cast<__half*>(hid16);
   if (pairs_f16) p.out16 = (__half*)pairs; else p.out = (float*)pairs;
   p.status = status; p.ready = ready;
-  if (img.fmt == kQ4K) return launch_fmt<false, kQ4K>(p, T, max_passes, launches, st);
-  if (img.fmt == kQ51) return launch_fmt<false, kQ51>(p, T, max_passes, launches, st);
-  return launch_fmt<false, kQ4CP>(p, T, max_passes, launches, st);
+  if (img.fmt == kQ4K) return launch_fmt<false, kQ4K, 4>(p, T, max_passes, launches, st);
+  if (img.fmt == kQ51) return launch_fmt<false, kQ51, 4>(p, T, max_passes, launches, st);
+  return decode ? launch_fmt<false, kQ4CP, 4>(p, T, max_passes, launches, st) : launch_fmt<false, kQ4CP, 8>(p, T, max_passes, launches, st);
 }
 
 }  // namespace b200moe

@@ -144,8 +144,8 @@ cudaError_t launch_down_simt(const Image& img, const float* hid_f32, int d, int 
 
 // ---- expert_gemv.cu (decode / verify path) ----
 int gemv_max_runs();
-int gemv_rows(int fmt);  // rows of an expert that one pass over its weights serves
-// The most passes that T tokens' pairs can make; the launches below take any number.
+int gemv_rows(int fmt, bool decode);  // rows of an expert that one pass over its weights serves, in decode calls or among longer ones'
+// The most passes that a decode call's pairs can make; the launches below take any number.
 int gemv_passes(int fmt, int T, int k, int E);
 int gemv_max_k();     // largest d
 int gemv_max_mid();   // largest mid
@@ -155,10 +155,10 @@ int gemv_max_mid();   // largest mid
 // route: the gate/up kernel does the routing, too (T*k <= 256; the lists above are then its results).
 // max_passes: no fewer than the listed runs make. launches: added to.
 cudaError_t launch_up_gemv(const Image& img, const Image* img_sh, const void* x_bf16, int T, int k, int E, int d, int mid,
-                           const int32_t* tokidx, const Run* runs, const int32_t* n_runs, int max_passes,
+                           const int32_t* tokidx, const Run* runs, const int32_t* n_runs, int max_passes, bool decode,
                            __half* hid16, int32_t* status, const RouteIn* route, int* launches, cudaStream_t st);
 cudaError_t launch_down_gemv(const Image& img, const Image* img_sh, const __half* hid16, int T, int k, int E, int d, int mid,
-                             const Run* runs, const int32_t* n_runs, int max_passes, void* pairs, bool pairs_f16, int32_t* status,
+                             const Run* runs, const int32_t* n_runs, int max_passes, bool decode, void* pairs, bool pairs_f16, int32_t* status,
                              int32_t* ready, int* launches, cudaStream_t st);
 
 // ---- decode.cu (q4cp decode / verify, T <= decode_max_tokens(), as one kernel) ----
