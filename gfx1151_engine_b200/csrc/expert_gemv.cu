@@ -15,7 +15,7 @@
 //     16 tokens of 64 x 2048 x 512: 31.0 / 90.1 / 204.7 and 47.1 us; four: 30.6 / 88.1 / 203.0 and 44.0), but of the 211
 //     experts of a 77-token prompt one pass of eight serves 191, one of four 171. Decode calls take four at any length, so
 //     that a token's bytes do not depend on the others of the call.
-//   * B never moves: a warp owns at most four K blocks (its slice) of all the rows its team works on, and the
+//   * B never moves: a warp owns at most four or five K blocks (its slice) of all the rows its team works on, and the
 //     activations of a slice are 8 registers per K block and lane.
 //   * q4cp: a code byte is decoded by one lookup in a 256-entry half2 table replicated per lane in shared memory
 //     (no bank conflicts; a line is 256 bytes, so the address is one byte permute): 32 of the 50 wavefronts per
@@ -60,8 +60,8 @@ struct Map {
   // the buffers let the slices drift further apart, 31.1 against 32.1 us at T = 1, 195.4 / 196.6 at T = 13, than two and
   // three; slices of three K blocks keep two and two.
   static constexpr int kRed = ROWS == 8 && KPW == 3 ? 2 : 4;
-  static constexpr int kGroup = KPW == 4 ? 2 : KPW;   // K blocks per ring slot
-  static constexpr int kGroups = KPW / kGroup;        // slots per unit
+  static constexpr int kGroup = KPW >= 4 ? 2 : KPW;             // K blocks per ring slot
+  static constexpr int kGroups = (KPW + kGroup - 1) / kGroup;  // slots per unit
   static constexpr uint32_t kLut = kOffLow;  // kQ4CP: 256 lines of {32 lanes x 4 B, first book}{32 x 4 B, second book}
   static constexpr uint32_t kRing = kLut + (FMT == kQ4CP ? 65536u : 0u);
   static constexpr uint32_t kSub = (uint32_t)sub_bytes(FMT), kSlot = kGroup * kSub;
@@ -577,7 +577,7 @@ k_gemv(const __grid_constant__ GemvParams p) {
 #pragma unroll
         for (int ii = 0; ii < M::kGroup; ii++) {
           const int i = gi * M::kGroup + ii;
-          if (i < nk) item(i, slot0 + ii * M::kSub, acc);
+          if (i < KPW && i < nk) item(i, slot0 + ii * M::kSub, acc);
         }
         __syncwarp();
         issue();  // the slot has been read
@@ -640,12 +640,24 @@ cudaError_t launch_gemv(const GemvParams& p, cudaStream_t st) {
 template <bool UP, int FMT, int ROWS>
 cudaError_t launch_one(GemvParams& p, cudaStream_t st) {
   const int KB = p.img.n_kblocks;
-  // The fewest K blocks per warp with which one team covers K, but two at least: more warps at work on a unit beat
-  // longer slices (K = 2560: 14 slices of three 85 us at T = 13, 10 of four 95); at K <= 1024 two and four are level.
-  const int kpw = KB > 48 ? 4 : KB > 32 ? 3 : 2;
+  // K blocks per warp: what leaves the fewest of the 16 warps idle or short of a block, and of equals the fewest. (At
+  // K = 1280 ten slices of two leave six warps idle: five of four, three units at a time, 58.4 -> 52.2 us of a 13-token call of
+  // 1280 x 768, 74.7 -> 64.5 of 1280 x 1024; K = 1536 8 slices of three instead of 12 of two, 44.0 -> 39.9.) Five only for eight
+  // rows per pass: 500 tokens of 2560 x 640 380 -> 370 us, 100 tokens 329 -> 316; with four rows, whose blocks are cheaper, 2560 x 640 is
+  // level and 2304 x 1024 loses 4 %.
+  constexpr int kMaxKpw = ROWS == 8 ? 5 : 4;
+  int kpw = 0, best = 0;
+  for (int n = 2; n <= kMaxKpw; n++) {
+    const int slices = (KB + n - 1) / n;
+    if (slices > kWarps) continue;
+    const int busy = KB * (kWarps / slices) * (60 / n);  // K blocks at work of 16 * n, times 960
+    if (busy > best) best = busy, kpw = n;
+  }
+  if (kpw == 0) return cudaErrorInvalidValue;
   p.slices = (KB + kpw - 1) / kpw;
   p.teams = kWarps / p.slices;
-  if (p.teams < 1) return cudaErrorInvalidValue;
+  if constexpr (kMaxKpw == 5)
+    if (kpw == 5) return launch_gemv<UP, FMT, 5, ROWS>(p, st);
   if (kpw == 4) return launch_gemv<UP, FMT, 4, ROWS>(p, st);
   if (kpw == 3) return launch_gemv<UP, FMT, 3, ROWS>(p, st);
   return launch_gemv<UP, FMT, 2, ROWS>(p, st);

@@ -11,6 +11,7 @@ import oracle
 from gfx1151_engine_b200 import synth
 from helpers import MAX_ABS_TOL, MEAN_REL_TOL, to_bf16_f32
 from test_gpu_parity import bits, make_op, run_layer
+from test_narrow_tiles import random_blob
 
 pytestmark = pytest.mark.gpu
 
@@ -52,3 +53,34 @@ def test_many_passes(cuda):
     """160 pairs on 512 experts (one row each) and on 12 experts (16 rows of some)."""
     for E in (512, 12):
         check(cuda, synth.LayerSpec(experts=E, topk=10, d=256, mid=128, shared=True), 93)
+
+
+# K blocks of gate/up and down where slices of three or four leave fewer warps idle than the shortest: 20 / 20, 24 / 6, 12 / 28
+@pytest.mark.parametrize("d,mid", [(1280, 1280), (1536, 384), (768, 1792)])
+@pytest.mark.parametrize("fmt", ["q4cp", "gguf"])
+def test_longer_slices(cuda, d, mid, fmt):
+    gguf = dict(fmt="gguf", gg_gu=pkg.GGML_Q4_K, gg_dn=pkg.GGML_Q5_1) if fmt == "gguf" else dict(shared=True)
+    check(cuda, synth.LayerSpec(experts=3, topk=2, d=d, mid=mid, **gguf), 94)
+
+
+@pytest.mark.parametrize("d,mid", [(2560, 640), (1280, 1280)])
+def test_slices_of_five_among_a_longer_call(cuda, d, mid):
+    """Experts with few rows of a 40-token call, whose GEMV cuts these shapes into slices of five K blocks."""
+    torch = cuda
+    E, k, T = 128, 8, 40
+    gu, dn = random_blob(torch, E * 2 * mid, d, None, 5), random_blob(torch, E * d, mid, None, 6)
+    x = torch.randn(T, d, device="cuda").bfloat16()
+    logits = torch.randn(T, E, device="cuda")
+    outs = []
+    for impl in (pkg.GEMM_AUTO, pkg.GEMM_SIMT):
+        op = pkg.MoeOperator(E, k, d, mid, T, gemm_impl=impl)
+        op.load_q4cp(0, gu, dn)
+        out = torch.full((T, d), float("nan"), dtype=torch.bfloat16, device="cuda")
+        op.moe_b(0, x, logits, out)
+        op.synchronize()
+        counts = np.diff(op.get_routing(T)[4])
+        outs.append(out.float())
+        op.close()
+    assert ((counts > 0) & (counts <= 8)).sum() * d * mid >= 160000000  # (the GEMV's share is worth its launches)
+    # 2-norm: bf16 roundings of both sides and fp16 ones of hidden values and pairs: sqrt(2 * 2^-18 + 2 * 2^-22) / sqrt(3) = 1.6e-3, twice
+    assert (outs[0] - outs[1]).norm() <= 3.3e-3 * outs[1].norm()
