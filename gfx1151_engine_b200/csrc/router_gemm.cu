@@ -8,6 +8,7 @@
 //     experts: two M=128 halves share every expert tile, so the weight matrix is read from L2
 //     once per 256 tokens. Products are exact; the fp32 accumulation differs from the
 //     reference's double sum by ~1e-6.
+//     Up to 4096 tokens (k_router_gemm_split): smaller tiles, whose K range a cluster of CTAs shares.
 //   * k_router_dots: few tokens (T <= 16): every logit as a double tree sum of the exact
 //     products, rounded to float (within 1e-9 of the reference's index-order sum, i.e. the same
 //     float except when the sum sits on a rounding boundary).
@@ -230,6 +231,130 @@ k_router_gemm(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
   }
 }
 
+// The same for few tokens: tiles of 128 tokens x 64 experts whose K blocks a cluster of up to eight CTAs shares. Each leaves its
+// sums in shared memory; they are added in the CTAs' order, an equal share of the columns by each. Bound by the latency of its few copies:
+// the large tiles leave most SMs idle (64 tokens x 512 experts of 2560: 2 CTAs, 37 us; 300: 4 CTAs, 63 us). Whole calls from hidden
+// states, large tiles / these, us: 20 tokens of 4096 x 1024 351 / 315, 1500 1058 / 1011, 3000 1386 / 1359, 6000 1975 / 1977; 300 tokens
+// of 2560 x 640 455 / 406, 4000 820 / 795, 9000 1273 / 1297; 64 experts of 2048 x 512, 100 tokens 102 / 84.
+constexpr int kRsMaxTokens = 4096;
+constexpr int kRsTileM = 128, kRsTileN = 64, kRsStages = 8;
+constexpr int kRsStageBytes = (kRsTileM + kRsTileN) * 128;
+constexpr int kRsSmem = kRsStages * kRsStageBytes + 1024 + 1024;
+static_assert(kRsTileM * kRsTileN * 4 <= kRsStages * kRsStageBytes, "the sums take the stages' place");
+
+__device__ __forceinline__ void rg_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__global__ void __launch_bounds__(kRgThreads, 1)
+k_router_gemm_split(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, int T, int E, int d,
+                    float* __restrict__ logits, int32_t* status) {
+  extern __shared__ __align__(1024) uint8_t rs_raw[];
+  const uint32_t raw0 = rg_smem_u32(rs_raw), base = (raw0 + 1023u) & ~1023u;
+  uint8_t* const sm = rs_raw + (base - raw0);
+  const uint32_t bars = base + kRsStages * kRsStageBytes;  // full[8], empty[8], acc_full
+  volatile int* abort_flag = (volatile int*)(sm + kRsStages * kRsStageBytes + 192);
+  uint32_t* tmem_slot = (uint32_t*)(sm + kRsStages * kRsStageBytes + 200);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint32_t rank, n_ranks;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(n_ranks));
+  const int m0 = blockIdx.y * kRsTileM, n0 = blockIdx.z * kRsTileN;  // (blockIdx.x: the place in the cluster)
+  const int KB = d / 64, kb0 = KB * (int)rank / (int)n_ranks, kb1 = KB * (int)(rank + 1) / (int)n_ranks;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kRsStages; i++) {
+      rg_mbar_init(bars + 8 * i, 1);
+      rg_mbar_init(bars + 8 * (kRsStages + i), 1);
+    }
+    rg_mbar_init(bars + 8 * (2 * kRsStages), 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(rg_smem_u32(tmem_slot)), "r"(kRsTileN) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      for (int kb = kb0; kb < kb1; kb++) {
+        const int i = kb - kb0, s = i % kRsStages, ph = (i / kRsStages) & 1;
+        if (!rg_wait(bars + 8 * (kRsStages + s), ph ^ 1, abort_flag, status, 11)) break;
+        rg_expect_tx(bars + 8 * s, kRsStageBytes);
+        rg_tma_2d(base + s * kRsStageBytes, &map_x, kb * 64, m0, bars + 8 * s);
+        rg_tma_2d(base + s * kRsStageBytes + kRsTileM * 128, &map_w, kb * 64, n0, bars + 8 * s);
+      }
+    }
+  } else if (warp == 1) {
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kRsTileN >> 3) << 17) | ((uint32_t)(kRsTileM >> 4) << 24);
+    for (int kb = kb0; kb < kb1; kb++) {
+      const int i = kb - kb0, s = i % kRsStages, ph = (i / kRsStages) & 1;
+      if (!__all_sync(0xffffffffu, rg_wait(bars + 8 * s, ph, abort_flag, status, 12))) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t a0 = base + s * kRsStageBytes;
+      if (rg_elect()) {
+#pragma unroll
+        for (int ks = 0; ks < 4; ks++)
+          rg_mma_ss(tmem, rg_desc(a0) + (uint64_t)(ks * 2), rg_desc(a0 + kRsTileM * 128) + (uint64_t)(ks * 2), idesc, (i | ks) != 0 ? 1u : 0u);
+        rg_commit(bars + 8 * (kRsStages + s));
+        if (kb == kb1 - 1) rg_commit(bars + 8 * (2 * kRsStages));
+      }
+      __syncwarp();
+    }
+  } else {
+    const int q = warp & 3, row = q * 32 + lane;
+    if (__all_sync(0xffffffffu, rg_wait(bars + 8 * (2 * kRsStages), 0, abort_flag, status, 13))) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      float* const sums = (float*)sm;  // [column][row]; every copy into the stages has been multiplied
+      for (int c0 = 0; c0 < kRsTileN; c0 += 16) {
+        uint32_t v[16];
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
+              "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+            : "r"(tmem + ((uint32_t)(q * 32) << 16) + c0)
+            : "memory");
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int j = 0; j < 16; j++) sums[(c0 + j) * kRsTileM + row] = __uint_as_float(v[j]);
+      }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  rg_cluster_sync();
+  const int per = kRsTileN / (int)n_ranks;  // columns of this CTA
+  if (threadIdx.x < kRsTileM && m0 + (int)threadIdx.x < T) {
+    float* dst = logits + (size_t)(m0 + threadIdx.x) * E;
+    for (int j = 0; j < per; j++) {
+      const int col = (int)rank * per + j;
+      const uint32_t at = base + (uint32_t)(col * kRsTileM + threadIdx.x) * 4;
+      float sum = 0.f;
+#pragma unroll 8
+      for (uint32_t r = 0; r < n_ranks; r++) {
+        uint32_t remote;
+        float v;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(at), "r"(r));
+        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote) : "memory");
+        sum += v;
+      }
+      if (n0 + col < E) dst[n0 + col] = sum;
+    }
+  }
+  // (no CTA leaves while another may read its sums)
+  __syncthreads();
+  rg_cluster_sync();
+  if (warp == 1) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kRsTileN) : "memory");
+  }
+}
+
 // ---- logits in double --------------------------------------------------------------------
 // A block takes kExTok tokens x 8 experts: the tokens' activations are staged in shared memory,
 // warp w owns expert 8*chunk + w and adds the tokens' dot products side by side in double (one
@@ -384,6 +509,7 @@ cudaError_t router_plan_create(RouterPlan** out) {
   RouterPlan* p = new RouterPlan();
   p->enc = (PFN_cuTensorMapEncodeTiled_v12000)fn;
   e = cudaFuncSetAttribute(k_router_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, kRgSmem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_router_gemm_split, cudaFuncAttributeMaxDynamicSharedMemorySize, kRsSmem);
   if (e != cudaSuccess) {
     delete p;
     return e;
@@ -394,10 +520,10 @@ cudaError_t router_plan_create(RouterPlan** out) {
 
 void router_plan_destroy(RouterPlan* p) { delete p; }
 
-static cudaError_t rg_encode(RouterPlan* p, CUtensorMap* map, const void* base, long long rows, long long cols) {
+static cudaError_t rg_encode(RouterPlan* p, CUtensorMap* map, const void* base, long long rows, long long cols, int box_rows) {
   cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
   cuuint64_t strides[1] = {(cuuint64_t)cols * 2};
-  cuuint32_t box[2] = {64, 256};
+  cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = p->enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
                       CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -408,8 +534,28 @@ static cudaError_t rg_encode(RouterPlan* p, CUtensorMap* map, const void* base, 
 cudaError_t launch_router_gemm(RouterPlan* p, const void* x_bf16, const void* w_bf16, int T, int E, int d,
                                float* logits, int32_t* status, cudaStream_t st) {
   CUtensorMap mx, mw;
-  cudaError_t e = rg_encode(p, &mx, x_bf16, T, d);
-  if (e == cudaSuccess) e = rg_encode(p, &mw, w_bf16, E, d);
+  if (T <= kRsMaxTokens) {
+    const int tiles = (T + kRsTileM - 1) / kRsTileM * ((E + kRsTileN - 1) / kRsTileN);
+    int ranks = 8;
+    while (ranks > 1 && (tiles * ranks > 148 || ranks > d / 64)) ranks /= 2;
+    cudaError_t e = rg_encode(p, &mx, x_bf16, T, d, kRsTileM);
+    if (e == cudaSuccess) e = rg_encode(p, &mw, w_bf16, E, d, kRsTileN);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(ranks, (T + kRsTileM - 1) / kRsTileM, (E + kRsTileN - 1) / kRsTileN);
+    cfg.blockDim = dim3(kRgThreads);
+    cfg.dynamicSmemBytes = kRsSmem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = ranks;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_router_gemm_split, mx, mw, T, E, d, logits, status);
+  }
+  cudaError_t e = rg_encode(p, &mx, x_bf16, T, d, kRgTileM);
+  if (e == cudaSuccess) e = rg_encode(p, &mw, w_bf16, E, d, kRgTileN);
   if (e != cudaSuccess) return e;
   dim3 grid((T + kRgTileM - 1) / kRgTileM, (E + kRgTileN - 1) / kRgTileN);
   k_router_gemm<<<grid, kRgThreads, kRgSmem, st>>>(mx, mw, T, E, d, logits, status);

@@ -117,3 +117,26 @@ def test_forward_hidden_prefill_matches_logits_entry(cuda):
     assert torch.equal(a.view(torch.int16), b.view(torch.int16))
     y_o, _, _ = oracle.moe_forward(spec, layer, synth.bf16_bits_to_f32(xb))
     assert_output_close(bf16_out_to_f32(torch, b), y_o, "forward from hidden states")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T", [17, 128, 129, 300, 1100, 4096, 4097])
+@pytest.mark.parametrize("E,d", [(16, 128), (65, 384), (512, 2560)])
+def test_gemm_tiles(cuda, T, E, d):
+    """Edges of the router GEMM's tiles, cluster sizes from one to eight, K blocks fewer than its CTAs."""
+    torch = cuda
+    op = pkg.MoeOperator(E, 2, d, 64, T)
+    x = torch.randn(T, d, device="cuda").bfloat16()
+    w = (torch.randn(E, d, device="cuda") * 0.02).bfloat16()
+    blob = torch.zeros(64 + E * 128 * d // 2 + E * 128 * (((d // 32 * 2) + 15) & ~15), dtype=torch.uint8, device="cuda")
+    down = torch.zeros(64 + E * d * 32 + E * d * 16, dtype=torch.uint8, device="cuda")
+    op.load_q4cp(0, blob, down)
+    op.load_router(0, w)
+    logits = torch.full((T, E), float("nan"), device="cuda")
+    op.router_logits(0, x, logits)
+    op.synchronize()
+    want = x.double() @ w.double().T
+    # exact products, fp32 sums (the tensor cores may cut off instead of rounding): d steps of 2^-23 of the terms' sum at most
+    bound = d * 2.0 ** -23 * (x.double().abs() @ w.double().abs().T)
+    assert ((logits.double() - want).abs() <= bound).all()
+    op.close()
