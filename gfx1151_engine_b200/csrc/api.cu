@@ -60,6 +60,9 @@ constexpr int kOneListRows = 48, kOneListTokens = 512;
 // (2.2 us an expert of 4096 x 1024) everywhere; 768, 1536 and 2304 differ by less than 1 %, with 4096 tokens level with none at 2304, 0.5 %
 // behind at 1536. The gate/up GEMM does not gain: 2544 / 2532 us with its expansion.
 constexpr int kPopularRows = 3 * kDenseGroup;
+// The two launches cost 6 us where no expert is popular (6635 tokens on 60 experts of 1536 x 256, top-2: 159 / 166 us), and can gain 13 % of the
+// down stage's 1 us per 5e8 rows x d x mid: the line lies where that is twice their cost.
+constexpr long long kPopularWork = 50000000000;
 // The shared expert's rows stay in narrow tiles while its gate/up GEMM has at most this many of them times row
 // blocks: they fill SMs beside the routed ones, so that more and shorter items end earlier. Wide / narrow: 144
 // items (768 tokens, mid 768) 288 / 282 us, 384 (1536, mid 1024) 871 / 868, 576 (2304, mid 1024) 906 / 937.
@@ -789,7 +792,7 @@ static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const
                                     : (long long)E * d * mid >= kBothLists);
   const bool narrow = !split && (few || (T <= kOneListTokens && T * k <= kOneListRows * E));
   const bool sh_narrow = few && (long long)(T / kTcNarrowN) * (mid / 64) <= kSharedNarrowItems;
-  const bool dense = !narrow && T >= kPopularRows && T > h->decode_max && h->dense_cap > 0 && !L.i4r && !L.dn.act_shift;
+  const bool dense = !narrow && T >= kPopularRows && (long long)T * k * d * mid >= kPopularWork && T > h->decode_max && h->dense_cap > 0 && !L.i4r && !L.dn.act_shift;
   const int min_few = range ? 0 : few_row_experts(h, L, T);
   const bool mixed = min_few > 0;
   const TileCut cut{narrow ? kTcNarrowN : h->tile_cap, sh_narrow ? kTcNarrowN : h->tile_cap, split ? kTcNarrowN : 0, second,

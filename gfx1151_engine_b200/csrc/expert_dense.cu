@@ -145,6 +145,9 @@ k_expert_dense(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   uint32_t* tmem_slot = (uint32_t*)(bar_ptr + kAccEmpty + 24);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_rank();
+  pdl_wait();
+  if (p.early_next) pdl_trigger();
+  if (p.n_dense[0] == 0) return;  // (all CTAs)
   if (threadIdx.x == 0) {
     for (int i = 0; i < kStages; i++) {
       mbar_init(bars + kFull + 8 * i, rank == 0 ? 3 : 2);  // this CTA's two copies (with byte counts); the other's relay
@@ -162,8 +165,6 @@ k_expert_dense(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
-  pdl_wait();
-  if (p.early_next) pdl_trigger();
   const int n_items = p.n_dense[0] * p.n_ntiles;
   tc_fence_before();
   __syncthreads();
