@@ -8,7 +8,7 @@
 //     experts: two M=128 halves share every expert tile, so the weight matrix is read from L2
 //     once per 256 tokens. Products are exact; the fp32 accumulation differs from the
 //     reference's double sum by ~1e-6.
-//     Up to 4096 tokens (k_router_gemm_split): smaller tiles, whose K range a cluster of CTAs shares.
+//     Few such tiles (k_router_gemm_split): smaller ones, whose K range a cluster of CTAs shares.
 //   * k_router_dots: few tokens (T <= 16): every logit as a double tree sum of the exact
 //     products, rounded to float (within 1e-9 of the reference's index-order sum, i.e. the same
 //     float except when the sum sits on a rounding boundary).
@@ -231,12 +231,12 @@ k_router_gemm(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
   }
 }
 
-// The same for few tokens: tiles of 128 tokens x 64 experts whose K blocks a cluster of up to eight CTAs shares. Each leaves its
+// The same where those tiles are few: tiles of 128 tokens x 64 experts whose K blocks a cluster of up to eight CTAs shares. Each leaves its
 // sums in shared memory; they are added in the CTAs' order, an equal share of the columns by each. Bound by the latency of its few copies:
 // the large tiles leave most SMs idle (64 tokens x 512 experts of 2560: 2 CTAs, 37 us; 300: 4 CTAs, 63 us). Whole calls from hidden
 // states, large tiles / these, us: 20 tokens of 4096 x 1024 351 / 315, 1500 1058 / 1011, 3000 1386 / 1359, 6000 1975 / 1977; 300 tokens
 // of 2560 x 640 455 / 406, 4000 820 / 795, 9000 1273 / 1297; 64 experts of 2048 x 512, 100 tokens 102 / 84.
-constexpr int kRsMaxTokens = 4096;
+constexpr int kRsMaxTiles = 40;  // of the large ones: 32 gain, 48 are level, 72 lose
 constexpr int kRsTileM = 128, kRsTileN = 64, kRsStages = 8;
 constexpr int kRsStageBytes = (kRsTileM + kRsTileN) * 128;
 constexpr int kRsSmem = kRsStages * kRsStageBytes + 1024 + 1024;
@@ -534,7 +534,8 @@ static cudaError_t rg_encode(RouterPlan* p, CUtensorMap* map, const void* base, 
 cudaError_t launch_router_gemm(RouterPlan* p, const void* x_bf16, const void* w_bf16, int T, int E, int d,
                                float* logits, int32_t* status, cudaStream_t st) {
   CUtensorMap mx, mw;
-  if (T <= kRsMaxTokens) {
+  const dim3 grid((T + kRgTileM - 1) / kRgTileM, (E + kRgTileN - 1) / kRgTileN);
+  if (grid.x * grid.y <= (unsigned)kRsMaxTiles) {
     const int tiles = (T + kRsTileM - 1) / kRsTileM * ((E + kRsTileN - 1) / kRsTileN);
     int ranks = 8;
     while (ranks > 1 && (tiles * ranks > 148 || ranks > d / 64)) ranks /= 2;
@@ -557,7 +558,6 @@ cudaError_t launch_router_gemm(RouterPlan* p, const void* x_bf16, const void* w_
   cudaError_t e = rg_encode(p, &mx, x_bf16, T, d, kRgTileM);
   if (e == cudaSuccess) e = rg_encode(p, &mw, w_bf16, E, d, kRgTileN);
   if (e != cudaSuccess) return e;
-  dim3 grid((T + kRgTileM - 1) / kRgTileM, (E + kRgTileN - 1) / kRgTileN);
   k_router_gemm<<<grid, kRgThreads, kRgSmem, st>>>(mx, mw, T, E, d, logits, status);
   return cudaGetLastError();
 }

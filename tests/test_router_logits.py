@@ -120,7 +120,7 @@ def test_forward_hidden_prefill_matches_logits_entry(cuda):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("T", [17, 128, 129, 300, 1100, 4096, 4097])
+@pytest.mark.parametrize("T", [17, 128, 129, 300, 1100, 5120, 5121])
 @pytest.mark.parametrize("E,d", [(16, 128), (65, 384), (512, 2560)])
 def test_gemm_tiles(cuda, T, E, d):
     """Edges of the router GEMM's tiles, cluster sizes from one to eight, K blocks fewer than its CTAs."""
