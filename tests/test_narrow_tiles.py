@@ -1,9 +1,8 @@
-"""Calls with few rows per expert run the grouped GEMMs in their narrow form (tiles of at most 64 rows,
-weights through a ring of bulk copies; at most 12 rows per expert on average), longer ones in the wide
-form; tiles of more than 64 rows in a call of the first kind are cut to 64 or run in the wide form beside the
-others. Against the oracle where that form can go wrong -- K block counts that are odd, one, or fewer than
-the ring's stages, experts whose rows end just behind a tile, every weight format -- and bit for bit
-against the wide form on both sides of the rule: a row's sums do not depend on the tile it is in."""
+"""Calls of the grouped GEMMs run tiles of at most 64 rows in the form for few rows (weights through a ring of bulk
+copies) and larger ones in the wide form, on two lists side by side or on one, by the call's sizes and the rows of all experts; popular
+experts' down GEMM runs on expanded weights. Against the oracle where those forms can go wrong -- K block counts that are odd, one, or
+fewer than the ring's stages, experts whose rows end just behind a tile, every weight format -- and bit for bit
+against one another on both sides of the rules: a row's sums do not depend on the tile it is in."""
 import numpy as np
 import pytest
 
