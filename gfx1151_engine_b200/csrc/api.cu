@@ -1013,10 +1013,10 @@ int b200moe_router_logits(b200moe_handle h, int layer, const void* x_bf16_dev, i
   if (T <= 16 || !h->rplan) {
     // few tokens: double sums (1e-9 from the reference), then the reference's arithmetic for
     // the experts that decide the top-k where two of them are within a few float ulps
-    CU_TRY(h, launch_router_dots(x_bf16_dev, L.router_w, T, E, d, logits_dev, st));
+    CU_TRY(h, launch_router_dots(x_bf16_dev, L.router_w, T, E, d, logits_dev, h->flag_count, st));
     CU_TRY(h, launch_router_flag(logits_dev, T, E, h->cfg.topk, 5e-7f, h->flag_list, h->flag_count, cap, st, h->status_dev));
   } else {
-    CU_TRY(h, launch_router_gemm(h->rplan, x_bf16_dev, L.router_w, T, E, d, logits_dev, h->status_dev, st));
+    CU_TRY(h, launch_router_gemm(h->rplan, x_bf16_dev, L.router_w, T, E, d, logits_dev, h->flag_count, h->status_dev, st));
     CU_TRY(h, launch_router_flag(logits_dev, T, E, h->cfg.topk, 1e-4f, h->flag_list, h->flag_count, cap, st, h->status_dev));
   }
   CU_TRY(h, launch_router_pairs(x_bf16_dev, L.router_w, h->flag_list, h->flag_count, cap, E, d, logits_dev, st));
@@ -1035,7 +1035,7 @@ int b200moe_forward_hidden(b200moe_handle h, int layer, const void* x_bf16_dev, 
   if (L.router_w && route_block_supported(T, c.topk) && !fused_decode(c)) {
     // few tokens: the routing kernel itself looks for near-ties (router_logits: two kernels and a memset more)
     cudaStream_t st = (cudaStream_t)stream;
-    CU_TRY(h, launch_router_dots(x_bf16_dev, L.router_w, T, c.experts, c.d_model, h->router_logits, st));
+    CU_TRY(h, launch_router_dots(x_bf16_dev, L.router_w, T, c.experts, c.d_model, h->router_logits, nullptr, st));
     h->launches++;
     if (h->prof) CU_TRY(h, cudaEventRecord(h->prof_ev[(size_t)h->prof_head * kProfEvents], st));
     return forward_impl(h, layer, x_bf16_dev, T, h->rb.topids, h->rb.topw, kIdStride, out_bf16_dev, st, h->prof, h->router_logits, L.router_w);

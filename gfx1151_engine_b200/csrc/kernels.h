@@ -184,14 +184,14 @@ cudaError_t launch_wait_flags(const int32_t* flags, int n, int32_t expected, int
 struct RouterPlan;
 cudaError_t router_plan_create(RouterPlan** out);
 void router_plan_destroy(RouterPlan* p);
-// logits[T][E] fp32 = x[T][d] (bf16) . w[E][d]^T (bf16) on the tensor cores (T > 16)
+// logits[T][E] fp32 = x[T][d] (bf16) . w[E][d]^T (bf16) on the tensor cores (T > 16); count <- 0, for launch_router_flag
 cudaError_t launch_router_gemm(RouterPlan* p, const void* x_bf16, const void* w_bf16, int T, int E, int d,
-                               float* logits, int32_t* status, cudaStream_t st);
-// few tokens: every logit as a double tree sum of the exact products, rounded to float
-cudaError_t launch_router_dots(const void* x_bf16, const void* w_bf16, int T, int E, int d, float* logits,
+                               float* logits, int32_t* count, int32_t* status, cudaStream_t st);
+// few tokens: every logit as a double tree sum of the exact products, rounded to float (count: may be null)
+cudaError_t launch_router_dots(const void* x_bf16, const void* w_bf16, int T, int E, int d, float* logits, int32_t* count,
                                cudaStream_t st);
 // pairs/count <- (token * E + expert) of the experts that decide a token's top-k, for tokens
-// where two of them are closer than rel_margin x magnitude (at most cap pairs are stored)
+// where two of them are closer than rel_margin x magnitude (at most cap pairs are stored, behind the *count there are)
 cudaError_t launch_router_flag(const float* logits, int T, int E, int k, float rel_margin, int32_t* pairs,
                                int32_t* count, int cap, cudaStream_t st, int32_t* status = nullptr);  // status {7, token}: list overflow
 // the listed logits in the reference's arithmetic

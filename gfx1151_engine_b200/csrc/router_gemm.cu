@@ -124,8 +124,9 @@ __device__ __forceinline__ bool rg_elect() {
 
 __global__ void __launch_bounds__(kRgThreads, 1)
 k_router_gemm(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, int T, int E,
-              int d, float* __restrict__ logits, int32_t* status) {
+              int d, float* __restrict__ logits, int32_t* __restrict__ count, int32_t* status) {
   extern __shared__ __align__(1024) uint8_t rg_raw[];
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *count = 0;  // of the list that k_router_flag writes
   const uint32_t raw0 = rg_smem_u32(rg_raw);
   const uint32_t base = (raw0 + 1023u) & ~1023u;            // stage buffers need 1 KB alignment
   uint8_t* const sm = rg_raw + (base - raw0);
@@ -248,8 +249,9 @@ __device__ __forceinline__ void rg_cluster_sync() {
 
 __global__ void __launch_bounds__(kRgThreads, 1)
 k_router_gemm_split(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, int T, int E, int d,
-                    float* __restrict__ logits, int32_t* status) {
+                    float* __restrict__ logits, int32_t* __restrict__ count, int32_t* status) {
   extern __shared__ __align__(1024) uint8_t rs_raw[];
+  if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0) *count = 0;  // of the list that k_router_flag writes
   const uint32_t raw0 = rg_smem_u32(rs_raw), base = (raw0 + 1023u) & ~1023u;
   uint8_t* const sm = rs_raw + (base - raw0);
   const uint32_t bars = base + kRsStages * kRsStageBytes;  // full[8], empty[8], acc_full
@@ -365,12 +367,13 @@ constexpr int kExExp = 8;
 template <int kExTok>
 __global__ void __launch_bounds__(256)
 k_router_dots(const uint16_t* __restrict__ x, const uint16_t* __restrict__ w, int n, int E, int d,
-              float* __restrict__ logits) {
+              float* __restrict__ logits, int32_t* __restrict__ count) {
   extern __shared__ __align__(16) uint16_t ex_x[];  // [kExTok][d] bf16 bits
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_groups = (n + kExTok - 1) / kExTok, n_chunks = (E + kExExp - 1) / kExExp;
   pdl_trigger();
   pdl_wait();
+  if (count != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *count = 0;
   for (long long job = blockIdx.x; job < (long long)n_groups * n_chunks; job += gridDim.x) {
     const int grp = (int)(job / n_chunks), chunk = (int)(job % n_chunks);
     __syncthreads();  // the previous job's reads of the staged rows are over
@@ -428,6 +431,8 @@ k_router_pairs(const uint16_t* __restrict__ x, const uint16_t* __restrict__ w, c
   __shared__ double s_prod[8][256];  // per warp: the products of 256 elements, for the index-order replay
   const int lane = threadIdx.x & 31;
   const int n_warps = gridDim.x * (blockDim.x >> 5);
+  pdl_trigger();
+  pdl_wait();
   const int n = min(*count, cap);
   for (int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += n_warps) {
     const int t = pairs[i] / E, e = pairs[i] % E;
@@ -447,6 +452,8 @@ k_router_flag(const float* __restrict__ logits, int T, int E, int k, float rel_m
               int32_t* __restrict__ count, int cap, int32_t* __restrict__ status) {
   const int lane = threadIdx.x & 31;
   const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  pdl_trigger();
+  pdl_wait();
   if (t >= T) return;
   float v[16], v0[16];
 #pragma unroll
@@ -532,7 +539,7 @@ static cudaError_t rg_encode(RouterPlan* p, CUtensorMap* map, const void* base, 
 }
 
 cudaError_t launch_router_gemm(RouterPlan* p, const void* x_bf16, const void* w_bf16, int T, int E, int d,
-                               float* logits, int32_t* status, cudaStream_t st) {
+                               float* logits, int32_t* count, int32_t* status, cudaStream_t st) {
   CUtensorMap mx, mw;
   const dim3 grid((T + kRgTileM - 1) / kRgTileM, (E + kRgTileN - 1) / kRgTileN);
   if (grid.x * grid.y <= (unsigned)kRsMaxTiles) {
@@ -553,25 +560,22 @@ cudaError_t launch_router_gemm(RouterPlan* p, const void* x_bf16, const void* w_
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_router_gemm_split, mx, mw, T, E, d, logits, status);
+    return cudaLaunchKernelEx(&cfg, k_router_gemm_split, mx, mw, T, E, d, logits, count, status);
   }
   cudaError_t e = rg_encode(p, &mx, x_bf16, T, d, kRgTileM);
   if (e == cudaSuccess) e = rg_encode(p, &mw, w_bf16, E, d, kRgTileN);
   if (e != cudaSuccess) return e;
-  k_router_gemm<<<grid, kRgThreads, kRgSmem, st>>>(mx, mw, T, E, d, logits, status);
+  k_router_gemm<<<grid, kRgThreads, kRgSmem, st>>>(mx, mw, T, E, d, logits, count, status);
   return cudaGetLastError();
 }
 
 cudaError_t launch_router_flag(const float* logits, int T, int E, int k, float rel_margin, int32_t* pairs,
                                int32_t* count, int cap, cudaStream_t st, int32_t* status) {
-  cudaError_t e = cudaMemsetAsync(count, 0, sizeof(int32_t), st);
-  if (e != cudaSuccess) return e;
-  k_router_flag<<<(T + 7) / 8, 256, 0, st>>>(logits, T, E, k, rel_margin, pairs, count, cap, status);
-  return cudaGetLastError();
+  return launch_pdl(k_router_flag, dim3((T + 7) / 8), dim3(256), 0, st, logits, T, E, k, rel_margin, pairs, count, cap, status);
 }
 
 template <int TOK>
-static cudaError_t launch_dots(const uint16_t* x, const uint16_t* w, int T, int E, int d, float* logits, cudaStream_t st) {
+static cudaError_t launch_dots(const uint16_t* x, const uint16_t* w, int T, int E, int d, float* logits, int32_t* count, cudaStream_t st) {
   const size_t smem = (size_t)TOK * d * 2;
   static size_t smem_set = 0;
   if (smem > smem_set) {
@@ -582,19 +586,19 @@ static cudaError_t launch_dots(const uint16_t* x, const uint16_t* w, int T, int 
   long long jobs = (long long)((T + TOK - 1) / TOK) * ((E + kExExp - 1) / kExExp);
   int blocks = (int)(jobs < 148 * 3 ? jobs : 148 * 3);
   if (blocks < 1) blocks = 1;
-  return launch_pdl(k_router_dots<TOK>, dim3(blocks), dim3(256), smem, st, x, w, T, E, d, logits);
+  return launch_pdl(k_router_dots<TOK>, dim3(blocks), dim3(256), smem, st, x, w, T, E, d, logits, count);
 }
 
-cudaError_t launch_router_dots(const void* x_bf16, const void* w_bf16, int T, int E, int d, float* logits,
+cudaError_t launch_router_dots(const void* x_bf16, const void* w_bf16, int T, int E, int d, float* logits, int32_t* count,
                                cudaStream_t st) {
   // As many tokens beside one another as still give every SM a block: 16 tokens x 64 experts in eights were
   // 16 blocks and 15 us.
   const long long chunks = (E + kExExp - 1) / kExExp;
   const uint16_t *x = (const uint16_t*)x_bf16, *w = (const uint16_t*)w_bf16;
-  if ((T + 7) / 8 * chunks >= 148) return launch_dots<8>(x, w, T, E, d, logits, st);
-  if ((T + 3) / 4 * chunks >= 148) return launch_dots<4>(x, w, T, E, d, logits, st);
-  if ((T + 1) / 2 * chunks >= 148) return launch_dots<2>(x, w, T, E, d, logits, st);
-  return launch_dots<1>(x, w, T, E, d, logits, st);
+  if ((T + 7) / 8 * chunks >= 148) return launch_dots<8>(x, w, T, E, d, logits, count, st);
+  if ((T + 3) / 4 * chunks >= 148) return launch_dots<4>(x, w, T, E, d, logits, count, st);
+  if ((T + 1) / 2 * chunks >= 148) return launch_dots<2>(x, w, T, E, d, logits, count, st);
+  return launch_dots<1>(x, w, T, E, d, logits, count, st);
 }
 
 cudaError_t launch_router_pairs(const void* x_bf16, const void* w_bf16, const int32_t* pairs, const int32_t* count,
@@ -602,8 +606,8 @@ cudaError_t launch_router_pairs(const void* x_bf16, const void* w_bf16, const in
   int blocks = (cap + 7) / 8;
   if (blocks > 148 * 8) blocks = 148 * 8;
   if (blocks < 1) blocks = 1;
-  k_router_pairs<<<blocks, 256, 0, st>>>((const uint16_t*)x_bf16, (const uint16_t*)w_bf16, pairs, count, cap, E, d, logits);
-  return cudaGetLastError();
+  return launch_pdl(k_router_pairs, dim3(blocks), dim3(256), 0, st, (const uint16_t*)x_bf16, (const uint16_t*)w_bf16, pairs, count, cap, E, d,
+                    logits);
 }
 
 }  // namespace b200moe
