@@ -640,7 +640,8 @@ cudaError_t launch_gemv(const GemvParams& p, cudaStream_t st) {
 template <bool UP, int FMT, int ROWS>
 cudaError_t launch_one(GemvParams& p, cudaStream_t st) {
   const int KB = p.img.n_kblocks;
-  // K blocks per warp: what leaves the fewest of the 16 warps idle or short of a block, and of equals the fewest. (At
+  // K blocks per warp: what leaves the fewest of the 16 warps idle or short of a block; in decode calls longer slices, whose chain is longer, only where
+  // they put an eighth more to work (K = 384: two slices of three instead of three of two, 16 against 15 warps: 26.6 against 25.9 us). (At
   // K = 1280 ten slices of two leave six warps idle: five of four, three units at a time, 58.4 -> 52.2 us of a 13-token call of
   // 1280 x 768, 74.7 -> 64.5 of 1280 x 1024; K = 1536 8 slices of three instead of 12 of two, 44.0 -> 39.9.) Five only for eight
   // rows per pass: 500 tokens of 2560 x 640 380 -> 370 us, 100 tokens 329 -> 316; with four rows, whose blocks are cheaper, 2560 x 640 is
@@ -651,7 +652,7 @@ cudaError_t launch_one(GemvParams& p, cudaStream_t st) {
     const int slices = (KB + n - 1) / n;
     if (slices > kWarps) continue;
     const int busy = KB * (kWarps / slices) * (60 / n);  // K blocks at work of 16 * n, times 960
-    if (busy > best) best = busy, kpw = n;
+    if (ROWS == 8 ? busy > best : 8 * busy >= 9 * best) best = busy, kpw = n;
   }
   if (kpw == 0) return cudaErrorInvalidValue;
   p.slices = (KB + kpw - 1) / kpw;
