@@ -308,3 +308,38 @@ def test_more_than_twelve_rows(cuda, E, k, d, mid, types):
 def test_popular_experts(cuda, E, k, d, mid, types):
     """Experts of 2304 rows and more: the down GEMM on expanded weights."""
     rows_agree(cuda, E, k, d, mid, types, 3200, [3200, 2304, 2303, 3071, 769])
+
+
+def test_popular_experts_captured(cuda):
+    """A captured call from hidden states (the router GEMM's clusters) with popular experts (pairs of SMs): replayed on other tokens."""
+    torch = cuda
+    E, k, d, mid, T = 16, 4, 2048, 2048, 3200
+    op = pkg.MoeOperator(E, k, d, mid, T)
+    op.load_q4cp(0, random_blob(torch, E * 2 * mid, d, None, 1), random_blob(torch, E * d, mid, None, 2))
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    w = torch.randn(E, d, device="cuda", generator=gen) * 0.02
+    mean = torch.randn(d, device="cuda", generator=gen)
+    w[[2, 5, 11]] += 0.01 * mean  # these experts' logits are the largest for most tokens
+    op.load_router(0, w.bfloat16())
+    tokens = [(mean + torch.randn(T, d, device="cuda", generator=gen)).bfloat16() for _ in range(2)]
+    want = []
+    for x in tokens:
+        out = torch.full((T, d), float("nan"), dtype=torch.bfloat16, device="cuda")
+        op.moe_hidden(0, x, out)
+        op.synchronize()
+        assert np.diff(op.get_routing(T)[4]).max() >= 2304
+        want.append(out)
+    assert all(torch.isfinite(y.float()).all() for y in want) and not torch.equal(want[0], want[1])
+    x, out = tokens[0].clone(), torch.empty((T, d), dtype=torch.bfloat16, device="cuda")
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        op.moe_hidden(0, x, out, stream=torch.cuda.current_stream().cuda_stream)
+    for y, z in zip(tokens, want):
+        x.copy_(y)
+        out.fill_(float("nan"))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, z)
+    del graph
+    op.synchronize()
+    op.close()
