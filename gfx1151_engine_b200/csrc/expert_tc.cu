@@ -120,7 +120,9 @@ constexpr int kTraceSlots = 512;
   } while (0)
 #endif
 
-template <bool UP, bool DUAL, int FMT>
+// SKIP: the list begins behind its first p.skip[0] tiles. (An instance of its own: the pointer that it takes costs registers in loops that
+// have none to spare, 183 -> 187 us of a Q8_0 gate/up launch.)
+template <bool UP, bool DUAL, int FMT, bool SKIP>
 __global__ void __launch_bounds__(kThreads, 1)
 k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ CUtensorMap map64,
             const __grid_constant__ CUtensorMap map128, const __grid_constant__ CUtensorMap map192,
@@ -147,7 +149,7 @@ k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ C
   uint32_t* tmem_slot = (uint32_t*)(smem + kOffBar + kNumBars * 8 + 8);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // (a launch beside another one starts only when its list is there, see below: with none, it just keeps the order)
-  if (p.beside && p.n_tiles[0] == (p.skip != nullptr ? p.skip[0] : 0)) {
+  if (p.beside && p.n_tiles[0] == (SKIP ? p.skip[0] : 0)) {
     pdl_trigger();
     if (blockIdx.x == 0) pdl_wait();
     return;
@@ -191,9 +193,9 @@ k_expert_tc(const __grid_constant__ CUtensorMap map16, const __grid_constant__ C
   // the wait to stay in front of the trigger, and nothing else between these launches.
   if (!p.beside) pdl_wait();
   if (p.early_next) pdl_trigger();
-  const int skip = p.skip != nullptr ? p.skip[0] : 0;
+  const int skip = SKIP ? p.skip[0] : 0;
   const int n_items = (p.n_tiles[0] - skip) * img.n_mtiles;
-  const Tile* const tiles = p.tiles + skip;
+  const Tile* const tiles = SKIP ? p.tiles + skip : p.tiles;
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -620,14 +622,14 @@ cudaError_t encode_pair(PFN_cuTensorMapEncodeTiled_v12000 enc, CUtensorMap* map,
   return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
-template <bool UP, bool DUAL, int FMT>
+template <bool UP, bool DUAL, int FMT, bool SKIP>
 cudaError_t launch_n(TcPlan* plan, const CUtensorMap* m, const Image& img,
                    const Tile* tiles, const int32_t* n_tiles, int max_tiles, __half* out, int out_ld,
                    int32_t* status, cudaStream_t st, const int32_t* rowmap, const int32_t* map_base, const int32_t* skip, bool beside) {
   constexpr int kSmemBytes = Map::kSmemBytes;
   static bool attr_set = false;  // one flag per template instance
   if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(k_expert_tc<UP, DUAL, FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(k_expert_tc<UP, DUAL, FMT, SKIP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          kSmemBytes);
     if (e != cudaSuccess) return e;
     attr_set = true;
@@ -642,7 +644,7 @@ cudaError_t launch_n(TcPlan* plan, const CUtensorMap* m, const Image& img,
   // With a margin the free SMs belong to another stream's exchange kernels. The CTAs of a dependent launch
   // would take them, shared memory and registers of a whole SM each, and only wait there: no early start
   // then, neither of this launch nor (early_next) of the one behind it.
-  return launch_opt(plan->margin == 0, k_expert_tc<UP, DUAL, FMT>, dim3(grid), dim3(kThreads), (size_t)kSmemBytes, st, m[0],
+  return launch_opt(plan->margin == 0, k_expert_tc<UP, DUAL, FMT, SKIP>, dim3(grid), dim3(kThreads), (size_t)kSmemBytes, st, m[0],
                     m[1], m[2], m[3], p);
 }
 
@@ -654,7 +656,11 @@ cudaError_t launch(TcPlan* plan, const CUtensorMap* m, const Image& img,
     if (o.rowmap != nullptr || o.skip != nullptr) return cudaErrorInvalidValue;
     return launch_few(plan, UP, m == plan->h, img, tiles, n_tiles, max_tiles, out, out_ld, status, st, o.beside);
   }
-  return launch_n<UP, DUAL, FMT>(plan, m, img, tiles, n_tiles, max_tiles, out, out_ld, status, st, o.rowmap,
+  if constexpr (!UP && !DUAL)
+    if (o.skip != nullptr) return launch_n<UP, DUAL, FMT, true>(plan, m, img, tiles, n_tiles, max_tiles, out, out_ld, status, st, o.rowmap,
+                                           o.map_base, o.skip, o.beside);
+  if (o.skip != nullptr) return cudaErrorInvalidValue;
+  return launch_n<UP, DUAL, FMT, false>(plan, m, img, tiles, n_tiles, max_tiles, out, out_ld, status, st, o.rowmap,
                                            o.map_base, o.skip, o.beside);
 }
 
