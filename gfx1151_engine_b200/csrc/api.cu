@@ -737,7 +737,7 @@ static bool fused_decode(const b200moe_config& c) {
 // there (kMinFewWork). 0: no call of this size does.
 static int few_row_experts(b200moe_handle h, const LayerWeights& L, int T) {
   const b200moe_config& c = h->cfg;
-  const int k = c.topk, E = c.experts, d = c.d_model, mid = c.d_mid, rows = std::min(gemv_rows(L.gu.fmt, false), gemv_rows(L.dn.fmt, false));
+  const int k = c.topk, E = c.experts, d = c.d_model, mid = c.d_mid, rows = std::min(gemv_rows(L.gu.fmt), gemv_rows(L.dn.fmt));
   const int least = (int)((kMinFewWork + (long long)d * mid - 1) / ((long long)d * mid));
   return T > 16 && T > h->decode_max && !L.i4r && c.gemm_impl == B200MOE_GEMM_AUTO && 4 * T * k <= 5 * rows * E && T * k <= kFewRows * E &&
                  std::min(E, T * k) >= least && (d << L.gu.act_shift) <= gemv_max_k() && (mid << L.dn.act_shift) <= gemv_max_mid()
@@ -797,7 +797,7 @@ static int forward_impl(b200moe_handle h, int layer, const void* x, int T, const
   const bool mixed = min_few > 0;
   const TileCut cut{narrow ? kTcNarrowN : h->tile_cap, sh_narrow ? kTcNarrowN : h->tile_cap, split ? kTcNarrowN : 0, second,
                     dense ? kPopularRows : 0, h->dense_cap,
-                    mixed ? std::min(gemv_rows(L.gu.fmt, false), gemv_rows(L.dn.fmt, false)) : 0, min_few};
+                    mixed ? std::min(gemv_rows(L.gu.fmt), gemv_rows(L.dn.fmt)) : 0, min_few};
   // (the shared expert's images are q4cp: it can ride along only with q4cp routed experts)
   const bool gemv = simt && c.gemm_impl == B200MOE_GEMM_AUTO &&
                     (!shared || (L.gu.fmt == kQ4CP && L.dn.fmt == kQ4CP)) &&

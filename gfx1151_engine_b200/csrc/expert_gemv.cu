@@ -9,13 +9,12 @@
 // on 512 code bytes, of which 16 were table lookups and 16 the activations, and stood at 2.7 TB/s. Here:
 //   * mma.m16n8k16 forms the products (exact) and sums (fp32). Its A operand is 16 weight rows: ldmatrix deals the
 //     packed codes of a row out to the four lanes of a quad, 8 codes each, a code BYTE becomes an fp16 pair. Scales
-//     stay in fp32: no sum runs over two 32-groups. The two groups of a K block stand in different columns of B (zeros
-//     elsewhere), so that a pass over the weights serves FOUR rows of an expert; for q4cp among longer calls one group per instruction
-//     and EIGHT rows. Eight cost twice the scale multiplications and partial sums (calls of T = 1 / 5 / 13 of 4096 x 1024 and of
-//     16 tokens of 64 x 2048 x 512: 31.0 / 90.1 / 204.7 and 47.1 us; four: 30.6 / 88.1 / 203.0 and 44.0), but of the 211
-//     experts of a 77-token prompt one pass of eight serves 191, one of four 171. Decode calls take four at any length, so
-//     that a token's bytes do not depend on the others of the call.
-//   * B never moves: a warp owns at most four or five K blocks (its slice) of all the rows its team works on, and the
+//     stay in fp32: no sum runs over two 32-groups. q4cp takes one group per instruction and FOUR or EIGHT rows of an expert per
+//     pass over the weights (kMeanRows4 below). Eight rows fill the columns of B; of four, the two groups stand in columns of their
+//     own (zeros elsewhere), so that a lane's two columns are the two groups of one row, scaled and added once: half the scale
+//     multiplications and partial sums. An instruction adds the same 16 products in either form, and zeros to the other group's
+//     columns: the sums are the same to the bit. The GGUF formats take half of each group per instruction, and four rows.
+//   * B never moves: a warp owns at most four K blocks (five among longer calls; its slice) of all the rows its team works on, and the
 //     activations of a slice are 8 registers per K block and lane.
 //   * q4cp: a code byte is decoded by one lookup in a 256-entry half2 table replicated per lane in shared memory
 //     (no bank conflicts; a line is 256 bytes, so the address is one byte permute): 32 of the 50 wavefronts per
@@ -499,11 +498,11 @@ k_gemv(const __grid_constant__ GemvParams p) {
       }
 #pragma unroll
     for (int b = 0; b < 2; b++) {
-      if (!kHalves) {
+      if (FMT == kQ4CP) {
+        float c[4];
 #pragma unroll
         for (int h = 0; h < 2; h++) {
           // the half's products: K slots 2t, 2t+1 are the codes of byte 2q, slots 2t+8, 2t+9 those of byte 2q+1
-          float c[4];
 #pragma unroll
           for (int q = 0; q < 2; q++) {
             uint32_t a[4];
@@ -511,13 +510,19 @@ k_gemv(const __grid_constant__ GemvParams p) {
             for (int i4 = 0; i4 < 4; i4++)
               a[i4] = lut32<M::kLut>(__byte_perm(m[b][2 * h + (i4 & 1)], b ? lut_b : lut_a, 0x5504 | (2 * q + (i4 >> 1)) << 4));
             const uint32_t b0 = h ? bw[i][2 * q] : bv[i][2 * q], b1 = h ? bw[i][2 * q + 1] : bv[i][2 * q + 1];
-            if (q == 0) mma16816_first(c, a[0], a[1], a[2], a[3], b0, b1);
+            if (q == 0 && !(kHalves && h == 1)) mma16816_first(c, a[0], a[1], a[2], a[3], b0, b1);
             else mma16816(c, a[0], a[1], a[2], a[3], b0, b1);
           }
+          if (!kHalves) {
 #pragma unroll
-          for (int r = 0; r < 2; r++)
+            for (int r = 0; r < 2; r++)
 #pragma unroll
-            for (int w = 0; w < kAcc; w++) acc[b][r][w] = fmaf(k[b][r][h], c[2 * r + w], acc[b][r][w]);
+              for (int w = 0; w < kAcc; w++) acc[b][r][w] = fmaf(k[b][r][h], c[2 * r + w], acc[b][r][w]);
+          }
+        }
+        if (kHalves) {
+#pragma unroll
+          for (int r = 0; r < 2; r++) acc[b][r][0] = fmaf(k[b][r][1], c[2 * r + 1], fmaf(k[b][r][0], c[2 * r], acc[b][r][0]));
         }
       } else {
         float c[4], c16[4];
@@ -526,9 +531,7 @@ k_gemv(const __grid_constant__ GemvParams p) {
           uint32_t a[4];
 #pragma unroll
           for (int h = 0; h < 4; h++) {
-            if (FMT == kQ4CP) {
-              a[h] = lut32<M::kLut>(__byte_perm(m[b][h], b ? lut_b : lut_a, 0x5504 | q << 4));
-            } else if (FMT == kQ4K) {
+            if (FMT == kQ4K) {
               // codes q and q + 4 of the word as the fp16 pair code * 2^-24, for odd q 16 times that (denormal numbers: exact, also in the products)
               a[h] = (q & 2 ? m[b][h] >> 8 : m[b][h]) & (q & 1 ? 0x00F000F0u : 0x000F000Fu);
             } else {
@@ -548,7 +551,7 @@ k_gemv(const __grid_constant__ GemvParams p) {
 #pragma unroll
         for (int r = 0; r < 2; r++) {
           acc[b][r][0] = fmaf(k[b][r][1], c[2 * r + 1], fmaf(k[b][r][0], c[2 * r], acc[b][r][0]));
-          if (FMT != kQ4CP) acc[b][r][0] = fmaf(k[b][r][3], xs[i][1], fmaf(k[b][r][2], xs[i][0], acc[b][r][0]));
+          acc[b][r][0] = fmaf(k[b][r][3], xs[i][1], fmaf(k[b][r][2], xs[i][0], acc[b][r][0]));
         }
       }
     }
@@ -638,26 +641,26 @@ cudaError_t launch_gemv(const GemvParams& p, cudaStream_t st) {
 
 // One launch for the passes pass0 .. pass0 + kMaxSubs - 1.
 template <bool UP, int FMT, int ROWS>
-cudaError_t launch_one(GemvParams& p, cudaStream_t st) {
+cudaError_t launch_one(GemvParams& p, bool decode, cudaStream_t st) {
   const int KB = p.img.n_kblocks;
   // K blocks per warp: what leaves the fewest of the 16 warps idle or short of a block; in decode calls longer slices, whose chain is longer, only where
   // they put an eighth more to work (K = 384: two slices of three instead of three of two, 16 against 15 warps: 26.6 against 25.9 us). (At
   // K = 1280 ten slices of two leave six warps idle: five of four, three units at a time, 58.4 -> 52.2 us of a 13-token call of
   // 1280 x 768, 74.7 -> 64.5 of 1280 x 1024; K = 1536 8 slices of three instead of 12 of two, 44.0 -> 39.9.) Five only for eight
-  // rows per pass: 500 tokens of 2560 x 640 380 -> 370 us, 100 tokens 329 -> 316; with four rows, whose blocks are cheaper, 2560 x 640 is
-  // level and 2304 x 1024 loses 4 %.
-  constexpr int kMaxKpw = ROWS == 8 ? 5 : 4;
+  // rows per pass among longer calls: 500 tokens of 2560 x 640 380 -> 370 us, 100 tokens 329 -> 316; with four rows, whose blocks are cheaper, 2560 x 640
+  // is level and 2304 x 1024 loses 4 %. The cut decides the order of the sums: one of the shape alone in all decode calls.
+  const bool longer = ROWS == 8 && !decode;
   int kpw = 0, best = 0;
-  for (int n = 2; n <= kMaxKpw; n++) {
+  for (int n = 2; n <= (longer ? 5 : 4); n++) {
     const int slices = (KB + n - 1) / n;
     if (slices > kWarps) continue;
     const int busy = KB * (kWarps / slices) * (60 / n);  // K blocks at work of 16 * n, times 960
-    if (ROWS == 8 ? busy > best : 8 * busy >= 9 * best) best = busy, kpw = n;
+    if (longer ? busy > best : 8 * busy >= 9 * best) best = busy, kpw = n;
   }
   if (kpw == 0) return cudaErrorInvalidValue;
   p.slices = (KB + kpw - 1) / kpw;
   p.teams = kWarps / p.slices;
-  if constexpr (kMaxKpw == 5)
+  if constexpr (ROWS == 8)
     if (kpw == 5) return launch_gemv<UP, FMT, 5, ROWS>(p, st);
   if (kpw == 4) return launch_gemv<UP, FMT, 4, ROWS>(p, st);
   if (kpw == 3) return launch_gemv<UP, FMT, 3, ROWS>(p, st);
@@ -667,10 +670,10 @@ cudaError_t launch_one(GemvParams& p, cudaStream_t st) {
 // Passes that the host cannot count take as many launches as could be needed (a call of up to 16 tokens: one). Each
 // waits for the one before; those beyond the last pass end at once.
 template <bool UP, int FMT, int ROWS>
-cudaError_t launch_fmt(GemvParams& p, int T, int max_passes, int* launches, cudaStream_t st) {
+cudaError_t launch_fmt(GemvParams& p, int T, int max_passes, bool decode, int* launches, cudaStream_t st) {
   if (p.n_sh > 0) max_passes = std::max(max_passes, (T + ROWS - 1) / ROWS);
   for (p.pass0 = 0; p.pass0 == 0 || p.pass0 < max_passes; p.pass0 += kMaxSubs) {
-    if (cudaError_t e = launch_one<UP, FMT, ROWS>(p, st)) return e;
+    if (cudaError_t e = launch_one<UP, FMT, ROWS>(p, decode, st)) return e;
     ++*launches;
   }
   return cudaSuccess;
@@ -687,12 +690,20 @@ int shared_ctas(int T, int k, int E, int rows) {
   return n > 74 ? 74 : n;
 }
 
+// Rows per pass of a decode call: eight cost an expert with up to four rows 1 to 5 % of the call more, four cost one with five to eight a second pass.
+// us of a call, four / eight: 512 experts of 4096 x 1024 + shared, top-10, T = 1 / 5 / 13 30.2 / 30.9, 83.1 / 87.3, 191.3 / 194.4; 512 of 2560 x
+// 640 + shared, 5 / 13 44.8 / 46.0, 85.1 / 88.4; 64 of 2048 x 512, top-8, 5 / 16 27.4 / 27.2, 38.1 / 38.6. Few experts of 4096 x 1024: 2.25 rows each
+// on average (top-4 of 16 and top-8 of 32 at T = 9) 37.0 / 37.6 and 57.8 / 59.1, 3.25 (T = 13) 42.4 / 39.1 and 67.9 / 61.8, 4.5 (top-8 of 16 at
+// T = 9) 50.0 / 40.8, 8 (T = 16) 68.7 / 51.8. The line lies at 11/4; both forms give the same bits.
+constexpr int kMeanRows4 = 11;
+int decode_rows(int fmt, int T, int k, int E) { return fmt == kQ4CP && T > 4 && 4ll * T * k > (long long)kMeanRows4 * E ? 8 : 4; }
+
 }  // namespace
 
 int gemv_max_runs() { return 192; }
-int gemv_rows(int fmt, bool decode) { return fmt == kQ4CP && !decode ? 8 : 4; }
+int gemv_rows(int fmt) { return fmt == kQ4CP ? 8 : 4; }
 int gemv_passes(int fmt, int T, int k, int E) {
-  const int rows = gemv_rows(fmt, true), runs = T * k < E ? T * k : E;
+  const int rows = decode_rows(fmt, T, k, E), runs = T * k < E ? T * k : E;
   return (T * k + runs * (rows - 1)) / rows;
 }
 int gemv_max_k() { return kWarps * 4 * kTileK; }
@@ -704,13 +715,15 @@ cudaError_t launch_up_gemv(const Image& img, const Image* img_sh, const void* x_
                            cudaStream_t st) {
   GemvParams p{};
   p.img = img;
-  if (img_sh) p.img_sh = *img_sh, p.n_sh = shared_ctas(T, k, E, gemv_rows(kQ4CP, true));
+  const int rows = decode ? decode_rows(img.fmt, T, k, E) : gemv_rows(img.fmt);
+  if (img_sh) p.img_sh = *img_sh, p.n_sh = shared_ctas(T, k, E, rows);
   p.runs = runs; p.n_runs = n_runs; p.K = d; p.mid = mid;
   p.x = (const uint16_t*)x_bf16; p.tokidx = tokidx; p.hid = hid16; p.status = status;
   if (route) p.route = *route, p.fused = 1;
-  if (img.fmt == kQ4K) return launch_fmt<true, kQ4K, 4>(p, T, max_passes, launches, st);
-  if (img.fmt == kQ51) return launch_fmt<true, kQ51, 4>(p, T, max_passes, launches, st);
-  return decode ? launch_fmt<true, kQ4CP, 4>(p, T, max_passes, launches, st) : launch_fmt<true, kQ4CP, 8>(p, T, max_passes, launches, st);
+  if (img.fmt == kQ4K) return launch_fmt<true, kQ4K, 4>(p, T, max_passes, decode, launches, st);
+  if (img.fmt == kQ51) return launch_fmt<true, kQ51, 4>(p, T, max_passes, decode, launches, st);
+  if (rows == 4) return launch_fmt<true, kQ4CP, 4>(p, T, max_passes, decode, launches, st);
+  return launch_fmt<true, kQ4CP, 8>(p, T, max_passes, decode, launches, st);
 }
 
 cudaError_t launch_down_gemv(const Image& img, const Image* img_sh, const __half* hid16, int T, int k, int E, int d, int mid,
@@ -718,14 +731,16 @@ cudaError_t launch_down_gemv(const Image& img, const Image* img_sh, const __half
                              int32_t* ready, int* launches, cudaStream_t st) {
   GemvParams p{};
   p.img = img;
-  if (img_sh) p.img_sh = *img_sh, p.n_sh = shared_ctas(T, k, E, gemv_rows(kQ4CP, true));
+  const int rows = decode ? decode_rows(img.fmt, T, k, E) : gemv_rows(img.fmt);
+  if (img_sh) p.img_sh = *img_sh, p.n_sh = shared_ctas(T, k, E, rows);
   p.runs = runs; p.n_runs = n_runs; p.K = mid; p.mid = mid;
   p.hid = const_cast<__half*>(hid16);
   if (pairs_f16) p.out16 = (__half*)pairs; else p.out = (float*)pairs;
   p.status = status; p.ready = ready;
-  if (img.fmt == kQ4K) return launch_fmt<false, kQ4K, 4>(p, T, max_passes, launches, st);
-  if (img.fmt == kQ51) return launch_fmt<false, kQ51, 4>(p, T, max_passes, launches, st);
-  return decode ? launch_fmt<false, kQ4CP, 4>(p, T, max_passes, launches, st) : launch_fmt<false, kQ4CP, 8>(p, T, max_passes, launches, st);
+  if (img.fmt == kQ4K) return launch_fmt<false, kQ4K, 4>(p, T, max_passes, decode, launches, st);
+  if (img.fmt == kQ51) return launch_fmt<false, kQ51, 4>(p, T, max_passes, decode, launches, st);
+  if (rows == 4) return launch_fmt<false, kQ4CP, 4>(p, T, max_passes, decode, launches, st);
+  return launch_fmt<false, kQ4CP, 8>(p, T, max_passes, decode, launches, st);
 }
 
 }  // namespace b200moe

@@ -144,7 +144,7 @@ cudaError_t launch_down_simt(const Image& img, const float* hid_f32, int d, int 
 
 // ---- expert_gemv.cu (decode / verify path) ----
 int gemv_max_runs();
-int gemv_rows(int fmt, bool decode);  // rows of an expert that one pass over its weights serves, in decode calls or among longer ones'
+int gemv_rows(int fmt);  // rows of an expert that one pass over its weights serves among a longer call's launches
 // The most passes that a decode call's pairs can make; the launches below take any number.
 int gemv_passes(int fmt, int T, int k, int E);
 int gemv_max_k();     // largest d
@@ -153,7 +153,7 @@ int gemv_max_mid();   // largest mid
 // hid16: fp16 [rows][mid] hidden activations silu(gate) * up, written by the gate/up kernel and
 // read by the down kernel.
 // route: the gate/up kernel does the routing, too (T*k <= 256; the lists above are then its results).
-// max_passes: no fewer than the listed runs make. launches: added to.
+// max_passes: no fewer than the listed runs make. decode: a decode call's, not among a longer one's. launches: added to.
 cudaError_t launch_up_gemv(const Image& img, const Image* img_sh, const void* x_bf16, int T, int k, int E, int d, int mid,
                            const int32_t* tokidx, const Run* runs, const int32_t* n_runs, int max_passes, bool decode,
                            __half* hid16, int32_t* status, const RouteIn* route, int* launches, cudaStream_t st);
