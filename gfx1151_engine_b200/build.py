@@ -11,7 +11,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libb200moe.so")
 SOURCES = ["api.cu", "repack.cu", "route.cu", "expert_simt.cu", "expert_gemv.cu", "expert_tc.cu", "expert_few.cu", "expert_dense.cu", "combine.cu", "route_static.cu", "router_gemm.cu", "files.cu", "decode.cu", "ep_host.cu", "rotate.cu"]
-HEADERS = ["common.cuh", "kernels.h", "tc.h", "tc_dev.cuh", "route_small.cuh", "route_block.cuh", "router_exact.cuh", os.path.join("..", "..", "include", "b200moe.h")]
+HEADERS = ["common.cuh", "kernels.h", "tc.h", "tc_dev.cuh", "per_device.h", "route_small.cuh", "route_block.cuh", "router_exact.cuh", os.path.join("..", "..", "include", "b200moe.h")]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo",

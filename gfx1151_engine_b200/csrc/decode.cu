@@ -1050,21 +1050,20 @@ cudaError_t launch_decode(const Image& gu, const Image& dn, const Image* sh_gu, 
                           const int32_t* ids, const float* w, int stride, const void* x_bf16, const uint16_t* gate_w, int T,
                           int E, int k, int d, int mid, __half* hid16, void* out_bf16, const float* hc_w4, void* hc_state,
                           const RouteBuffers& rb, unsigned long long* bar, int32_t* status, cudaStream_t st, unsigned long long* trace) {
-  static bool attr_done = false;
-  static int sms = 0;
-  const int smem = (int)(kDecSmemEnd - 1024);
-  if (!attr_done) {
-    cudaError_t e = cudaFuncSetAttribute(k_decode, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    int dev = 0, per_sm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  constexpr int smem = (int)(kDecSmemEnd - 1024);
+  static OncePerDevice once;
+  cudaError_t e = once([] {
+    cudaError_t r = cudaFuncSetAttribute(k_decode, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     // the grid-wide barrier needs every block resident at once: one block per SM must fit
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_decode, kDecThreads, smem);
-    if (e != cudaSuccess) return e;
-    if (per_sm < 1 || sms < 1) return cudaErrorLaunchOutOfResources;
-    attr_done = true;
-  }
+    int per_sm = 0;
+    if (r == cudaSuccess) r = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_decode, kDecThreads, smem);
+    if (r == cudaSuccess && per_sm < 1) r = cudaErrorLaunchOutOfResources;
+    return r;
+  });
+  int sms = 0;
+  if (e == cudaSuccess) e = sm_count(&sms);
+  if (e == cudaSuccess && sms < 1) e = cudaErrorLaunchOutOfResources;
+  if (e != cudaSuccess) return e;
   DecParams p{};
   p.gu = gu;
   p.dn = dn;

@@ -305,12 +305,8 @@ cudaError_t launch_expand(const TcPlan* plan, const Image& img, const int32_t* e
 
 cudaError_t launch_down_dense(const TcPlan* plan, const Tile* tiles, const int32_t* n_dense, int d, int mid, __half* pairs16, int32_t* status,
                               cudaStream_t st) {
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(k_expert_dense, cudaFuncAttributeMaxDynamicSharedMemorySize, kDenseSmem);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
+  static OncePerDevice once;
+  if (cudaError_t e = once([] { return cudaFuncSetAttribute(k_expert_dense, cudaFuncAttributeMaxDynamicSharedMemorySize, kDenseSmem); })) return e;
   const DenseParams p{tiles, n_dense, pairs16, d, mid / kTileK, d / 256, status, 1};
   return launch_pdl(k_expert_dense, dim3(plan->sms / 2 * 2), dim3(kDenseThreads), (size_t)kDenseSmem, st, plan->h[2], plan->w_dense, p);
 }

@@ -517,12 +517,9 @@ k_expert_few(const __grid_constant__ CUtensorMap map16, const __grid_constant__ 
 template <bool UP, bool DUAL, int FMT>
 cudaError_t launch(const TcPlan* plan, const CUtensorMap* m, const Image& img, const Tile* tiles, const int32_t* n_tiles, int max_tiles,
                    __half* out, int out_ld, int32_t* status, cudaStream_t st, bool beside) {
-  static bool attr_set = false;  // one flag per template instance
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(k_expert_few<UP, DUAL, FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
+  static OncePerDevice once;  // one per template instance
+  if (cudaError_t e = once([] { return cudaFuncSetAttribute(k_expert_few<UP, DUAL, FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes); }))
+    return e;
   FewParams p{img, tiles, n_tiles, out, out_ld, status, beside ? 1 : 0, plan->margin == 0};
   const long long max_items = (long long)max_tiles * img.n_mtiles;
   const int usable = plan->sms - plan->margin > 1 ? plan->sms - plan->margin : 1;

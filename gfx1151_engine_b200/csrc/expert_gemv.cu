@@ -626,16 +626,11 @@ k_gemv(const __grid_constant__ GemvParams p) {
 template <bool UP, int FMT, int KPW, int ROWS>
 cudaError_t launch_gemv(const GemvParams& p, cudaStream_t st) {
   constexpr int smem = Map<FMT, KPW, ROWS>::kBytes;
-  static bool attr_done = false;
-  static int sms = 0;
-  if (!attr_done) {
-    cudaError_t e = cudaFuncSetAttribute(k_gemv<UP, FMT, KPW, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    attr_done = true;
-  }
+  static OncePerDevice once;
+  if (cudaError_t e = once([] { return cudaFuncSetAttribute(k_gemv<UP, FMT, KPW, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); }))
+    return e;
+  int sms = 0;
+  if (cudaError_t e = sm_count(&sms)) return e;
   return launch_pdl(k_gemv<UP, FMT, KPW, ROWS>, dim3(sms), dim3(kThreads), (size_t)smem, st, p);
 }
 

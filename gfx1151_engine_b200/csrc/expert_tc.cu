@@ -627,13 +627,9 @@ cudaError_t launch_n(TcPlan* plan, const CUtensorMap* m, const Image& img,
                    const Tile* tiles, const int32_t* n_tiles, int max_tiles, __half* out, int out_ld,
                    int32_t* status, cudaStream_t st, const int32_t* rowmap, const int32_t* map_base, const int32_t* skip, bool beside) {
   constexpr int kSmemBytes = Map::kSmemBytes;
-  static bool attr_set = false;  // one flag per template instance
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(k_expert_tc<UP, DUAL, FMT, SKIP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         kSmemBytes);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
+  static OncePerDevice once;  // one per template instance
+  if (cudaError_t e = once([] { return cudaFuncSetAttribute(k_expert_tc<UP, DUAL, FMT, SKIP>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes); }))
+    return e;
   static const int l2_ahead = getenv("B200MOE_TC_L2_AHEAD") ? atoi(getenv("B200MOE_TC_L2_AHEAD")) : 3;
   KParams p{img, tiles, n_tiles, out, out_ld, status, (UP != (getenv("B200MOE_TC_TRACE_DOWN") != nullptr)) ? plan->trace : nullptr,
             l2_ahead, rowmap, map_base, skip, beside ? 1 : 0, plan->margin == 0};

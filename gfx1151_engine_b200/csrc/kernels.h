@@ -3,6 +3,7 @@
 // none synchronises or allocates.
 #pragma once
 #include "common.cuh"
+#include "per_device.h"
 
 #include <cstdlib>
 #include <utility>

@@ -577,12 +577,8 @@ cudaError_t launch_router_flag(const float* logits, int T, int E, int k, float r
 template <int TOK>
 static cudaError_t launch_dots(const uint16_t* x, const uint16_t* w, int T, int E, int d, float* logits, int32_t* count, cudaStream_t st) {
   const size_t smem = (size_t)TOK * d * 2;
-  static size_t smem_set = 0;
-  if (smem > smem_set) {
-    cudaError_t e = cudaFuncSetAttribute(k_router_dots<TOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    smem_set = smem;
-  }
+  static OncePerDevice once;  // (227 KB: all that a block can have, whatever the layer's d)
+  if (cudaError_t e = once([] { return cudaFuncSetAttribute(k_router_dots<TOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024); })) return e;
   long long jobs = (long long)((T + TOK - 1) / TOK) * ((E + kExExp - 1) / kExExp);
   int blocks = (int)(jobs < 148 * 3 ? jobs : 148 * 3);
   if (blocks < 1) blocks = 1;
