@@ -9,8 +9,10 @@
 // output columns of its token and stores whole sectors without a transposition. Bound by the tensor pipe: 1473 TFLOP/s at 145k rows
 // of 4096 x 1024 (0.90 of the measured burst), where the dequant-GEMM's down launch makes 1018: its tiles of 8 pairs of K blocks are too
 // short to hide the handshake between decoding and MMAs. Two warps issue the copies: a thread starts one every ~170
-// cycles, and a K block's MMAs take 512. Arrivals from the other CTA carry no cluster-wide fence (they publish nothing that was
-// written by ordinary stores): with .release.cluster on the relay's arrival a K block took 1800 cycles.
+// cycles, and a K block's MMAs take 512. Both CTAs' copies complete on the first one's barriers, so
+// that no thread relays "landed" between them; what else crosses (an accumulator is free) is an arrival with .release.cluster, and all waits are
+// .acquire.cluster. That costs 0.6 %: 708 us of a 16384-token call's launch against 704 with arrivals and waits of one CTA's scope and a relay. A
+// relay with .release.cluster took 1800 cycles per K block, a fence.acq_rel.cluster behind the MMA warp's waits 775 each.
 #include "tc_dev.cuh"
 
 namespace b200moe {
@@ -91,7 +93,7 @@ k_expand(const Image img, const int32_t* __restrict__ experts, const int32_t* __
 constexpr int kStages = 6;
 constexpr int kOperand = 128 * 128;         // bytes of 128 rows x 64 halfs
 constexpr int kStageBytes = 2 * kOperand;   // 128 rows of activations, 128 of weights
-constexpr int kDenseThreads = 256;          // warps 0 and 3 copies, 1 MMAs or relay, 2 tensor memory, 4-7 epilogue
+constexpr int kDenseThreads = 256;          // warps 0 and 3 copies, 1 MMAs (of both CTAs, in the first), 2 tensor memory, 4-7 epilogue
 constexpr int kDenseSmem = kStages * kStageBytes + 1024 + 1024;  // + alignment + barriers
 constexpr int kAcc = 256;                   // columns of an accumulator
 
@@ -118,8 +120,16 @@ __device__ __forceinline__ uint32_t of_leader(uint32_t addr) {  // the same plac
   asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(addr));
   return r;
 }
+// Orders what this thread did before for the other CTA's thread that waits for it (mbar_wait<true>).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t addr) {
-  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
+}
+// A copy into this CTA's shared memory whose bytes are counted on a barrier of the pair's other CTA, or its own.
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
+      "l"(map), "r"(x), "r"(y), "r"(bar)
+      : "memory");
 }
 __device__ __forceinline__ void commit_pair(uint32_t bar) {  // arrives on that barrier of both CTAs
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
@@ -150,7 +160,7 @@ k_expert_dense(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   if (p.n_dense[0] == 0) return;  // (all CTAs)
   if (threadIdx.x == 0) {
     for (int i = 0; i < kStages; i++) {
-      mbar_init(bars + kFull + 8 * i, rank == 0 ? 3 : 2);  // this CTA's two copies (with byte counts); the other's relay
+      mbar_init(bars + kFull + 8 * i, 2);  // the first CTA's two copying warps, with both CTAs' byte counts (the second's is not used)
       mbar_init(bars + kEmpty + 8 * i, 1);
     }
     for (int i = 0; i < 2; i++) {
@@ -185,11 +195,13 @@ k_expert_dense(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
         const Tile t = p.tiles[it / p.n_ntiles];
         const int row = (warp == 0 ? t.first : (t.expert * p.n_ntiles + it % p.n_ntiles) * 256) + (int)rank * 128;
         for (int kb = 0; kb < KB; kb++) {
-          ok = mbar_wait(bars + kEmpty + 8 * stage, ph ^ 1, abort_flag, p.status, 21);
+          ok = mbar_wait<true>(bars + kEmpty + 8 * stage, ph ^ 1, abort_flag, p.status, 21);
           if (!ok) break;
+          // (the second CTA's bytes may come in before the first has announced them: the phase ends with its arrivals at the earliest, and
+          // is the same, since a stage is free only when the MMAs that waited for the phase before are done)
           const uint32_t bar = bars + kFull + 8 * stage;
-          mbar_expect_tx(bar, kOperand);
-          tma_load_2d(ring + stage * kStageBytes + off, map, kb * kTileK, row, bar);
+          if (rank == 0) mbar_expect_tx(bar, 2 * kOperand);
+          tma_load_2d_pair(ring + stage * kStageBytes + off, map, kb * kTileK, row, of_leader(bar));
           if (++stage == (uint32_t)kStages) {
             stage = 0;
             ph ^= 1;
@@ -197,36 +209,19 @@ k_expert_dense(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
         }
       }
     }
-  } else if (warp == 1 && rank != 0) {
-    // ================= relay: "this CTA's copies have landed" to the leader =================
-    if (lane == 0) {
-      uint32_t stage = 0, ph = 0;
-      bool ok = true;
-      for (int it = cluster; it < n_items && ok; it += n_clusters) {
-        for (int kb = 0; kb < KB; kb++) {
-          ok = mbar_wait(bars + kFull + 8 * stage, ph, abort_flag, p.status, 22);
-          if (!ok) break;
-          mbar_arrive_cluster(of_leader(bars + kFull + 8 * stage));
-          if (++stage == (uint32_t)kStages) {
-            stage = 0;
-            ph ^= 1;
-          }
-        }
-      }
-    }
-  } else if (warp == 1) {
+  } else if (warp == 1 && rank == 0) {
     // ================= MMA issue, for both CTAs =================
     const uint32_t idesc = (1u << 4) | (256u / 8 << 17) | (256u / 16 << 24);  // D fp32, A and B fp16, both K-major
     uint32_t stage = 0, ph = 0, li = 0;
     bool ok = true;
     for (int it = cluster; it < n_items && ok; it += n_clusters, li++) {
       const uint32_t acc = li & 1, accph = (li >> 1) & 1;
-      ok = __all_sync(0xffffffffu, mbar_wait(bars + kAccEmpty + 8 * acc, accph ^ 1, abort_flag, p.status, 23));
+      ok = __all_sync(0xffffffffu, mbar_wait<true>(bars + kAccEmpty + 8 * acc, accph ^ 1, abort_flag, p.status, 23));
       if (!ok) break;
       tc_fence_after();
       const uint32_t d_tmem = tmem + acc * kAcc;
       for (int kb = 0; kb < KB; kb++) {
-        ok = __all_sync(0xffffffffu, mbar_wait(bars + kFull + 8 * stage, ph, abort_flag, p.status, 24));
+        ok = __all_sync(0xffffffffu, mbar_wait<true>(bars + kFull + 8 * stage, ph, abort_flag, p.status, 24));
         if (!ok) break;
         tc_fence_after();
         if (elect_one()) {
@@ -251,7 +246,7 @@ k_expert_dense(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
       const Tile t = p.tiles[it / p.n_ntiles];
       const int nt = it % p.n_ntiles;
       const uint32_t acc = li & 1, accph = (li >> 1) & 1;
-      if (!__all_sync(0xffffffffu, mbar_wait(bars + kAccFull + 8 * acc, accph, abort_flag, p.status, 25))) break;
+      if (!__all_sync(0xffffffffu, mbar_wait<true>(bars + kAccFull + 8 * acc, accph, abort_flag, p.status, 25))) break;
       tc_fence_after();
       const uint32_t src = tmem + ((uint32_t)(quarter * 32) << 16) + acc * kAcc;
       const int r = (int)rank * 128 + quarter * 32 + lane;

@@ -38,15 +38,27 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
                : "memory");
 }
+// CLUSTER: also what other CTAs of the cluster did before they arrived is seen behind the wait (an arrival of theirs with .release.cluster).
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
   uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity), "r"(20000u)  // suspend-time hint (ns): sleep in hardware, not in a poll loop
-      : "memory");
+  // %3: suspend-time hint (ns): sleep in hardware, not in a poll loop
+  if constexpr (CLUSTER)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity), "r"(20000u)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity), "r"(20000u)
+        : "memory");
   return ok != 0;
 }
 // One lane of a converged warp. Code around it stays warp-uniform, which lets the compiler
@@ -70,13 +82,14 @@ __device__ __forceinline__ unsigned long long now_ns() {
 // `nap_ns` > 0 makes the waiting warp sleep between polls: warps that poll in a tight loop
 // take issue slots from the warp that shares their scheduler, and the thread that issues
 // the MMAs must not be slowed down by waiters.
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
                                           int32_t* status, int where, unsigned nap_ns = 0) {
-  if (mbar_try(bar, parity)) return true;
+  if (mbar_try<CLUSTER>(bar, parity)) return true;
   const unsigned long long t0 = now_ns();
   for (uint32_t spin = 1;; spin++) {
     if (nap_ns) __nanosleep(nap_ns);
-    if (mbar_try(bar, parity)) return true;
+    if (mbar_try<CLUSTER>(bar, parity)) return true;
     if ((spin & 255u) == 0) {
       if (*abort_flag) return false;
       if (now_ns() - t0 > (unsigned long long)kWaitLimitNs) {

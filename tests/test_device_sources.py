@@ -1,0 +1,21 @@
+"""What the kernels' correctness rests on and no run shows, read from their sources."""
+import glob
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "gfx1151_engine_b200", "csrc")
+
+
+def source(name):
+    text = open(os.path.join(CSRC, name)).read()
+    return re.sub(r"//[^\n]*", "", text)
+
+
+def test_hand_overs_between_ctas_have_the_clusters_scope():
+    """A thread's arrival on another CTA's barrier publishes something that CTA goes on with: the default scope, one CTA, does
+    not. Copies of a pair of CTAs complete on the barrier that is waited on, and every wait of that kernel acquires at the cluster's scope."""
+    for path in glob.glob(os.path.join(CSRC, "*.cu*")):
+        assert not re.search(r"mbarrier\.arrive(\.expect_tx)?\.shared::cluster", source(os.path.basename(path))), path
+    dense = source("expert_dense.cu")
+    assert ".cta_group::2 [%0]" in dense and "tma_load_2d(" not in dense
+    assert "mbar_wait(" not in dense and dense.count("mbar_wait<true>(") == 4
