@@ -84,6 +84,18 @@ __device__ __forceinline__ bool rg_wait(uint32_t bar, uint32_t parity, volatile 
     }
   }
 }
+// All threads, behind a barrier of the CTA: where a wait gave up, copies still in flight get time to land before the CTA's shared
+// memory goes away.
+__device__ __forceinline__ void rg_settle(volatile int* abort_flag) {
+  if (*abort_flag) {
+    unsigned long long t0, t1;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+    do {
+      __nanosleep(1000);
+      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
+    } while (t1 - t0 < 200000ull);
+  }
+}
 __device__ __forceinline__ void rg_tma_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
@@ -226,6 +238,8 @@ k_router_gemm(const __grid_constant__ CUtensorMap map_x, const __grid_constant__
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  rg_settle(abort_flag);
+  __syncthreads();
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
@@ -349,6 +363,7 @@ k_router_gemm_split(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     }
   }
   // (no CTA leaves while another may read its sums)
+  rg_settle(abort_flag);
   __syncthreads();
   rg_cluster_sync();
   if (warp == 1) {

@@ -19,3 +19,16 @@ def test_hand_overs_between_ctas_have_the_clusters_scope():
     dense = source("expert_dense.cu")
     assert ".cta_group::2 [%0]" in dense and "tma_load_2d(" not in dense
     assert "mbar_wait(" not in dense and dense.count("mbar_wait<true>(") == 4
+
+
+def test_aborted_kernels_wait_for_their_copies():
+    """A kernel whose bounded wait gave up (abort_flag) lets copies in flight land before it frees its tensor memory and leaves."""
+    found = 0
+    for path in glob.glob(os.path.join(CSRC, "*.cu")):
+        for kernel in source(os.path.basename(path)).split("__global__")[1:]:
+            if "abort_flag" not in kernel or "dealloc" not in kernel:
+                continue
+            end = kernel[:kernel.index("dealloc")][-900:]
+            assert re.search(r"rg_settle\(abort_flag\)|if \(\*abort_flag\) \{[^}]*now_ns\(\) - t0 < 200000ull", end), path
+            found += 1
+    assert found == 5
