@@ -353,6 +353,7 @@ k_expert_few(const __grid_constant__ CUtensorMap map16, const __grid_constant__ 
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(pending);
+      pending = 0;  // (a wait below that gives up leaves the loop: no second arrival behind it)
     };
     // A parity wait for a stage is good only when the use before it has completed. With an even number of stages that was
     // this set's own; with an odd one the other set's quad qi - 3, whose MMAs this set then waits for first.
@@ -363,7 +364,6 @@ k_expert_few(const __grid_constant__ CUtensorMap map16, const __grid_constant__ 
     for (uint32_t qi = (uint32_t)set; qi < total; qi += 2) {
       if (kOdd) {
         if (pending) signal();
-        pending = 0;
         if (!slot_free()) break;
       }
       if (!c_ready && !__all_sync(0xffffffffu, mbar_wait(bars + 8 * (kBarCFull + stage), ph, abort_flag, p.status, 11))) break;

@@ -32,3 +32,10 @@ def test_aborted_kernels_wait_for_their_copies():
             assert re.search(r"rg_settle\(abort_flag\)|if \(\*abort_flag\) \{[^}]*now_ns\(\) - t0 < 200000ull", end), path
             found += 1
     assert found == 5
+
+
+def test_an_arrival_is_made_once():
+    """The few-row GEMM's dequantising warps tell of a quad's stores later; once told, it is not told again when a wait behind it gives up."""
+    few = source("expert_few.cu")
+    signal = few[few.index("auto signal = [&]() {"):]
+    assert re.search(r"mbar_arrive\(pending\);\s*pending = 0;", signal[:signal.index("};")])
