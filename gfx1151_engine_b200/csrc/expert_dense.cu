@@ -61,10 +61,6 @@ k_expand(const Image img, const int32_t* __restrict__ experts, const int32_t* __
       RowMetaTc sc{0, 0, 0, 0};
       if (FMT == kQ4CP) {
         sc.a = __ldg((const uint32_t*)pm);
-      } else if (FMT == kQ4K) {
-        const uint2 t = __ldg((const uint2*)pm);
-        sc.a = t.x;
-        sc.b = t.y;
       } else {
         const uint4 t = __ldg((const uint4*)pm);
         sc = RowMetaTc{t.x, t.y, t.z, t.w};
@@ -104,7 +100,6 @@ struct DenseParams {
   int out_ld;
   int KB, n_ntiles;          // K / 64, tiles of 256 weight rows per expert
   int32_t* status;
-  int early_next;
 };
 
 __device__ __forceinline__ uint32_t cluster_rank() {
@@ -156,7 +151,7 @@ k_expert_dense(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_rank();
   pdl_wait();
-  if (p.early_next) pdl_trigger();
+  pdl_trigger();  // (behind the wait: the launches behind this one run beside it)
   if (p.n_dense[0] == 0) return;  // (all CTAs)
   if (threadIdx.x == 0) {
     for (int i = 0; i < kStages; i++) {
@@ -292,7 +287,7 @@ cudaError_t expand(const TcPlan* plan, const Image& img, const int32_t* experts,
 
 cudaError_t launch_expand(const TcPlan* plan, const Image& img, const int32_t* experts, const int32_t* n_dense, __half* out,
                           cudaStream_t st) {
-  if (img.act_shift || img.paired) return cudaErrorNotSupported;
+  if (img.act_shift || img.paired || plan->margin > 0) return cudaErrorNotSupported;
   if (img.fmt == kQ51) return expand<kQ51>(plan, img, experts, n_dense, out, st);
   if (img.fmt != kQ4CP) return cudaErrorNotSupported;
   return expand<kQ4CP>(plan, img, experts, n_dense, out, st);
@@ -300,9 +295,10 @@ cudaError_t launch_expand(const TcPlan* plan, const Image& img, const int32_t* e
 
 cudaError_t launch_down_dense(const TcPlan* plan, const Tile* tiles, const int32_t* n_dense, int d, int mid, __half* pairs16, int32_t* status,
                               cudaStream_t st) {
+  if (plan->margin > 0) return cudaErrorNotSupported;  // its pairs fill the GPU and start early: not beside exchange kernels
   static OncePerDevice once;
   if (cudaError_t e = once([] { return cudaFuncSetAttribute(k_expert_dense, cudaFuncAttributeMaxDynamicSharedMemorySize, kDenseSmem); })) return e;
-  const DenseParams p{tiles, n_dense, pairs16, d, mid / kTileK, d / 256, status, 1};
+  const DenseParams p{tiles, n_dense, pairs16, d, mid / kTileK, d / 256, status};
   return launch_pdl(k_expert_dense, dim3(plan->sms / 2 * 2), dim3(kDenseThreads), (size_t)kDenseSmem, st, plan->h[2], plan->w_dense, p);
 }
 

@@ -17,7 +17,7 @@ cudaError_t launch_expand(const TcPlan* plan, const Image& img, const int32_t* e
 cudaError_t launch_down_dense(const TcPlan* plan, const Tile* tiles, const int32_t* n_dense, int d, int mid, __half* pairs16, int32_t* status,
                               cudaStream_t st);
 // Leave `sms` SMs free of the persistent GEMM CTAs (for communication kernels that must run
-// at the same time).
+// at the same time). The two launches above are refused on such a plan.
 void tc_set_sm_margin(TcPlan* plan, int sms);
 
 // Largest number of rows in one grouped-GEMM tile (the MMA N extent), and in one of a narrow launch.

@@ -39,3 +39,11 @@ def test_an_arrival_is_made_once():
     few = source("expert_few.cu")
     signal = few[few.index("auto signal = [&]() {"):]
     assert re.search(r"mbar_arrive\(pending\);\s*pending = 0;", signal[:signal.index("};")])
+
+
+def test_popular_experts_gemm_keeps_out_of_plans_with_a_margin():
+    """Launches that fill the GPU and let the next one start early are refused where SMs are to stay free for exchange kernels."""
+    dense = source("expert_dense.cu")
+    for name in ("launch_expand", "launch_down_dense"):
+        body = dense[dense.index("cudaError_t %s(" % name):]
+        assert re.match(r"[^{]*\{[^;]*plan->margin > 0\) return cudaErrorNotSupported;", body), name
