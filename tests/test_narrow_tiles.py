@@ -2,7 +2,11 @@
 copies) and larger ones in the wide form, on two lists side by side or on one, by the call's sizes and the rows of all experts; popular
 experts' down GEMM runs on expanded weights. Against the oracle where those forms can go wrong -- K block counts that are odd, one, or
 fewer than the ring's stages, experts whose rows end just behind a tile, every weight format -- and bit for bit
-against one another on both sides of the rules: a row's sums do not depend on the tile it is in."""
+against one another on both sides of the rules: a row's sums do not depend on the tile it is in. The rules' lines are read from the
+sources, and each call is checked to lie on the side that it stands for."""
+import os
+import re
+
 import numpy as np
 import pytest
 
@@ -15,6 +19,37 @@ from test_gpu_parity import bits, make_op, run_layer
 from test_i4r_gpu import make_i4r_op, run as run_i4r
 
 pytestmark = pytest.mark.gpu
+
+CSRC = os.path.join(os.path.dirname(pkg.__file__), "csrc")
+SOURCES = "".join(open(os.path.join(CSRC, f)).read() for f in ("api.cu", "kernels.h", "tc.h", "common.cuh"))
+
+
+def line(name):
+    """The value of a constant of the rules."""
+    return int(re.search(r"\b%s = (\d+)" % name, SOURCES).group(1))
+
+
+WIDE_ROWS, FEW_ROWS = line("kTcTileN"), line("kTcNarrowN")
+
+
+def form(E, k, d, mid, T):
+    """What a tensor-core call of T > 16 tokens runs: "few" (one list of tiles of 64 rows), "wide" (one of 192), or "both" (the
+    device chooses: two launches more)."""
+    few, second = T * k <= line("kFewRows") * E, line("kSecondListCycles") * 148 * 8192 // (3 * d * mid)
+    if (line("kTileCostFew") * 2 * T * k > (2 * FEW_ROWS + 1) * second) if few else E * d * mid >= line("kBothLists"):
+        return "both"
+    return "few" if few or (T <= line("kOneListTokens") and T * k <= line("kOneListRows") * E) else "wide"
+
+
+def device_choice(counts, d, mid):
+    """Where the device chooses: the form that it takes for these experts' rows."""
+    wide_cost, few_cost = line("kTileCostWide"), line("kTileCostFew")
+    wide, few = sum(-(-c // WIDE_ROWS) for c in counts), sum(-(-c // FEW_ROWS) for c in counts)
+    ragged = sum(0 < c % WIDE_ROWS <= FEW_ROWS for c in counts)
+    both = wide_cost * (wide - ragged) + few_cost * ragged + line("kSecondListCycles") * 148 * 8192 // (3 * d * mid)
+    if few_cost * few <= min(wide_cost * wide, both):
+        return "few"
+    return "wide" if wide_cost * wide <= both else "both"
 
 
 def popular(logits, experts):
@@ -41,11 +76,12 @@ def test_narrow_tiles_against_oracle(cuda, shape, T):
     op.close()
 
 
-def test_both_sides_of_the_rule_agree(cuda):
-    """T*k = 12*E is the last narrow call; one token more runs wide."""
-    spec = synth.LayerSpec(experts=32, topk=4, d=512, mid=256, shared=True)
+# the last calls of tiles of 64 rows alone, by the rows per expert and by the tokens; one token more runs the wide form alone
+@pytest.mark.parametrize("E,T", [(32, 384), (64, 512)])
+def test_both_sides_of_the_rule_agree(cuda, E, T):
+    spec = synth.LayerSpec(experts=E, topk=4, d=512, mid=256, shared=True)
+    assert [form(E, 4, 512, 256, n) for n in (T, T + 1)] == ["few", "wide"]
     layer = synth.make_layer(spec, seed=82)
-    T = 12 * spec.experts // spec.topk
     logits = popular(synth.make_logits(synth.rng_for(82, 1), T + 1, spec.experts, zipf=True), [5, 17])
     xb = synth.make_x(synth.rng_for(82, 9), T + 1, spec.d)
     op = make_op(cuda, spec, T + 1, layer=layer)
@@ -58,7 +94,7 @@ def test_both_sides_of_the_rule_agree(cuda):
 @pytest.mark.parametrize("types", [(pkg.GGML_Q4_K, pkg.GGML_Q5_1), (pkg.GGML_Q5_K, pkg.GGML_Q5_1), (pkg.GGML_Q8_0, pkg.GGML_Q8_0),
                                    (pkg.GGML_IQ4_XS, pkg.GGML_IQ4_XS)])
 def test_narrow_gguf_equals_wide(cuda, types):
-    """The GGUF images (more metadata per tile, two planes for Q8_0): the same rows in a narrow and in a wide call."""
+    """The GGUF images (more metadata per tile, two planes for Q8_0): the same rows in a call of the few-row and in one of the wide form."""
     torch = cuda
     E, k, d, mid = 16, 2, 512, 256
     gen = np.random.default_rng(83)
@@ -73,7 +109,8 @@ def test_narrow_gguf_equals_wide(cuda, types):
             b[:, 2:4] = np.full(len(b), 5e-4 if per == 256 else -1e-1, "<f2").view(np.uint8).reshape(-1, 2)
         return torch.from_numpy(b.reshape(-1)).cuda()
 
-    T = 200
+    T = 600
+    assert form(E, k, d, mid, T) == "wide" and form(E, k, d, mid, 90) == "few"
     op = pkg.MoeOperator(E, k, d, mid, T)
     op.load_gguf(0, blocks(E * mid, d, types[0]), blocks(E * mid, d, types[0]), blocks(E * d, mid, types[1]),
                  type_gu=types[0], type_dn=types[1])
@@ -133,29 +170,33 @@ def ids_of_counts(E, k, T, counts):
     return ids
 
 
-# Calls of T = 12*E/k tokens on a layer of 4096 x 1024, whose line for the second list lies at 12 tiles saved: no
-# expert over a narrow tile (64 rows); 16 experts just over one, so that every block has work in both forms; rows on
-# both sides of a narrow tile and of a full one (192), 12 and 13 saved
+# Calls of T = 12*E/k tokens on a layer of 4096 x 1024, where the device chooses: no expert over a small tile (64 rows) or four just over one
+# (tiles of 64 rows alone), 16 just over one or a few of all tokens (two lists), and a few of all tokens with hardly any others (wide
+# tiles alone), with rows on both sides of a small tile and of a full one (192)
 @pytest.mark.parametrize("fmt", ["q4cp", "i4r"])
 def test_both_forms_in_one_call(cuda, fmt):
-    """Tiles of more than 64 rows run in the wide form, the others of the same call in the narrow one: bit for
-    bit the rows of a call of one token more, which runs the wide form alone."""
+    """Tiles of more than 64 rows run in the wide form, the others of the same call in the few-row one, or all in either: bit for
+    bit the rows of a longer call, which runs the wide form alone."""
     torch = cuda
     E, k, d, mid = 96, 4, 4096, 1024
     T = 12 * E // k
+    whole = line("kOneListTokens") + 1
+    assert form(E, k, d, mid, T) == "both" and form(E, k, d, mid, whole) == "wide"
     if fmt == "i4r":
         L = synth.make_i4r_layer(E, d, mid, seed=87)
-        op = make_i4r_op(torch, E, k, d, mid, T + 1, L)
+        op = make_i4r_op(torch, E, k, d, mid, whole, L)
     else:
         spec = synth.LayerSpec(experts=E, topk=k, d=d, mid=mid, shared=True)
-        op = make_op(torch, spec, T + 1, layer=synth.make_layer(spec, seed=87))
-    w = synth.rng_for(87, 1).uniform(0.2, 1.0, size=(T + 1, 16)).astype(np.float32) / k
-    xb = synth.make_x(synth.rng_for(87, 9), T + 1, d)
-    for counts in ([64, 64], [65] * 16, [288, 257, 193, 130, 129, 64, 64], [288, 257, 193, 130, 129, 65, 64]):
+        op = make_op(torch, spec, whole, layer=synth.make_layer(spec, seed=87))
+    w = synth.rng_for(87, 1).uniform(0.2, 1.0, size=(whole, 16)).astype(np.float32) / k
+    xb = synth.make_x(synth.rng_for(87, 9), whole, d)
+    for counts, choice in (([64, 64], "few"), ([65] * 4, "few"), ([65] * 16, "both"), ([288] * 3, "both"),
+                           ([288, 257, 257, 257], "both"), ([288] * 4, "wide"), ([288, 288, 193, 193, 65, 64, 49, 12], "wide")):
         ids = ids_of_counts(E, k, T, counts)
-        ids = np.concatenate([ids, ids[-1:]])
+        assert device_choice(np.bincount(ids[:, :k].reshape(-1), minlength=E), d, mid) == choice, counts
+        ids = np.concatenate([ids, np.repeat(ids[-1:], whole - T, axis=0)])
         outs = []
-        for n in (T, T + 1):
+        for n in (T, whole):
             before = op.launches
             out = torch.full((n, d), float("nan"), dtype=torch.bfloat16, device="cuda")
             op.moe_q4w_run(0, bf16_tensor(torch, xb[:n], (n, d)), torch.from_numpy(ids[:n]).cuda(), torch.from_numpy(w[:n]).cuda(), out)
@@ -255,8 +296,9 @@ def random_blob(torch, rows, cols, fmt, seed):
     return b.reshape(-1)
 
 
-def rows_agree(torch, E, k, d, mid, types, T, counts):
-    """A call's rows, bit for bit those of calls of 17 tokens, and the fp32 kernels' results within the roundings' bound."""
+def rows_agree(torch, E, k, d, mid, types, T, counts, extra=None):
+    """A call's rows, bit for bit those of calls of 17 tokens, and the fp32 kernels' results within the roundings' bound. extra:
+    (n, m): the call makes m more launches than one of its first n tokens."""
     ids = torch.from_numpy(ids_of_counts(E, k, T, counts)).cuda()
     w = torch.from_numpy(synth.rng_for(88, 1).uniform(0.2, 1.0, size=(T, 16)).astype(np.float32) / k).cuda()
     x = bf16_tensor(torch, synth.make_x(synth.rng_for(88, 9), T, d), (T, d))
@@ -279,10 +321,17 @@ def rows_agree(torch, E, k, d, mid, types, T, counts):
 
     tc, simt = make(pkg.GEMM_TC), make(pkg.GEMM_SIMT)
     for _ in range(2):
+        before = tc.launches
         whole = run(tc, 0, T)
+        launches = tc.launches - before
+        assert np.array_equal(np.diff(tc.get_routing(T)[4])[:len(counts)], counts)
         assert torch.isfinite(whole.float()).all()
         for t0 in (0, 17, T // 2, T - 17):
             assert torch.equal(whole[t0:t0 + 17], run(tc, t0, 17)), t0
+        if extra is not None:
+            before = tc.launches
+            assert torch.equal(run(tc, 0, extra[0]), whole[:extra[0]])
+            assert launches - (tc.launches - before) == extra[1]
     # 2-norm: both sides round to bf16 (a uniform error of 2^-9 at most: 2^-9 / sqrt(3) rms each), the tensor cores also gate, up and down
     # weights and the hidden values to fp16 (2^-11 / sqrt(3) each): sqrt(2 * 2^-18 + 4 * 2^-22) / sqrt(3) = 1.7e-3; twice that
     want = run(simt, 0, T).float()
@@ -301,19 +350,76 @@ def test_more_than_twelve_rows(cuda, E, k, d, mid, types):
     rows_agree(cuda, E, k, d, mid, types, max(13 * E // k + 1, 320), counts)
 
 
+def popular_calls(E, k, d, mid, T):
+    """A call of T tokens has the popular experts' launches, with room to the line; one of `line` tokens, where no expert can have
+    enough rows, has not, and is otherwise made of the same launches."""
+    least = 3 * line("kDenseGroup")
+    assert T > least and T * k * d * mid > 1.5 * line("kPopularWork")
+    assert form(E, k, d, mid, T) == form(E, k, d, mid, least - 1) != "few"
+    return least - 1
+
+
 # one group of rows more or less than the line, a whole number of them and not; two places for three popular experts (12800 rows, mid
-# 5376); an odd number of K blocks; a layer of two lists
-@pytest.mark.parametrize("E,k,d,mid,types", [(16, 4, 2048, 2048, (None, None)), (16, 4, 768, 5376, (None, None)), (16, 4, 2048, 2048, (pkg.GGML_Q5_K, pkg.GGML_Q5_1)),
-                                             (16, 4, 3840, 1088, (None, None)), (64, 4, 2816, 2816, (None, None))])
+# 6144); an odd number of K blocks; a layer of two lists
+@pytest.mark.parametrize("E,k,d,mid,types", [(16, 4, 2560, 2560, (None, None)), (16, 4, 1280, 6144, (None, None)), (16, 4, 2560, 2560, (pkg.GGML_Q5_K, pkg.GGML_Q5_1)),
+                                             (16, 4, 4096, 1600, (None, None)), (64, 4, 3072, 3072, (None, None))])
 def test_popular_experts(cuda, E, k, d, mid, types):
-    """Experts of 2304 rows and more: the down GEMM on expanded weights."""
-    rows_agree(cuda, E, k, d, mid, types, 3200, [3200, 2304, 2303, 3071, 769])
+    """Experts of 2304 rows and more: the down GEMM on expanded weights (two launches)."""
+    n = popular_calls(E, k, d, mid, 3200)
+    rows_agree(cuda, E, k, d, mid, types, 3200, [3200, 2304, 2303, 3071, 769], (n, 2))
+
+
+# one list and two
+@pytest.mark.parametrize("E,d,mid", [(16, 2560, 2560), (64, 3072, 3072)])
+def test_popular_experts_beside_a_shared_one(cuda, E, d, mid):
+    """The longest row of launches beside one another (popular experts, few rows, shared expert, wide tiles), stored and added into a residual state."""
+    torch = cuda
+    k, T = 4, 3200
+    n = popular_calls(E, k, d, mid, T)
+    counts = [3200, 2304, 2303, 3071, 769]
+    ids = ids_of_counts(E, k, T, counts)
+    lg = np.zeros((T, E), np.float32)
+    np.put_along_axis(lg, ids[:, :k].astype(np.int64), 8.0 + 0.25 * np.arange(k, dtype=np.float32), axis=1)
+    lg = torch.from_numpy(lg).cuda()
+    x = bf16_tensor(torch, synth.make_x(synth.rng_for(89, 9), T, d), (T, d))
+    gate_w = (torch.randn(d, device="cuda") * 0.02).bfloat16()
+    blobs = [random_blob(torch, r, c, None, i) for i, (r, c) in enumerate([(E * 2 * mid, d), (E * d, mid), (mid, d), (mid, d), (d, mid)])]
+
+    def make(impl):
+        op = pkg.MoeOperator(E, k, d, mid, T, has_shared=True, gemm_impl=impl)
+        op.load_q4cp(0, *blobs[:2])
+        op.load_shared_q4cp(0, *blobs[2:], gate_w)
+        return op
+
+    def run(op, t0, m):
+        before = op.launches
+        out = torch.full((m, d), float("nan"), dtype=torch.bfloat16, device="cuda")
+        op.moe_b(0, x[t0:t0 + m].contiguous(), lg[t0:t0 + m].contiguous(), out)
+        op.synchronize()
+        return out, op.launches - before
+
+    tc, simt = make(pkg.GEMM_TC), make(pkg.GEMM_SIMT)
+    whole, launches = run(tc, 0, T)
+    assert np.array_equal(np.diff(tc.get_routing(T)[4])[:5], counts) and torch.isfinite(whole.float()).all()
+    part, fewer = run(tc, 0, n)
+    assert torch.equal(part, whole[:n]) and launches == fewer + 2
+    for t0 in (0, 1600, T - 17):
+        assert torch.equal(run(tc, t0, 17)[0], whole[t0:t0 + 17]), t0
+    want = run(simt, 0, T)[0].float()
+    assert (whole.float() - want).norm() <= 3.4e-3 * want.norm()   # (rows_agree's bound)
+    state = torch.zeros((T, 4, d), dtype=torch.bfloat16, device="cuda")
+    tc.moe_b_hc(0, x, lg, torch.zeros((T, 4), device="cuda"), state)     # gates of 2 * sigmoid(0) = 1
+    tc.synchronize()
+    assert torch.equal(state, whole[:, None].expand(T, 4, d))
+    tc.close()
+    simt.close()
 
 
 def test_popular_experts_captured(cuda):
     """A captured call from hidden states (the router GEMM's clusters) with popular experts (pairs of SMs): replayed on other tokens."""
     torch = cuda
-    E, k, d, mid, T = 16, 4, 2048, 2048, 3200
+    E, k, d, mid, T = 16, 4, 2560, 2560, 3200
+    n = popular_calls(E, k, d, mid, T)
     op = pkg.MoeOperator(E, k, d, mid, T)
     op.load_q4cp(0, random_blob(torch, E * 2 * mid, d, None, 1), random_blob(torch, E * d, mid, None, 2))
     gen = torch.Generator(device="cuda").manual_seed(3)
@@ -325,9 +431,14 @@ def test_popular_experts_captured(cuda):
     want = []
     for x in tokens:
         out = torch.full((T, d), float("nan"), dtype=torch.bfloat16, device="cuda")
+        before = op.launches
         op.moe_hidden(0, x, out)
         op.synchronize()
+        launches = op.launches - before
         assert np.diff(op.get_routing(T)[4]).max() >= 2304
+        before = op.launches
+        op.moe_hidden(0, x[:n].contiguous(), torch.empty_like(out[:n]))
+        assert launches == op.launches - before + 2
         want.append(out)
     assert all(torch.isfinite(y.float()).all() for y in want) and not torch.equal(want[0], want[1])
     x, out = tokens[0].clone(), torch.empty((T, d), dtype=torch.bfloat16, device="cuda")
