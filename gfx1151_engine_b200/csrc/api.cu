@@ -40,8 +40,9 @@ struct LayerWeights {
 // a cold L2, wide form alone / both lists: 512 experts of 4096 x 1024, even routing: 614 tokens 1152 / 814, 1200 1236 /
 // 931, 2048 1306 / 1091, 3200 1478 / 1373, 4096 1616 / 1625, 8192 2274 / 2245; the benchmark's skew: 614 402 / 343,
 // 2048 775 / 705, 4096 1308 / 1221, 8192 2304 / 2201, Q4_K / Q5_1 8192 2379 / 2264; 512 of 2560 x 640, 2048 tokens even 640
-// / 542, skewed 415 / 398, 4096 even 788 / 789, skewed 665 / 645; i4r 2048 tokens 706 / 572. Layers below this many weights of a projection
-// do not win the second list's launches back (64 of 2048 x 512, 1000 tokens 107 / 115, skewed 116 / 128).
+// / 542, skewed 415 / 398, 4096 even 788 / 789, skewed 665 / 645; i4r 2048 tokens 706 / 572. A small layer, 6.7e7 weights
+// of a projection, does not win the second list's launches back (64 of 2048 x 512, 1000 tokens 107 / 115, skewed 116 / 128); the smallest
+// measured above the line has 8.4e8. Layers in between were not measured: those below the line run the wide form alone.
 constexpr long long kBothLists = 500000000;
 // What the second list costs: launches, set-up and last items of two GEMM stages, in cycles of every SM. 5000 / 15000 /
 // 30000: 64 of 2048 x 512, 200 tokens, skewed 87 / 71 / 71 us, 400 tokens 95 / 87 / 87; 512 of 2560 x 640 + shared, 300 tokens, skewed 211 / 199 / 213.
@@ -68,14 +69,15 @@ constexpr long long kPopularWork = 50000000000;
 // items (768 tokens, mid 768) 288 / 282 us, 384 (1536, mid 1024) 871 / 868, 576 (2304, mid 1024) 906 / 937.
 constexpr int kSharedNarrowItems = 384;
 // Experts of a call of the first kind (kFewRows) with no more rows than one pass of the decode GEMV serves (8, 4 in the GGUF
-// formats) take the GEMV, with the tensor-core launches beside it for the rest. That costs two more launches, 10 to 15 us, and is
-// done where the GEMV's share is worth them: 160 million weights of a projection in such experts, which only the device can
-// count (k_route_scan). It is not asked where the average is above 5/4 of those rows: even routing then leaves less
-// than a third of the experts there. Without / with, us, cold L2: 512 experts of 4096 x 1024, 24 tokens 321 / 325 and (skew 1)
-// 124 / 132, 77 with a shared expert 634 / 640 and (0.5) 370 / 388, 400 tokens 792 / 824; Q4_K / Q5_1, 24 tokens 363 / 349, 77 710
-// / 695, 200 (0.5) 572 / 577; 512 of 2560 x 640 + shared, 500 tokens 378 / 398 and (0.5) 347 / 372. So it is no longer the
-// faster form for q4cp; it stays for its precision: the GEMV multiplies exact weights in fp32, the tensor cores weights rounded to fp16.
-// The two round differently (fp32 scales and sums by slices against fp16 weights), so that an output of such a call depends on the
+// formats) take the GEMV, with the tensor-core launches beside it for the rest: for its precision, since it multiplies exact
+// weights in fp32 where the tensor cores take weights rounded to fp16. Error against 64 bits without / with: 24 tokens of 512 experts of 4096 x
+// 1024 1.757e-3 / 1.731e-3, in Q4_K / Q5_1 1.781e-3 / 1.679e-3. It is the faster form in the GGUF formats with even routing only. Without / with, us, cold L2: 24
+// tokens 319 / 324 and (skew 1) 120 / 130, 77 with a shared expert 632 / 642 and (0.5) 368 / 390, 400 tokens 783 / 820 and (0.5)
+// 671 / 695; Q4_K / Q5_1, 24 tokens 357 / 351, 77 704 / 693 and (0.5) 384 / 392, 200 (0.5) 570 / 573; 512 of 2560 x 640 + shared, 100 tokens 323 /
+// 330, 500 376 / 390 and (0.5) 357 / 368. So the line says where precision may cost that much, not where time is won: experts that hold 160
+// million weights of a projection, which only the device can count (k_route_scan), drawn when the GEMV was the faster form above it and two
+// launches more, 10 to 15 us, than a smaller call can bear. It is not asked where the average is above 5/4 of those rows: even routing
+// then leaves less than a third of the experts there. The two round differently (fp32 scales and sums by slices against fp16 weights), so that an output of such a call depends on the
 // other tokens by rounding; calls that must not have GEMM_TC.
 constexpr long long kMinFewWork = 160000000;
 
@@ -1033,7 +1035,7 @@ int b200moe_forward_hidden(b200moe_handle h, int layer, const void* x_bf16_dev, 
   const b200moe_config& c = h->cfg;
   LayerWeights& L = h->layers[layer];
   if (L.router_w && route_block_supported(T, c.topk) && !fused_decode(c)) {
-    // few tokens: the routing kernel itself looks for near-ties (router_logits: two kernels and a memset more)
+    // few tokens: the routing kernel itself looks for near-ties (router_logits: two kernels more)
     cudaStream_t st = (cudaStream_t)stream;
     CU_TRY(h, launch_router_dots(x_bf16_dev, L.router_w, T, c.experts, c.d_model, h->router_logits, nullptr, st));
     h->launches++;

@@ -10,8 +10,8 @@
 //               codes at a time (a table lookup per code byte, see Map in expert_tc.cu), into tensor memory. The stores are
 //               waited for behind the next quad's first 32 codes.
 //   warps 20-23 epilogue, 16 rows of the expert at a time; two accumulators, three slots of 128 columns for the weights
-// What bounds it: of a 128 x 64 block's 255 cycles (10 rows; 512 experts of 4096 x 1024, 600 tokens, 505 us of the gate/up
-// launch at 3.5 TB/s) the table lookups take 126 by themselves, the stores to tensor memory another 90 (they and the loads share
+// What bounds it: of a 128 x 64 block's 255 cycles (12 rows; 512 experts of 4096 x 1024, 600 tokens, 505 us of the gate/up
+// launch at 4.8 TB/s) the table lookups take 126 by themselves, the stores to tensor memory another 90 (they and the loads share
 // a pipe), the MMAs' reads of it the rest; weights from L2 instead of HBM gain 2 %, no epilogue 1 %. The HBM's share is 200. Before,
 // with pairs of K blocks as the unit, a relay warp and two more barrier checks of the MMA warp (each ~180 cycles of its
 // serial chain): 375 cycles, 650 us. Steps: quads alone 714 us; activations counted by the weights' barrier, checks ahead of their

@@ -17,8 +17,8 @@
 //   * B never moves: a warp owns at most four K blocks (five among longer calls; its slice) of all the rows its team works on, and the
 //     activations of a slice are 8 registers per K block and lane.
 //   * q4cp: a code byte is decoded by one lookup in a 256-entry half2 table replicated per lane in shared memory
-//     (no bank conflicts; a line is 256 bytes, so the address is one byte permute): 32 of the 50 wavefronts per
-//     32 x 64 block, which keep the load pipe busy for two thirds of a 13-token launch, its ends included. GGUF: the codes are masked into fp16 bit patterns,
+//     (no bank conflicts; a line is 256 bytes, so the address is one byte permute): 32 of the 49 wavefronts per
+//     32 x 64 block, which keep the load pipe busy for three quarters of a 13-token launch, its ends included. GGUF: the codes are masked into fp16 bit patterns,
 //     code * 2^-24 (denormal, exact), no lookup; 2^24 goes into the fp32 constants. Issue slots bound those.
 //   * Weights come by bulk copies into a ring of two or three slots of two K blocks per warp (74 to 123 KB in flight per
 //     SM), one copy and one wait per slot; the image keeps a slice's K blocks together (common.cuh).

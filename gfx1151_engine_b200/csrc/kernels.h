@@ -14,8 +14,8 @@ namespace b200moe {
 // the next kernel of the stream may start its prologue (code-book tables, index setup) while
 // this one drains. A kernel launched this way must call pdl_wait() before it touches anything
 // an earlier kernel of the stream wrote (or still reads); pdl_trigger() lets its own successor
-// start early. (One exception: k_expert_tc and k_expert_few launches with TcLaunch::beside rely on the wait of the
-// k_expert_tc or k_gemv launch in front of them, which triggers behind it.) B200MOE_NO_PDL=1 in the environment turns the attribute off (plain launches).
+// start early. (One exception: k_expert_tc and k_expert_few launches with TcLaunch::beside rely on the wait of the launch in front of
+// them, k_expert_tc, k_expert_few, k_gemv or k_expert_dense, each of which triggers behind its wait, or, itself beside another, waits at its end.) B200MOE_NO_PDL=1 in the environment turns the attribute off (plain launches).
 // launch_opt(false, ...) is a plain launch of the same kernel.
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
@@ -91,11 +91,12 @@ struct RouteBuffers {
 };
 cudaError_t launch_router_topk(const float* logits, int T, int E, int k, int32_t* ids, float* w,
                                int stride, cudaStream_t st);
+// What a tile costs in the wide and in the few-row form, cycles per 128 x 64 block of weights.
+constexpr int kTileCostWide = 380, kTileCostFew = 270;
 // How the work lists are cut: at most `routed` rows in a tile of a routed expert, `shared` in one of the shared
 // expert. narrow > 0: the device chooses between tiles of `routed` rows on tiles, tiles of `narrow` rows on tiles_narrow, and
-// both lists, where the ragged tiles of at most `narrow` rows go on tiles_narrow and the others on tiles.
-// What a tile costs in the one and in the other form (cycles per 128 x 64 block of weights), and the second list's launches in that unit.
-constexpr int kTileCostWide = 380, kTileCostFew = 270;
+// both lists, where the ragged tiles of at most `narrow` rows go on tiles_narrow and the others on tiles; second: what the
+// second list's launches cost, in the tiles' unit.
 struct TileCut {
   int routed, shared, narrow = 0, second = 0;
   // > 0: the rows of the first dense_cap experts of at least so many are on tiles_dense, too, kDenseGroup at a time.

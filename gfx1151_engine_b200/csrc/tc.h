@@ -27,7 +27,7 @@ constexpr int kTcNarrowN = 64;
 struct TcLaunch {
   bool narrow = false;  // every tile of the list has at most kTcNarrowN rows
   // The launch may run at the same time as the one in front of it in the stream, which must be another
-  // of these launches or the decode GEMV's on other rows; it is complete only when that one is.
+  // of these launches (either form), the popular experts' GEMM or the decode GEMV's, on other rows; it is complete only when that one is.
   bool beside = false;
   // down GEMM; rowmap + map_base (device, both or neither): result row r >= map_base[0] of the tile list goes
   // to pairs16[rowmap[r - map_base[0]]] instead of pairs16[r].

@@ -1,4 +1,4 @@
-// tc_dev.cuh -- device helpers of the grouped dequant-GEMMs (expert_tc.cu, expert_few.cu): barriers with
+// tc_dev.cuh -- device helpers of the grouped GEMMs (expert_tc.cu, expert_few.cu, expert_dense.cu): barriers with
 // bounded waits, TMA, tcgen05, and the decoding of packed weights. Included by .cu files only.
 #pragma once
 #include "kernels.h"
@@ -180,8 +180,7 @@ __device__ __forceinline__ uint32_t instr_desc(int n) {
   return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 }
 
-// finite values saturate to the fp16 range (as on the GEMV path), NaN stays NaN
-// fp32 -> fp16, finite values saturating to the fp16 range, NaN staying NaN: one conversion
+// fp32 -> fp16, finite values saturating to the fp16 range (as on the GEMV path), NaN staying NaN: one conversion
 __device__ __forceinline__ __half f16_sat(float v) {
   unsigned short h;
   asm("cvt.rn.satfinite.f16.f32 %0, %1;" : "=h"(h) : "f"(v));
